@@ -152,8 +152,8 @@ struct Finest {
   double *visc = nullptr, *dens = nullptr;  // [nvnod]
   double *G64 = nullptr;              // [120][nel]: G[p][3n+c]
   double *M64 = nullptr;              // [10][nel] packed lower 4x4
-  double *Fbe = nullptr;              // [30][nel]
-  double *BCe = nullptr;              // [30][nel] K_unmasked * Ufix per element
+  double *Fbe = nullptr;              // [nel][30]
+  double *BCe = nullptr;              // [nel][30] K_unmasked * Ufix per element
   double *Fb = nullptr;               // [ndof] assembled, rotated
   double *LiMM = nullptr;             // [nvnod] inverse lumped M
   int *err = nullptr;                 // device error flags
@@ -188,7 +188,7 @@ struct SetupArgs {
   int pa_ld;
   uint32_t *emask;          // [nel] free-dof bits or nullptr
   const double *ufix;       // [3*nnod] prescribed values (rotated frame) or nullptr
-  double *BCe;              // [30][nel] element K_unmasked * ufix (when ufix != nullptr)
+  double *BCe;              // [nel][30] element K_unmasked * ufix (when ufix != nullptr)
   int *err;
 };
 

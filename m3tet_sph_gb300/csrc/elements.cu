@@ -323,14 +323,14 @@ __global__ void __launch_bounds__(SETUP_THREADS) k_element_setup(SetupArgs a) {
     for (int cc = 0; cc < 3; ++cc) {
       double v = 0.0;
       for (int c = 0; c < 3; ++c) v += sQ[(n * 9 + c * 3 + cc) * EB + el] * F[c];
-      a.Fbe[(size_t)(3 * n + cc) * nel + e] = v;
+      a.Fbe[(size_t)e * 30 + 3 * n + cc] = v;
     }
   }
   if (a.ufix) {
     __syncthreads();
     for (int t = tid; t < 30 * EB; t += SETUP_THREADS) {
-      const int q = t / EB, el = t % EB, e = e0 + el;
-      if (e < nel) a.BCe[(size_t)q * nel + e] = sBC[q * EB + el];
+      const int el = t / 30, q = t - 30 * el, e = e0 + el;
+      if (e < nel) a.BCe[(size_t)e * 30 + q] = sBC[q * EB + el];
     }
   }
 }
@@ -652,147 +652,225 @@ int ebe_apply(const Level &L, const T *K, const T *x, T *y, cudaStream_t s) {
 template int ebe_apply<double>(const Level &, const double *, const double *, double *, cudaStream_t);
 template int ebe_apply<float>(const Level &, const float *, const float *, float *, cudaStream_t);
 
-// assemble element vectors V[q][nel] (q < nq) into node dofs / pressure nodes, per colour
-__global__ void k_scatter_elvec(const double *__restrict__ V, int nq, int per_node, const int *__restrict__ el2nod,
-                                int nel, int e_begin, int e_end, double *__restrict__ out) {
-  const int e = e_begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= e_end) return;
-  for (int q = 0; q < nq; ++q) {
-    const int n = q / per_node, c = q % per_node;
-    const int nod = el2nod[(size_t)n * nel + e];
-    out[per_node * nod + c] += V[(size_t)q * nel + e];
-  }
-}
-
-int scatter_elvec(const Level &L, const double *V, int nq, int per_node, double *out, size_t nout, cudaStream_t s) {
-  M3_CUDA(cudaMemsetAsync(out, 0, sizeof(double) * nout, s));
-  const int nc = (int)L.cstart.size() - 1;
-  for (int c = 0; c < nc; ++c) {
-    const int b = L.cstart[c], e = L.cstart[c + 1];
-    if (e <= b) continue;
-    k_scatter_elvec<<<(e - b + 127) / 128, 128, 0, s>>>(V, nq, per_node, L.el2nod, L.nel, b, e, out); count_launch();
-  }
-  M3_CUDA(cudaGetLastError());
-  return M3SPH_OK;
-}
-
-// diagonal of the element matrices -> inverse diagonal (0 on fixed dofs)
-template <typename T>
-__global__ void k_diag_scatter(const T *__restrict__ K, const int *__restrict__ el2nod, int nel, int e_begin,
-                               int e_end, double *__restrict__ D) {
-  const int e = e_begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= e_end) return;
-  for (int q = 0; q < 30; ++q) {
-    const int nod = el2nod[(size_t)(q / 3) * nel + e];
-    D[3 * nod + q % 3] += (double)K[kidx<T>(pack_idx(q, q), e, nel)];
-  }
-}
-
-__global__ void k_invert_diag(const double *D, const uint8_t *mask, int n, double *Di64, float *Di32) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double v = (mask[i] && D[i] != 0.0) ? 1.0 / D[i] : 0.0;
-  if (Di64) Di64[i] = v;
-  if (Di32) Di32[i] = (float)v;
-}
-
-template <typename T>
-int level_inverse_diag(Level &L, const T *K, double *work, cudaStream_t s) {
-  M3_CUDA(cudaMemsetAsync(work, 0, sizeof(double) * L.ndof, s));
-  const int nc = (int)L.cstart.size() - 1;
-  for (int c = 0; c < nc; ++c) {
-    const int b = L.cstart[c], e = L.cstart[c + 1];
-    if (e <= b) continue;
-    k_diag_scatter<T><<<(e - b + 127) / 128, 128, 0, s>>>(K, L.el2nod, L.nel, b, e, work); count_launch();
-  }
-  k_invert_diag<<<(L.ndof + 255) / 256, 256, 0, s>>>(work, L.freemask, L.ndof, L.Dinv64, L.Dinv32); count_launch();
-  M3_CUDA(cudaGetLastError());
-  return M3SPH_OK;
-}
-template int level_inverse_diag<double>(Level &, const double *, double *, cudaStream_t);
-template int level_inverse_diag<float>(Level &, const float *, double *, cudaStream_t);
-
 // ----------------------------------------------------------------------------------------
-// gradient / divergence / pressure-mass applications (finest level, per colour)
+// level diagonals, gradient, divergence and pressure mass: element products, then sums per node
+//
+// One launch per colour (about 40) left each launch with a few CTAs whose threads read, add and write
+// their nodes one after the other: 20-40 us per launch at 3,840 to 245,760 elements, 0.5-0.9 ms per
+// gradient. Element products go to an element-output array instead and every node sums its entries
+// in element order from the g_ptr / g_idx table (no atomics, the result does not depend on
+// scheduling); a gradient is then two launches bound by the 960 B of G per element.
 // ----------------------------------------------------------------------------------------
-// y(3*nnod) += G q  (G[p][3n+c])
-__global__ void k_grad(const double *__restrict__ G, const int *__restrict__ el2nod, int nel, int eb, int ee,
-                       const double *__restrict__ q, double *__restrict__ y) {
-  const int e = eb + blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ee) return;
-  double qe[4];
-  for (int p = 0; p < 4; ++p) qe[p] = q[el2nod[(size_t)p * nel + e]];
-  for (int n = 0; n < 10; ++n) {
-    const int nod = el2nod[(size_t)n * nel + e];
-    for (int c = 0; c < 3; ++c) {
-      double v = 0.0;
-      for (int p = 0; p < 4; ++p) v += G[(size_t)(p * 30 + 3 * n + c) * nel + e] * qe[p];
-      y[3 * nod + c] += v;
+// inverse diagonal of the finest level: node n sums the diagonal entries of its (element, local
+// node) entries; 0 on fixed dofs
+__global__ void k_diag_nodes(const int *__restrict__ ptr, const int *__restrict__ idx, int nnod,
+                             const double *__restrict__ K, int nel, const uint8_t *__restrict__ mask,
+                             double *__restrict__ Di64, float *__restrict__ Di32) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= nnod) return;
+  double d[3] = {0.0, 0.0, 0.0};
+  for (int j = ptr[n]; j < ptr[n + 1]; ++j) {
+    const int o = idx[j], e = o / 30, q = o - 30 * e;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) d[c] += K[kidx<double>(pack_idx(q + c, q + c), e, nel)];
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const size_t i = 3 * (size_t)n + c;
+    const double v = (mask[i] && d[c] != 0.0) ? 1.0 / d[c] : 0.0;
+    Di64[i] = v;
+    Di32[i] = (float)v;
+  }
+}
+// the same on a coarse level, whose node entries are the contributions of the diagonal block
+template <typename T>
+__global__ void k_diag_blocks(const int *__restrict__ ptr, const int *__restrict__ col, const int *__restrict__ cptr,
+                              const int *__restrict__ contrib, int nnod, const T *__restrict__ K, int nel,
+                              const uint8_t *__restrict__ mask, double *__restrict__ Di64, float *__restrict__ Di32) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= nnod) return;
+  double d[3] = {0.0, 0.0, 0.0};
+  for (int k = ptr[n]; k < ptr[n + 1]; ++k) {
+    if (col[k] != n) continue;
+    for (int j = cptr[k]; j < cptr[k + 1]; ++j) {
+      const int code = contrib[j], e = code / 100, q = 3 * (code % 10);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) d[c] += (double)K[kidx<T>(pack_idx(q + c, q + c), e, nel)];
     }
   }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const size_t i = 3 * (size_t)n + c;
+    const double v = (mask[i] && d[c] != 0.0) ? 1.0 / d[c] : 0.0;
+    Di64[i] = v;
+    Di32[i] = (float)v;
+  }
 }
-// s(nvnod) += G^T z
-__global__ void k_div(const double *__restrict__ G, const int *__restrict__ el2nod, int nel, int eb, int ee,
-                      const double *__restrict__ z, double *__restrict__ s) {
-  const int e = eb + blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ee) return;
-  double ze[30];
+
+int level_inverse_diag(Level &L, const double *K, cudaStream_t s) {
+  if (L.g_ptr)
+    k_diag_nodes<<<(L.nnod + 127) / 128, 128, 0, s>>>(L.g_ptr, L.g_idx, L.nnod, K, L.nel, L.freemask, L.Dinv64, L.Dinv32);
+  else
+    k_diag_blocks<double><<<(L.nnod + 127) / 128, 128, 0, s>>>(L.bsr_ptr, L.bsr_col, L.bsr_cptr, L.bsr_contrib, L.nnod, K,
+                                                              L.nel, L.freemask, L.Dinv64, L.Dinv32);
+  count_launch();
+  M3_CUDA(cudaGetLastError());
+  return M3SPH_OK;
+}
+int level_inverse_diag(Level &L, const float *K, cudaStream_t s) {
+  k_diag_blocks<float><<<(L.nnod + 127) / 128, 128, 0, s>>>(L.bsr_ptr, L.bsr_col, L.bsr_cptr, L.bsr_contrib, L.nnod, K,
+                                                           L.nel, L.freemask, L.Dinv64, L.Dinv32);
+  count_launch();
+  M3_CUDA(cudaGetLastError());
+  return M3SPH_OK;
+}
+
+// element outputs of G q, 30 consecutive values per element (staged in shared memory: coalesced)
+constexpr int GR_T = 64;
+__global__ void __launch_bounds__(GR_T) k_grad_elem(const double *__restrict__ G, const int *__restrict__ el2nod, int nel,
+                                                    const double *__restrict__ q, double *__restrict__ ye) {
+  __shared__ double sy[GR_T * 31];
+  const int e0 = blockIdx.x * GR_T, e = e0 + threadIdx.x;
+  if (e < nel) {
+    double qe[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) qe[p] = q[el2nod[(size_t)p * nel + e]];
+#pragma unroll
+    for (int k = 0; k < 30; ++k) {
+      double v = 0.0;
+#pragma unroll
+      for (int p = 0; p < 4; ++p) v += __ldcs(G + (size_t)(p * 30 + k) * nel + e) * qe[p];
+      sy[threadIdx.x * 31 + k] = v;
+    }
+  }
+  __syncthreads();
+  const int nv = min(GR_T, nel - e0) * 30;
+  double *out = ye + (size_t)e0 * 30;
+  for (int i = threadIdx.x; i < nv; i += GR_T) out[i] = sy[(i / 30) * 31 + i % 30];
+}
+// element outputs of G' z: 4 consecutive values per element
+__global__ void __launch_bounds__(128) k_div_elem(const double *__restrict__ G, const int *__restrict__ el2nod, int nel,
+                                                  const double *__restrict__ z, double *__restrict__ se) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= nel) return;
+  double v[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
   for (int n = 0; n < 10; ++n) {
     const int nod = el2nod[(size_t)n * nel + e];
-    for (int c = 0; c < 3; ++c) ze[3 * n + c] = z[3 * nod + c];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double zc = z[3 * (size_t)nod + c];
+#pragma unroll
+      for (int p = 0; p < 4; ++p) v[p] += __ldcs(G + (size_t)(p * 30 + 3 * n + c) * nel + e) * zc;
+    }
   }
-  for (int p = 0; p < 4; ++p) {
-    double v = 0.0;
-    for (int q = 0; q < 30; ++q) v += G[(size_t)(p * 30 + q) * nel + e] * ze[q];
-    s[el2nod[(size_t)p * nel + e]] += v;
-  }
+  double2 *out = reinterpret_cast<double2 *>(se + 4 * (size_t)e);
+  out[0] = make_double2(v[0], v[1]);
+  out[1] = make_double2(v[2], v[3]);
 }
-// y(nvnod) += M d (packed lower 4x4) or lumped row sums if d == nullptr
-__global__ void k_mass(const double *__restrict__ M, const int *__restrict__ el2nod, int nel, int eb, int ee,
-                       const double *__restrict__ d, double *__restrict__ y) {
-  const int e = eb + blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ee) return;
+// element outputs of M d (packed lower 4x4), d = r .* w (w null: d = r; r null: lumped row sums)
+__global__ void __launch_bounds__(128) k_mass_elem(const double *__restrict__ M, const int *__restrict__ el2nod, int nel,
+                                                   const double *__restrict__ r, const double *__restrict__ w,
+                                                   double *__restrict__ se) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= nel) return;
   double de[4], ye[4] = {0, 0, 0, 0};
-  int nod[4];
+#pragma unroll
   for (int p = 0; p < 4; ++p) {
-    nod[p] = el2nod[(size_t)p * nel + e];
-    de[p] = d ? d[nod[p]] : 1.0;
+    const int nod = el2nod[(size_t)p * nel + e];
+    de[p] = r ? (w ? r[nod] * w[nod] : r[nod]) : 1.0;
   }
   int k = 0;
+#pragma unroll
   for (int c = 0; c < 4; ++c)
-    for (int r = c; r < 4; ++r) {
+#pragma unroll
+    for (int q = c; q < 4; ++q) {
       const double v = M[(size_t)k * nel + e];
       ++k;
-      ye[r] += v * de[c];
-      if (r != c) ye[c] += v * de[r];
+      ye[q] += v * de[c];
+      if (q != c) ye[c] += v * de[q];
     }
-  for (int p = 0; p < 4; ++p) y[nod[p]] += ye[p];
+  double2 *out = reinterpret_cast<double2 *>(se + 4 * (size_t)e);
+  out[0] = make_double2(ye[0], ye[1]);
+  out[1] = make_double2(ye[2], ye[3]);
+}
+// vertex sums of 4-value element outputs (a vertex's entries in the node table are local nodes 0-3)
+__device__ __forceinline__ double vertex_sum(const int *__restrict__ ptr, const int *__restrict__ idx, int v,
+                                             const double *__restrict__ se) {
+  double t = 0.0;
+  for (int j = ptr[v]; j < ptr[v + 1]; ++j) {
+    const int o = idx[j], e = o / 30, a = (o - 30 * e) / 3;
+    if (a < 4) t += se[4 * (size_t)e + a];
+  }
+  return t;
+}
+__global__ void k_vertex_gather(const int *__restrict__ ptr, const int *__restrict__ idx, int nv,
+                                const double *__restrict__ se, double scale, double *__restrict__ out) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v < nv) out[v] = scale * vertex_sum(ptr, idx, v, se);
+}
+// d = w r + w (r - M (w r)): the pressure preconditioner's two lumped sweeps
+__global__ void k_vertex_precond(const int *__restrict__ ptr, const int *__restrict__ idx, int nv,
+                                 const double *__restrict__ se, const double *__restrict__ r,
+                                 const double *__restrict__ w, double *__restrict__ d) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= nv) return;
+  const double rv = r[v], wv = w[v];
+  d[v] = rv * wv + wv * (rv - vertex_sum(ptr, idx, v, se));
+}
+// node sums of 30-value element outputs on the free dofs, mode 0: the sum; mode 1: Fb + sum - bc (the
+// velocity right-hand side); 0 on fixed dofs (mask null: every dof)
+__global__ void k_node_gather_rhs(const int *__restrict__ ptr, const int *__restrict__ idx, int nnod,
+                                  const double *__restrict__ ye, const uint8_t *__restrict__ mask,
+                                  const double *__restrict__ Fb, const double *__restrict__ bc, double *__restrict__ y) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= nnod) return;
+  double t[3] = {0.0, 0.0, 0.0};
+  for (int j = ptr[n]; j < ptr[n + 1]; ++j) {
+    const double *v = ye + idx[j];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) t[c] += v[c];
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const size_t i = 3 * (size_t)n + c;
+    y[i] = (mask && !mask[i]) ? 0.0 : (Fb ? Fb[i] + t[c] - bc[i] : t[c]);
+  }
 }
 
-int grad_apply(const Level &L, const double *G, const double *q, double *y, cudaStream_t s) {
-  M3_CUDA(cudaMemsetAsync(y, 0, sizeof(double) * L.ndof, s));
-  for (size_t c = 0; c + 1 < L.cstart.size(); ++c) {
-    const int b = L.cstart[c], e = L.cstart[c + 1];
-    if (e > b) k_grad<<<(e - b + 127) / 128, 128, 0, s>>>(G, L.el2nod, L.nel, b, e, q, y); count_launch();
-  }
+// y = G q; with a mask: on free dofs only; with Fb, bc: y = Fb + G q - bc on free dofs
+int grad_apply(const Level &L, const double *G, const double *q, const uint8_t *mask, const double *Fb, const double *bc,
+               double *y, cudaStream_t s) {
+  k_grad_elem<<<(L.nel + GR_T - 1) / GR_T, GR_T, 0, s>>>(G, L.el2nod, L.nel, q, L.ye64); count_launch();
+  k_node_gather_rhs<<<(L.nnod + 127) / 128, 128, 0, s>>>(L.g_ptr, L.g_idx, L.nnod, L.ye64, mask, Fb, bc, y); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
-int div_apply(const Level &L, const double *G, const double *z, double *out, cudaStream_t s) {
-  M3_CUDA(cudaMemsetAsync(out, 0, sizeof(double) * L.nvnod, s));
-  for (size_t c = 0; c + 1 < L.cstart.size(); ++c) {
-    const int b = L.cstart[c], e = L.cstart[c + 1];
-    if (e > b) k_div<<<(e - b + 127) / 128, 128, 0, s>>>(G, L.el2nod, L.nel, b, e, z, out); count_launch();
-  }
+// out = scale G' z
+int div_apply(const Level &L, const double *G, const double *z, double scale, double *out, cudaStream_t s) {
+  k_div_elem<<<(L.nel + 127) / 128, 128, 0, s>>>(G, L.el2nod, L.nel, z, L.ye64); count_launch();
+  k_vertex_gather<<<(L.nvnod + 127) / 128, 128, 0, s>>>(L.g_ptr, L.g_idx, L.nvnod, L.ye64, scale, out); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
-int mass_apply(const Level &L, const double *M, const double *d, double *out, cudaStream_t s) {
-  M3_CUDA(cudaMemsetAsync(out, 0, sizeof(double) * L.nvnod, s));
-  for (size_t c = 0; c + 1 < L.cstart.size(); ++c) {
-    const int b = L.cstart[c], e = L.cstart[c + 1];
-    if (e > b) k_mass<<<(e - b + 127) / 128, 128, 0, s>>>(M, L.el2nod, L.nel, b, e, d, out); count_launch();
-  }
+// row sums of the pressure mass matrix
+int mass_lump(const Level &L, const double *M, double *out, cudaStream_t s) {
+  k_mass_elem<<<(L.nel + 127) / 128, 128, 0, s>>>(M, L.el2nod, L.nel, nullptr, nullptr, L.ye64); count_launch();
+  k_vertex_gather<<<(L.nvnod + 127) / 128, 128, 0, s>>>(L.g_ptr, L.g_idx, L.nvnod, L.ye64, 1.0, out); count_launch();
+  M3_CUDA(cudaGetLastError());
+  return M3SPH_OK;
+}
+// d = w r + w (r - M (w r)) with w the inverse lumped mass
+int mass_precondition(const Level &L, const double *M, const double *r, const double *w, double *d, cudaStream_t s) {
+  k_mass_elem<<<(L.nel + 127) / 128, 128, 0, s>>>(M, L.el2nod, L.nel, r, w, L.ye64); count_launch();
+  k_vertex_precond<<<(L.nvnod + 127) / 128, 128, 0, s>>>(L.g_ptr, L.g_idx, L.nvnod, L.ye64, r, w, d); count_launch();
+  M3_CUDA(cudaGetLastError());
+  return M3SPH_OK;
+}
+// node sums of element vectors V [nel][30]
+int gather_elvec(const Level &L, const double *V, double *out, cudaStream_t s) {
+  k_node_gather_rhs<<<(L.nnod + 127) / 128, 128, 0, s>>>(L.g_ptr, L.g_idx, L.nnod, V, nullptr, nullptr, nullptr, out);
+  count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
@@ -964,15 +1042,5 @@ template int bsr_assemble<double>(const Level &, const double *, double *, cudaS
 template int bsr_assemble<float>(const Level &, const float *, float *, cudaStream_t);
 template int bsr_apply<double>(const Level &, const double *, const double *, double *, cudaStream_t);
 template int bsr_apply<float>(const Level &, const float *, const float *, float *, cudaStream_t);
-
-__global__ void k_f64_to_f32(const double *a, float *b, size_t n) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i < n) b[i] = (float)a[i];
-}
-int convert_f64_f32(const double *a, float *b, size_t n, cudaStream_t s) {
-  k_f64_to_f32<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a, b, n); count_launch();
-  M3_CUDA(cudaGetLastError());
-  return M3SPH_OK;
-}
 
 }  // namespace m3sph

@@ -622,8 +622,7 @@ __global__ void k_interp_p2(SlmMesh m, const int *__restrict__ els, const double
   }
 }
 
-// quasi-cubic: element P1 gradients of vertex values and distance weights, per element (original
-// ids); the nodal sums are gathered per colour of the Stokes colouring (atomic-free)
+// quasi-cubic: element P1 gradients of vertex values and distance weights, per element (original ids)
 __global__ void k_cubic_elgrad(SlmMesh m, const double *__restrict__ X, const double *__restrict__ B,
                                int method_wght, double *__restrict__ gel, double *__restrict__ wel) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -653,21 +652,29 @@ __global__ void k_cubic_elgrad(SlmMesh m, const double *__restrict__ X, const do
     wel[(size_t)i * m.nel + e] = w;
   }
 }
-// per colour of the Stokes level-0 colouring (stored order -> original ids via perm)
-__global__ void k_cubic_scatter(const int *__restrict__ perm, int nel, int eb, int ee, const int *__restrict__ el2nod_orig,
-                                const double *__restrict__ gel, const double *__restrict__ wel, double *__restrict__ gn,
-                                double *__restrict__ wn, int nvnod) {
-  const int p = eb + blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= ee) return;
-  const int e = perm[p];
-  for (int i = 0; i < 4; ++i) {
-    const int v = el2nod_orig[(size_t)i * nel + e];
-    const double w = wel[(size_t)i * nel + e];
-    gn[v] += w * gel[e];
-    gn[nvnod + v] += w * gel[nel + e];
-    gn[2 * (size_t)nvnod + v] += w * gel[2 * (size_t)nel + e];
-    wn[v] += w;
+// nodal sums of the weighted element gradients: vertex v over its elements in element order (one launch
+// per colour, 40 launches of a few CTAs each, took 0.33-0.39 ms at 30,720-245,760 elements)
+__global__ void k_cubic_nodes(SlmMesh m, const double *__restrict__ gel, const double *__restrict__ wel,
+                              double *__restrict__ gn, double *__restrict__ wn) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= m.nvnod) return;
+  double g0 = 0.0, g1 = 0.0, g2 = 0.0, ws = 0.0;
+  for (int k = m.v2e_ptr[v]; k < m.v2e_ptr[v + 1]; ++k) {
+    const int e = m.v2e[k];
+    int i = 0;
+#pragma unroll
+    for (int q = 1; q < 4; ++q)
+      if (m.el2nod[(size_t)q * m.nel + e] == v) i = q;
+    const double w = wel[(size_t)i * m.nel + e];
+    g0 += w * gel[e];
+    g1 += w * gel[(size_t)m.nel + e];
+    g2 += w * gel[2 * (size_t)m.nel + e];
+    ws += w;
   }
+  gn[v] = g0;
+  gn[m.nvnod + (size_t)v] = g1;
+  gn[2 * (size_t)m.nvnod + v] = g2;
+  wn[v] = ws;
 }
 
 __global__ void k_cubic_interp(SlmMesh m, const double *__restrict__ X, const int *__restrict__ els,
@@ -1166,13 +1173,7 @@ static int slm_cubic_gradients(m3sph_mesh *M, SlmState *S, const double *B, int 
   Level &L0 = M->lev[0];
   const int nel = L0.nel, nv = L0.nvnod;
   k_cubic_elgrad<<<(nel + 127) / 128, 128, 0, s>>>(S->view, M->fin.gcoord, B, method_wght, S->gel, S->wel); count_launch();
-  M3_CUDA(cudaMemsetAsync(S->gn, 0, sizeof(double) * 3 * nv, s));
-  M3_CUDA(cudaMemsetAsync(S->wn, 0, sizeof(double) * nv, s));
-  for (size_t c = 0; c + 1 < L0.cstart.size(); ++c) {
-    const int b = L0.cstart[c], e = L0.cstart[c + 1];
-    if (e > b) k_cubic_scatter<<<(e - b + 127) / 128, 128, 0, s>>>(L0.perm, nel, b, e, S->el2nod, S->gel, S->wel,
-                                                                   S->gn, S->wn, nv); count_launch();
-  }
+  k_cubic_nodes<<<(nv + 127) / 128, 128, 0, s>>>(S->view, S->gel, S->wel, S->gn, S->wn); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
@@ -1558,12 +1559,6 @@ __global__ void k_cubic_interp_caller(SlmMesh m, const double *__restrict__ X, c
                                       const double *__restrict__ gn, const double *__restrict__ wn,
                                       const double *__restrict__ gel, int monotonic, double *__restrict__ out);
 
-// zero n doubles (the nodal sums): a kernel of this module rather than cudaMemsetAsync, so that
-// nothing the call uses is loaded outside noalloc_prepare
-__global__ void k_noalloc_zero(double *a, size_t n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) a[i] = 0.0;
-}
-
 // Run once per handle, from m3sph_mesh_create with the handle's device current. With CUDA's lazy
 // module loading, the first use of this file's module -- the scratch lookup or the first launch of
 // one of its kernels -- is where the driver loads the code and commits the 8 MiB array; doing both
@@ -1574,9 +1569,8 @@ static int noalloc_prepare(int device) {
   if (st) return st;
   cudaFuncAttributes fa;
   M3_CUDA(cudaFuncGetAttributes(&fa, k_cubic_elgrad));
-  M3_CUDA(cudaFuncGetAttributes(&fa, k_cubic_scatter));
+  M3_CUDA(cudaFuncGetAttributes(&fa, k_cubic_nodes));
   M3_CUDA(cudaFuncGetAttributes(&fa, k_cubic_interp_caller));
-  M3_CUDA(cudaFuncGetAttributes(&fa, k_noalloc_zero));
   return M3SPH_OK;
 }
 
@@ -1663,14 +1657,7 @@ extern "C" int m3sph_interp3d_cubic_noalloc(m3sph_mesh *M, const int32_t *els, c
   double *gel = scr, *wel = gel + 3 * nel, *gn = wel + 4 * nel, *wn = gn + 3 * nv;
   cudaStream_t s = M->stream;
   k_cubic_elgrad<<<(unsigned)((nel + 127) / 128), 128, 0, s>>>(S->view, M->fin.gcoord, V, method_wght, gel, wel); count_launch();
-  // the array keeps the previous call's contents: the nodal sums must start at zero
-  k_noalloc_zero<<<(unsigned)std::min<size_t>((4 * nv + 255) / 256, 1024), 256, 0, s>>>(gn, 4 * nv); count_launch();
-  // (gn (3 nv) and wn (nv) are contiguous)
-  for (size_t c = 0; c + 1 < L0.cstart.size(); ++c) {
-    const int b = L0.cstart[c], e = L0.cstart[c + 1];
-    if (e > b) k_cubic_scatter<<<(e - b + 127) / 128, 128, 0, s>>>(L0.perm, (int)nel, b, e, S->el2nod, gel, wel, gn,
-                                                                   wn, (int)nv); count_launch();
-  }
+  k_cubic_nodes<<<(unsigned)((nv + 127) / 128), 128, 0, s>>>(S->view, gel, wel, gn, wn); count_launch();
   k_cubic_interp_caller<<<(npt + 127) / 128, 128, 0, s>>>(S->view, M->fin.gcoord, els, lc, npt, V, gn, wn, gel,
                                                            monotonic, Vi); count_launch();
   M3_CUDA(cudaGetLastError());

@@ -44,11 +44,14 @@ int pa_apply_f32(const Level &L, const float *x, float *y, cudaStream_t s);
 int pa_apply_jac_f32(const Level &L, float w, const float *r, const float *Di, float *d, cudaStream_t s);
 int stream_set_outer_warps(int n);
 int stream_set_f32_variant(int v);
-int scatter_elvec(const Level &L, const double *V, int nq, int per_node, double *out, size_t nout, cudaStream_t s);
-template <typename T> int level_inverse_diag(Level &L, const T *K, double *work, cudaStream_t s);
-int grad_apply(const Level &L, const double *G, const double *q, double *y, cudaStream_t s);
-int div_apply(const Level &L, const double *G, const double *z, double *out, cudaStream_t s);
-int mass_apply(const Level &L, const double *M, const double *d, double *out, cudaStream_t s);
+int gather_elvec(const Level &L, const double *V, double *out, cudaStream_t s);
+int level_inverse_diag(Level &L, const double *K, cudaStream_t s);
+int level_inverse_diag(Level &L, const float *K, cudaStream_t s);
+int grad_apply(const Level &L, const double *G, const double *q, const uint8_t *mask, const double *Fb, const double *bc,
+               double *y, cudaStream_t s);
+int div_apply(const Level &L, const double *G, const double *z, double scale, double *out, cudaStream_t s);
+int mass_lump(const Level &L, const double *M, double *out, cudaStream_t s);
+int mass_precondition(const Level &L, const double *M, const double *r, const double *w, double *d, cudaStream_t s);
 template <typename T> int galerkin(const Level &F, const T *Kf, Level &C, T *Kc, cudaStream_t s);
 template <typename T> int bsr_assemble(const Level &L, const T *K, T *B, cudaStream_t s);
 template <typename T> int bsr_apply(const Level &L, const T *B, const T *x, T *y, cudaStream_t s);
@@ -754,28 +757,28 @@ static int rebuild_operator(m3sph_mesh *M) {
     return M3SPH_ERR_BAD_INPUT;
   }
   // assembled force vector, lumped pressure mass, boundary-condition rhs
-  M3_TRY(scatter_elvec(L0, M->fin.Fbe, 30, 3, M->fin.Fb, L0.ndof, s));
-  M3_TRY(mass_apply(L0, M->fin.M64, nullptr, W->pt, s));
+  M3_TRY(gather_elvec(L0, M->fin.Fbe, M->fin.Fb, s));
+  M3_TRY(mass_lump(L0, M->fin.M64, W->pt, s));
   k_recip<<<(L0.nvnod + 255) / 256, 256, 0, s>>>(W->pt, M->fin.LiMM, L0.nvnod); count_launch();
   if (M->has_nonzero_fix) {
-    M3_TRY(scatter_elvec(L0, M->fin.BCe, 30, 3, M->bc_rhs, L0.ndof, s));
+    M3_TRY(gather_elvec(L0, M->fin.BCe, M->bc_rhs, s));
   } else {
     M3_CUDA(cudaMemsetAsync(M->bc_rhs, 0, sizeof(double) * L0.ndof, s));
   }
   // level diagonals and Galerkin coarse operators
-  M3_TRY(level_inverse_diag<double>(L0, L0.K64, W->tmp, s));
+  M3_TRY(level_inverse_diag(L0, L0.K64, s));
   for (int i = 1; i < M->nmg; ++i) {
     Level &F = M->lev[i - 1], &C = M->lev[i];
     if (M->precision == 0) {
       if (!C.K64) M3_TRY(dalloc(&C.K64, (size_t)kpad<double>() * C.nel));
       M3_TRY(galerkin<double>(F, F.K64, C, C.K64, s));
-      M3_TRY(level_inverse_diag<double>(C, C.K64, W->tmp, s));
+      M3_TRY(level_inverse_diag(C, C.K64, s));
       if (!C.B64) M3_TRY(dalloc(&C.B64, 9 * (size_t)C.nnzb));
       M3_TRY(bsr_assemble<double>(C, C.K64, C.B64, s));
     } else {
       if (!C.K32) M3_TRY(dalloc(&C.K32, (size_t)kpad<float>() * C.nel));
       M3_TRY(galerkin<float>(F, F.K32, C, C.K32, s));
-      M3_TRY(level_inverse_diag<float>(C, C.K32, W->tmp, s));
+      M3_TRY(level_inverse_diag(C, C.K32, s));
       if (!C.B32) M3_TRY(dalloc(&C.B32, 9 * (size_t)C.nnzb));
       M3_TRY(bsr_assemble<float>(C, C.K32, C.B32, s));
     }
@@ -1278,21 +1281,9 @@ __global__ void k_shift(double *a, double c, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) a[i] += c;
 }
-__global__ void k_precond_p1(const double *r, const double *LiMM, double *d, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) d[i] = r[i] * LiMM[i];
-}
-__global__ void k_precond_p2(const double *r, const double *Md, const double *LiMM, double *d, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) d[i] += LiMM[i] * (r[i] - Md[i]);
-}
 __global__ void k_rhs(const double *Fb, const double *GP, const double *bc, const uint8_t *mask, double *out, size_t n) {
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i < n) out[i] = mask[i] ? Fb[i] + GP[i] - bc[i] : 0.0;
-}
-__global__ void k_scale(double *a, double c, size_t n) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i < n) a[i] *= c;
 }
 // Cartesian component r of node n's velocity from its rotated-frame dofs (U_xyz = RR U)
 __device__ __forceinline__ double rotate_back_comp(const double *U, const double *RR, int nnod, int n, int r) {
@@ -1329,14 +1320,10 @@ static int remove_mean(m3sph_mesh *M, double *a) {
   return M3SPH_OK;
 }
 
+// Rhs = Fb + G P - bc on the free dofs
 static int build_rhs(m3sph_mesh *M, const double *P, double *Rhs) {
-  Work *W = get_work(M);
   Level &L0 = M->lev[0];
-  M3_TRY(grad_apply(L0, M->fin.G64, P, W->y, M->stream));
-  k_rhs<<<(unsigned)((L0.ndof + 255) / 256), 256, 0, M->stream>>>(M->fin.Fb, W->y, M->bc_rhs, L0.freemask, Rhs,
-                                                                  L0.ndof);
-  M3_CUDA(cudaGetLastError());
-  return M3SPH_OK;
+  return grad_apply(L0, M->fin.G64, P, L0.freemask, M->fin.Fb, M->bc_rhs, Rhs, M->stream);
 }
 
 // coupled FP64 relative residual
@@ -1360,7 +1347,7 @@ static int coupled_residual(m3sph_mesh *M, const double *U, const double *P, dou
   M3_TRY(dot(W->tmp, W->tmp, n, M->red, M->scal + 10, s));
   M3_TRY(read_scal(M, 10, ru));
   // rp = -G' U, mean removed
-  M3_TRY(div_apply(L0, M->fin.G64, U, W->pt, s));
+  M3_TRY(div_apply(L0, M->fin.G64, U, 1.0, W->pt, s));
   M3_TRY(remove_mean(M, W->pt));
   double rp;
   M3_TRY(dot(W->pt, W->pt, np, M->red, M->scal + 10, s));
@@ -1370,13 +1357,7 @@ static int coupled_residual(m3sph_mesh *M, const double *U, const double *P, dou
 }
 
 static int precondition_P(m3sph_mesh *M, const double *r, double *d) {
-  Work *W = get_work(M);
-  const int np = M->lev[0].nvnod;
-  k_precond_p1<<<(np + 255) / 256, 256, 0, M->stream>>>(r, M->fin.LiMM, d, np); count_launch();
-  M3_TRY(mass_apply(M->lev[0], M->fin.M64, d, W->pSq, M->stream));   // pSq used as temp (Md)
-  k_precond_p2<<<(np + 255) / 256, 256, 0, M->stream>>>(r, W->pSq, M->fin.LiMM, d, np); count_launch();
-  M3_CUDA(cudaGetLastError());
-  return M3SPH_OK;
+  return mass_precondition(M->lev[0], M->fin.M64, r, M->fin.LiMM, d, M->stream);
 }
 
 // Patera solve on device-resident data: the initial pressure must be in the workspace pressure
@@ -1404,8 +1385,7 @@ static int solve_core(m3sph_mesh *M, const m3sph_opts *opts, m3sph_info &inf) {
   M3_TRY(mgpcg(M, W->Rhs, U, rtol_U * rtol_restart, false, itmax_U, cs));
   inf.nitU += cs.it;
   // initial pressure residual r = -G'U
-  M3_TRY(div_apply(L0, M->fin.G64, U, r, s));
-  k_scale<<<(np + 255) / 256, 256, 0, s>>>(r, -1.0, np); count_launch();
+  M3_TRY(div_apply(L0, M->fin.G64, U, -1.0, r, s));
   M3_TRY(remove_mean(M, r));
   double rr;
   M3_TRY(pdot(M, r, r, rr));
@@ -1437,12 +1417,11 @@ static int solve_core(m3sph_mesh *M, const m3sph_opts *opts, m3sph_info &inf) {
     M3_TRY(remove_mean(M, q));
     M3_TRY(pdot(M, r, d, rd));
     rdlast = rd;
-    M3_TRY(grad_apply(L0, M->fin.G64, q, y, s));
-    M3_TRY(apply_mask(y, L0.freemask, n, s));
+    M3_TRY(grad_apply(L0, M->fin.G64, q, L0.freemask, nullptr, nullptr, y, s));
     M3_CUDA(cudaMemsetAsync(z, 0, sizeof(double) * n, s));
     M3_TRY(mgpcg(M, y, z, tol_Z, true, itmax_U, cs));
     inf.nitZ += cs.it;
-    M3_TRY(div_apply(L0, M->fin.G64, z, Sq, s));
+    M3_TRY(div_apply(L0, M->fin.G64, z, 1.0, Sq, s));
     double qSq;
     M3_TRY(pdot(M, q, Sq, qSq));
     M3_CUDA(cudaMemcpyAsync(W->prl, r, sizeof(double) * np, cudaMemcpyDeviceToDevice, s));
@@ -1473,8 +1452,7 @@ static int solve_core(m3sph_mesh *M, const m3sph_opts *opts, m3sph_info &inf) {
         M3_TRY(build_rhs(M, Pd, W->Rhs));
         M3_TRY(mgpcg(M, W->Rhs, U, tol_U_restart, true, itmax_U, cs));
         inf.nitU += cs.it;
-        M3_TRY(div_apply(L0, M->fin.G64, U, r, s));
-        k_scale<<<(np + 255) / 256, 256, 0, s>>>(r, -1.0, np); count_launch();
+        M3_TRY(div_apply(L0, M->fin.G64, U, -1.0, r, s));
         M3_TRY(remove_mean(M, r));
         M3_TRY(pdot(M, r, r, rr));
         norm_rP = std::sqrt(rr) / sqp;
@@ -1490,8 +1468,7 @@ static int solve_core(m3sph_mesh *M, const m3sph_opts *opts, m3sph_info &inf) {
       M3_TRY(build_rhs(M, Pd, W->Rhs));
       M3_TRY(mgpcg(M, W->Rhs, U, tol_U_restart, true, itmax_U, cs));
       inf.nitU += cs.it;
-      M3_TRY(div_apply(L0, M->fin.G64, U, r, s));
-      k_scale<<<(np + 255) / 256, 256, 0, s>>>(r, -1.0, np); count_launch();
+      M3_TRY(div_apply(L0, M->fin.G64, U, -1.0, r, s));
       double rt;
       M3_TRY(pdot(M, r, r, rt));
       const double norm_rP_true = std::sqrt(rt) / sqp;
@@ -1757,7 +1734,7 @@ extern "C" int m3sph_grad_apply(m3sph_mesh *M, const double *q, double *y) {
   Level &L0 = M->lev[0];
   cudaStream_t s = M->stream;
   M3_CUDA(cudaMemcpyAsync(W->pt, q, sizeof(double) * L0.nvnod, cudaMemcpyHostToDevice, s));
-  M3_TRY(grad_apply(L0, M->fin.G64, W->pt, W->y, s));
+  M3_TRY(grad_apply(L0, M->fin.G64, W->pt, nullptr, nullptr, nullptr, W->y, s));
   M3_CUDA(cudaMemcpyAsync(y, W->y, sizeof(double) * L0.ndof, cudaMemcpyDeviceToHost, s));
   M3_CUDA(cudaStreamSynchronize(s));
   return M3SPH_OK;
@@ -1769,7 +1746,7 @@ extern "C" int m3sph_div_apply(m3sph_mesh *M, const double *z, double *out) {
   Level &L0 = M->lev[0];
   cudaStream_t s = M->stream;
   M3_CUDA(cudaMemcpyAsync(W->tmp, z, sizeof(double) * L0.ndof, cudaMemcpyHostToDevice, s));
-  M3_TRY(div_apply(L0, M->fin.G64, W->tmp, W->pt, s));
+  M3_TRY(div_apply(L0, M->fin.G64, W->tmp, 1.0, W->pt, s));
   M3_CUDA(cudaMemcpyAsync(out, W->pt, sizeof(double) * L0.nvnod, cudaMemcpyDeviceToHost, s));
   M3_CUDA(cudaStreamSynchronize(s));
   return M3SPH_OK;
