@@ -95,17 +95,16 @@ int upload_shape_tables();
 struct Level {
   int nel = 0, nnod = 0, nvnod = 0, ndof = 0;
   int nfree = 0;
-  std::vector<int> cstart;            // colour ranges in stored element order (host)
-  int *el2nod = nullptr;              // [10][nel], 0-based, stored (colour) order
-  int *perm = nullptr;                // stored -> original element id
-  int *invperm = nullptr;             // original -> stored
+  std::vector<int> cstart;            // colour ranges of `corder` (host)
+  int *el2nod = nullptr;              // [10][nel], 0-based
+  int *corder = nullptr;              // [nel] element ids sorted by colour (per-colour kernels)
   uint8_t *freemask = nullptr;        // [ndof], 1 = free dof
   double *K64 = nullptr;              // [465][nel] rotated, masked element matrices
   float *K32 = nullptr;
   float *KL32 = nullptr;              // K64 - K32 rounded to FP32 (finest level, mixed precision)
   double *Dinv64 = nullptr;           // [ndof] inverse diagonal (0 on fixed dofs)
   float *Dinv32 = nullptr;
-  // children (coarse levels): fine stored index of child k, and parent-local vertex indices
+  // children (coarse levels): fine index of child k, and parent-local vertex indices
   int *child = nullptr;               // [8][nel]
   uint32_t *child_vloc = nullptr;     // [8][nel], 4 x 4-bit parent-local node index (0..9)
   // transfer to the next coarser level (levels 0..nmg-2)
@@ -119,7 +118,7 @@ struct Level {
   int *bsr_cptr = nullptr, *bsr_contrib = nullptr;   // per block: contributions e*100 + a*10 + b
   double *B64 = nullptr;                         // [nnzb][9]
   float *B32 = nullptr;
-  // streamed apply (finest level): phase 1 streams the element matrices in chunks of 32 stored
+  // streamed apply (finest level): phase 1 streams the element matrices in chunks of 32
   // elements and writes element outputs Ye; phase 2 sums them per node in a fixed order
   int nchunk = 0, sa_grid = 0;
   int *chunk_conn = nullptr;          // [nchunk][10][32] node ids of the chunk's elements (0: unused lane)
@@ -138,15 +137,15 @@ struct Level {
   float4 *pa_trig = nullptr;          // [nnod] (cos theta, sin theta, cos phi, sin phi)
   bool pa_ready = false;              // pa32 / pa_emask written by the last operator set-up
   // host copies needed at set-up
-  std::vector<int> h_el2nod_orig;     // [nel][10] original order, 0-based
+  std::vector<int> h_el2nod_orig;     // [nel][10], 0-based
 };
 
 struct Finest {
   double *gcoord = nullptr;           // [3][nnod]
   double *gcoord_sph = nullptr;       // [3][nnod]
   double *RR = nullptr;               // [9][nnod] (theta,phi,r)->(x,y,z), row-major 3x3
-  uint8_t *cls = nullptr;             // [nel] stored order
-  int *iso_slot = nullptr;            // [nel] stored order, -1 if not iso
+  uint8_t *cls = nullptr;             // [nel]
+  int *iso_slot = nullptr;            // [nel], -1 if not iso
   double *cubic = nullptr;            // [60][niso] (theta,phi,r) x 20 nodes, X-90 frame
   int niso = 0;
   double *visc = nullptr, *dens = nullptr;  // [nvnod]
@@ -173,7 +172,7 @@ struct Coarse {
 
 struct SetupArgs {
   int nel, nnod;
-  const int *el2nod;        // [10][nel] stored order
+  const int *el2nod;        // [10][nel]
   const uint8_t *cls;
   const int *iso_slot;
   const double *cubic;      // [60][niso]

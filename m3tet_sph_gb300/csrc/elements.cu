@@ -360,11 +360,13 @@ template <> __device__ __forceinline__ double lane<double2, double>(const double
 
 template <typename T>
 __global__ void __launch_bounds__(128) k_ebe_apply(const T *__restrict__ K, const int *__restrict__ el2nod, int nel,
-                                                   int e_begin, int e_end, const T *__restrict__ x, T *__restrict__ y) {
+                                                   const int *__restrict__ corder, int e_begin, int e_end,
+                                                   const T *__restrict__ x, T *__restrict__ y) {
   using VT = typename Vec<T>::type;
   constexpr int V = KVec<T>::V;
-  const int e = e_begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= e_end) return;
+  const int i0 = e_begin + blockIdx.x * blockDim.x + threadIdx.x;
+  if (i0 >= e_end) return;
+  const int e = corder[i0];
   int nod[10];
 #pragma unroll
   for (int n = 0; n < 10; ++n) nod[n] = __ldg(el2nod + (size_t)n * nel + e);
@@ -402,10 +404,12 @@ __global__ void __launch_bounds__(128) k_ebe_apply(const T *__restrict__ K, cons
 // multiply-add instead of one FP64 FMA, which GB300 issues at 1/62 of its FP32 rate.
 
 __global__ void __launch_bounds__(128) k_ebe_apply_df(const float *__restrict__ Kh, const float *__restrict__ Kl,
-                                                      const int *__restrict__ el2nod, int nel, int e_begin, int e_end,
+                                                      const int *__restrict__ el2nod, int nel,
+                                                      const int *__restrict__ corder, int e_begin, int e_end,
                                                       const double *__restrict__ x, double *__restrict__ y) {
-  const int e = e_begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= e_end) return;
+  const int i0 = e_begin + blockIdx.x * blockDim.x + threadIdx.x;
+  if (i0 >= e_end) return;
+  const int e = corder[i0];
   int nod[10];
 #pragma unroll
   for (int n = 0; n < 10; ++n) nod[n] = __ldg(el2nod + (size_t)n * nel + e);
@@ -451,7 +455,7 @@ int ebe_apply_df(const Level &L, const float *Kh, const float *Kl, const double 
   for (int c = 0; c < nc; ++c) {
     const int b = L.cstart[c], e = L.cstart[c + 1];
     if (e <= b) continue;
-    k_ebe_apply_df<<<(e - b + 127) / 128, 128, 0, s>>>(Kh, Kl, L.el2nod, L.nel, b, e, x, y); count_launch();
+    k_ebe_apply_df<<<(e - b + 127) / 128, 128, 0, s>>>(Kh, Kl, L.el2nod, L.nel, L.corder, b, e, x, y); count_launch();
   }
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
@@ -459,8 +463,7 @@ int ebe_apply_df(const Level &L, const float *Kh, const float *Kl, const double 
 
 // ----------------------------------------------------------------------------------------
 // split element-by-element apply: a CTA of 4 warps handles 32 elements of one colour; warp w
-// streams the w-th quarter of the packed matrix (lanes = elements, so every load of a warp is
-// one contiguous 512-byte segment), partial results are summed in shared memory and scattered.
+// reads the w-th quarter of the packed matrix (lanes = elements of the colour), partial results are summed in shared memory and scattered.
 // Packed entry k -> (row, col) is resolved at compile time.
 // ----------------------------------------------------------------------------------------
 
@@ -566,15 +569,15 @@ __device__ __forceinline__ void run_part(const Op &op, int e, size_t nel, const 
 }
 
 template <class Op, typename XT>
-__global__ void __launch_bounds__(128) k_ebe_apply_split(Op op, const int *__restrict__ el2nod, int nel, int e_begin,
-                                                         int e_end, const XT *__restrict__ x, XT *__restrict__ y) {
+__global__ void __launch_bounds__(128) k_ebe_apply_split(Op op, const int *__restrict__ el2nod, int nel,
+                                                         const int *__restrict__ corder, int e_begin, int e_end, const XT *__restrict__ x, XT *__restrict__ y) {
   using A = typename Op::acc_t;
   __shared__ XT sY[4][30][33];
   __shared__ int sNod[10][32];
   const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
   const int e0 = e_begin + blockIdx.x * 32;
-  const int e = e0 + lane;
-  const bool valid = e < e_end;
+  const bool valid = e0 + lane < e_end;
+  const int e = valid ? corder[e0 + lane] : 0;
   if (part == 0)
 #pragma unroll
     for (int n = 0; n < 10; ++n) sNod[n][lane] = valid ? __ldg(el2nod + (size_t)n * nel + e) : 0;
@@ -621,7 +624,7 @@ static int ebe_apply_split(const Level &L, const Op &op, const XT *x, XT *y, cud
   for (int c = 0; c < nc; ++c) {
     const int b = L.cstart[c], e = L.cstart[c + 1];
     if (e <= b) continue;
-    k_ebe_apply_split<Op, XT><<<(e - b + 31) / 32, 128, 0, s>>>(op, L.el2nod, L.nel, b, e, x, y); count_launch();
+    k_ebe_apply_split<Op, XT><<<(e - b + 31) / 32, 128, 0, s>>>(op, L.el2nod, L.nel, L.corder, b, e, x, y); count_launch();
   }
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
@@ -644,7 +647,7 @@ int ebe_apply(const Level &L, const T *K, const T *x, T *y, cudaStream_t s) {
   for (int c = 0; c < nc; ++c) {
     const int b = L.cstart[c], e = L.cstart[c + 1];
     if (e <= b) continue;
-    k_ebe_apply<T><<<(e - b + 127) / 128, 128, 0, s>>>(K, L.el2nod, L.nel, b, e, x, y); count_launch();
+    k_ebe_apply<T><<<(e - b + 127) / 128, 128, 0, s>>>(K, L.el2nod, L.nel, L.corder, b, e, x, y); count_launch();
   }
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;

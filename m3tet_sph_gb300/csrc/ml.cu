@@ -112,11 +112,11 @@ __device__ __forceinline__ void forward_strip(int row0, const __nv_bfloat16 *sX,
 }
 
 // ---------------------------------------------------------------------------------------
-// features of one element from a residual vector (level operator in stored order)
+// features of one element from a residual vector 
 // ---------------------------------------------------------------------------------------
 struct FeatLevel {
   int nel;
-  const int *el2nod;     // [10][nel] stored order
+  const int *el2nod;     // [10][nel]
   const float *lvisc;    // [10][nel] standardised log-viscosity
   const float *geo;      // [12][nel]
 };
@@ -214,7 +214,7 @@ __global__ void k_ml_gather(int nnod, int nel, const int *__restrict__ ptr, cons
 // ---------------------------------------------------------------------------------------
 // Fused sweep on the 5th-generation tensor cores (the default inference path).
 //
-// Persistent CTAs of 8 warps take tiles of 128 consecutive stored elements (tile = MMA M = TMEM
+// Persistent CTAs of 8 warps take tiles of 128 consecutive elements (tile = MMA M = TMEM
 // lanes). Warps 4-7 gather: thread g computes the 52 features of element g of a tile (the local
 // residual r0 - kd is formed here) and writes them, BF16, as row g of a K-major 128-byte-swizzled
 // A tile; two A tiles alternate, so the gather of the next tile overlaps the MMAs and the GELU of
@@ -352,18 +352,17 @@ __device__ __forceinline__ float element_features_packed(const FeatLevel &L, int
   return s;
 }
 
-// features of every element of a level in original element order (rows of IN values) and the
-// residual norms s, for checks against a CPU restatement
-__global__ void k_ml_feature_rows(FeatLevel L, const int *__restrict__ perm, const float *__restrict__ z,
+// features of every element of a level (rows of IN values) and the residual norms s, for checks
+// against a CPU restatement
+__global__ void k_ml_feature_rows(FeatLevel L, const float *__restrict__ z,
                                   float *__restrict__ X, float *__restrict__ S) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= L.nel) return;
   float x[IN];
   const float s = element_features_f32(L, e, z, x);
-  const int o = perm[e];
 #pragma unroll
-  for (int q = 0; q < IN; ++q) X[(size_t)o * IN + q] = x[q];
-  S[o] = s;
+  for (int q = 0; q < IN; ++q) X[(size_t)e * IN + q] = x[q];
+  S[e] = s;
 }
 
 // z = (r0 - kd) Dinv in FP32 (kd may be null), the per-dof input of the features
@@ -856,15 +855,12 @@ int ml_build(m3sph_mesh *M) {
   S->nlev = std::min(2, M->nmg);
   for (int j = 0; j < S->nlev; ++j) {
     Level &L = M->lev[j];
-    std::vector<int> perm(L.nel), invp(L.nel);
-    M3_CUDA(cudaMemcpy(perm.data(), L.perm, sizeof(int) * L.nel, cudaMemcpyDeviceToHost));
-    for (int p = 0; p < L.nel; ++p) invp[perm[p]] = p;
     std::vector<int> ptr(L.nnod + 1, 0), code((size_t)L.nel * 10);
     for (size_t i = 0; i < (size_t)L.nel * 10; ++i) ptr[L.h_el2nod_orig[i] + 1]++;
     for (int n = 0; n < L.nnod; ++n) ptr[n + 1] += ptr[n];
     std::vector<int> fill(ptr.begin(), ptr.end() - 1);
     for (int e = 0; e < L.nel; ++e)
-      for (int a = 0; a < 10; ++a) code[fill[L.h_el2nod_orig[(size_t)e * 10 + a]]++] = invp[e] * 10 + a;
+      for (int a = 0; a < 10; ++a) code[fill[L.h_el2nod_orig[(size_t)e * 10 + a]]++] = e * 10 + a;
     MlLevel &ml = S->lev[j];
     M3_TRY(ml_alloc(&ml.n2e_ptr, ptr.size()));
     M3_TRY(ml_alloc(&ml.n2e_code, code.size()));
@@ -1051,12 +1047,14 @@ bool ml_ready(m3sph_mesh *M) { return M->ml && mls(M)->trained; }
 // Training pair of element e: features of the residual, and as target the element's error values scaled
 // like the network output (1 / local residual norm), zero on fixed dofs and clamped against outliers.
 constexpr float TARGET_CLIP = 20.f;
-__global__ void k_ml_samples(FeatLevel L, const double *__restrict__ r, const double *__restrict__ Dinv,
+// Samples are taken in colour order (`corder`), so a stride spreads over the whole shell.
+__global__ void k_ml_samples(FeatLevel L, const int *__restrict__ corder, const double *__restrict__ r,
+                             const double *__restrict__ Dinv,
                              const double *__restrict__ err, const uint8_t *__restrict__ mask, int stride, int offset,
                              long base, long cap, __nv_bfloat16 *__restrict__ Xo, float *__restrict__ Tg) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int e = offset + i * stride;
-  if (e >= L.nel) return;
+  if (offset + i * stride >= L.nel) return;
+  const int e = corder[offset + i * stride];
   const long row = base + i;
   if (row >= cap) return;
   __nv_bfloat16 xr[INP];
@@ -1081,8 +1079,8 @@ int ml_add_samples(m3sph_mesh *M, const double *r, const double *err, int stride
   const long room = S->cap - S->count;
   if (room <= 0) return M3SPH_OK;
   FeatLevel f{L0.nel, L0.el2nod, S->lev[0].lvisc, S->lev[0].geo};
-  k_ml_samples<<<(n + 127) / 128, 128, 0, M->stream>>>(f, r, L0.Dinv64, err, L0.freemask, stride, offset, S->count,
-                                                        S->cap, S->X, S->T);
+  k_ml_samples<<<(n + 127) / 128, 128, 0, M->stream>>>(f, L0.corder, r, L0.Dinv64, err, L0.freemask, stride, offset,
+                                                        S->count, S->cap, S->X, S->T);
   count_launch();
   M3_CUDA(cudaGetLastError());
   S->count = std::min<long>(S->cap, S->count + n);
@@ -1094,7 +1092,7 @@ int ml_feature_rows(m3sph_mesh *M, int j, const float *z, float *X, float *Sn) {
   MlState *S = mls(M);
   Level &L = M->lev[j];
   FeatLevel f{L.nel, L.el2nod, S->lev[j].lvisc, S->lev[j].geo};
-  k_ml_feature_rows<<<(L.nel + 127) / 128, 128, 0, M->stream>>>(f, L.perm, z, X, Sn);
+  k_ml_feature_rows<<<(L.nel + 127) / 128, 128, 0, M->stream>>>(f, z, X, Sn);
   count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;

@@ -29,7 +29,7 @@ int ebe_apply_df(const Level &L, const float *Kh, const float *Kl, const double 
 int ebe_apply_split_f32(const Level &L, const float *K, const float *x, float *y, cudaStream_t s);
 int ebe_apply_split_f64(const Level &L, const double *K, const double *x, double *y, cudaStream_t s);
 int ebe_apply_split_df(const Level &L, const float *Kh, const float *Kl, const double *x, double *y, cudaStream_t s);
-int stream_build(Level &L, const std::vector<int> &perm, cudaStream_t s);
+int stream_build(Level &L, cudaStream_t s);
 int stream_apply_f32(const Level &L, const float *K, const float *x, float *y, cudaStream_t s);
 int stream_apply_jac_f32(const Level &L, const float *K, float w, const float *r, const float *Di, float *d,
                          cudaStream_t s);
@@ -166,7 +166,7 @@ static void dfree(void *p) {
   if (p) cudaFree(p);
 }
 
-// ---- greedy element colouring: elements sharing a vertex get different colours ----
+// ---- greedy element colouring (per-colour kernels): elements sharing a vertex get different colours ----
 static int color_elements(const std::vector<int> &el, int nel, int nvert_ids, std::vector<int> &color, int &ncolor) {
   std::vector<uint64_t> used(2 * (size_t)nvert_ids, 0);
   color.assign(nel, -1);
@@ -226,11 +226,9 @@ extern "C" int m3sph_device_count(int *count) {
 }
 
 // block sparsity pattern of a level and the element contributions of every block
-static int build_bsr(m3sph_mesh *M, Level &L, const std::vector<int> &perm) {
+static int build_bsr(m3sph_mesh *M, Level &L) {
   const int nel = L.nel, nnod = L.nnod;
-  std::vector<int> invp(nel);
-  for (int p = 0; p < nel; ++p) invp[perm[p]] = p;
-  // node -> (stored element, local index)
+  // node -> (element, local index)
   std::vector<int> nptr(nnod + 1, 0);
   for (size_t i = 0; i < (size_t)nel * 10; ++i) nptr[L.h_el2nod_orig[i] + 1]++;
   for (int n = 0; n < nnod; ++n) nptr[n + 1] += nptr[n];
@@ -239,7 +237,7 @@ static int build_bsr(m3sph_mesh *M, Level &L, const std::vector<int> &perm) {
     for (int a = 0; a < 10; ++a) {
       const int n = L.h_el2nod_orig[(size_t)e * 10 + a];
       const int pos = nfill[n]++;
-      nel_of[pos] = invp[e];
+      nel_of[pos] = e;
       nloc[pos] = a;
     }
   std::vector<int> ptr(nnod + 1, 0), col, cptr(1, 0), contrib;
@@ -249,9 +247,8 @@ static int build_bsr(m3sph_mesh *M, Level &L, const std::vector<int> &perm) {
   for (int i = 0; i < nnod; ++i) {
     row.clear();
     for (int k = nptr[i]; k < nptr[i + 1]; ++k) {
-      const int p = nel_of[k], a = nloc[k];
-      const int e = perm[p];
-      for (int b = 0; b < 10; ++b) row.push_back({L.h_el2nod_orig[(size_t)e * 10 + b], p * 100 + a * 10 + b});
+      const int e = nel_of[k], a = nloc[k];
+      for (int b = 0; b < 10; ++b) row.push_back({L.h_el2nod_orig[(size_t)e * 10 + b], e * 100 + a * 10 + b});
     }
     std::sort(row.begin(), row.end());
     for (size_t k = 0; k < row.size(); ++k) {
@@ -304,24 +301,24 @@ static int build_level(m3sph_mesh *M, int img, const m3sph_level &in, Level &L) 
   for (int e = 0; e < in.nel; ++e) cnt[color[e] + 1]++;
   for (int c = 0; c < ncolor; ++c) cnt[c + 1] += cnt[c];
   L.cstart = cnt;
-  std::vector<int> perm(in.nel), invperm(in.nel), fill(cnt.begin(), cnt.end() - 1);
-  for (int e = 0; e < in.nel; ++e) {
-    const int pos = fill[color[e]]++;
-    perm[pos] = e;
-    invperm[e] = pos;
-  }
+  // Elements keep the caller's order: the 8 children of a parent are consecutive on every level, so
+  // neighbours in memory are neighbours in space and the nodes that a warp gathers share cache lines.
+  // (Colour order, which only the per-colour kernels need, spread a warp's nodes over the whole
+  // vector: the partially assembled apply took 104 us at 491,520 elements.) The per-colour kernels go
+  // through the list `corder`.
+  std::vector<int> corder(in.nel), fill(cnt.begin(), cnt.end() - 1);
+  for (int e = 0; e < in.nel; ++e) corder[fill[color[e]]++] = e;
   std::vector<int> el_soa((size_t)in.nel * 10);
-  for (int p = 0; p < in.nel; ++p)
-    for (int n = 0; n < 10; ++n) el_soa[(size_t)n * in.nel + p] = L.h_el2nod_orig[(size_t)perm[p] * 10 + n];
+  for (int e = 0; e < in.nel; ++e)
+    for (int n = 0; n < 10; ++n) el_soa[(size_t)n * in.nel + e] = L.h_el2nod_orig[(size_t)e * 10 + n];
   M3_TRY(upload(&L.el2nod, el_soa.data(), el_soa.size(), s));
-  M3_TRY(upload(&L.perm, perm.data(), perm.size(), s));
-  M3_TRY(upload(&L.invperm, invperm.data(), invperm.size(), s));
+  M3_TRY(upload(&L.corder, corder.data(), corder.size(), s));
   M3_TRY(dalloc(&L.freemask, L.ndof));
   M3_CUDA(cudaMemsetAsync(L.freemask, 1, L.ndof, s));
   M3_TRY(dalloc(&L.Dinv64, L.ndof));
   M3_TRY(dalloc(&L.Dinv32, L.ndof));
-  if (img > 0) M3_TRY(build_bsr(M, L, perm));
-  if (img == 0) M3_TRY(stream_build(L, perm, s));
+  if (img > 0) M3_TRY(build_bsr(M, L));
+  if (img == 0) M3_TRY(stream_build(L, s));
   M3_CUDA(cudaStreamSynchronize(s));
   return M3SPH_OK;
 }
@@ -334,9 +331,6 @@ static int build_transfer(m3sph_mesh *M, Level &F, Level &C, const uint8_t *ispl
     set_error("fine level must have 8 children per coarse element");
     return M3SPH_ERR_BAD_INPUT;
   }
-  std::vector<int> hperm_c(C.nel), hinv_f(F.nel);
-  M3_CUDA(cudaMemcpy(hperm_c.data(), C.perm, sizeof(int) * C.nel, cudaMemcpyDeviceToHost));
-  M3_CUDA(cudaMemcpy(hinv_f.data(), F.invperm, sizeof(int) * F.nel, cudaMemcpyDeviceToHost));
   std::vector<int> child((size_t)8 * C.nel);
   std::vector<uint32_t> vloc((size_t)8 * C.nel);
   // parent-local index of each child vertex
@@ -360,13 +354,11 @@ static int build_transfer(m3sph_mesh *M, Level &F, Level &C, const uint8_t *ispl
       vloc_orig[fe] = code;
     }
   }
-  for (int pc = 0; pc < C.nel; ++pc) {
-    const int p = hperm_c[pc];
+  for (int p = 0; p < C.nel; ++p)
     for (int k = 0; k < 8; ++k) {
-      child[(size_t)k * C.nel + pc] = hinv_f[8 * p + k];
-      vloc[(size_t)k * C.nel + pc] = vloc_orig[8 * p + k];
+      child[(size_t)k * C.nel + p] = 8 * p + k;
+      vloc[(size_t)k * C.nel + p] = vloc_orig[8 * p + k];
     }
-  }
   M3_TRY(upload(&C.child, child.data(), child.size(), s));
   M3_TRY(upload(&C.child_vloc, vloc.data(), vloc.size(), s));
   // transfer rows: parent of the first element listing the node (intermesh_transfer_matrix.m:19-23)
@@ -428,7 +420,7 @@ static int build_transfer(m3sph_mesh *M, Level &F, Level &C, const uint8_t *ispl
 static void clear_graphs(m3sph_mesh *M);
 
 static void free_level(Level &L) {
-  for (void *p : {(void *)L.el2nod, (void *)L.perm, (void *)L.invperm, (void *)L.freemask, (void *)L.K64,
+  for (void *p : {(void *)L.el2nod, (void *)L.corder, (void *)L.freemask, (void *)L.K64,
                   (void *)L.K32, (void *)L.KL32, (void *)L.Dinv64, (void *)L.Dinv32, (void *)L.child, (void *)L.child_vloc,
                   (void *)L.P_ptr, (void *)L.P_col, (void *)L.P_w, (void *)L.R_ptr, (void *)L.R_col, (void *)L.R_w,
                   (void *)L.bsr_ptr, (void *)L.bsr_col, (void *)L.bsr_cptr, (void *)L.bsr_contrib, (void *)L.B64,
@@ -535,8 +527,6 @@ extern "C" int m3sph_mesh_create(int32_t nmg, const m3sph_level *levels, int32_t
     const double Rm[9] = {cp * ct, -sp, cp * st_, sp * ct, cp, sp * st_, -st_, 0.0, ct};
     for (int q = 0; q < 9; ++q) RR[(size_t)q * nnod + n] = Rm[q];
   }
-  std::vector<int> hperm(nel);
-  M3_CUDA(cudaMemcpy(hperm.data(), L0.perm, sizeof(int) * nel, cudaMemcpyDeviceToHost));
   std::vector<uint8_t> cls(nel);
   std::vector<int> iso_slot(nel, -1), iso_of_orig(nel, -1);
   for (int i = 0; i < f0.niso; ++i) {
@@ -548,18 +538,17 @@ extern "C" int m3sph_mesh_create(int32_t nmg, const m3sph_level *levels, int32_t
     iso_of_orig[e - 1] = i;
   }
   for (int p = 0; p < nel; ++p) {
-    const int e = hperm[p];
-    cls[p] = f0.elclass[e];
+    cls[p] = f0.elclass[p];
     if (cls[p] > 3) {
       set_error("element class out of range");
       return fail(M3SPH_ERR_BAD_INPUT);
     }
     if (cls[p] == M3SPH_IN_CONE_ISO) {
-      if (iso_of_orig[e] < 0) {
+      if (iso_of_orig[p] < 0) {
         set_error("in-cone isoparametric element without cubic geometry");
         return fail(M3SPH_ERR_BAD_INPUT);
       }
-      iso_slot[p] = iso_of_orig[e];
+      iso_slot[p] = iso_of_orig[p];
     }
   }
   F.niso = f0.niso;
@@ -1764,31 +1753,28 @@ extern "C" int m3sph_element_matrices(m3sph_mesh *M, double *K, double *G, doubl
   Level &L0 = M->lev[0];
   const int nel = L0.nel;
   std::vector<double> hk((size_t)kpad<double>() * nel), hg(120 * (size_t)nel), hm(10 * (size_t)nel);
-  std::vector<int> perm(nel);
   M3_CUDA(cudaMemcpy(hk.data(), L0.K64, sizeof(double) * hk.size(), cudaMemcpyDeviceToHost));
   M3_CUDA(cudaMemcpy(hg.data(), M->fin.G64, sizeof(double) * hg.size(), cudaMemcpyDeviceToHost));
   M3_CUDA(cudaMemcpy(hm.data(), M->fin.M64, sizeof(double) * hm.size(), cudaMemcpyDeviceToHost));
-  M3_CUDA(cudaMemcpy(perm.data(), L0.perm, sizeof(int) * nel, cudaMemcpyDeviceToHost));
   for (int p = 0; p < nel; ++p) {
-    const int e = perm[p];
     if (K)
       for (int c = 0; c < 30; ++c)
         for (int r = c; r < 30; ++r) {
           const double v = hk[kidx<double>(pack_idx(r, c), p, nel)];
-          K[(size_t)e * 900 + r * 30 + c] = v;
-          K[(size_t)e * 900 + c * 30 + r] = v;
+          K[(size_t)p * 900 + r * 30 + c] = v;
+          K[(size_t)p * 900 + c * 30 + r] = v;
         }
     if (G)
       for (int pp = 0; pp < 4; ++pp)
-        for (int q = 0; q < 30; ++q) G[(size_t)e * 120 + q * 4 + pp] = hg[(size_t)(pp * 30 + q) * nel + p];
+        for (int q = 0; q < 30; ++q) G[(size_t)p * 120 + q * 4 + pp] = hg[(size_t)(pp * 30 + q) * nel + p];
     if (Mm) {
       int k = 0;
       for (int c = 0; c < 4; ++c)
         for (int r = c; r < 4; ++r) {
           const double v = hm[(size_t)k * nel + p];
           ++k;
-          Mm[(size_t)e * 16 + r * 4 + c] = v;
-          Mm[(size_t)e * 16 + c * 4 + r] = v;
+          Mm[(size_t)p * 16 + r * 4 + c] = v;
+          Mm[(size_t)p * 16 + c * 4 + r] = v;
         }
     }
   }

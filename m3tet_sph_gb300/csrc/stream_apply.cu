@@ -1,7 +1,7 @@
 // Streamed element-by-element apply of the finest-level FP32 operator, y = sum_e K_e x_e
 // (the matrix-free product of mgpcg_solver_p.m:388-596 with the stored element matrices).
 //
-// Phase 1, one persistent launch: CTAs take chunks of 32 consecutive stored elements by ticket.
+// Phase 1, one persistent launch: CTAs take chunks of 32 consecutive elements by ticket.
 //   * a producer warp streams a chunk's packed matrices into a 3-stage shared-memory ring with one
 //     2D TMA tensor load (117 rows x 512 B, L2 evict-first) and the chunk's connectivity with one
 //     bulk copy, both completing on mbarriers;
@@ -602,7 +602,7 @@ static cudaError_t g_encode_status = cudaSuccess;
 template <class Op> static int rowlane_attrs();
 static int f32_attrs();
 
-int stream_build(Level &L, const std::vector<int> &perm, cudaStream_t s) {
+int stream_build(Level &L, cudaStream_t s) {
   std::call_once(g_encode_once, [] {
     void *fn = nullptr;
     cudaDriverEntryPointQueryResult q;
@@ -614,14 +614,14 @@ int stream_build(Level &L, const std::vector<int> &perm, cudaStream_t s) {
   const int nel = L.nel, nnod = L.nnod;
   L.nchunk = (nel + sa::E - 1) / sa::E;
   L.nchunk8 = (nel + sr::E - 1) / sr::E;
-  // node -> (element, local node) table in stored element order
+  // node -> (element, local node) table in element order
   std::vector<int> ptr(nnod + 1, 0), idx((size_t)nel * 10);
   for (int p = 0; p < nel; ++p)
-    for (int n = 0; n < 10; ++n) ptr[L.h_el2nod_orig[(size_t)perm[p] * 10 + n] + 1]++;
+    for (int n = 0; n < 10; ++n) ptr[L.h_el2nod_orig[(size_t)p * 10 + n] + 1]++;
   for (int i = 0; i < nnod; ++i) ptr[i + 1] += ptr[i];
   std::vector<int> fill(ptr.begin(), ptr.end() - 1);
   for (int p = 0; p < nel; ++p)
-    for (int n = 0; n < 10; ++n) idx[fill[L.h_el2nod_orig[(size_t)perm[p] * 10 + n]]++] = p * 30 + 3 * n;
+    for (int n = 0; n < 10; ++n) idx[fill[L.h_el2nod_orig[(size_t)p * 10 + n]]++] = p * 30 + 3 * n;
   M3_CUDA(cudaMalloc(&L.chunk_conn, sizeof(int) * (size_t)L.nchunk * 10 * sa::E));
   M3_CUDA(cudaMalloc(&L.ye32, sizeof(float) * (size_t)nel * 30));
   M3_CUDA(cudaMalloc(&L.chunk_conn8, sizeof(int) * (size_t)L.nchunk8 * 10 * sr::E));
