@@ -130,12 +130,17 @@ struct Level {
   int *g_idx = nullptr;               // [10 nel] offsets e * 30 + 3 * local node into Ye, element order
   int *sa_err = nullptr;              // bounded waits of the streamed apply that gave up (bit mask)
   // partially assembled FP32 operator (finest level): per integration point the 3x3 factor
-  // sqrt(w eta) d xi / d x, [NIP][9][nel]; per element the free-dof bits; per node RR's angles
+  // sqrt(w eta) d xi / d x, tiles of 64 elements [tile][NIP][9][32][2] (lane, lane + 32); per node RR's angles; slots: the
+  // nodes of every tile
   float *pa32 = nullptr;
-  int pa_ld = 0;                      // row stride of pa32 (floats, multiple of 4)
-  uint32_t *pa_emask = nullptr;       // [nel] bit 3 n + c set when dof c of local node n is free
   float4 *pa_trig = nullptr;          // [nnod] (cos theta, sin theta, cos phi, sin phi)
-  bool pa_ready = false;              // pa32 / pa_emask written by the last operator set-up
+  float4 *pa_xc = nullptr;            // [nnod] operand, masked, global Cartesian components
+  float4 *pa_yb = nullptr;            // [slots] sums of a tile's element outputs, node-major
+  int *pa_tptr = nullptr;             // [tiles + 1] first slot of a tile
+  int2 *pa_slot = nullptr;            // [slots] {position in pa_yb, begin | end << 16 of its entries}
+  uint16_t *pa_ent = nullptr;         // [tiles][640] entries: 3 a * 65 + element of the tile
+  int *pa_nptr = nullptr;             // [nnod + 1] a node's range of pa_yb
+  bool pa_ready = false;              // pa32 written by the last operator set-up
   // host copies needed at set-up
   std::vector<int> h_el2nod_orig;     // [nel][10], 0-based
 };
@@ -170,6 +175,18 @@ struct Coarse {
   double *t64 = nullptr;              // [n] refinement residual
 };
 
+// Cartesian copy of a nodal vector for the partially assembled operator: a pass that writes (theta,
+// phi, r) values of a node also writes xc[node] when xc is set
+struct PaCart {
+  const float4 *trig = nullptr;       // [nnod] (cos theta, sin theta, cos phi, sin phi)
+  float4 *xc = nullptr;
+};
+// masked local (theta, phi, r) values of a node -> global Cartesian components
+__device__ __forceinline__ float4 pa_to_cart(const float4 tr, float x0, float x1, float x2) {
+  const float a = tr.x * x0 + tr.y * x2;             // ct x0 + st x2
+  return make_float4(tr.z * a - tr.w * x1, tr.w * a + tr.z * x1, tr.x * x2 - tr.y * x0, 0.f);
+}
+
 struct SetupArgs {
   int nel, nnod;
   const int *el2nod;        // [10][nel]
@@ -183,9 +200,7 @@ struct SetupArgs {
   double g, Bscale, Dens0, minVisc, maxVisc;
   double *K64; float *K32; double *G64; double *M64; double *Fbe;
   float *KL32;              // low FP32 part of K64 - K32 (double-float outer operator) or nullptr
-  float *PA32;              // [NIP * 9][pa_ld] partially assembled factors or nullptr
-  int pa_ld;
-  uint32_t *emask;          // [nel] free-dof bits or nullptr
+  float *PA32;              // [tile][NIP][9][32][2] partially assembled factors or nullptr
   const double *ufix;       // [3*nnod] prescribed values (rotated frame) or nullptr
   double *BCe;              // [nel][30] element K_unmasked * ufix (when ufix != nullptr)
   int *err;
@@ -201,7 +216,8 @@ int diffusion_resident(m3sph_mesh *M, double *T, double dt, int *nit);
 int stokes_set_pressure(m3sph_mesh *M, const double *P);
 int ml_build(m3sph_mesh *M);
 int ml_features(m3sph_mesh *M, const double *h_visc);
-template <typename T> int ml_sweep(m3sph_mesh *M, int j, const T *r0, const T *kd, const T *Dinv, T *tmp, T *d);
+template <typename T>
+int ml_sweep(m3sph_mesh *M, int j, const T *r0, const T *kd, const T *Dinv, T *tmp, T *d, const PaCart &pc);
 int ml_init_kernels();
 int ml_set_infer(int v);
 int ml_check(m3sph_mesh *M);

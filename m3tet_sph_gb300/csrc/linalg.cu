@@ -272,25 +272,27 @@ __global__ void __launch_bounds__(256) k_restrict(const int *__restrict__ ptr, c
     out[3 * (size_t)i + lane] = mask[3 * (size_t)i + lane] ? v : T(0);
   }
 }
-// out = add + P xc (masked); add may alias out
+// out = add + P xc (masked); add may alias out; pc: also the Cartesian copy of out
 template <typename T>
 __global__ void k_prolong(const int *__restrict__ ptr, const int *__restrict__ col, const float *__restrict__ w,
-                          int nrow, const T *__restrict__ xc, const T *add, const uint8_t *__restrict__ mask, T *out) {
+                          int nrow, const T *__restrict__ xc, const T *add, const uint8_t *__restrict__ mask, T *out,
+                          PaCart pc) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nrow) return;
-  T s0 = 0, s1 = 0, s2 = 0;
+  T t[3] = {0, 0, 0};
   for (int k = ptr[i]; k < ptr[i + 1]; ++k) {
     const int j = col[k];
     const T wk = (T)w[k];
-    s0 += wk * xc[3 * j];
-    s1 += wk * xc[3 * j + 1];
-    s2 += wk * xc[3 * j + 2];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) t[c] += wk * xc[3 * j + c];
   }
+#pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const T s = c == 0 ? s0 : (c == 1 ? s1 : s2);
     const T base = add ? add[3 * i + c] : T(0);
-    out[3 * i + c] = mask[3 * i + c] ? base + s : T(0);
+    t[c] = mask[3 * i + c] ? base + t[c] : T(0);
+    out[3 * i + c] = t[c];
   }
+  if (pc.xc) pc.xc[i] = pa_to_cart(pc.trig[i], (float)t[0], (float)t[1], (float)t[2]);
 }
 template <typename T>
 int restrict_(const Level &F, const Level &C, const T *a, const T *b, T *out, cudaStream_t s) {
@@ -301,15 +303,18 @@ int restrict_(const Level &F, const Level &C, const T *a, const T *b, T *out, cu
   return M3SPH_OK;
 }
 template <typename T>
-int prolong(const Level &F, const Level &C, const T *xc, const T *add, T *out, cudaStream_t s) {
-  k_prolong<T><<<(F.nnod + 255) / 256, 256, 0, s>>>(F.P_ptr, F.P_col, F.P_w, F.nnod, xc, add, F.freemask, out); count_launch();
+int prolong(const Level &F, const Level &C, const T *xc, const T *add, T *out, const PaCart &pc, cudaStream_t s) {
+  k_prolong<T><<<(F.nnod + 255) / 256, 256, 0, s>>>(F.P_ptr, F.P_col, F.P_w, F.nnod, xc, add, F.freemask, out, pc);
+  count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
 template int restrict_<double>(const Level &, const Level &, const double *, const double *, double *, cudaStream_t);
 template int restrict_<float>(const Level &, const Level &, const float *, const float *, float *, cudaStream_t);
-template int prolong<double>(const Level &, const Level &, const double *, const double *, double *, cudaStream_t);
-template int prolong<float>(const Level &, const Level &, const float *, const float *, float *, cudaStream_t);
+template int prolong<double>(const Level &, const Level &, const double *, const double *, double *, const PaCart &,
+                             cudaStream_t);
+template int prolong<float>(const Level &, const Level &, const float *, const float *, float *, const PaCart &,
+                            cudaStream_t);
 
 // ---------------------------------------------------------------------------------------
 // coarsest level: dense assembly, in-place Gauss-Jordan inverse (SPD, no pivoting), GEMV

@@ -187,11 +187,30 @@ __global__ void __launch_bounds__(256) k_ml_infer(FeatLevel L, MlpDev w, const T
   }
 }
 
+// d_n += v on free dofs (a non-finite value is dropped); pc: also the Cartesian copy of d
+template <typename T>
+__device__ __forceinline__ void ml_add_node(int n, float v0, float v1, float v2, const uint8_t *__restrict__ mask,
+                                            T *__restrict__ d, const PaCart &pc) {
+  const float v[3] = {v0, v1, v2};
+  float x[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const size_t i = 3 * (size_t)n + c;
+    T t = d[i];
+    if (mask[i] && isfinite(v[c])) {
+      t += (T)v[c];
+      d[i] = t;
+    }
+    x[c] = mask[i] ? (float)t : 0.f;
+  }
+  if (pc.xc) pc.xc[n] = pa_to_cart(pc.trig[n], x[0], x[1], x[2]);
+}
+
 // d[3n+c] += omega * sum over (element, local node) of node n of C[3a+c][e] / multiplicity(n)
 template <typename T>
 __global__ void k_ml_gather(int nnod, int nel, const int *__restrict__ ptr, const int *__restrict__ code,
                             const float *__restrict__ C, const uint8_t *__restrict__ mask, float omega,
-                            T *__restrict__ d) {
+                            T *__restrict__ d, PaCart pc) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= nnod) return;
   const int b = ptr[n], e = ptr[n + 1];
@@ -206,9 +225,7 @@ __global__ void k_ml_gather(int nnod, int nel, const int *__restrict__ ptr, cons
   // a non-finite correction (an unusable network) is dropped; the outer CG's rate check then
   // switches the smoother off
   const float w = omega / (float)(e - b);
-  if (mask[3 * n] && isfinite(s0)) d[3 * n] += (T)(w * s0);
-  if (mask[3 * n + 1] && isfinite(s1)) d[3 * n + 1] += (T)(w * s1);
-  if (mask[3 * n + 2] && isfinite(s2)) d[3 * n + 2] += (T)(w * s2);
+  ml_add_node<T>(n, w * s0, w * s1, w * s2, mask, d, pc);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -571,7 +588,7 @@ __global__ void __launch_bounds__(tc::THREADS, 2) k_ml_sweep_tc(FeatLevel L, Mlp
 template <typename T>
 __global__ void k_ml_gather_rows(int nnod, const int *__restrict__ ptr, const int *__restrict__ code,
                                  const float *__restrict__ C, const uint8_t *__restrict__ mask, float omega,
-                                 T *__restrict__ d) {
+                                 T *__restrict__ d, PaCart pc) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= nnod) return;
   const int b = ptr[n], e = ptr[n + 1];
@@ -593,9 +610,7 @@ __global__ void k_ml_gather_rows(int nnod, const int *__restrict__ ptr, const in
     }
   }
   const float w = omega / (float)(e - b);
-  if (mask[3 * n] && isfinite(s0)) d[3 * n] += (T)(w * s0);
-  if (mask[3 * n + 1] && isfinite(s1)) d[3 * n + 1] += (T)(w * s1);
-  if (mask[3 * n + 2] && isfinite(s2)) d[3 * n + 2] += (T)(w * s2);
+  ml_add_node<T>(n, w * s0, w * s1, w * s2, mask, d, pc);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1000,7 +1015,7 @@ int ml_check(m3sph_mesh *M) {
 
 // d += PoU(MLP(features(r0 - kd))) on level j (kd may be null: residual r0)
 template <typename T>
-int ml_sweep(m3sph_mesh *M, int j, const T *r0, const T *kd, const T *Dinv, T *tmp, T *d) {
+int ml_sweep(m3sph_mesh *M, int j, const T *r0, const T *kd, const T *Dinv, T *tmp, T *d, const PaCart &pc) {
   MlState *S = mls(M);
   Level &L = M->lev[j];
   cudaStream_t s = M->stream;
@@ -1012,7 +1027,7 @@ int ml_sweep(m3sph_mesh *M, int j, const T *r0, const T *kd, const T *Dinv, T *t
     k_ml_scale<T><<<(unsigned)((L.ndof + 255) / 256), 256, 0, s>>>(r0, kd, Dinv, S->lev[j].z, L.ndof); count_launch();
     k_ml_sweep_tc<<<grid, tc::THREADS, tc::SMEM_ALLOC, s>>>(f, w, S->lev[j].z, S->lev[j].C, S->err); count_launch();
     k_ml_gather_rows<T><<<(L.nnod + 127) / 128, 128, 0, s>>>(L.nnod, S->lev[j].n2e_ptr, S->lev[j].n2e_code,
-                                                              S->lev[j].C, L.freemask, M->ml_omega, d); count_launch();
+                                                              S->lev[j].C, L.freemask, M->ml_omega, d, pc); count_launch();
     M3_CUDA(cudaGetLastError());
     return M3SPH_OK;
   }
@@ -1023,12 +1038,14 @@ int ml_sweep(m3sph_mesh *M, int j, const T *r0, const T *kd, const T *Dinv, T *t
   }
   k_ml_infer<T><<<(L.nel + INF_ROWS - 1) / INF_ROWS, 256, INF_SMEM, s>>>(f, w, r, Dinv, S->lev[j].C); count_launch();
   k_ml_gather<T><<<(L.nnod + 127) / 128, 128, 0, s>>>(L.nnod, L.nel, S->lev[j].n2e_ptr, S->lev[j].n2e_code,
-                                                       S->lev[j].C, L.freemask, M->ml_omega, d); count_launch();
+                                                       S->lev[j].C, L.freemask, M->ml_omega, d, pc); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
-template int ml_sweep<float>(m3sph_mesh *, int, const float *, const float *, const float *, float *, float *);
-template int ml_sweep<double>(m3sph_mesh *, int, const double *, const double *, const double *, double *, double *);
+template int ml_sweep<float>(m3sph_mesh *, int, const float *, const float *, const float *, float *, float *,
+                             const PaCart &);
+template int ml_sweep<double>(m3sph_mesh *, int, const double *, const double *, const double *, double *, double *,
+                              const PaCart &);
 
 int ml_init_kernels() {
   M3_CUDA(cudaFuncSetAttribute(k_ml_infer<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)INF_SMEM));

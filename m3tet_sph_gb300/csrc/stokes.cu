@@ -38,10 +38,11 @@ int stream_apply_f64(const Level &L, const double *K, const double *x, double *y
 int stream_check(const Level &L, cudaStream_t s);
 int pa_upload_tables();
 int ml_feature_rows(m3sph_mesh *M, int j, const float *z, float *X, float *Sn);
-int pa_row_stride(int nel);
-int pa_build_trig(const double *RR, int nnod, float4 *trig, cudaStream_t s);
-int pa_apply_f32(const Level &L, const float *x, float *y, cudaStream_t s);
-int pa_apply_jac_f32(const Level &L, float w, const float *r, const float *Di, float *d, cudaStream_t s);
+size_t pa_factor_floats(int nel);
+int pa_build(Level &L, const double *RR, cudaStream_t s);
+int pa_jac_first_f32(const Level &L, float w, const float *r, const float *Di, float *d, cudaStream_t s);
+int pa_apply_f32(const Level &L, const float *x, float *y, bool have_cart, cudaStream_t s);
+int pa_apply_jac_f32(const Level &L, float w, const float *r, const float *Di, float *d, bool have_cart, cudaStream_t s);
 int stream_set_outer_warps(int n);
 int stream_set_f32_variant(int v);
 int gather_elvec(const Level &L, const double *V, double *out, cudaStream_t s);
@@ -69,7 +70,8 @@ int f2d(const float *a, double *b, size_t n, cudaStream_t s);
 template <typename T> int jac_first(T w, const T *r0, const T *Di, T *d, size_t n, cudaStream_t s);
 template <typename T> int jac(T w, const T *r0, const T *Kd, const T *Di, T *d, size_t n, cudaStream_t s);
 template <typename T> int restrict_(const Level &F, const Level &C, const T *a, const T *b, T *out, cudaStream_t s);
-template <typename T> int prolong(const Level &F, const Level &C, const T *xc, const T *add, T *out, cudaStream_t s);
+template <typename T>
+int prolong(const Level &F, const Level &C, const T *xc, const T *add, T *out, const PaCart &pc, cudaStream_t s);
 template <typename T>
 int dense_inverse_blocked(const Level &L, const T *B, T *A, T *work, const int *cmap, int nf, cudaStream_t s);
 int dense_inverse_from64(const Level &L, const double *B64, float *B32tmp, float *A, float *work, const int *cmap,
@@ -425,7 +427,8 @@ static void free_level(Level &L) {
                   (void *)L.P_ptr, (void *)L.P_col, (void *)L.P_w, (void *)L.R_ptr, (void *)L.R_col, (void *)L.R_w,
                   (void *)L.bsr_ptr, (void *)L.bsr_col, (void *)L.bsr_cptr, (void *)L.bsr_contrib, (void *)L.B64,
                   (void *)L.B32, (void *)L.chunk_conn, (void *)L.ye32, (void *)L.g_ptr, (void *)L.g_idx, (void *)L.sa_err,
-                  (void *)L.chunk_conn8, (void *)L.ye64, (void *)L.pa32, (void *)L.pa_emask, (void *)L.pa_trig})
+                  (void *)L.chunk_conn8, (void *)L.ye64, (void *)L.pa32, (void *)L.pa_trig, (void *)L.pa_xc,
+                  (void *)L.pa_yb, (void *)L.pa_tptr, (void *)L.pa_slot, (void *)L.pa_ent, (void *)L.pa_nptr})
     dfree(p);
   L = Level();
 }
@@ -708,21 +711,11 @@ static int rebuild_operator(m3sph_mesh *M) {
   a.BCe = nullptr;
   a.KL32 = L0.KL32;
   a.PA32 = nullptr;
-  a.emask = nullptr;
   L0.pa_ready = false;
   if (M->precision == 1 && g_pa_apply) {
-    if (!L0.pa32) {
-      L0.pa_ld = pa_row_stride(L0.nel);
-      M3_TRY(dalloc(&L0.pa32, (size_t)NIP * 9 * L0.pa_ld));
-    }
-    if (!L0.pa_emask) M3_TRY(dalloc(&L0.pa_emask, (size_t)L0.nel));
-    if (!L0.pa_trig) {
-      M3_TRY(dalloc(&L0.pa_trig, (size_t)L0.nnod));
-      M3_TRY(pa_build_trig(M->fin.RR, L0.nnod, L0.pa_trig, s));
-    }
+    if (!L0.pa32) M3_TRY(dalloc(&L0.pa32, pa_factor_floats(L0.nel)));
+    if (!L0.pa_trig) M3_TRY(pa_build(L0, M->fin.RR, s));
     a.PA32 = L0.pa32;
-    a.pa_ld = L0.pa_ld;
-    a.emask = L0.pa_emask;
   }
   if (M->has_nonzero_fix) {
     a.ufix = M->Ufix;
@@ -994,11 +987,18 @@ static int stream_apply_T(const Level &L, const float *K, const float *x, float 
 static int stream_apply_T(const Level &L, const double *K, const double *x, double *y, cudaStream_t s) {
   return stream_apply_f64(L, K, x, y, s);
 }
+// the level whose FP32 operator is the partially assembled one
 template <typename T>
-static int level_op(const Level &L, int img, const T *x, T *y, cudaStream_t s) {
+static bool pa_level(const Level &L, int img) {
+  return std::is_same<T, float>::value && img == 0 && g_pa_apply && L.pa_ready;
+}
+// have_cart: the operand's Cartesian copy is up to date (passes that write a partially assembled
+// level's vector in the V-cycle leave it so)
+template <typename T>
+static int level_op(const Level &L, int img, const T *x, T *y, cudaStream_t s, bool have_cart = false) {
   if (img > 0 && levB<T>(L)) return bsr_apply<T>(L, levB<T>(L), x, y, s);
   if constexpr (std::is_same<T, float>::value) {
-    if (img == 0 && g_pa_apply && L.pa_ready) return pa_apply_f32(L, x, y, s);
+    if (pa_level<T>(L, img)) return pa_apply_f32(L, x, y, have_cart, s);
   }
   if ((std::is_same<T, float>::value ? g_stream_apply : g_stream_outer) && L.nchunk && levK<T>(L))
     return stream_apply_T(L, levK<T>(L), x, y, s);
@@ -1013,13 +1013,22 @@ template <> const float *levDi<float>(const Level &L) { return L.Dinv32; }
 // kd = K d, then d += w (r - kd) / diag; fused into one pass on the streamed finest level (kd is
 // then not written)
 template <typename T>
-static int level_op_jac(const Level &L, int img, T w, const T *r, T *d, T *kd, cudaStream_t s) {
+static int level_op_jac(const Level &L, int img, T w, const T *r, T *d, T *kd, cudaStream_t s, bool have_cart) {
   if constexpr (std::is_same<T, float>::value) {
-    if (img == 0 && g_pa_apply && L.pa_ready) return pa_apply_jac_f32(L, w, r, L.Dinv32, d, s);
+    if (pa_level<T>(L, img)) return pa_apply_jac_f32(L, w, r, L.Dinv32, d, have_cart, s);
     if (img == 0 && g_stream_apply && L.nchunk && L.K32) return stream_apply_jac_f32(L, L.K32, w, r, L.Dinv32, d, s);
   }
   M3_TRY(level_op<T>(L, img, d, kd, s));
   return jac<T>(w, r, kd, levDi<T>(L), d, L.ndof, s);
+}
+
+// first Jacobi sweep from zero, d = w r / diag
+template <typename T>
+static int level_jac_first(const Level &L, int img, T w, const T *r, T *d, cudaStream_t s) {
+  if constexpr (std::is_same<T, float>::value) {
+    if (pa_level<T>(L, img)) return pa_jac_first_f32(L, w, r, L.Dinv32, d, s);
+  }
+  return jac_first<T>(w, r, levDi<T>(L), d, L.ndof, s);
 }
 
 // the coarsest-level solve of the V-cycle: one GEMV with the dense inverse, or on the plain FP64
@@ -1048,59 +1057,60 @@ static int vcycle_T(m3sph_mesh *M, std::vector<T *> &r, std::vector<T *> &d, std
   // learned levels: the two finest (schedules 0, 1, 3) or the finest only (schedule 2)
   const int nml = M->ml_schedule == 2 ? 1 : 2;
   const bool one = M->ml_schedule == 1 || M->ml_schedule == 2;
+  // every pass that writes d on a partially assembled level also writes its Cartesian copy (the
+  // learned sweeps and the prolongation through `xc`), so the products that follow need no pass of
+  // their own for it
   for (int j = 0; j < nm - 1; ++j) {
     const Level &L = M->lev[j];
     const double *w = j == 0 ? WD0 : WDc;
     const size_t n = L.ndof;
-    if (ml && j < nml && one) {
-      // one learned sweep from zero, then the residual for the restriction
+    const PaCart pc = pa_level<T>(L, j) ? PaCart{L.pa_trig, L.pa_xc} : PaCart{};
+    auto sweep = [&](const T *k) { return ml_sweep<T>(M, j, r[j], k, levDi<T>(L), tmp[j], d[j], pc); };
+    auto op = [&]() { return level_op<T>(L, j, d[j], kd[j], s, true); };
+    auto op_jac = [&](double wk) { return level_op_jac<T>(L, j, (T)wk, r[j], d[j], kd[j], s, true); };
+    if (ml && j < nml) {
       M3_CUDA(cudaMemsetAsync(d[j], 0, sizeof(T) * n, s));
-      M3_TRY(ml_sweep<T>(M, j, r[j], nullptr, levDi<T>(L), tmp[j], d[j]));
-      M3_TRY(level_op<T>(L, j, d[j], kd[j], s));
-    } else if (ml && j < nml && M->ml_schedule == 3) {
-      // learned sweep from zero, one weighted Jacobi sweep, residual
-      M3_CUDA(cudaMemsetAsync(d[j], 0, sizeof(T) * n, s));
-      M3_TRY(ml_sweep<T>(M, j, r[j], nullptr, levDi<T>(L), tmp[j], d[j]));
-      M3_TRY(level_op_jac<T>(L, j, (T)w[2], r[j], d[j], kd[j], s));
-      M3_TRY(level_op<T>(L, j, d[j], kd[j], s));
-    } else if (ml && j < nml) {
-      // learned sweep, weighted Jacobi sweep, learned sweep
-      M3_CUDA(cudaMemsetAsync(d[j], 0, sizeof(T) * n, s));
-      M3_TRY(ml_sweep<T>(M, j, r[j], nullptr, levDi<T>(L), tmp[j], d[j]));
-      M3_TRY(level_op<T>(L, j, d[j], kd[j], s));
-      M3_TRY(jac<T>((T)w[1], r[j], kd[j], levDi<T>(L), d[j], n, s));
-      M3_TRY(level_op<T>(L, j, d[j], kd[j], s));
-      M3_TRY(ml_sweep<T>(M, j, r[j], kd[j], levDi<T>(L), tmp[j], d[j]));
-      M3_TRY(level_op<T>(L, j, d[j], kd[j], s));
+      M3_TRY(sweep(nullptr));
+      if (!one && M->ml_schedule == 3) {
+        // learned sweep from zero, one weighted Jacobi sweep
+        M3_TRY(op_jac(w[2]));
+      } else if (!one) {
+        // learned sweep, weighted Jacobi sweep, learned sweep
+        M3_TRY(op_jac(w[1]));
+        M3_TRY(op());
+        M3_TRY(sweep(kd[j]));
+      }
     } else {
-      M3_TRY(jac_first<T>((T)w[0], r[j], levDi<T>(L), d[j], n, s));
-      for (int k = 1; k < 3; ++k) M3_TRY(level_op_jac<T>(L, j, (T)w[k], r[j], d[j], kd[j], s));
-      M3_TRY(level_op<T>(L, j, d[j], kd[j], s));
+      M3_TRY(level_jac_first<T>(L, j, (T)w[0], r[j], d[j], s));
+      for (int k = 1; k < 3; ++k) M3_TRY(op_jac(w[k]));
     }
+    M3_TRY(op());                        // the residual for the restriction
     M3_TRY(restrict_<T>(L, M->lev[j + 1], r[j], kd[j], r[j + 1], s));
   }
   M3_TRY(coarse_solve<T>(M, Ainv, r[nm - 1], d[nm - 1]));
   for (int j = nm - 2; j >= 0; --j) {
     const Level &L = M->lev[j];
     const double *w = j == 0 ? WU0 : WUc;
-    const size_t n = L.ndof;
-    M3_TRY(prolong<T>(L, M->lev[j + 1], d[j + 1], d[j], d[j], s));
+    const PaCart pc = pa_level<T>(L, j) ? PaCart{L.pa_trig, L.pa_xc} : PaCart{};
+    auto sweep = [&](const T *k) { return ml_sweep<T>(M, j, r[j], k, levDi<T>(L), tmp[j], d[j], pc); };
+    auto op = [&]() { return level_op<T>(L, j, d[j], kd[j], s, true); };
+    auto op_jac = [&](double wk) { return level_op_jac<T>(L, j, (T)wk, r[j], d[j], kd[j], s, true); };
+    M3_TRY(prolong<T>(L, M->lev[j + 1], d[j + 1], d[j], d[j], pc, s));
     if (ml && j < nml && one) {
-      M3_TRY(level_op<T>(L, j, d[j], kd[j], s));
-      M3_TRY(ml_sweep<T>(M, j, r[j], kd[j], levDi<T>(L), tmp[j], d[j]));
+      M3_TRY(op());
+      M3_TRY(sweep(kd[j]));
     } else if (ml && j < nml && M->ml_schedule == 3) {
-      M3_TRY(level_op_jac<T>(L, j, (T)w[0], r[j], d[j], kd[j], s));
-      M3_TRY(level_op<T>(L, j, d[j], kd[j], s));
-      M3_TRY(ml_sweep<T>(M, j, r[j], kd[j], levDi<T>(L), tmp[j], d[j]));
+      M3_TRY(op_jac(w[0]));
+      M3_TRY(op());
+      M3_TRY(sweep(kd[j]));
     } else if (ml && j < nml) {
-      M3_TRY(level_op<T>(L, j, d[j], kd[j], s));
-      M3_TRY(ml_sweep<T>(M, j, r[j], kd[j], levDi<T>(L), tmp[j], d[j]));
-      M3_TRY(level_op<T>(L, j, d[j], kd[j], s));
-      M3_TRY(jac<T>((T)w[1], r[j], kd[j], levDi<T>(L), d[j], n, s));
-      M3_TRY(level_op<T>(L, j, d[j], kd[j], s));
-      M3_TRY(ml_sweep<T>(M, j, r[j], kd[j], levDi<T>(L), tmp[j], d[j]));
+      M3_TRY(op());
+      M3_TRY(sweep(kd[j]));
+      M3_TRY(op_jac(w[1]));
+      M3_TRY(op());
+      M3_TRY(sweep(kd[j]));
     } else {
-      for (int k = 0; k < 3; ++k) M3_TRY(level_op_jac<T>(L, j, (T)w[k], r[j], d[j], kd[j], s));
+      for (int k = 0; k < 3; ++k) M3_TRY(op_jac(w[k]));
     }
   }
   return M3SPH_OK;
@@ -1844,7 +1854,8 @@ extern "C" int m3sph_ml_sweep32(m3sph_mesh *M, int32_t img, const float *r, cons
   M3_CUDA(cudaMemcpyAsync(W->r32[img], r, sizeof(float) * n, cudaMemcpyHostToDevice, s));
   if (kd) M3_CUDA(cudaMemcpyAsync(W->kd32[img], kd, sizeof(float) * n, cudaMemcpyHostToDevice, s));
   M3_CUDA(cudaMemcpyAsync(W->d32[img], d, sizeof(float) * n, cudaMemcpyHostToDevice, s));
-  M3_TRY(ml_sweep<float>(M, img, W->r32[img], kd ? W->kd32[img] : nullptr, L.Dinv32, W->t32[img], W->d32[img]));
+  M3_TRY(ml_sweep<float>(M, img, W->r32[img], kd ? W->kd32[img] : nullptr, L.Dinv32, W->t32[img], W->d32[img],
+                         PaCart{}));
   M3_CUDA(cudaMemcpyAsync(d, W->d32[img], sizeof(float) * n, cudaMemcpyDeviceToHost, s));
   M3_CUDA(cudaStreamSynchronize(s));
   return ml_check(M);
@@ -1937,7 +1948,7 @@ extern "C" int m3sph_prolong(m3sph_mesh *M, int32_t img, const double *xc, doubl
   Level &F = M->lev[img], &C = M->lev[img + 1];
   cudaStream_t s = M->stream;
   M3_CUDA(cudaMemcpyAsync(W->r64[img + 1], xc, sizeof(double) * C.ndof, cudaMemcpyHostToDevice, s));
-  M3_TRY(prolong<double>(F, C, W->r64[img + 1], nullptr, W->d64[img], s));
+  M3_TRY(prolong<double>(F, C, W->r64[img + 1], nullptr, W->d64[img], PaCart{}, s));
   M3_CUDA(cudaMemcpyAsync(xf, W->d64[img], sizeof(double) * F.ndof, cudaMemcpyDeviceToHost, s));
   M3_CUDA(cudaStreamSynchronize(s));
   return M3SPH_OK;

@@ -1,0 +1,47 @@
+"""Finest-level element passes on meshes whose element count is not a multiple of their tiles and blocks
+(64 and 128 elements): partially assembled FP32 apply, gradient, divergence and inverse diagonal against
+the FP64 element matrices summed on the host."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# (surface level, layers, MG levels): 60, 240, 480, 720 and 3,840 elements
+SIZES = [(0, 1, 1), (1, 1, 2), (1, 2, 2), (1, 3, 1), (2, 4, 2)]
+
+
+@pytest.fixture(params=SIZES, ids=lambda p: f"L{p[0]}x{p[1]}")
+def dm(request, built_lib):
+    from m3tet_sph_gb300 import stokes, workloads
+    level, layers, nmg = request.param
+    w = workloads.make_workload('c2', level=level, nlayer=layers, nmg=nmg)
+    d = stokes.DeviceMesh(w['levels'])
+    d.setup(w['visc'], w['dens'], w['ifix'], w['vfix'], w['phys'], precision=1)
+    yield w, d
+    d.close()
+
+
+def test_element_passes(dm):
+    w, d = dm
+    f = w['levels'][0]
+    EL, n, nv = f['EL2NOD'], 3 * f['nnod'], d.nvnod
+    K, G, _ = d.element_matrices()
+    dof = (3 * EL[:, :, None] + np.arange(3)).reshape(len(EL), 30)
+    rng = np.random.default_rng(5)
+    x, q = rng.standard_normal(n), rng.standard_normal(nv)
+    free = np.ones(n, bool)
+    free[w['ifix']] = False
+    # K is masked: fixed rows and columns are zero
+    y = np.bincount(dof.ravel(), np.einsum('eij,ej->ei', K, x[dof]).ravel(), n)
+    y32 = d.level_apply32(0, x.astype(np.float32))
+    # FP32 rounding (6e-8) over sums of a few hundred terms of either sign
+    assert np.linalg.norm(y32 - y) <= 1e-5 * np.linalg.norm(y)
+    assert np.all(y32[~free] == 0)
+    # FP64 sums of at most a few hundred terms
+    g = np.bincount(dof.ravel(), np.einsum('eip,ep->ei', G, q[EL[:, :4]]).ravel(), n)
+    assert np.linalg.norm(d.grad(q) - g) <= 1e-13 * np.linalg.norm(g)
+    s = np.bincount(EL[:, :4].ravel(), np.einsum('eip,ei->ep', G, x[dof]).ravel(), nv)
+    assert np.linalg.norm(d.div(x) - s) <= 1e-13 * np.linalg.norm(s)
+    D = np.bincount(dof.ravel(), np.einsum('eii->ei', K).ravel(), n)
+    Di = np.where(free & (D != 0), 1.0 / np.where(D != 0, D, 1.0), 0.0)
+    assert np.allclose(d.level_inverse_diag32(0), Di, rtol=1e-6, atol=0)
