@@ -91,31 +91,64 @@ template <typename R> struct PointFramesT {
 };
 using PointFrames = PointFramesT<double>;
 
-__device__ __forceinline__ void point_frames(double th, double ph, double r, PointFrames &f) {
-  f.p0[0] = th; f.p0[1] = ph; f.p0[2] = r;
+// 180 deg about z: for angles in their usual range the longitude moves by pi (no trigonometry)
+__device__ __forceinline__ void frame_z180(double th, double ph, double r, double *o) {
+  if (th >= 0.0 && th <= M_PI && ph >= 0.0 && ph < 2.0 * M_PI) {
+    o[0] = th;
+    o[1] = ph < M_PI ? ph + M_PI : ph - M_PI;
+    o[2] = r;
+  } else {
+    double x, y, z;
+    sph2cart_d(th, ph, r, x, y, z);
+    c2s(-x, -y, z, o[0], o[1], o[2]);
+  }
+}
+// 90 deg about x
+__device__ __forceinline__ void frame_x90(double th, double ph, double r, double *o) {
   double x, y, z;
   sph2cart_d(th, ph, r, x, y, z);
-  c2s(-x, -y, z, f.pz[0], f.pz[1], f.pz[2]);     // 180 deg about z
-  c2s(x, -z, y, f.px[0], f.px[1], f.px[2]);      // 90 deg about x
+  c2s(x, -z, y, o[0], o[1], o[2]);
+}
+__device__ __forceinline__ void point_frames(double th, double ph, double r, PointFrames &f) {
+  f.p0[0] = th; f.p0[1] = ph; f.p0[2] = r;
+  frame_z180(th, ph, r, f.pz);
+  frame_x90(th, ph, r, f.px);
+}
+// the frames in FP32 without FP64 trigonometry (GB300 issues FP64 at 1/64 of its FP32 rate): what the
+// FP32 walk and pre-filter need, both with margins far above FP32 rounding
+__device__ __forceinline__ void point_frames_f32(double th, double ph, double r, PointFramesT<float> &g) {
+  double z[3];
+  frame_z180(th, ph, r, z);
+  const float thf = (float)th, phf = (float)ph, rf = (float)r;
+  g.p0[0] = thf; g.p0[1] = phf; g.p0[2] = rf;
+  for (int k = 0; k < 3; ++k) g.pz[k] = (float)z[k];
+  float st, ct, sp, cp;
+  sincosf(thf, &st, &ct);
+  sincosf(phf, &sp, &cp);
+  const float x = rf * st * cp, y = rf * st * sp, zz = rf * ct;       // (x, -z, y)
+  g.px[0] = atan2f(sqrtf(x * x + zz * zz), y);
+  g.px[1] = atan2f(-zz, x);
+  if (g.px[1] < 0.f) g.px[1] += 6.2831853f;
+  g.px[2] = sqrtf(x * x + y * y + zz * zz);
 }
 
-// barycentric determinant ratio of local_coords_3d_sph.m:94-147 for vertex a (b,c,d the others)
-template <typename R>
-__device__ __forceinline__ R dratio(const R (&t)[4], const R (&p)[4], const R (&q)[4], int b, int c, int d, R tp, R pp,
-                                    R rp, int a) {
-  auto D = [&](R ta, R pa, R ra) {
-    return (t[b] - ta) * (p[c] - pa) * (q[d] - ra) + (t[c] - ta) * (p[d] - pa) * (q[b] - ra) +
-           (t[d] - ta) * (p[b] - pa) * (q[c] - ra) - (q[b] - ra) * (p[c] - pa) * (t[d] - ta) -
-           (q[c] - ra) * (p[d] - pa) * (t[b] - ta) - (q[d] - ra) * (p[b] - pa) * (t[c] - ta);
-  };
-  return D(tp, pp, rp) / D(t[a], p[a], q[a]);
-}
-
+// barycentric coordinates 0..2 of pt in a straight-in-frame element (the determinant ratios of
+// local_coords_3d_sph.m:94-147), all from differences to vertex 3, which lies on the faces opposite
+// vertices 0..2: 45 multiply-adds and one division in place of six determinants
 template <typename R>
 __device__ __forceinline__ void lc_straight(const R (&t)[4], const R (&p)[4], const R (&q)[4], const R *pt, R *lc) {
-  lc[0] = dratio<R>(t, p, q, 1, 2, 3, pt[0], pt[1], pt[2], 0);
-  lc[1] = dratio<R>(t, p, q, 0, 2, 3, pt[0], pt[1], pt[2], 1);
-  lc[2] = dratio<R>(t, p, q, 0, 1, 3, pt[0], pt[1], pt[2], 2);
+  R a[3], b[3], c[3], d[3];
+  a[0] = t[0] - t[3]; a[1] = p[0] - p[3]; a[2] = q[0] - q[3];
+  b[0] = t[1] - t[3]; b[1] = p[1] - p[3]; b[2] = q[1] - q[3];
+  c[0] = t[2] - t[3]; c[1] = p[2] - p[3]; c[2] = q[2] - q[3];
+  d[0] = pt[0] - t[3]; d[1] = pt[1] - p[3]; d[2] = pt[2] - q[3];
+  const R bc0 = b[1] * c[2] - b[2] * c[1], bc1 = b[2] * c[0] - b[0] * c[2], bc2 = b[0] * c[1] - b[1] * c[0];
+  const R ca0 = c[1] * a[2] - c[2] * a[1], ca1 = c[2] * a[0] - c[0] * a[2], ca2 = c[0] * a[1] - c[1] * a[0];
+  const R ab0 = a[1] * b[2] - a[2] * b[1], ab1 = a[2] * b[0] - a[0] * b[2], ab2 = a[0] * b[1] - a[1] * b[0];
+  const R id = R(1) / (a[0] * bc0 + a[1] * bc1 + a[2] * bc2);
+  lc[0] = (d[0] * bc0 + d[1] * bc1 + d[2] * bc2) * id;
+  lc[1] = (d[0] * ca0 + d[1] * ca1 + d[2] * ca2) * id;
+  lc[2] = (d[0] * ab0 + d[1] * ab1 + d[2] * ab2) * id;
 }
 
 // own-frame local coordinates of point f in element e from the frame coordinates S0/SZ/SX (FP64 or
@@ -251,47 +284,41 @@ struct GapBest {
   __device__ int pick() const { return non >= 0 ? non : iso; }
 };
 
-// one element of a ring or of the brute-force set: a candidate (within the tie band, appended to the
-// warp's shared list; the rule does not depend on the order) or a gap contender
 // an FP32 pre-filter skips the FP64 evaluation of elements the point is far from: FP32 barycentrics
 // err by ~1e-5 here, so an element whose FP32 need exceeds the largest gap tolerance by PRE_MARGIN
 // can be neither a tie candidate nor a gap contender in FP64
 constexpr float PRE_MARGIN = 1e-3f;
-__device__ __forceinline__ PointFramesT<float> frames_f32(const PointFrames &f) {
-  PointFramesT<float> g;
-  for (int k = 0; k < 3; ++k) {
-    g.p0[k] = (float)f.p0[k];
-    g.pz[k] = (float)f.pz[k];
-    g.px[k] = (float)f.px[k];
-  }
-  return g;
+__device__ __forceinline__ bool far_f32(const SlmMesh &m, int e, const PointFramesT<float> &g) {
+  float l[3];
+  local_coords_t<float>(m, m.S0f, m.SZf, m.SXf, e, g, l);
+  const float l4 = 1.0f - l[0] - l[1] - l[2];
+  const float nf = fmaxf(fmaxf(-fminf(fminf(l[0], l[1]), fminf(l[2], l4)), 0.0f),
+                         fmaxf(fmaxf(l[0], l[1]), fmaxf(l[2], l4)) - 1.0f);
+  return nf > (float)((GAP_QMAX + 1) * GAP_STEP) + PRE_MARGIN;        // NaN is not far
 }
+// flags of a candidate within the tie band
+__device__ __forceinline__ uint8_t cand_flags(int cls, double mx) {
+  return (uint8_t)((cls == M3SPH_IN_CONE_ISO ? 1 : 0) | (frame_rank(cls) << 1) | (mx >= 1.0 - TIE_BAND ? 8 : 0));
+}
+// an element the FP32 filter keeps: tie candidate, gap contender or neither
 __device__ __forceinline__ void eval_shared(const SlmMesh &m, int e, const PointFrames &f,
                                             const PointFramesT<float> &g, int *ids, uint8_t *fl, int *n,
                                             GapBest &G) {
-  {
-    float l[3];
-    local_coords_t<float>(m, m.S0f, m.SZf, m.SXf, e, g, l);
-    const float l4 = 1.0f - l[0] - l[1] - l[2];
-    const float nf = fmaxf(fmaxf(-fminf(fminf(l[0], l[1]), fminf(l[2], l4)), 0.0f),
-                           fmaxf(fmaxf(l[0], l[1]), fmaxf(l[2], l4)) - 1.0f);
-    if (nf > (float)((GAP_QMAX + 1) * GAP_STEP) + PRE_MARGIN) return;   // NaN falls through to FP64
-  }
+  if (far_f32(m, e, g)) return;
   double lc[3], mn, mx;
   int am;
   const double step = local_coords(m, e, f, lc);
   bary_minmax(lc, mn, mx, am);
   const double need = fmax(-mn, mx - 1.0);
   const int cls = m.cls[e];
-  const bool iso = cls == M3SPH_IN_CONE_ISO;
   if (need <= TIE_BAND) {
     const int slot = atomicAdd(n, 1);
     if (slot < MAX_CAND) {
       ids[slot] = e;
-      fl[slot] = (uint8_t)((iso ? 1 : 0) | (frame_rank(cls) << 1) | (mx >= 1.0 - TIE_BAND ? 8 : 0));
+      fl[slot] = cand_flags(cls, mx);
     }
   } else if (need <= (GAP_QMAX + 1) * GAP_STEP) {
-    G.add(e, (int)ceil(need / GAP_STEP - 1e-9), iso, step);
+    G.add(e, (int)ceil(need / GAP_STEP - 1e-9), cls == M3SPH_IN_CONE_ISO, step);
   }
 }
 
@@ -311,6 +338,21 @@ __device__ __forceinline__ int gap_reduce(const GapBest &G, int &q) {
     if (oi >= 0 && (iso_e < 0 || os < iso_s || (os == iso_s && oi < iso_e))) { iso_e = oi; iso_s = os; }
   }
   return non >= 0 ? non : iso_e;
+}
+
+// element and local coordinates of a point; adjust: adjust_local_coords
+// (locate_points_interp_vars_3d_sph.m:180-198)
+__device__ __forceinline__ void store_point(int i, int npt, int e, double (&lc)[3], int adjust, int *__restrict__ els,
+                                            double *__restrict__ lc_out) {
+  if (adjust) {
+    for (int k = 0; k < 3; ++k) lc[k] = fmin(fmax(lc[k], 0.0), 1.0);
+    const double sm = lc[0] + lc[1] + lc[2];
+    if (sm > 1.0) for (int k = 0; k < 3; ++k) lc[k] /= sm;
+  }
+  els[i] = e;
+  lc_out[i] = lc[0];
+  lc_out[npt + i] = lc[1];
+  lc_out[2 * (size_t)npt + i] = lc[2];
 }
 
 // rule 1 / rule 2 on the warp's shared candidate list (duplicates removed first), by lane 0;
@@ -345,93 +387,76 @@ __device__ void finish_point(const SlmMesh &m, const PointFrames &f, int i, int 
   }
   double lc[3];
   local_coords(m, e, f, lc);
-  if (adjust) {   // adjust_local_coords (locate_points_interp_vars_3d_sph.m:180-198)
-    for (int k = 0; k < 3; ++k) lc[k] = fmin(fmax(lc[k], 0.0), 1.0);
-    const double sm = lc[0] + lc[1] + lc[2];
-    if (sm > 1.0) for (int k = 0; k < 3; ++k) lc[k] /= sm;
-  }
-  els[i] = e;
-  lc_out[i] = lc[0];
-  lc_out[npt + i] = lc[1];
-  lc_out[2 * npt + i] = lc[2];
+  store_point(i, npt, e, lc, adjust, els, lc_out);
   status[i] = (uint8_t)kind;
 }
 
-// Rules 1-2 for the points k_locate listed: one warp per point over the elements sharing a vertex
-// with the walk's element (placed points) or with any of those (points the walk could not place).
-constexpr int RING_WARPS = 8;
+// elements around element e0 visited once each by the lanes of a warp: depth 1 those sharing a vertex
+// with e0, depth 2 those sharing a vertex with any of these; visit(e, live) is called by whole warps
 constexpr int RING_VTAB = 256;   // open-addressing table of the 1-ring's vertices (2-ring search)
-__global__ void __launch_bounds__(RING_WARPS * 32) k_resolve_ring(SlmMesh m, const double *__restrict__ P, int npt,
-                                                                 const int *__restrict__ todo, int ntodo,
-                                                                 int *__restrict__ els, double *__restrict__ lc_out,
-                                                                 uint8_t *__restrict__ status, int adjust) {
-  __shared__ int s_id[RING_WARPS][MAX_CAND];
-  __shared__ uint8_t s_fl[RING_WARPS][MAX_CAND];
-  __shared__ int s_n[RING_WARPS];
-  __shared__ int s_vt[RING_WARPS][RING_VTAB];
-  const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int w = blockIdx.x * RING_WARPS + wl;
-  if (w >= ntodo) return;
-  const int i = todo[w];
-  const int e0 = els[i];
-  const int depth = (status[i] & 1) ? 1 : 2;
-  if (lane == 0) s_n[wl] = 0;
-  PointFrames f;
-  point_frames(P[i], P[npt + i], P[2 * npt + i], f);
-  const PointFramesT<float> g32 = frames_f32(f);
+template <class V>
+__device__ __forceinline__ void ring_visit(const SlmMesh &m, int e0, int depth, int lane, int *vt, V visit) {
   int v0[4], len[4];
   for (int k = 0; k < 4; ++k) {
     v0[k] = m.el2nod[(size_t)k * m.nel + e0];
     len[k] = m.v2e_ptr[v0[k] + 1] - m.v2e_ptr[v0[k]];
   }
   const int tot = len[0] + len[1] + len[2] + len[3];
-  GapBest G;
-  __syncwarp();
   if (depth == 1) {
-    // an element of the 1-ring is visited once: from the first of e0's vertices it contains
-    for (int t = lane; t < tot; t += 32) {
-      int k = 0, o = t;
-      while (o >= len[k]) o -= len[k++];
-      const int e1 = m.v2e[m.v2e_ptr[v0[k]] + o];
-      bool dup = false;
-      for (int j = 0; j < 4; ++j) {
-        const int v = m.el2nod[(size_t)j * m.nel + e1];
-        for (int kk = 0; kk < k; ++kk) dup |= v == v0[kk];
-      }
-      if (!dup) eval_shared(m, e1, f, g32, s_id[wl], s_fl[wl], &s_n[wl], G);
-    }
-  } else {
-    // vertices of the 1-ring, deduplicated in a shared hash table (-1 = empty)
-    for (int t = lane; t < RING_VTAB; t += 32) s_vt[wl][t] = -1;
-    __syncwarp();
-    for (int t = lane; t < tot; t += 32) {
-      int k = 0, o = t;
-      while (o >= len[k]) o -= len[k++];
-      const int e1 = m.v2e[m.v2e_ptr[v0[k]] + o];
-      for (int j = 0; j < 4; ++j) {
-        const int v = m.el2nod[(size_t)j * m.nel + e1];
-        int h = (int)(((unsigned)v * 2654435761u) % RING_VTAB);
-        for (int probe = 0; probe < RING_VTAB; ++probe) {
-          const int old = atomicCAS(&s_vt[wl][h], -1, v);
-          if (old == -1 || old == v) break;
-          h = (h + 1) % RING_VTAB;
+    // an element of the 1-ring is visited from the first of e0's vertices it contains
+    for (int t0 = 0; t0 < tot; t0 += 32) {
+      const int t = t0 + lane;
+      bool live = t < tot;
+      int e1 = e0;
+      if (live) {
+        int k = 0, o = t;
+        while (o >= len[k]) o -= len[k++];
+        e1 = m.v2e[m.v2e_ptr[v0[k]] + o];
+        for (int j = 0; j < 4; ++j) {
+          const int v = m.el2nod[(size_t)j * m.nel + e1];
+          for (int kk = 0; kk < k; ++kk) live &= v != v0[kk];
         }
       }
+      visit(e1, live);
     }
-    __syncwarp();
-    // an element of the 2-ring is visited once: from the vertex in the table's lowest slot
-    for (int slot = 0; slot < RING_VTAB; ++slot) {
-      const int v = s_vt[wl][slot];
-      if (v < 0) continue;
-      for (int k = m.v2e_ptr[v] + lane; k < m.v2e_ptr[v + 1]; k += 32) {
-        const int e1 = m.v2e[k];
+    return;
+  }
+  // vertices of the 1-ring, deduplicated in a shared hash table (-1 = empty)
+  for (int t = lane; t < RING_VTAB; t += 32) vt[t] = -1;
+  __syncwarp();
+  for (int t = lane; t < tot; t += 32) {
+    int k = 0, o = t;
+    while (o >= len[k]) o -= len[k++];
+    const int e1 = m.v2e[m.v2e_ptr[v0[k]] + o];
+    for (int j = 0; j < 4; ++j) {
+      const int v = m.el2nod[(size_t)j * m.nel + e1];
+      int h = (int)(((unsigned)v * 2654435761u) % RING_VTAB);
+      for (int probe = 0; probe < RING_VTAB; ++probe) {
+        const int old = atomicCAS(&vt[h], -1, v);
+        if (old == -1 || old == v) break;
+        h = (h + 1) % RING_VTAB;
+      }
+    }
+  }
+  __syncwarp();
+  // an element of the 2-ring is visited from its vertex in the table's lowest slot
+  for (int slot = 0; slot < RING_VTAB; ++slot) {
+    const int v = vt[slot];
+    if (v < 0) continue;
+    const int kb = m.v2e_ptr[v], ke = m.v2e_ptr[v + 1];
+    for (int k0 = kb; k0 < ke; k0 += 32) {
+      const int k = k0 + lane;
+      bool live = k < ke;
+      int e1 = e0;
+      if (live) {
+        e1 = m.v2e[k];
         bool dup = false;
         for (int j = 0; j < 4 && !dup; ++j) {
           const int vj = m.el2nod[(size_t)j * m.nel + e1];
           if (vj == v) continue;
           int h = (int)(((unsigned)vj * 2654435761u) % RING_VTAB);
           for (int probe = 0; probe < RING_VTAB; ++probe) {
-            const int tv = s_vt[wl][h];
+            const int tv = vt[h];
             if (tv < 0) break;
             if (tv == vj) {
               dup = h < slot;
@@ -440,46 +465,180 @@ __global__ void __launch_bounds__(RING_WARPS * 32) k_resolve_ring(SlmMesh m, con
             h = (h + 1) % RING_VTAB;
           }
         }
-        if (!dup) eval_shared(m, e1, f, g32, s_id[wl], s_fl[wl], &s_n[wl], G);
+        live = !dup;
       }
+      visit(e1, live);
     }
   }
   __syncwarp();
-  int q;
-  const int gap_e = gap_reduce(G, q);
-  if (lane != 0) return;
-  finish_point(m, f, i, npt, s_id[wl], s_fl[wl], s_n[wl], gap_e, q, 1, adjust, els, lc_out, status);
 }
 
-// one thread per point: walk from the guess to the containing element; points that may tie and
-// points the walk could not place are listed for k_resolve_ring.
-// status bits: 1 placed, 2 tie, 4 gap (tolerance), 8 not placed yet (brute force next), 16 placed by
-// brute force, 32 ambiguous for the reference, 64 candidate list overflow, 128 ring resolution pending
-__global__ void k_locate(SlmMesh m, const double *__restrict__ P, int npt, const int *__restrict__ guess,
-                         const int *__restrict__ node_guess, int *__restrict__ els, double *__restrict__ lc_out,
-                         uint8_t *__restrict__ status, int adjust, int *__restrict__ ring_todo,
-                         int *__restrict__ ring_count) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= npt) return;
-  PointFrames f;
-  point_frames(P[i], P[npt + i], P[2 * npt + i], f);
-  int e = guess ? guess[i] : -1;
-  if ((e < 0 || e >= m.nel) && node_guess) e = node_guess[i];
-  if ((e < 0 || e >= m.nel) && m.grid)
-    e = m.grid[grid_cell(m.gnt, m.gnp, m.gnr, m.grmin, m.grmax, cos(P[i]), P[npt + i], P[2 * npt + i])];
-  if (e < 0 || e >= m.nel) e = 0;
-  int prev = -1, found = -1;
-  // walk in FP32 (the FP64 pipe issues at 1/64 of the FP32 rate) until the FP32 barycentrics place
-  // the point inside within a margin well above their rounding; the FP64 walk below then decides
-  int steps32 = 0;
-  {
-    PointFramesT<float> g;
-    for (int k = 0; k < 3; ++k) {
-      g.p0[k] = (float)f.p0[k];
-      g.pz[k] = (float)f.pz[k];
-      g.px[k] = (float)f.px[k];
+// Rules 1-2 for the points k_place listed, over the elements sharing a vertex with the walk's element
+// (placed points) or with any of those (points the walk could not place).
+//
+// FP64 bounds it: an FP64 instruction takes the SM 16 cycles whatever the number of active lanes. So a
+// block takes 32 points at a time: one warp forms the X-90 frames of all of them, one point per lane,
+// while the warps (4 points each) filter the rings in FP32 and list what is left, about 8 elements a
+// point; the FP64 coordinates of the 4 points' lists are then formed together by the lanes of a warp,
+// and one lane per point applies the rules. (One warp per point, every lane forming the point's frames
+// and each round of 32 ring elements its FP64 coordinates, took 1,069 us for the 43,554 departure points of
+// the 30,720-element shell and 6,464 us for the listed ones of 1.5M random points there; now 316 and
+// 1,287 us.)
+constexpr int RING_WARPS = 8, RING_PTS = 32, RING_PPW = RING_PTS / RING_WARPS;
+constexpr int RING_CAP = 48;     // listed elements per point; more (never on a shell mesh): one by one
+struct RingSmem {
+  double px[3][RING_PTS];
+  double need[RING_PTS][RING_CAP], step[RING_PTS][RING_CAP], lc[RING_PTS][RING_CAP][3];
+  int id[RING_PTS][RING_CAP];
+  int n[RING_PTS];
+  int vt[RING_WARPS][RING_VTAB];
+};
+__global__ void __launch_bounds__(RING_WARPS * 32, 2) k_resolve_ring(SlmMesh m, const double *__restrict__ P, int npt,
+                                                                 const int *__restrict__ todo, const int *__restrict__ ntodo,
+                                                                 int *__restrict__ els, double *__restrict__ lc_out,
+                                                                 uint8_t *__restrict__ status, int adjust) {
+  extern __shared__ __align__(16) unsigned char ring_raw[];
+  RingSmem &S = *reinterpret_cast<RingSmem *>(ring_raw);
+  const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int total = *ntodo;
+  for (int base = blockIdx.x * RING_PTS; base < total; base += gridDim.x * RING_PTS) {
+    const int nloc = min(RING_PTS, total - base);
+    if (wl == 0 && lane < nloc) {
+      const int i = todo[base + lane];
+      double x[3];
+      frame_x90(P[i], P[npt + i], P[2 * (size_t)npt + i], x);
+      for (int k = 0; k < 3; ++k) S.px[k][lane] = x[k];
     }
-    for (; steps32 < WALK_MAX_STEPS; ++steps32) {
+    for (int w = 0; w < RING_PPW; ++w) {
+      const int pt = wl * RING_PPW + w;
+      int cnt = 0;
+      if (pt < nloc) {
+        const int i = todo[base + pt];
+        PointFramesT<float> g;
+        point_frames_f32(P[i], P[npt + i], P[2 * (size_t)npt + i], g);
+        ring_visit(m, els[i], (status[i] & 1) ? 1 : 2, lane, S.vt[wl], [&](int e, bool live) {
+          const bool keep = live && !far_f32(m, e, g);
+          const unsigned mask = __ballot_sync(0xffffffffu, keep);
+          const int at = cnt + __popc(mask & ((1u << lane) - 1u));
+          if (keep && at < RING_CAP) S.id[pt][at] = e;
+          cnt += __popc(mask);
+        });
+      }
+      if (lane == 0) S.n[pt] = cnt;
+    }
+    __syncthreads();
+    // FP64 coordinates of the listed elements of the warp's points
+    int off[RING_PPW + 1];
+    off[0] = 0;
+    for (int w = 0; w < RING_PPW; ++w) off[w + 1] = off[w] + min(S.n[wl * RING_PPW + w], RING_CAP);
+    for (int t = lane; t < off[RING_PPW]; t += 32) {
+      int w = 0;
+      while (t >= off[w + 1]) ++w;
+      const int pt = wl * RING_PPW + w, k = t - off[w], i = todo[base + pt], e = S.id[pt][k];
+      PointFrames f;
+      f.p0[0] = P[i];
+      f.p0[1] = P[npt + i];
+      f.p0[2] = P[2 * (size_t)npt + i];
+      frame_z180(f.p0[0], f.p0[1], f.p0[2], f.pz);
+      for (int c = 0; c < 3; ++c) f.px[c] = S.px[c][pt];
+      double lc[3], mn, mx;
+      int am;
+      S.step[pt][k] = local_coords(m, e, f, lc);
+      bary_minmax(lc, mn, mx, am);
+      S.need[pt][k] = fmax(-mn, mx - 1.0);
+      for (int c = 0; c < 3; ++c) S.lc[pt][k][c] = lc[c];
+    }
+    __syncwarp();
+    if (lane < RING_PPW && wl * RING_PPW + lane < nloc) {
+      const int pt = wl * RING_PPW + lane, i = todo[base + pt], nc = S.n[pt];
+      int ids[MAX_CAND], n = 0;
+      uint8_t fl[MAX_CAND];
+      GapBest G;
+      if (nc <= RING_CAP) {
+        for (int k = 0; k < nc; ++k) {
+          const int e = S.id[pt][k], cls = m.cls[e];
+          const double need = S.need[pt][k], *l = S.lc[pt][k];
+          if (need <= TIE_BAND) {
+            bool dup = false;
+            for (int q = 0; q < n; ++q) dup |= ids[q] == e;
+            if (dup) continue;
+            const double mx = fmax(fmax(l[0], l[1]), fmax(l[2], 1.0 - l[0] - l[1] - l[2]));
+            ids[n] = e;
+            fl[n++] = cand_flags(cls, mx);
+          } else if (need <= (GAP_QMAX + 1) * GAP_STEP) {
+            G.add(e, (int)ceil(need / GAP_STEP - 1e-9), cls == M3SPH_IN_CONE_ISO, S.step[pt][k]);
+          }
+        }
+        int e = -1, kind = 0;
+        if (n > 0) {
+          int amb = 0;
+          e = tie_rule(ids, fl, n, &amb);
+          kind = 1 | (n >= 2 ? 2 : 0) | (amb ? 32 : 0);
+        } else if (G.q <= GAP_QMAX) {
+          e = G.pick();
+          kind = 4;
+        }
+        if (e < 0) {
+          status[i] = 8;
+        } else {
+          int k = 0;
+          while (S.id[pt][k] != e) ++k;
+          double lc[3] = {S.lc[pt][k][0], S.lc[pt][k][1], S.lc[pt][k][2]};
+          store_point(i, npt, e, lc, adjust, els, lc_out);
+          status[i] = (uint8_t)kind;
+        }
+      }
+    }
+    __syncwarp();
+    // points with more listed elements than a list holds: the whole ring again, lists per warp in
+    // the pieces of the point's own arrays
+    for (int w = 0; w < RING_PPW; ++w) {
+      const int pt = wl * RING_PPW + w;
+      if (S.n[pt] <= RING_CAP) continue;
+      const int i = todo[base + pt];
+      int *ids = reinterpret_cast<int *>(S.need[pt]), *n = S.id[pt];
+      uint8_t *fl = reinterpret_cast<uint8_t *>(S.step[pt]);
+      if (lane == 0) *n = 0;
+      __syncwarp();
+      PointFrames f;
+      point_frames(P[i], P[npt + i], P[2 * (size_t)npt + i], f);
+      PointFramesT<float> g;
+      point_frames_f32(P[i], P[npt + i], P[2 * (size_t)npt + i], g);
+      GapBest G;
+      ring_visit(m, els[i], (status[i] & 1) ? 1 : 2, lane, S.vt[wl], [&](int e, bool live) {
+        if (live) eval_shared(m, e, f, g, ids, fl, n, G);
+      });
+      __syncwarp();
+      int q;
+      const int gap_e = gap_reduce(G, q);
+      if (lane == 0) finish_point(m, f, i, npt, ids, fl, *n, gap_e, q, 1, adjust, els, lc_out, status);
+      __syncwarp();
+    }
+    __syncthreads();                                 // lists and frames are free for the next 32 points
+  }
+}
+static_assert(MAX_CAND * sizeof(int) <= sizeof(double) * RING_CAP && MAX_CAND <= sizeof(double) * RING_CAP,
+              "candidate lists fit in a point's arrays");
+
+// One thread per point: FP32 walk from the guess to the element that contains the point within the FP32
+// margin. Points are then listed by what their FP64 coordinates cost (original and Z-180 frames, X-90
+// frame, isoparametric), so that k_place runs warps of one kind.
+__global__ void k_walk32(SlmMesh m, const double *__restrict__ P, int npt, const int *__restrict__ guess,
+                         const int *__restrict__ node_guess, int *__restrict__ els, int *__restrict__ list,
+                         int *__restrict__ cnt) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  int kind = -1;
+  if (i < npt) {
+    const double th = P[i], ph = P[npt + i], r = P[2 * (size_t)npt + i];
+    PointFramesT<float> g;
+    point_frames_f32(th, ph, r, g);
+    int e = guess ? guess[i] : -1;
+    if ((e < 0 || e >= m.nel) && node_guess) e = node_guess[i];
+    if ((e < 0 || e >= m.nel) && m.grid)
+      e = m.grid[grid_cell(m.gnt, m.gnp, m.gnr, m.grmin, m.grmax, (double)cosf((float)th), ph, r)];
+    if (e < 0 || e >= m.nel) e = 0;
+    int prev = -1;
+    for (int step = 0; step < WALK_MAX_STEPS; ++step) {
       float l[3];
       local_coords_t<float>(m, m.S0f, m.SZf, m.SXf, e, g, l);
       const float b[4] = {l[0], l[1], l[2], 1.0f - l[0] - l[1] - l[2]};
@@ -503,94 +662,138 @@ __global__ void k_locate(SlmMesh m, const double *__restrict__ P, int npt, const
       prev = e;
       e = nb;
     }
+    els[i] = e;
+    const int cls = m.cls[e];
+    kind = cls < M3SPH_IN_CONE_NO_ISO ? 0 : (cls == M3SPH_IN_CONE_ISO ? 2 : 1);
   }
-  prev = -1;
-  double lc[3] = {0, 0, 0};
-  uint8_t st = 0;
-  for (int step = 0; step < WALK_MAX_STEPS; ++step) {
-    double mn, mx;
-    int am;
-    local_coords(m, e, f, lc);
-    bary_minmax(lc, mn, mx, am);
-    if (mn >= 0.0 && mx <= 1.0) {
-      found = e;
-      break;
-    }
-    // leave through the face opposite the most negative barycentric; avoid stepping straight back
-    int nb = m.nbr[(size_t)am * m.nel + e];
-    if (nb == prev || nb < 0) {
-      const double b[4] = {lc[0], lc[1], lc[2], 1.0 - lc[0] - lc[1] - lc[2]};
-      int alt = -1;
-      double amin = 1e300;
-      for (int k = 0; k < 4; ++k) {
-        if (k == am || b[k] >= 0.0) continue;
-        const int c = m.nbr[(size_t)k * m.nel + e];
-        if (c >= 0 && c != prev && b[k] < amin) { amin = b[k]; alt = c; }
-      }
-      if (alt < 0) break;
-      nb = alt;
-    }
-    prev = e;
-    e = nb;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const unsigned mask = __ballot_sync(0xffffffffu, kind == c);
+    if (!mask) continue;
+    int at = 0;
+    if (lane == __ffs(mask) - 1) at = atomicAdd(cnt + c, __popc(mask));
+    at = __shfl_sync(0xffffffffu, at, __ffs(mask) - 1) + __popc(mask & ((1u << lane) - 1u));
+    if (kind == c) list[(size_t)c * npt + at] = i;
   }
-  if (found >= 0) {
-    st = 1;
-    // the point may tie with other elements (within the band of a face, edge or vertex, or inside a
-    // face that borders another frame or an isoparametric element, where the own-frame shapes
-    // overlap): the ring is resolved by k_resolve_ring, one warp per such point
-    const double b[4] = {lc[0], lc[1], lc[2], 1.0 - lc[0] - lc[1] - lc[2]};
+}
+
+// (FP32 walk and FP64 walk of unsorted points in one kernel, all three frames in FP64: 3,420 us for 1.5M
+// random points in the 30,720-element shell; k_walk32 466 us + k_place 614 us.)
+// One thread per listed point: FP64 walk from the FP32 element; points that may tie and points the walk
+// could not place are listed for k_resolve_ring. A point's X-90 frame is formed when the first element
+// that needs it is met.
+// status bits: 1 placed, 2 tie, 4 gap (tolerance), 8 not placed yet (brute force next), 16 placed by
+// brute force, 32 ambiguous for the reference, 64 candidate list overflow, 128 ring resolution pending
+__global__ void k_place(SlmMesh m, const double *__restrict__ P, int npt, int *__restrict__ els,
+                        double *__restrict__ lc_out, uint8_t *__restrict__ status, const int *__restrict__ list,
+                        const int *__restrict__ cnt, int *__restrict__ ring_todo, int *__restrict__ ring_count) {
+  const int lane = threadIdx.x & 31, nwarp = (int)((gridDim.x * blockDim.x) >> 5);
+  const int w0 = (cnt[0] + 31) >> 5, w1 = w0 + ((cnt[1] + 31) >> 5), w2 = w1 + ((cnt[2] + 31) >> 5);
+  for (int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); w < w2; w += nwarp) {
+    const int c = w < w0 ? 0 : (w < w1 ? 1 : 2);
+    const int k = ((w - (c == 0 ? 0 : (c == 1 ? w0 : w1))) << 5) + lane;
     bool trig = false;
-    const uint8_t fmask = m.iface[found];
-    for (int k = 0; k < 4; ++k)
-      trig |= b[k] < TIE_TRIGGER || b[k] > 1.0 - TIE_TRIGGER || (((fmask >> k) & 1) && b[k] < IFACE_TRIGGER);
-    if (trig) {
-      st = 1 | 128;
-      ring_todo[atomicAdd(ring_count, 1)] = i;
+    int i = 0;
+    if (k < cnt[c]) {
+      i = list[(size_t)c * npt + k];
+      PointFrames f;
+      f.p0[0] = P[i];
+      f.p0[1] = P[npt + i];
+      f.p0[2] = P[2 * (size_t)npt + i];
+      frame_z180(f.p0[0], f.p0[1], f.p0[2], f.pz);
+      bool have_px = false;
+      int e = els[i], prev = -1, found = -1;
+      double lc[3] = {0, 0, 0};
+      for (int step = 0; step < WALK_MAX_STEPS; ++step) {
+        if (!have_px && m.cls[e] >= M3SPH_IN_CONE_NO_ISO) {
+          frame_x90(f.p0[0], f.p0[1], f.p0[2], f.px);
+          have_px = true;
+        }
+        double mn, mx;
+        int am;
+        local_coords(m, e, f, lc);
+        bary_minmax(lc, mn, mx, am);
+        if (mn >= 0.0 && mx <= 1.0) {
+          found = e;
+          break;
+        }
+        // leave through the face opposite the most negative barycentric; avoid stepping straight back
+        int nb = m.nbr[(size_t)am * m.nel + e];
+        if (nb == prev || nb < 0) {
+          const double b[4] = {lc[0], lc[1], lc[2], 1.0 - lc[0] - lc[1] - lc[2]};
+          int alt = -1;
+          double amin = 1e300;
+          for (int q = 0; q < 4; ++q) {
+            if (q == am || b[q] >= 0.0) continue;
+            const int cand = m.nbr[(size_t)q * m.nel + e];
+            if (cand >= 0 && cand != prev && b[q] < amin) { amin = b[q]; alt = cand; }
+          }
+          if (alt < 0) break;
+          nb = alt;
+        }
+        prev = e;
+        e = nb;
+      }
+      uint8_t st = 128;
+      if (found >= 0) {
+        // the point may tie with other elements (within the band of a face, edge or vertex, or inside a
+        // face that borders another frame or an isoparametric element, where the own-frame shapes
+        // overlap)
+        const double b[4] = {lc[0], lc[1], lc[2], 1.0 - lc[0] - lc[1] - lc[2]};
+        const uint8_t fmask = m.iface[found];
+        for (int q = 0; q < 4; ++q)
+          trig |= b[q] < TIE_TRIGGER || b[q] > 1.0 - TIE_TRIGGER || (((fmask >> q) & 1) && b[q] < IFACE_TRIGGER);
+        st = trig ? (1 | 128) : 1;
+      } else {
+        found = e;                   // the walk's last element: centre of the 2-ring search
+        trig = true;
+      }
+      els[i] = found;
+      status[i] = st;
+      if (!trig) {
+        lc_out[i] = lc[0];
+        lc_out[npt + i] = lc[1];
+        lc_out[2 * (size_t)npt + i] = lc[2];
+      }
     }
-  } else {
-    found = e;                   // the walk's last element: centre of the 2-ring search
-    st = 128;
-    ring_todo[atomicAdd(ring_count, 1)] = i;
+    const unsigned mask = __ballot_sync(0xffffffffu, trig);
+    if (mask) {
+      int at = 0;
+      if (lane == __ffs(mask) - 1) at = atomicAdd(ring_count, __popc(mask));
+      at = __shfl_sync(0xffffffffu, at, __ffs(mask) - 1) + __popc(mask & ((1u << lane) - 1u));
+      if (trig) ring_todo[at] = i;
+    }
   }
-  if (st & 128) {                // resolved later from the centre element stored in els
-    els[i] = found;
-    status[i] = st;
-    return;
-  }
-  els[i] = found;
-  lc_out[i] = lc[0];
-  lc_out[npt + i] = lc[1];
-  lc_out[2 * npt + i] = lc[2];
-  status[i] = st;
 }
 
 // brute force over all elements for points no ring could place (status 8): one warp per point, the
 // same rule over every element
 constexpr int BRUTE_WARPS = 8;
 __global__ void __launch_bounds__(BRUTE_WARPS * 32) k_locate_brute(SlmMesh m, const double *__restrict__ P, int npt,
-                                                                  const int *__restrict__ todo, int ntodo,
+                                                                  const int *__restrict__ todo, const int *__restrict__ ntodo,
                                                                   int *__restrict__ els, double *__restrict__ lc_out,
                                                                   uint8_t *status, int adjust) {
   __shared__ int s_id[BRUTE_WARPS][MAX_CAND];
   __shared__ uint8_t s_fl[BRUTE_WARPS][MAX_CAND];
   __shared__ int s_n[BRUTE_WARPS];
-  const int wl = threadIdx.x >> 5;
-  const int w = blockIdx.x * BRUTE_WARPS + wl;
-  const int lane = threadIdx.x & 31;
-  if (w >= ntodo) return;
-  if (lane == 0) s_n[wl] = 0;
-  __syncwarp();
-  const int i = todo[w];
-  PointFrames f;
-  point_frames(P[i], P[npt + i], P[2 * npt + i], f);
-  GapBest G;
-  const PointFramesT<float> g32 = frames_f32(f);
-  for (int e = lane; e < m.nel; e += 32) eval_shared(m, e, f, g32, s_id[wl], s_fl[wl], &s_n[wl], G);
-  __syncwarp();
-  int q;
-  const int gap_e = gap_reduce(G, q);
-  if (lane != 0) return;
-  finish_point(m, f, i, npt, s_id[wl], s_fl[wl], s_n[wl], gap_e, q, 16, adjust, els, lc_out, status);
+  const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int total = *ntodo;
+  for (int w = blockIdx.x * BRUTE_WARPS + wl; w < total; w += gridDim.x * BRUTE_WARPS) {
+    __syncwarp();
+    if (lane == 0) s_n[wl] = 0;
+    __syncwarp();
+    const int i = todo[w];
+    PointFrames f;
+    point_frames(P[i], P[npt + i], P[2 * (size_t)npt + i], f);
+    PointFramesT<float> g;
+    point_frames_f32(P[i], P[npt + i], P[2 * (size_t)npt + i], g);
+    GapBest G;
+    for (int e = lane; e < m.nel; e += 32) eval_shared(m, e, f, g, s_id[wl], s_fl[wl], &s_n[wl], G);
+    __syncwarp();
+    int q;
+    const int gap_e = gap_reduce(G, q);
+    if (lane == 0) finish_point(m, f, i, npt, s_id[wl], s_fl[wl], s_n[wl], gap_e, q, 16, adjust, els, lc_out, status);
+  }
 }
 
 // P2 interpolation (interp3d_tet.m:39-69): V is [nvar][nnod], out [nvar][npt]
@@ -849,13 +1052,13 @@ struct SlmState {
   float *S0f = nullptr, *SZf = nullptr, *SXf = nullptr;
   uint8_t *cls = nullptr, *iface = nullptr;
   int *ring_count = nullptr;          // [16]: 0 points listed for k_resolve_ring, 1 for the brute force,
-                                      // 2.. status counts (k_status_counts)
+                                      // 2.. status counts (k_status_counts), 9.. points per kind
   double *S0 = nullptr, *SZ = nullptr, *SX = nullptr;
   // work
   double *P = nullptr, *lc = nullptr, *V = nullptr, *out = nullptr, *upu = nullptr, *rpu = nullptr, *U = nullptr;
   double *gel = nullptr, *wel = nullptr, *gn = nullptr, *wn = nullptr;
   double *Xc = nullptr, *kk = nullptr, *acc = nullptr;   // RK4 point, stage slope, weighted sum
-  int *els = nullptr, *guess = nullptr, *todo = nullptr;
+  int *els = nullptr, *guess = nullptr, *todo = nullptr, *list = nullptr;   // list: [3][points] by kind
   uint8_t *status = nullptr;
   size_t cap = 0;
   SlmMesh view{};
@@ -892,7 +1095,7 @@ int slm_build(m3sph_mesh *M, const m3sph_level &f0) {
                     (void *)S->V, (void *)S->out, (void *)S->upu, (void *)S->rpu, (void *)S->U, (void *)S->gel,
                     (void *)S->wel, (void *)S->gn, (void *)S->wn, (void *)S->Xc, (void *)S->kk, (void *)S->acc,
                     (void *)S->els, (void *)S->guess,
-                    (void *)S->todo, (void *)S->status, (void *)S->grid, (void *)S->S0f, (void *)S->SZf,
+                    (void *)S->todo, (void *)S->list, (void *)S->status, (void *)S->grid, (void *)S->S0f, (void *)S->SZf,
                     (void *)S->SXf, (void *)S->iface, (void *)S->ring_count})
       if (q) cudaFree(q);
     delete S;
@@ -1031,6 +1234,7 @@ int slm_build(m3sph_mesh *M, const m3sph_level &f0) {
       (st = sl_upload(&S->SXf, SXf.data(), SXf.size(), s)))
     return st;
   M3_CUDA(cudaStreamSynchronize(s));
+  M3_CUDA(cudaFuncSetAttribute(k_resolve_ring, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RingSmem)));
   S->view = SlmMesh{nel, nnod, nv, S->el2nod, S->nbr, S->cls, S->S0, S->SZ, S->SX, S->v2e_ptr, S->v2e, S->iface,
                     S->S0f, S->SZf, S->SXf, S->grid, gnt, gnp, gnr, grmin, grmax};
   S->built = true;
@@ -1042,7 +1246,7 @@ int slm_build(m3sph_mesh *M, const m3sph_level &f0) {
 static int slm_reserve(SlmState *S, size_t npt, int nel, int nnod, int nv) {
   if (npt <= S->cap && S->P) return M3SPH_OK;
   for (void *q : {(void *)S->P, (void *)S->lc, (void *)S->V, (void *)S->out, (void *)S->upu, (void *)S->rpu,
-                  (void *)S->U, (void *)S->els, (void *)S->guess, (void *)S->todo, (void *)S->status})
+                  (void *)S->U, (void *)S->els, (void *)S->guess, (void *)S->todo, (void *)S->list, (void *)S->status})
     if (q) cudaFree(q);
   const size_t n = std::max(npt, (size_t)nnod);
   int st;
@@ -1050,7 +1254,7 @@ static int slm_reserve(SlmState *S, size_t npt, int nel, int nnod, int nv) {
       (st = sl_alloc(&S->out, 3 * n)) || (st = sl_alloc(&S->upu, 3 * (size_t)nnod)) ||
       (st = sl_alloc(&S->rpu, 3 * (size_t)nnod)) || (st = sl_alloc(&S->U, 3 * (size_t)nnod)) ||
       (st = sl_alloc(&S->els, n)) || (st = sl_alloc(&S->guess, n)) || (st = sl_alloc(&S->todo, n)) ||
-      (st = sl_alloc(&S->status, n)))
+      (st = sl_alloc(&S->list, 3 * n)) || (st = sl_alloc(&S->status, n)))
     return st;
   if (!S->gel) {
     if ((st = sl_alloc(&S->gel, 3 * (size_t)nel)) || (st = sl_alloc(&S->wel, 4 * (size_t)nel)) ||
@@ -1116,34 +1320,25 @@ __global__ void k_status_counts(const uint8_t *__restrict__ status, int npt, int
 static int slm_locate(m3sph_mesh *M, SlmState *S, int npt, bool use_guess, bool node_guess, bool adjust,
                       m3sph_locate_info *info) {
   cudaStream_t s = M->stream;
-  M3_CUDA(cudaMemsetAsync(S->ring_count, 0, 16 * sizeof(int), s));
-  k_locate<<<(npt + 127) / 128, 128, 0, s>>>(S->view, S->P, npt, use_guess ? S->guess : nullptr,
-                                              node_guess ? S->node_guess : nullptr, S->els, S->lc, S->status,
-                                              adjust ? 1 : 0, S->todo, S->ring_count); count_launch();
-  M3_CUDA(cudaGetLastError());
-  int nring = 0;
-  M3_CUDA(cudaMemcpyAsync(&nring, S->ring_count, sizeof(int), cudaMemcpyDeviceToHost, s));
-  M3_CUDA(cudaStreamSynchronize(s));
-  if (nring > 0) {
-    k_resolve_ring<<<(nring + RING_WARPS - 1) / RING_WARPS, RING_WARPS * 32, 0, s>>>(S->view, S->P, npt, S->todo, nring,
-                                                                                     S->els, S->lc, S->status,
-                                                                                     adjust ? 1 : 0); count_launch();
-    M3_CUDA(cudaGetLastError());
-  }
+  // counters: [0] ring points, [1] brute-force points, [2..8] status counts, [9..11] points per kind. The
+  // passes read the counts they need on the device, so the host waits once, for the status counts.
+  int *cnt = S->ring_count;
+  M3_CUDA(cudaMemsetAsync(cnt, 0, 16 * sizeof(int), s));
+  const int b128 = (npt + 127) / 128;
+  k_walk32<<<b128, 128, 0, s>>>(S->view, S->P, npt, use_guess ? S->guess : nullptr, node_guess ? S->node_guess : nullptr,
+                                S->els, S->list, cnt + 9); count_launch();
+  k_place<<<std::min(b128 + 3, 152 * 16), 128, 0, s>>>(S->view, S->P, npt, S->els, S->lc, S->status, S->list, cnt + 9,
+                                                       S->todo, cnt); count_launch();
+  k_resolve_ring<<<std::min((npt + RING_PTS - 1) / RING_PTS, 152 * 2), RING_WARPS * 32, sizeof(RingSmem), s>>>(
+      S->view, S->P, npt, S->todo, cnt, S->els, S->lc, S->status, adjust ? 1 : 0); count_launch();
   // unplaced points: listed on the device, brute force over the list
-  k_status_compact<<<(npt + 255) / 256, 256, 0, s>>>(S->status, npt, S->todo, S->ring_count + 1); count_launch();
-  int nt = 0;
-  M3_CUDA(cudaMemcpyAsync(&nt, S->ring_count + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
-  M3_CUDA(cudaStreamSynchronize(s));
-  if (nt > 0) {
-    k_locate_brute<<<(nt + BRUTE_WARPS - 1) / BRUTE_WARPS, BRUTE_WARPS * 32, 0, s>>>(S->view, S->P, npt, S->todo, nt,
-                                                                                    S->els, S->lc, S->status,
-                                                                                    adjust ? 1 : 0); count_launch();
-    M3_CUDA(cudaGetLastError());
-  }
-  k_status_counts<<<std::min((npt + 255) / 256, 1216), 256, 0, s>>>(S->status, npt, S->ring_count + 2); count_launch();
+  k_status_compact<<<(npt + 255) / 256, 256, 0, s>>>(S->status, npt, S->todo, cnt + 1); count_launch();
+  k_locate_brute<<<std::min((npt + BRUTE_WARPS - 1) / BRUTE_WARPS, 152 * 4), BRUTE_WARPS * 32, 0, s>>>(
+      S->view, S->P, npt, S->todo, cnt + 1, S->els, S->lc, S->status, adjust ? 1 : 0); count_launch();
+  k_status_counts<<<std::min((npt + 255) / 256, 1216), 256, 0, s>>>(S->status, npt, cnt + 2); count_launch();
+  M3_CUDA(cudaGetLastError());
   int hc[7];
-  M3_CUDA(cudaMemcpyAsync(hc, S->ring_count + 2, sizeof(hc), cudaMemcpyDeviceToHost, s));
+  M3_CUDA(cudaMemcpyAsync(hc, cnt + 2, sizeof(hc), cudaMemcpyDeviceToHost, s));
   M3_CUDA(cudaStreamSynchronize(s));
   const int nwalk = hc[0], ntie = hc[1], ngap = hc[2], nbrute = hc[3], nlost = hc[4], nambig = hc[5],
             noverflow = hc[6];

@@ -7,7 +7,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 # (surface level, layers, MG levels): 60, 240, 480, 720 and 3,840 elements
-SIZES = [(0, 1, 1), (1, 1, 2), (1, 2, 2), (1, 3, 1), (2, 4, 2)]
+SIZES = [(0, 1, 1), (1, 1, 1), (1, 2, 2), (1, 3, 1), (2, 4, 2)]
 
 
 @pytest.fixture(params=SIZES, ids=lambda p: f"L{p[0]}x{p[1]}")
