@@ -165,10 +165,10 @@ struct Finest {
 
 struct Coarse {
   int n = 0;                          // dofs of the coarsest level
-  int nf = 0;                         // its free dofs: the dense inverse is nf x nf
+  int nf = 0;                         // its free dofs: the dense inverse is nf rows of dense_ld(nf) values
   int *fidx = nullptr;                // [nf] compact -> level dof
   int *cmap = nullptr;                // [n] level dof -> compact index, -1 for a fixed dof
-  double *A64 = nullptr;              // dense inverse (n x n)
+  double *A64 = nullptr;              // dense inverse
   float *A32 = nullptr;
   bool refine64 = false;              // FP64 path: FP32 inverse + iterative refinement against B64
   float *B32tmp = nullptr;            // [9][nnzb] FP32 copy of the coarsest FP64 blocks (refinement)

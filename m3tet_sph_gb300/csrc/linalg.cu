@@ -325,7 +325,7 @@ template int prolong<float>(const Level &, const Level &, const float *, const f
 // the compact map cmap (-1 for a fixed dof)
 template <typename T>
 __global__ void k_dense_from_bsr(const int *__restrict__ ptr, const int *__restrict__ col, const T *__restrict__ B,
-                                 int nrow, size_t nnzb, const int *__restrict__ cmap, int nf, T *__restrict__ A) {
+                                 int nrow, size_t nnzb, const int *__restrict__ cmap, int ld, T *__restrict__ A) {
   const int i = blockIdx.x;
   if (i >= nrow) return;
   for (int k = ptr[i] + threadIdx.x; k < ptr[i + 1]; k += blockDim.x) {
@@ -337,240 +337,367 @@ __global__ void k_dense_from_bsr(const int *__restrict__ ptr, const int *__restr
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
         const int b = cmap[3 * j + q];
-        if (b >= 0) A[(size_t)a * nf + b] = B[(size_t)(p * 3 + q) * nnzb + k];
+        if (b >= 0) A[(size_t)a * ld + b] = B[(size_t)(p * 3 + q) * nnzb + k];
       }
     }
   }
 }
 // ---------------------------------------------------------------------------------------
-// blocked Gauss-Jordan inverse of the SPD coarsest matrix, 128-wide panels (no pivoting):
-// per panel k, with D = A_kk, C = A_:k (saved) and R = D^-1 A_k: :
+// blocked Gauss-Jordan inverse of the SPD coarsest matrix, panels of NB (no pivoting). Per panel k, with
+// D = A_kk, C = A_:k and R = D^-1 A_k: :
 //   A_ij -= C_i R_j (i, j outside panel k), A_kj = R_j, A_ik = -C_i D^-1, A_kk = D^-1.
-// Three launches per panel; the rank-128 update is a 128x128-tile GEMM in shared memory with an
-// 8x8 register block per thread (16-byte shared loads, K chunks copied with cp.async one chunk
-// ahead of the FMAs). The inner dimension runs in chunks of GJK(T) (32 FP32, 16 FP64)
-// so that the two staged tiles stay near 33 KB.
+// The matrix stays symmetric up to sign -- A_ij = A_ji' when both or neither of panels i, j have been
+// swept, A_ij = -A_ji' when one has -- so only tiles on and below the diagonal are kept and updated (half
+// the work of the full form): C_i of an unswept panel i is the stored tile, of a swept one minus the
+// transpose of tile (k, i), and R_j = +-D^-1 C_j'. The upper triangle is filled in at the end.
+//
+// Three launches per panel:
+//  * k_gjb_diag inverts D in one CTA, the block held in registers (an RT x RT piece per thread), by
+//    16-wide sub-panels: the 16 x 16 pivot block by one warp through shuffles, the rest as rank-16
+//    updates. (One pivot at a time in shared memory took 975 us per panel in FP32 and 3,941 us in FP64;
+//    now 74 us, and 129 us for the 64-wide FP64 block.)
+//  * k_gjb_panels saves C (transposed) and forms R;
+//  * k_gjb_update is a tile GEMM: NB x NB tiles, 256 threads, an RT x RT register block per thread read
+//    from shared memory as 16-byte vectors, chunks of the inner dimension brought in by 16-byte
+//    asynchronous copies two chunks ahead (panels are padded to whole tiles with zeros, so the copies
+//    need no bounds). FP32 issue bounds it: 588 us per panel at 14.8k free dofs = 48 TFLOP/s (the full
+//    form with 4-byte copies: 1,886 us).
+// NB is 64 in FP64: the diagonal block is inverted on one SM, whose FP64 rate (2 FMA a cycle) makes a
+// 128-wide block cost 0.5 ms.
 // ---------------------------------------------------------------------------------------
-constexpr int GJB = 128;
-template <typename T> struct GjChunk { static constexpr int K = sizeof(T) == 4 ? 32 : 16; };
+template <typename T> struct Gj;
+template <> struct Gj<float> { static constexpr int NB = 128, KC = 16; using V = float4; static constexpr int VN = 4; };
+template <> struct Gj<double> { static constexpr int NB = 64, KC = 8; using V = double2; static constexpr int VN = 2; };
+constexpr int GJ_ST = 3;             // chunk stages
+constexpr int GJ_SB = 16;            // sub-panel width of the diagonal block
 
-// D^-1 of the nb x nb diagonal block (one CTA, unblocked Gauss-Jordan in dynamic shared memory:
-// GJB x (GJB+1) values + two pivot vectors)
+// values of the work array: D^-1, its transpose, the saved column panel and the row panel
+template <typename T> size_t gj_work(int n) {
+  const size_t NB = Gj<T>::NB, npad = (n + NB - 1) / NB * NB;
+  return 2 * NB * NB + 2 * NB * npad;
+}
+size_t dense_inverse_work64(int n) { return gj_work<double>(n); }
+size_t dense_inverse_work32(int n) { return gj_work<float>(n); }
+// row stride of the dense inverse: whole 16-byte vectors
+int dense_ld(int n) { return (n + 3) & ~3; }
+
 template <typename T>
-__global__ void __launch_bounds__(256) k_gjb_diag(const T *__restrict__ A, int n, int kb, int nb, T *__restrict__ Dinv) {
-  extern __shared__ __align__(16) unsigned char gj_smem[];
-  T(*a)[GJB + 1] = reinterpret_cast<T(*)[GJB + 1]>(gj_smem);
-  T *colp = reinterpret_cast<T *>(gj_smem) + GJB * (GJB + 1), *rowp = colp + GJB;
-  for (int t = threadIdx.x; t < GJB * GJB; t += blockDim.x) {
-    const int r = t / GJB, c = t % GJB;
-    a[r][c] = (r < nb && c < nb) ? A[(size_t)(kb + r) * n + kb + c] : (r == c ? T(1) : T(0));
+__global__ void __launch_bounds__(256) k_gjb_diag(const T *__restrict__ A, int ld, int kb, int nb, T *__restrict__ Dinv,
+                                                  T *__restrict__ DinvT) {
+  constexpr int NB = Gj<T>::NB, RT = NB / 16, SB = GJ_SB;
+  __shared__ T sC[NB][SB + 1], sK[SB][NB], sR[SB][NB], sD[SB][SB + 1];
+  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16, r0 = ty * RT, c0 = tx * RT;
+  T a[RT][RT];
+#pragma unroll
+  for (int i = 0; i < RT; ++i)
+#pragma unroll
+    for (int j = 0; j < RT; ++j) {
+      const int r = r0 + i, c = c0 + j;
+      a[i][j] = (r < nb && c < nb) ? A[(size_t)(kb + r) * ld + kb + c] : (r == c ? T(1) : T(0));
+    }
+  for (int p0 = 0; p0 < NB; p0 += SB) {
+    const bool inr = r0 >= p0 && r0 < p0 + SB, inc = c0 >= p0 && c0 < p0 + SB;    // RT divides SB
+#pragma unroll
+    for (int i = 0; i < RT; ++i)
+#pragma unroll
+      for (int j = 0; j < RT; ++j) {
+        if (inc) sC[r0 + i][c0 + j - p0] = a[i][j];
+        if (inr) sK[r0 + i - p0][c0 + j] = a[i][j];
+      }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      // 16 x 16 pivot block: lane (h, c) holds rows 8h..8h+7 of column c
+      const int lane = threadIdx.x, c = lane & 15, h = lane >> 4;
+      T d[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) d[r] = sK[8 * h + r][p0 + c];
+#pragma unroll
+      for (int p = 0; p < SB; ++p) {
+        const int hp = p >> 3;
+        const T piv = __shfl_sync(0xffffffffu, d[p & 7], p + 16 * hp);
+        const T rp = __shfl_sync(0xffffffffu, d[p & 7], c + 16 * hp);
+        const T inv = T(1) / piv, row = c == p ? inv : rp * inv;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const T cv = __shfl_sync(0xffffffffu, d[r], p + 16 * h);
+          if (8 * h + r == p) d[r] = row;
+          else d[r] = c == p ? -cv * inv : d[r] - cv * row;
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 8; ++r) sD[8 * h + r][c] = d[r];
+    }
+    __syncthreads();
+    // R = D^-1 A_k: , with D^-1 itself in the panel's own columns
+    for (int q = threadIdx.x; q < SB * NB; q += 256) {
+      const int r = q / NB, c = q % NB;
+      T v = T(0);
+      if (c >= p0 && c < p0 + SB) {
+        v = sD[r][c - p0];
+      } else {
+#pragma unroll
+        for (int m = 0; m < SB; ++m) v += sD[r][m] * sK[m][c];
+      }
+      sR[r][c] = v;
+    }
+    __syncthreads();
+    if (inr) {
+#pragma unroll
+      for (int i = 0; i < RT; ++i)
+#pragma unroll
+        for (int j = 0; j < RT; ++j) a[i][j] = sR[r0 + i - p0][c0 + j];
+    } else {
+      if (inc) {
+#pragma unroll
+        for (int i = 0; i < RT; ++i)
+#pragma unroll
+          for (int j = 0; j < RT; ++j) a[i][j] = T(0);
+      }
+#pragma unroll 4
+      for (int m = 0; m < SB; ++m) {
+        T x[RT], y[RT];
+#pragma unroll
+        for (int i = 0; i < RT; ++i) x[i] = sC[r0 + i][m];
+#pragma unroll
+        for (int j = 0; j < RT; ++j) y[j] = sR[m][c0 + j];
+#pragma unroll
+        for (int i = 0; i < RT; ++i)
+#pragma unroll
+          for (int j = 0; j < RT; ++j) a[i][j] -= x[i] * y[j];
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < RT; ++i)
+#pragma unroll
+    for (int j = 0; j < RT; ++j) {
+      Dinv[(r0 + i) * NB + c0 + j] = a[i][j];
+      DinvT[(c0 + j) * NB + r0 + i] = a[i][j];
+    }
+}
+
+// acc = sum_m X[m][row] Y[m][col] over m < NB, X and Y with row strides ldx, ldy (16-byte aligned).
+// Thread (ty, tx) owns rows and columns in groups of four consecutive indices: gj_idx
+template <typename T>
+__device__ __forceinline__ int gj_idx(int t, int a) {
+  constexpr int NG = Gj<T>::NB / 64;                 // groups per thread
+  return (a >> 2) * (Gj<T>::NB / NG) + 4 * t + (a & 3);
+}
+__device__ __forceinline__ void gj_ld4(const float *p, float *v) {
+  const float4 q = *reinterpret_cast<const float4 *>(p);
+  v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+}
+__device__ __forceinline__ void gj_ld4(const double *p, double *v) {
+  const double2 a = *reinterpret_cast<const double2 *>(p), b = *reinterpret_cast<const double2 *>(p + 2);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ void gj_st4(float *p, const float *v) {
+  *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void gj_st4(double *p, const double *v) {
+  *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
+  *reinterpret_cast<double2 *>(p + 2) = make_double2(v[2], v[3]);
+}
+template <typename T> constexpr size_t gj_smem() { return sizeof(T) * GJ_ST * 2 * Gj<T>::KC * Gj<T>::NB; }
+template <typename T, int RT>
+__device__ __forceinline__ void gj_tile(T (&acc)[RT][RT], const T *__restrict__ X, size_t ldx, const T *__restrict__ Y,
+                                        size_t ldy) {
+  constexpr int NB = Gj<T>::NB, KC = Gj<T>::KC, NCH = NB / KC, VN = 16 / sizeof(T), PR = NB / VN;
+  extern __shared__ __align__(16) unsigned char gj_raw[];
+  T(*sm)[2][KC][NB] = reinterpret_cast<T(*)[2][KC][NB]>(gj_raw);
+  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+#pragma unroll
+  for (int a = 0; a < RT; ++a)
+#pragma unroll
+    for (int b = 0; b < RT; ++b) acc[a][b] = T(0);
+  auto issue = [&](int ch) {
+    if (ch < NCH) {
+      for (int q = threadIdx.x; q < KC * PR; q += 256) {
+        const int m = q / PR, v = (q % PR) * VN, k = ch * KC + m;
+        const uint32_t dx = (uint32_t)__cvta_generic_to_shared(&sm[ch % GJ_ST][0][m][v]);
+        const uint32_t dy = (uint32_t)__cvta_generic_to_shared(&sm[ch % GJ_ST][1][m][v]);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dx), "l"(X + k * ldx + v) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dy), "l"(Y + k * ldy + v) : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int ch = 0; ch < GJ_ST - 1; ++ch) issue(ch);
+  for (int ch = 0; ch < NCH; ++ch) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(GJ_ST - 2) : "memory");
+    __syncthreads();                     // chunk ch has landed, everyone is done with chunk ch - 1
+    issue(ch + GJ_ST - 1);
+    const T(*xs)[NB] = sm[ch % GJ_ST][0], (*ys)[NB] = sm[ch % GJ_ST][1];
+#pragma unroll
+    for (int m = 0; m < KC; ++m) {
+      T xv[RT], yv[RT];
+#pragma unroll
+      for (int g = 0; g < RT; g += 4) {
+        gj_ld4(&xs[m][gj_idx<T>(ty, g)], xv + g);
+        gj_ld4(&ys[m][gj_idx<T>(tx, g)], yv + g);
+      }
+#pragma unroll
+      for (int a = 0; a < RT; ++a)
+#pragma unroll
+        for (int b = 0; b < RT; ++b) acc[a][b] += xv[a] * yv[b];
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// block j: saved column panel Ct[m][i] = C_i[m] for its rows i and row panel R = +-D^-1 C_j' for its
+// columns (minus for panels already swept, j < kblk); zero padding past n
+template <typename T>
+__global__ void __launch_bounds__(256) k_gjb_panels(const T *__restrict__ A, int ld, int n, int kblk, int nb,
+                                                    const T *__restrict__ DinvT, size_t npad, T *__restrict__ R, T *Ct) {
+  constexpr int NB = Gj<T>::NB, RT = NB / 16;
+  __shared__ T tr[32][33];
+  const int j = blockIdx.x, j0 = j * NB, kb = kblk * NB;
+  const bool swept = j < kblk;
+  if (swept) {
+    // C_i = -A_ki' : row m of tile (k, j) is column m of C
+    for (int q = threadIdx.x; q < NB * NB; q += 256) {
+      const int m = q / NB, c = q % NB;
+      Ct[m * npad + j0 + c] = (m < nb) ? -A[(size_t)(kb + m) * ld + j0 + c] : T(0);
+    }
+  } else {
+    // tile (j, k), transposed 32 x 32 at a time
+    const int lx = threadIdx.x % 32, ly = threadIdx.x / 32;
+    for (int b = 0; b < (NB / 32) * (NB / 32); ++b) {
+      const int i0 = (b / (NB / 32)) * 32, m0 = (b % (NB / 32)) * 32;
+      __syncthreads();
+      for (int y = ly; y < 32; y += 8) {
+        const int i = j0 + i0 + y, m = m0 + lx;
+        tr[y][lx] = (i < n && m < nb) ? A[(size_t)i * ld + kb + m] : T(0);
+      }
+      __syncthreads();
+      for (int y = ly; y < 32; y += 8) Ct[(size_t)(m0 + y) * npad + j0 + i0 + lx] = tr[lx][y];
+    }
   }
   __syncthreads();
-  for (int p = 0; p < GJB; ++p) {
-    if (threadIdx.x < GJB) {
-      colp[threadIdx.x] = a[threadIdx.x][p];
-      rowp[threadIdx.x] = a[p][threadIdx.x] / a[p][p];
-    }
-    __syncthreads();
-    const T piv = colp[p];
-    for (int t = threadIdx.x; t < GJB * GJB; t += blockDim.x) {
-      const int r = t / GJB, c = t % GJB;
-      T v;
-      if (r == p) v = (c == p) ? T(1) / piv : rowp[c];
-      else if (c == p) v = -colp[r] / piv;
-      else v = a[r][c] - colp[r] * rowp[c];
-      a[r][c] = v;
-    }
-    __syncthreads();
-  }
-  for (int t = threadIdx.x; t < GJB * GJB; t += blockDim.x) Dinv[t] = a[t / GJB][t % GJB];
-}
-
-// 128x128 tile product acc = X (rows i0.., inner dimension 0..127) * Y (inner, cols j0..), X and Y
-// read through the loaders (row / column index fastest across threads, so global reads coalesce
-// and shared stores do not conflict). 256 threads; thread (ty, tx) owns rows 4ty..4ty+3 and
-// 64+4ty..64+4ty+3 and the same columns with tx, read from shared memory as 16-byte vectors
-// (a quarter-warp's vectors are consecutive: no bank conflicts).
-template <typename T> struct GjVec;
-template <> struct GjVec<float> {
-  static __device__ __forceinline__ void ld4(const float *p, float *v) {
-    const float4 q = *reinterpret_cast<const float4 *>(p);
-    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-  }
-};
-template <> struct GjVec<double> {
-  static __device__ __forceinline__ void ld4(const double *p, double *v) {
-    const double2 a = *reinterpret_cast<const double2 *>(p), b = *reinterpret_cast<const double2 *>(p + 2);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-  }
-};
-constexpr int GJ_LD = GJB + 4;       // shared row stride (16-byte aligned rows)
-__device__ __forceinline__ int gj_row(int t, int a) { return (a < 4 ? 0 : 64) + 4 * t + (a & 3); }
-
-// asynchronous 4- or 8-byte global -> shared copies (cp.async), grouped per K chunk
-template <typename T>
-__device__ __forceinline__ void gj_cp(T *dst, const T *src) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  if constexpr (sizeof(T) == 4)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void gj_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void gj_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// dynamic shared memory of the tile product: two buffers of X and Y chunks
-template <typename T> constexpr size_t gj_tile_smem() { return sizeof(T) * 2 * 2 * GjChunk<T>::K * GJ_LD; }
-
-// the loaders return the source address of an operand element, or nullptr for a zero; chunks of
-// the inner dimension are copied asynchronously one chunk ahead of the FMAs (double buffer)
-template <typename T, typename LX, typename LY>
-__device__ __forceinline__ void gj_tile_mma(T (&acc)[8][8], LX srcx, LY srcy) {
-  constexpr int KC = GjChunk<T>::K, NCH = GJB / KC;
-  extern __shared__ __align__(16) unsigned char gj_tile_raw[];
-  T(*xs)[KC][GJ_LD] = reinterpret_cast<T(*)[KC][GJ_LD]>(gj_tile_raw);               // [2][KC][GJ_LD]
-  T(*ys)[KC][GJ_LD] = reinterpret_cast<T(*)[KC][GJ_LD]>(gj_tile_raw + sizeof(T) * 2 * KC * GJ_LD);
+  T acc[RT][RT];
+  gj_tile<T, RT>(acc, DinvT, NB, Ct + j0, npad);
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
 #pragma unroll
-  for (int a = 0; a < 8; ++a)
+  for (int a = 0; a < RT; ++a)
 #pragma unroll
-    for (int b = 0; b < 8; ++b) acc[a][b] = T(0);
-  auto issue = [&](int ch) {
-    const int buf = ch & 1, k0 = ch * KC;
-    for (int q = threadIdx.x; q < GJB * KC; q += blockDim.x) {
-      const int r = q % GJB, m = q / GJB;
-      const T *px = srcx(r, k0 + m), *py = srcy(k0 + m, r);
-      if (px) gj_cp(&xs[buf][m][r], px); else xs[buf][m][r] = T(0);
-      if (py) gj_cp(&ys[buf][m][r], py); else ys[buf][m][r] = T(0);
-    }
-    gj_commit();
-  };
-  issue(0);
-  for (int ch = 0; ch < NCH; ++ch) {
-    if (ch + 1 < NCH) {
-      issue(ch + 1);
-      gj_wait<1>();
-    } else {
-      gj_wait<0>();
-    }
-    __syncthreads();
-    const int buf = ch & 1;
-#pragma unroll 4
-    for (int m = 0; m < KC; ++m) {
-      T xv[8], yv[8];
-      GjVec<T>::ld4(&xs[buf][m][4 * ty], xv);
-      GjVec<T>::ld4(&xs[buf][m][64 + 4 * ty], xv + 4);
-      GjVec<T>::ld4(&ys[buf][m][4 * tx], yv);
-      GjVec<T>::ld4(&ys[buf][m][64 + 4 * tx], yv + 4);
+    for (int g = 0; g < RT; g += 4) {
+      T v[4];
 #pragma unroll
-      for (int a = 0; a < 8; ++a)
-#pragma unroll
-        for (int b = 0; b < 8; ++b) acc[a][b] += xv[a] * yv[b];
-    }
-    __syncthreads();                     // buffer `buf` is refilled by the next issue
-  }
-}
-
-// column panel C (n x 128, saved transposed as Ct [128][n] before the update overwrites it) and
-// row panel R = D^-1 A_k: (128 x n); block x handles columns [128x, 128x+128) of R and rows
-// [128x, 128x+128) of C
-template <typename T>
-__global__ void __launch_bounds__(256) k_gjb_panels(const T *__restrict__ A, int n, int kb, int nb,
-                                                    const T *__restrict__ Dinv, T *__restrict__ R, T *__restrict__ Cc) {
-  const int j0 = blockIdx.x * GJB;
-  for (int q = threadIdx.x; q < GJB * GJB; q += blockDim.x) {
-    const int r = q % GJB, c = q / GJB;
-    const int i = j0 + r;
-    if (i < n) Cc[(size_t)c * n + i] = c < nb ? A[(size_t)i * n + kb + c] : T(0);
-  }
-  T acc[8][8];
-  gj_tile_mma<T>(
-      acc, [&](int r, int m) -> const T * { return Dinv + r * GJB + m; },
-      [&](int m, int c) -> const T * { return (m < nb && j0 + c < n) ? A + (size_t)(kb + m) * n + j0 + c : nullptr; });
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-#pragma unroll
-  for (int a = 0; a < 8; ++a)
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      const int j = j0 + gj_row(tx, b);
-      if (j < n) R[(size_t)gj_row(ty, a) * n + j] = acc[a][b];
+      for (int b = 0; b < 4; ++b) v[b] = swept ? -acc[a][g + b] : acc[a][g + b];
+      gj_st4(&R[gj_idx<T>(ty, a) * npad + j0 + gj_idx<T>(tx, g)], v);
     }
 }
 
-// the update of one 128x128 tile (by, bx): outside panel k A -= C R; row panel R; column panel
-// -C D^-1; diagonal block D^-1
+// tile (bi, bj), bj <= bi, of the update: A - C R outside panel k; the panel's row R; its column
+// -C D^-1 = -R'; the diagonal block D^-1
 template <typename T>
-__global__ void __launch_bounds__(256) k_gjb_update(T *__restrict__ A, int n, int kblk, int nb,
-                                                    const T *__restrict__ Dinv, const T *__restrict__ R,
-                                                    const T *__restrict__ Cc) {
-  const int bi = blockIdx.y, bj = blockIdx.x;
-  const int i0 = bi * GJB, j0 = bj * GJB, kb = kblk * GJB;
-  const bool rowk = bi == kblk, colk = bj == kblk;
-  if (rowk && colk) {
-    for (int q = threadIdx.x; q < GJB * GJB; q += blockDim.x) {
-      const int r = q / GJB, c = q % GJB;
-      if (r < nb && c < nb) A[(size_t)(kb + r) * n + kb + c] = Dinv[q];
-    }
-    return;
-  }
-  if (rowk) {
-    for (int q = threadIdx.x; q < GJB * GJB; q += blockDim.x) {
-      const int r = q / GJB, c = q % GJB;
-      if (r < nb && j0 + c < n) A[(size_t)(kb + r) * n + j0 + c] = R[(size_t)r * n + j0 + c];
-    }
-    return;
-  }
-  T acc[8][8];
-  gj_tile_mma<T>(
-      acc, [&](int r, int m) -> const T * { return (i0 + r < n) ? Cc + (size_t)m * n + i0 + r : nullptr; },
-      [&](int m, int c) -> const T * {
-        return colk ? Dinv + m * GJB + c : ((j0 + c < n) ? R + (size_t)m * n + j0 + c : nullptr);
-      });
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-#pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    const int i = i0 + gj_row(ty, a);
-    if (i >= n) continue;
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      const int j = j0 + gj_row(tx, b);
-      if (j >= n) continue;
-      if (colk) {
-        if (j - kb < nb) A[(size_t)i * n + j] = -acc[a][b];           // -C D^-1
+__global__ void __launch_bounds__(256, 2) k_gjb_update(T *__restrict__ A, int ld, int n, int kblk, int nb,
+                                                       const T *__restrict__ Dinv, size_t npad, const T *__restrict__ R,
+                                                       const T *__restrict__ Ct) {
+  constexpr int NB = Gj<T>::NB, RT = NB / 16;
+  __shared__ T tr[32][33];
+  int bi = (int)((sqrtf(8.f * blockIdx.x + 1.f) - 1.f) * 0.5f);
+  while ((size_t)bi * (bi + 1) / 2 > blockIdx.x) --bi;
+  while ((size_t)(bi + 1) * (bi + 2) / 2 <= blockIdx.x) ++bi;
+  const int bj = (int)(blockIdx.x - (size_t)bi * (bi + 1) / 2);
+  const int i0 = bi * NB, j0 = bj * NB, kb = kblk * NB;
+  if (bi == kblk) {
+    for (int q = threadIdx.x; q < NB * NB; q += 256) {
+      const int r = q / NB, c = q % NB;
+      if (r >= nb) break;
+      if (bj == kblk) {
+        if (c < nb) A[(size_t)(kb + r) * ld + kb + c] = Dinv[q];
       } else {
-        A[(size_t)i * n + j] -= acc[a][b];                           // A - C R
+        A[(size_t)(kb + r) * ld + j0 + c] = R[r * npad + j0 + c];
       }
     }
+    return;
+  }
+  if (bj == kblk) {
+    const int lx = threadIdx.x % 32, ly = threadIdx.x / 32;
+    for (int b = 0; b < (NB / 32) * (NB / 32); ++b) {
+      const int r0 = (b / (NB / 32)) * 32, m0 = (b % (NB / 32)) * 32;
+      __syncthreads();
+      for (int y = ly; y < 32; y += 8) tr[y][lx] = R[(size_t)(m0 + y) * npad + i0 + r0 + lx];
+      __syncthreads();
+      for (int y = ly; y < 32; y += 8) {
+        const int i = i0 + r0 + y, m = m0 + lx;
+        if (i < n && m < nb) A[(size_t)i * ld + kb + m] = -tr[lx][y];
+      }
+    }
+    return;
+  }
+  T acc[RT][RT];
+  gj_tile<T, RT>(acc, Ct + i0, npad, R + j0, npad);
+  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+#pragma unroll
+  for (int a = 0; a < RT; ++a) {
+    const int i = i0 + gj_idx<T>(ty, a);
+    if (i >= n) continue;
+#pragma unroll
+    for (int g = 0; g < RT; g += 4) {
+      const int j = j0 + gj_idx<T>(tx, g);
+      if (j >= ld) continue;                         // ld is a multiple of 4: whole vectors
+      T *p = A + (size_t)i * ld + j, v[4];
+      gj_ld4(p, v);
+#pragma unroll
+      for (int b = 0; b < 4; ++b) v[b] -= acc[a][g + b];
+      gj_st4(p, v);
+    }
   }
 }
 
-// in-place inverse of the n x n SPD matrix A; work holds GJB*GJB + 2*GJB*n values
+// upper triangle from the lower one
 template <typename T>
-int gj_blocked_inverse(T *A, int n, T *work, cudaStream_t s) {
-  T *Dinv = work, *R = work + GJB * GJB, *Cc = R + (size_t)GJB * n;
-  const int nbk = (n + GJB - 1) / GJB;
-  const size_t dsmem = sizeof(T) * ((size_t)GJB * (GJB + 1) + 2 * GJB);
-  M3_CUDA(cudaFuncSetAttribute(k_gjb_diag<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsmem));
-  M3_CUDA(cudaFuncSetAttribute(k_gjb_panels<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gj_tile_smem<T>()));
-  M3_CUDA(cudaFuncSetAttribute(k_gjb_update<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gj_tile_smem<T>()));
-  for (int k = 0; k < nbk; ++k) {
-    const int kb = k * GJB, nb = std::min(GJB, n - kb);
-    k_gjb_diag<T><<<1, 256, dsmem, s>>>(A, n, kb, nb, Dinv); count_launch();
-    k_gjb_panels<T><<<nbk, 256, gj_tile_smem<T>(), s>>>(A, n, kb, nb, Dinv, R, Cc); count_launch();
-    k_gjb_update<T><<<dim3(nbk, nbk), 256, gj_tile_smem<T>(), s>>>(A, n, k, nb, Dinv, R, Cc); count_launch();
+__global__ void __launch_bounds__(256) k_gjb_mirror(T *__restrict__ A, int ld, int n) {
+  __shared__ T tr[32][33];
+  const int bi = blockIdx.y, bj = blockIdx.x;
+  if (bj > bi) return;
+  const int lx = threadIdx.x % 32, ly = threadIdx.x / 32;
+  for (int y = ly; y < 32; y += 8) {
+    const int i = bi * 32 + y, j = bj * 32 + lx;
+    if (i < n && j < n) tr[y][lx] = A[(size_t)i * ld + j];
   }
+  __syncthreads();
+  for (int y = ly; y < 32; y += 8) {
+    const int i = bj * 32 + y, j = bi * 32 + lx;
+    if (i < n && j < n && j > i) A[(size_t)i * ld + j] = tr[lx][y];
+  }
+}
+
+// in-place inverse of the n x n SPD matrix A with row stride ld; work holds gj_work(n) values
+template <typename T>
+int gj_blocked_inverse(T *A, int ld, int n, T *work, cudaStream_t s) {
+  constexpr int NB = Gj<T>::NB;
+  const int nbk = (n + NB - 1) / NB;
+  const size_t npad = (size_t)nbk * NB;
+  T *Dinv = work, *DinvT = Dinv + NB * NB, *R = DinvT + NB * NB, *Ct = R + NB * npad;
+  M3_CUDA(cudaFuncSetAttribute(k_gjb_panels<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gj_smem<T>()));
+  M3_CUDA(cudaFuncSetAttribute(k_gjb_update<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gj_smem<T>()));
+  for (int k = 0; k < nbk; ++k) {
+    const int kb = k * NB, nb = std::min(NB, n - kb);
+    k_gjb_diag<T><<<1, 256, 0, s>>>(A, ld, kb, nb, Dinv, DinvT); count_launch();
+    k_gjb_panels<T><<<nbk, 256, gj_smem<T>(), s>>>(A, ld, n, k, nb, DinvT, npad, R, Ct); count_launch();
+    k_gjb_update<T><<<(unsigned)((size_t)nbk * (nbk + 1) / 2), 256, gj_smem<T>(), s>>>(A, ld, n, k, nb, Dinv, npad, R, Ct);
+    count_launch();
+  }
+  const unsigned g = (unsigned)((n + 31) / 32);
+  k_gjb_mirror<T><<<dim3(g, g), 256, 0, s>>>(A, ld, n); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
 
-// dense coarse matrix (from the level's block rows) and its blocked Gauss-Jordan inverse; with a
-// `lowp` target the FP64 matrix is rounded to FP32 first and A receives nothing
-// free-dof inverse of the level matrix: A (nf x nf) = (K restricted to the free dofs)^-1
+// free-dof inverse of the level matrix (from its block rows): A (nf rows of dense_ld(nf) values) = (K
+// restricted to the free dofs)^-1
 template <typename T>
 int dense_inverse_blocked(const Level &L, const T *B, T *A, T *work, const int *cmap, int nf, cudaStream_t s) {
-  M3_CUDA(cudaMemsetAsync(A, 0, sizeof(T) * (size_t)nf * nf, s));
-  k_dense_from_bsr<T><<<L.nnod, 64, 0, s>>>(L.bsr_ptr, L.bsr_col, B, L.nnod, (size_t)L.nnzb, cmap, nf, A); count_launch();
-  return gj_blocked_inverse<T>(A, nf, work, s);
+  const int ld = dense_ld(nf);
+  M3_CUDA(cudaMemsetAsync(A, 0, sizeof(T) * (size_t)nf * ld, s));
+  k_dense_from_bsr<T><<<L.nnod, 64, 0, s>>>(L.bsr_ptr, L.bsr_col, B, L.nnod, (size_t)L.nnzb, cmap, ld, A); count_launch();
+  return gj_blocked_inverse<T>(A, ld, nf, work, s);
 }
 template int dense_inverse_blocked<double>(const Level &, const double *, double *, double *, const int *, int,
                                            cudaStream_t);
@@ -580,25 +707,25 @@ template int dense_inverse_blocked<float>(const Level &, const float *, float *,
 // y[fidx[row]] = sum_j A[row][j] x[fidx[j]] over the nf free dofs (one warp per row); the fixed
 // entries of y are zeroed beforehand
 template <typename T>
-__global__ void k_dense_gemv(const T *__restrict__ A, int nf, const int *__restrict__ fidx, const T *__restrict__ x,
+__global__ void k_dense_gemv(const T *__restrict__ A, int ld, int nf, const int *__restrict__ fidx, const T *__restrict__ x,
                              T *__restrict__ y) {
   const int row = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= nf) return;
   T s = 0;
-  for (int j = lane; j < nf; j += 32) s += A[(size_t)row * nf + j] * x[fidx[j]];
+  for (int j = lane; j < nf; j += 32) s += A[(size_t)row * ld + j] * x[fidx[j]];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (lane == 0) y[fidx[row]] = s;
 }
 // the same with A in FP32 and x, y in FP64 (FP64 accumulation): the refined FP64 coarse solve
-__global__ void k_dense_gemv_mixed(const float *__restrict__ A, int nf, const int *__restrict__ fidx,
+__global__ void k_dense_gemv_mixed(const float *__restrict__ A, int ld, int nf, const int *__restrict__ fidx,
                                    const double *__restrict__ x, double *__restrict__ y, int accumulate) {
   const int row = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= nf) return;
   double s = 0.0;
-  for (int j = lane; j < nf; j += 32) s += (double)A[(size_t)row * nf + j] * x[fidx[j]];
+  for (int j = lane; j < nf; j += 32) s += (double)A[(size_t)row * ld + j] * x[fidx[j]];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (lane == 0) y[fidx[row]] = accumulate ? y[fidx[row]] + s : s;
@@ -616,11 +743,11 @@ int coarse_refined(const Level &L, const float *A32, const double *B64, const do
   const int n = L.ndof;
   const unsigned g = (unsigned)((nf + 7) / 8);
   M3_CUDA(cudaMemsetAsync(d, 0, sizeof(double) * n, s));
-  k_dense_gemv_mixed<<<g, 256, 0, s>>>(A32, nf, fidx, r, d, 0); count_launch();
+  k_dense_gemv_mixed<<<g, 256, 0, s>>>(A32, dense_ld(nf), nf, fidx, r, d, 0); count_launch();
   for (int k = 0; k < sweeps; ++k) {
     M3_TRY(bsr_apply<double>(L, B64, d, t, s));
     k_sub_masked<<<(n + 255) / 256, 256, 0, s>>>(r, t, L.freemask, t, n); count_launch();
-    k_dense_gemv_mixed<<<g, 256, 0, s>>>(A32, nf, fidx, t, d, 1); count_launch();
+    k_dense_gemv_mixed<<<g, 256, 0, s>>>(A32, dense_ld(nf), nf, fidx, t, d, 1); count_launch();
   }
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
@@ -643,7 +770,7 @@ template <typename T>
 int dense_gemv(const T *A, int n, int nf, const int *fidx, const T *x, T *y, cudaStream_t s) {
   M3_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * n, s));
   if (nf > 0) {
-    k_dense_gemv<T><<<(nf + 7) / 8, 256, 0, s>>>(A, nf, fidx, x, y);
+    k_dense_gemv<T><<<(nf + 7) / 8, 256, 0, s>>>(A, dense_ld(nf), nf, fidx, x, y);
     count_launch();
   }
   M3_CUDA(cudaGetLastError());

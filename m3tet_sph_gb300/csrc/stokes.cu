@@ -79,6 +79,9 @@ int dense_inverse_from64(const Level &L, const double *B64, float *B32tmp, float
 int coarse_refined(const Level &L, const float *A32, const double *B64, const double *r, double *d, double *t,
                    int sweeps, const int *fidx, int nf, cudaStream_t s);
 template <typename T> int dense_gemv(const T *A, int n, int nf, const int *fidx, const T *x, T *y, cudaStream_t s);
+size_t dense_inverse_work64(int n);
+size_t dense_inverse_work32(int n);
+int dense_ld(int n);
 size_t element_setup_smem();
 
 // ---- errors and counters ----
@@ -647,9 +650,8 @@ static int alloc_work(m3sph_mesh *M) {
     M3_TRY(dalloc(&W->t64[i], n)); M3_TRY(dalloc(&W->t32[i], n));
   }
   const size_t nc = M->lev[nmg - 1].ndof;
-  // blocked Gauss-Jordan: the 128x128 diagonal inverse and the 128-wide row and column panels
-  M3_TRY(dalloc(&W->cwork64, 128 * 128 + 2 * 128 * nc));
-  M3_TRY(dalloc(&W->cwork32, 128 * 128 + 2 * 128 * nc));
+  M3_TRY(dalloc(&W->cwork64, dense_inverse_work64((int)nc)));
+  M3_TRY(dalloc(&W->cwork32, dense_inverse_work32((int)nc)));
   const size_t n0 = M->lev[0].ndof, np = M->lev[0].nvnod;
   M3_TRY(dalloc(&W->r, n0)); M3_TRY(dalloc(&W->d, n0)); M3_TRY(dalloc(&W->q, n0));
   M3_TRY(dalloc(&W->Kq, n0)); M3_TRY(dalloc(&W->tmp, n0));
@@ -766,7 +768,7 @@ static int rebuild_operator(m3sph_mesh *M) {
     }
   }
   // coarsest-level solve (stands in for cholesky_factorization / cholesky_solve): the dense
-  // inverse by blocked Gauss-Jordan (128-wide panels), applied as one GEMV per V-cycle. FP32 V-cycle: FP32 inverse.
+  // inverse by blocked Gauss-Jordan, applied as one GEMV per V-cycle. FP32 V-cycle: FP32 inverse.
   // Plain FP64 path: the FP64 inverse up to g_coarse_f64_direct_max dofs; above, the FP32 inverse
   // of the FP64 operator refined against it to FP64 rounding in every coarse solve (an FP64 dense
   // inverse costs 2 n^3 FP64 flops, ~10 s at n = 17,334 on this part's FP64 rate).
@@ -801,16 +803,16 @@ static int rebuild_operator(m3sph_mesh *M) {
   const int nf = M->coarse.nf;
   if (M->nmg > 1) {
     if (M->precision == 0 && nc <= g_coarse_f64_direct_max) {
-      if (!M->coarse.A64) M3_TRY(dalloc(&M->coarse.A64, (size_t)nc * nc));
+      if (!M->coarse.A64) M3_TRY(dalloc(&M->coarse.A64, (size_t)nc * dense_ld(nc)));
       M3_TRY(dense_inverse_blocked<double>(Lc, Lc.B64, M->coarse.A64, W->cwork64, M->coarse.cmap, nf, s));
     } else if (M->precision == 0) {
       M->coarse.refine64 = true;
-      if (!M->coarse.A32) M3_TRY(dalloc(&M->coarse.A32, (size_t)nc * nc));
+      if (!M->coarse.A32) M3_TRY(dalloc(&M->coarse.A32, (size_t)nc * dense_ld(nc)));
       if (!M->coarse.B32tmp) M3_TRY(dalloc(&M->coarse.B32tmp, 9 * (size_t)Lc.nnzb));
       if (!M->coarse.t64) M3_TRY(dalloc(&M->coarse.t64, (size_t)nc));
       M3_TRY(dense_inverse_from64(Lc, Lc.B64, M->coarse.B32tmp, M->coarse.A32, W->cwork32, M->coarse.cmap, nf, s));
     } else {
-      if (!M->coarse.A32) M3_TRY(dalloc(&M->coarse.A32, (size_t)nc * nc));
+      if (!M->coarse.A32) M3_TRY(dalloc(&M->coarse.A32, (size_t)nc * dense_ld(nc)));
       M3_TRY(dense_inverse_blocked<float>(Lc, Lc.B32, M->coarse.A32, W->cwork32, M->coarse.cmap, nf, s));
     }
   }

@@ -45,3 +45,25 @@ def test_element_passes(dm):
     D = np.bincount(dof.ravel(), np.einsum('eii->ei', K).ravel(), n)
     Di = np.where(free & (D != 0), 1.0 / np.where(D != 0, D, 1.0), 0.0)
     assert np.allclose(d.level_inverse_diag32(0), Di, rtol=1e-6, atol=0)
+
+
+@pytest.mark.parametrize("level,layers", [(1, 2), (1, 4), (2, 2)])
+def test_coarse_inverse_panel_edges(level, layers, built_lib):
+    """Coarsest levels whose free dofs do not fill the last panel (378, 630 and 1,458 dofs in all): the
+    FP64 inverse and the FP32 inverse refined against the FP64 operator give the same V-cycle. Three
+    refinements leave (FP32 rounding x condition)^4, far below FP64 rounding; 1e-11 covers the
+    conditioning of the levels above."""
+    from m3tet_sph_gb300 import stokes, workloads
+    w = workloads.make_workload('c2', level=level, nlayer=layers, nmg=2)
+    d = stokes.DeviceMesh(w['levels'])
+    try:
+        r = np.random.default_rng(3).standard_normal(d.ndof)
+        out = []
+        for direct_max in (6000, 0):
+            d.set_option("coarse_f64_direct_max", direct_max)
+            d.setup(w['visc'], w['dens'], w['ifix'], w['vfix'], w['phys'], precision=0)
+            out.append(d.vcycle(r))
+        assert np.linalg.norm(out[1] - out[0]) < 1e-11 * np.linalg.norm(out[0])
+    finally:
+        d.set_option("coarse_f64_direct_max", 6000)
+        d.close()
