@@ -27,21 +27,27 @@ int upload_shape_tables() {
 
 // ----------------------------------------------------------------------------------------
 // element matrix set-up (FP64): one CTA handles EB elements
+//
+// FP64 issue bounds it (2 FMA a cycle per SM). The stiffness block of nodes i, j is formed from the 3x3
+// moment H = sum_q w eta grad Ni grad Nj' alone (9 FMA per point, the weights folded into the stored
+// gradients as sqrt(w eta)): K[p][q] = d_pq tr H + H[q][p] - 2/3 H[p][q]. Gradients come from the four
+// barycentric gradients, and the boundary-condition products run only in elements with a nonzero
+// prescribed velocity. (All nine entries of the block formed at every point and the boundary products
+// in every element: 19.4 ms at 245,760 elements; now 10.4 ms.)
 // ----------------------------------------------------------------------------------------
 constexpr int EB = 32;
 constexpr int SETUP_THREADS = 256;
 // shared-memory layout per CTA, all arrays [..][EB]
-constexpr int SM_DN = NIP * 10 * 3;     // dN/dx at each IP
-constexpr int SM_W = NIP;               // weight
-constexpr int SM_W2 = NIP;              // weight * viscosity
+constexpr int SM_DN = NIP * 10 * 3;     // dN/dx at each IP times sqrt(weight * viscosity)
+constexpr int SM_W = NIP;               // weight / sqrt(weight * viscosity)
 constexpr int SM_W3 = NIP;              // weight / viscosity
 constexpr int SM_FG = NIP;              // weight * buoyancy
 constexpr int SM_DIR = NIP * 3;         // radial unit vector in element frame
 constexpr int SM_VC = 60;               // frame (theta,phi,r) of 4 (or 20) geometry nodes
 constexpr int SM_Q = 90;                // per node: Q = R_cls * RR (3x3)
 constexpr int SM_BC = 30;               // unmasked K * Ufix per element dof
-constexpr int SM_PER_EL = SM_DN + SM_W + SM_W2 + SM_W3 + SM_FG + SM_DIR + SM_VC + SM_Q + SM_BC;
-size_t element_setup_smem() { return sizeof(double) * SM_PER_EL * EB + sizeof(int) * 2 * EB; }
+constexpr int SM_PER_EL = SM_DN + SM_W + SM_W3 + SM_FG + SM_DIR + SM_VC + SM_Q + SM_BC;
+size_t element_setup_smem() { return sizeof(double) * SM_PER_EL * EB + sizeof(int) * 3 * EB; }
 
 
 
@@ -56,8 +62,7 @@ __global__ void __launch_bounds__(SETUP_THREADS) k_element_setup(SetupArgs a) {
   extern __shared__ double sm[];
   double *sDN = sm;                          // [ip][n][k][EB]
   double *sW = sDN + SM_DN * EB;
-  double *sW2 = sW + SM_W * EB;
-  double *sW3 = sW2 + SM_W2 * EB;
+  double *sW3 = sW + SM_W * EB;
   double *sFG = sW3 + SM_W3 * EB;
   double *sDIR = sFG + SM_FG * EB;           // [ip][3][EB]
   double *sVC = sDIR + SM_DIR * EB;          // [k][node][EB], node < 4 (or 20 for iso)
@@ -65,6 +70,7 @@ __global__ void __launch_bounds__(SETUP_THREADS) k_element_setup(SetupArgs a) {
   double *sBC = sQ + SM_Q * EB;              // [30][EB]
   int *sMask = reinterpret_cast<int *>(sBC + SM_BC * EB);
   int *sCls = sMask + EB;
+  int *sBcOn = sCls + EB;                    // a nonzero prescribed velocity in the element
   const int e0 = blockIdx.x * EB;
   const int tid = threadIdx.x;
   const int nel = a.nel;
@@ -72,7 +78,7 @@ __global__ void __launch_bounds__(SETUP_THREADS) k_element_setup(SetupArgs a) {
   // phase 0: frame coordinates, per-node rotations and dof masks
   if (tid < EB) {
     const int el = tid, e = e0 + el;
-    int cls = 0, mask = 0;
+    int cls = 0, mask = 0, bc_on = 0;
     if (e < nel) {
       cls = a.cls[e];
       int v[4];
@@ -117,8 +123,11 @@ __global__ void __launch_bounds__(SETUP_THREADS) k_element_setup(SetupArgs a) {
         for (int q = 0; q < 9; ++q) sQ[(n * 9 + q) * EB + el] = Q[q];
         for (int c = 0; c < 3; ++c)
           if (a.freemask[3 * nod + c]) mask |= 1 << (3 * n + c);
+        if (a.ufix)
+          for (int c = 0; c < 3; ++c) bc_on |= a.ufix[3 * (size_t)nod + c] != 0.0;
       }
     }
+    sBcOn[el] = bc_on;
     sMask[el] = mask;
     sCls[el] = cls;
     for (int q = 0; q < 30; ++q) sBC[q * EB + el] = 0.0;
@@ -183,10 +192,6 @@ __global__ void __launch_bounds__(SETUP_THREADS) k_element_setup(SetupArgs a) {
     double Jd[3][3];      // Jd[c][j] = d loc_j / d cart_c
     for (int c = 0; c < 3; ++c)
       for (int j = 0; j < 3; ++j) Jd[c][j] = JSC[c][0] * Ji[0][j] + JSC[c][1] * Ji[1][j] + JSC[c][2] * Ji[2][j];
-    for (int n = 0; n < 10; ++n)
-      for (int c = 0; c < 3; ++c)
-        sDN[((ip * 10 + n) * 3 + c) * EB + el] =
-            Jd[c][0] * c_sf.dNU[ip][n][0] + Jd[c][1] * c_sf.dNU[ip][n][1] + Jd[c][2] * c_sf.dNU[ip][n][2];
     const double w = detCS * detSL * c_sf.ipw[ip];
     double visc = 0.0, dens = 0.0;
     for (int v = 0; v < 4; ++v) {
@@ -197,12 +202,30 @@ __global__ void __launch_bounds__(SETUP_THREADS) k_element_setup(SetupArgs a) {
     if (a.minVisc > 0.0) visc = fmax(visc, a.minVisc);
     if (a.maxVisc > 0.0) visc = fmin(visc, a.maxVisc);
     if (!(visc > 0.0)) atomicOr(a.err, 4);
-    sW[ip * EB + el] = w;
-    sW2[ip * EB + el] = w * visc;
+    // gradients scaled by sqrt(w eta): vertices (4 L_v - 1) grad L_v, edges 4 (L_b grad L_a + L_a grad L_b)
+    const double sq = sqrt(w * visc);
+    {
+      double L[4];
+      for (int v = 0; v < 4; ++v) L[v] = c_sf.NP[ip][v];
+      for (int c = 0; c < 3; ++c) {
+        const double g0 = sq * Jd[c][0], g1 = sq * Jd[c][1], g2 = sq * Jd[c][2], g3 = -(g0 + g1 + g2);
+        double *o = sDN + (ip * 30 + c) * EB + el;
+        o[0 * EB] = (4.0 * L[0] - 1.0) * g0;
+        o[3 * EB] = (4.0 * L[1] - 1.0) * g1;
+        o[6 * EB] = (4.0 * L[2] - 1.0) * g2;
+        o[9 * EB] = (4.0 * L[3] - 1.0) * g3;
+        o[12 * EB] = 4.0 * L[1] * g0 + 4.0 * L[0] * g1;
+        o[15 * EB] = 4.0 * L[2] * g1 + 4.0 * L[1] * g2;
+        o[18 * EB] = 4.0 * L[3] * g2 + 4.0 * L[2] * g3;
+        o[21 * EB] = 4.0 * L[3] * g0 + 4.0 * L[0] * g3;
+        o[24 * EB] = 4.0 * L[2] * g0 + 4.0 * L[0] * g2;
+        o[27 * EB] = 4.0 * L[3] * g1 + 4.0 * L[1] * g3;
+      }
+    }
+    sW[ip * EB + el] = w / sq;
     if (a.PA32) {
       // sqrt(w eta) d xi_j / d x_c in global Cartesian components: frame = R_cls global, so
       // d xi / d x_global = R_cls^T Jd (Z-180: diag(-1,-1,1); X-90: frame (x, -z, y))
-      const double sq = sqrt(w * visc);
       float *pa = a.PA32 + ((size_t)(e >> 6) * NIP + ip) * (9 * 64) + 2 * (e & 31) + ((e >> 5) & 1);
       for (int j = 0; j < 3; ++j) {
         double g0 = Jd[0][j], g1 = Jd[1][j], g2 = Jd[2][j];
@@ -235,23 +258,27 @@ __global__ void __launch_bounds__(SETUP_THREADS) k_element_setup(SetupArgs a) {
     int i = 0, rem = blk;
     while (rem > i) { rem -= i + 1; ++i; }        // blk -> (i, j), j <= i
     const int j = rem;
-    double B[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+    double H[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+#pragma unroll 2
     for (int ip = 0; ip < NIP; ++ip) {
-      const double w2 = sW2[ip * EB + el];
       double di[3], dj[3];
+#pragma unroll
       for (int c = 0; c < 3; ++c) {
         di[c] = sDN[((ip * 10 + i) * 3 + c) * EB + el];
         dj[c] = sDN[((ip * 10 + j) * 3 + c) * EB + el];
       }
-      const double lap = di[0] * dj[0] + di[1] * dj[1] + di[2] * dj[2];
+#pragma unroll
       for (int p = 0; p < 3; ++p)
-        for (int q = 0; q < 3; ++q) {
-          // K[(i,p),(j,q)] = w2 (d_pq gradNi.gradNj + d_q Ni d_p Nj - 2/3 d_p Ni d_q Nj)
-          double v = di[q] * dj[p] + C2 * di[p] * dj[q];
-          if (p == q) v += lap;
-          B[p][q] += w2 * v;
-        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) H[p][q] += di[p] * dj[q];
     }
+    // K[(i,p),(j,q)] = d_pq (gradNi.gradNj) + d_q Ni d_p Nj - 2/3 d_p Ni d_q Nj
+    double B[3][3];
+    const double tr = H[0][0] + H[1][1] + H[2][2];
+#pragma unroll
+    for (int p = 0; p < 3; ++p)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) B[p][q] = (p == q ? tr : 0.0) + H[q][p] + C2 * H[p][q];
     double Qi[9], Qj[9];
     for (int q = 0; q < 9; ++q) { Qi[q] = sQ[(i * 9 + q) * EB + el]; Qj[q] = sQ[(j * 9 + q) * EB + el]; }
     // T = B Qj ; Kl = Qi^T T
@@ -259,7 +286,7 @@ __global__ void __launch_bounds__(SETUP_THREADS) k_element_setup(SetupArgs a) {
     for (int p = 0; p < 3; ++p)
       for (int q = 0; q < 3; ++q) T[p][q] = B[p][0] * Qj[0 * 3 + q] + B[p][1] * Qj[1 * 3 + q] + B[p][2] * Qj[2 * 3 + q];
     const int mask = sMask[el];
-    const bool bc = a.ufix != nullptr;
+    const bool bc = a.ufix != nullptr && sBcOn[el];
     int ni = 0, nj = 0;
     if (bc) {
       ni = a.el2nod[(size_t)i * nel + e];
