@@ -60,6 +60,53 @@ __device__ __forceinline__ void df_mac(float vh, float vl, float xh, float xl, f
   sl += err + e;
 }
 
+// Block reduction whose last block finishes it: v[k] summed over the grid in a fixed order (threads of a
+// block by shuffles, then blocks in order), so the result does not depend on scheduling. `cnt` is 0 before
+// and after. Returns true in the last block, whose thread 0 holds the sums. Blocks of up to 256 threads.
+#ifdef __CUDACC__
+template <int NV>
+__device__ __forceinline__ bool block_reduce_last(double (&v)[NV], double *partials, unsigned *cnt) {
+  __shared__ double sh[NV][8];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  auto block_sum = [&]() {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+      if (lane == 0) sh[k][wid] = v[k];
+    }
+    __syncthreads();
+    if (wid == 0) {
+#pragma unroll
+      for (int k = 0; k < NV; ++k) {
+        double t = lane < nw ? sh[k][lane] : 0.0;
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        v[k] = t;
+      }
+    }
+  };
+  block_sum();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) partials[k * gridDim.x + blockIdx.x] = v[k];
+    __threadfence();
+    last = atomicInc(cnt, gridDim.x - 1) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    v[k] = 0.0;
+    for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x) v[k] += __ldcg(partials + k * gridDim.x + i);
+  }
+  block_sum();
+  return true;
+}
+#endif
+
 template <typename T> constexpr int kpad() { return ((NPACK + KVec<T>::V - 1) / KVec<T>::V) * KVec<T>::V; }
 
 void set_error(const std::string &msg);
@@ -166,13 +213,14 @@ struct Finest {
 struct Coarse {
   int n = 0;                          // dofs of the coarsest level
   int nf = 0;                         // its free dofs: the dense inverse is nf rows of dense_ld(nf) values
-  int *fidx = nullptr;                // [nf] compact -> level dof
   int *cmap = nullptr;                // [n] level dof -> compact index, -1 for a fixed dof
   double *A64 = nullptr;              // dense inverse
   float *A32 = nullptr;
   bool refine64 = false;              // FP64 path: FP32 inverse + iterative refinement against B64
   float *B32tmp = nullptr;            // [9][nnzb] FP32 copy of the coarsest FP64 blocks (refinement)
   double *t64 = nullptr;              // [n] refinement residual
+  double *x64 = nullptr;              // [dense_ld(nf)] operand of the coarse solve on the free dofs (compact)
+  float *x32 = nullptr;
 };
 
 // Cartesian copy of a nodal vector for the partially assembled operator: a pass that writes (theta,
@@ -186,6 +234,16 @@ __device__ __forceinline__ float4 pa_to_cart(const float4 tr, float x0, float x1
   const float a = tr.x * x0 + tr.y * x2;             // ct x0 + st x2
   return make_float4(tr.z * a - tr.w * x1, tr.w * a + tr.z * x1, tr.x * x2 - tr.y * x0, 0.f);
 }
+
+// threads of a node-sum pass that go to the nv vertices, four each, in whole warps; edge nodes follow, one
+// thread each
+__host__ __device__ __forceinline__ int gather_threads4(int nv) { return (4 * nv + 31) & ~31; }
+
+// scratch of a grid reduction
+struct Reduction {
+  double *partials;
+  unsigned *cnt;
+};
 
 struct SetupArgs {
   int nel, nnod;
@@ -280,6 +338,7 @@ struct m3sph_mesh {
   void *slm = nullptr;                // advection / point-location state
   void (*slm_free)(void *) = nullptr;
   double *red = nullptr;              // reduction partials
+  unsigned *red_cnt = nullptr;        // finished blocks of a reduction (0 between kernels)
   double *scal = nullptr;             // device scalars
   double *h_scal = nullptr;           // pinned host mirror
 };

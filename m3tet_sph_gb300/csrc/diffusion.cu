@@ -15,7 +15,7 @@
 
 namespace m3sph {
 
-int dot(const double *a, const double *b, size_t n, double *partials, double *out, cudaStream_t s);
+int dot(const double *a, const double *b, size_t n, double *partials, unsigned *cnt, double *out, cudaStream_t s);
 
 // children of a P2 tetrahedron (local node numbers 0..9) for the three interior diagonals, and the
 // diagonals' end nodes (tetmesh_p2_to_p1.m): the table that the reference's split follows
@@ -364,7 +364,7 @@ int diffusion_resident(m3sph_mesh *M, double *T, double dt, int *nit) {
   const int nfree = n - D->nfix;
   const double sq = std::sqrt((double)std::max(1, nfree));
   double rr = 0.0;
-  M3_TRY(dot(D->r, D->r, n, M->red, M->scal + 20, s));
+  M3_TRY(dot(D->r, D->r, n, M->red, M->red_cnt, M->scal + 20, s));
   M3_TRY(read2(M, 20, rr));
   double norm_r = std::sqrt(rr) / sq;
   const double tol = D->tol * norm_r;
@@ -380,21 +380,21 @@ int diffusion_resident(m3sph_mesh *M, double *T, double dt, int *nit) {
         // beta = (r - rlast) . d / rdlast (Polak-Ribiere)
         k_diff_sub<<<g, 256, 0, s>>>(n, D->r, D->rl, D->Aq); count_launch();
         double num;
-        M3_TRY(dot(D->Aq, D->d, n, M->red, M->scal + 21, s));
+        M3_TRY(dot(D->Aq, D->d, n, M->red, M->red_cnt, M->scal + 21, s));
         M3_TRY(read2(M, 21, num));
         beta = num / rd;
       }
       k_diff_dir<<<g, 256, 0, s>>>(n, D->d, beta, D->q, it == 1); count_launch();
-      M3_TRY(dot(D->r, D->d, n, M->red, M->scal + 22, s));
+      M3_TRY(dot(D->r, D->d, n, M->red, M->red_cnt, M->scal + 22, s));
       M3_TRY(read2(M, 22, rd));
       M3_TRY(diff_apply(M, D, D->q, 1.0, c, true, D->Aq));
       double qAq;
-      M3_TRY(dot(D->q, D->Aq, n, M->red, M->scal + 23, s));
+      M3_TRY(dot(D->q, D->Aq, n, M->red, M->red_cnt, M->scal + 23, s));
       M3_TRY(read2(M, 23, qAq));
       M3_CUDA(cudaMemcpyAsync(D->rl, D->r, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
       const double alpha = rd / qAq;
       k_diff_step<<<g, 256, 0, s>>>(n, alpha, D->q, D->Aq, T, D->r); count_launch();
-      M3_TRY(dot(D->r, D->r, n, M->red, M->scal + 20, s));
+      M3_TRY(dot(D->r, D->r, n, M->red, M->red_cnt, M->scal + 20, s));
       M3_TRY(read2(M, 20, rr));
       norm_r = std::sqrt(rr) / sq;
       if (std::isnan(norm_r)) {

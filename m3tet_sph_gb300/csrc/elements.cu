@@ -1028,11 +1028,13 @@ __global__ void k_bsr_assemble(const T *__restrict__ K, int nel, int nnzb, const
 }
 
 // y = B x for a 3x3-block CSR matrix with blocks stored [9][nnzb]: one warp per block row, lane l
-// takes blocks ptr[i] + l, ptr[i] + l + 32, ... (all loads of a warp coalesced), then a shuffle sum
-template <typename T>
+// takes blocks ptr[i] + l, ptr[i] + l + 32, ... (all loads of a warp coalesced), then a shuffle sum.
+// JAC: one weighted Jacobi sweep y = x + w (r - B x) Di (y another vector than x)
+template <typename T, bool JAC>
 __global__ void __launch_bounds__(256) k_bsr_spmv(const int *__restrict__ ptr, const int *__restrict__ col,
                                                   const T *__restrict__ B, int nrow, size_t nnzb,
-                                                  const T *__restrict__ x, T *__restrict__ y) {
+                                                  const T *__restrict__ x, T *__restrict__ y, T w,
+                                                  const T *__restrict__ r, const T *__restrict__ Di) {
   const int i = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (i >= nrow) return;
@@ -1051,7 +1053,12 @@ __global__ void __launch_bounds__(256) k_bsr_spmv(const int *__restrict__ ptr, c
     s1 += __shfl_xor_sync(0xffffffffu, s1, o);
     s2 += __shfl_xor_sync(0xffffffffu, s2, o);
   }
-  if (lane < 3) y[3 * (size_t)i + lane] = lane == 0 ? s0 : lane == 1 ? s1 : s2;
+  if (lane < 3) {
+    const size_t q = 3 * (size_t)i + lane;
+    const T v = lane == 0 ? s0 : lane == 1 ? s1 : s2;
+    if constexpr (JAC) y[q] = x[q] + w * (r[q] - v) * Di[q];
+    else y[q] = v;
+  }
 }
 
 template <typename T>
@@ -1062,12 +1069,25 @@ int bsr_assemble(const Level &L, const T *K, T *B, cudaStream_t s) {
 }
 template <typename T>
 int bsr_apply(const Level &L, const T *B, const T *x, T *y, cudaStream_t s) {
-  k_bsr_spmv<T><<<(unsigned)(((size_t)L.nnod * 32 + 255) / 256), 256, 0, s>>>(L.bsr_ptr, L.bsr_col, B, L.nnod,
-                                                                             (size_t)L.nnzb, x, y);
+  k_bsr_spmv<T, false><<<(unsigned)(((size_t)L.nnod * 32 + 255) / 256), 256, 0, s>>>(
+      L.bsr_ptr, L.bsr_col, B, L.nnod, (size_t)L.nnzb, x, y, T(0), nullptr, nullptr);
   count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
+// y = x + w (r - B x) Di
+template <typename T>
+int bsr_apply_jac(const Level &L, const T *B, T w, const T *r, const T *Di, const T *x, T *y, cudaStream_t s) {
+  k_bsr_spmv<T, true><<<(unsigned)(((size_t)L.nnod * 32 + 255) / 256), 256, 0, s>>>(L.bsr_ptr, L.bsr_col, B, L.nnod,
+                                                                                   (size_t)L.nnzb, x, y, w, r, Di);
+  count_launch();
+  M3_CUDA(cudaGetLastError());
+  return M3SPH_OK;
+}
+template int bsr_apply_jac<double>(const Level &, const double *, double, const double *, const double *, const double *,
+                                   double *, cudaStream_t);
+template int bsr_apply_jac<float>(const Level &, const float *, float, const float *, const float *, const float *, float *,
+                                  cudaStream_t);
 template int bsr_assemble<double>(const Level &, const double *, double *, cudaStream_t);
 template int bsr_assemble<float>(const Level &, const float *, float *, cudaStream_t);
 template int bsr_apply<double>(const Level &, const double *, const double *, double *, cudaStream_t);

@@ -7,147 +7,108 @@ namespace m3sph {
 
 constexpr int RED_THREADS = 256;
 constexpr int RED_BLOCKS = 608;      // 4 CTAs per SM on 152 SMs
-
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-template <int NV>
-__device__ __forceinline__ void block_sums(double (&v)[NV], double *partials) {
-  __shared__ double sh[NV][RED_THREADS / 32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    const double s = warp_sum(v[k]);
-    if (lane == 0) sh[k][wid] = s;
-  }
-  __syncthreads();
-  if (wid == 0) {
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      double s = lane < RED_THREADS / 32 ? sh[k][lane] : 0.0;
-      s = warp_sum(s);
-      if (lane == 0) partials[k * gridDim.x + blockIdx.x] = s;
-    }
-  }
-}
-
-// final pass: out[k] = sum of partials[k][0..nb)
-template <int NV>
-__global__ void k_finish(const double *partials, int nb, double *out) {
-  double v[NV];
-#pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    double s = 0.0;
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) s += partials[k * nb + i];
-    v[k] = s;
-  }
-  __shared__ double sh[NV][32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    const double s = warp_sum(v[k]);
-    if (lane == 0) sh[k][wid] = s;
-  }
-  __syncthreads();
-  if (wid == 0) {
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      double s = lane < (int)(blockDim.x / 32) ? sh[k][lane] : 0.0;
-      s = warp_sum(s);
-      if (lane == 0) out[k] = s;
-    }
-  }
+// blocks of a reduction over n values: at least 4 values per thread (a fixed number for a given n)
+unsigned red_blocks(size_t n) {
+  return (unsigned)std::max<size_t>(1, std::min<size_t>(RED_BLOCKS, (n + 4 * RED_THREADS - 1) / (4 * RED_THREADS)));
 }
 
 // out[0] = a.b
-__global__ void k_dot(const double *__restrict__ a, const double *__restrict__ b, size_t n, double *partials) {
+__global__ void k_dot(const double *__restrict__ a, const double *__restrict__ b, size_t n, double *partials,
+                      unsigned *cnt, double *out) {
   double v[1] = {0.0};
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     v[0] += a[i] * b[i];
-  block_sums<1>(v, partials);
+  if (block_reduce_last<1>(v, partials, cnt) && threadIdx.x == 0) out[0] = v[0];
 }
-// out[0] = a.b, out[1] = c.b
-__global__ void k_dot2(const double *__restrict__ a, const double *__restrict__ c, const double *__restrict__ b,
-                       size_t n, double *partials) {
+// out[0] = a.b, out[1] = c.b (b in the precision of the preconditioner)
+template <typename T>
+__global__ void k_dot2(const double *__restrict__ a, const double *__restrict__ c, const T *__restrict__ b, size_t n,
+                       double *partials, unsigned *cnt, double *out) {
   double v[2] = {0.0, 0.0};
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    v[0] += a[i] * b[i];
-    v[1] += c[i] * b[i];
+    const double bi = (double)b[i];
+    v[0] += a[i] * bi;
+    v[1] += c[i] * bi;
   }
-  block_sums<2>(v, partials);
+  if (block_reduce_last<2>(v, partials, cnt) && threadIdx.x == 0) {
+    out[0] = v[0];
+    out[1] = v[1];
+  }
 }
 // out[0] = sum(a)
-__global__ void k_sum(const double *__restrict__ a, size_t n, double *partials) {
+__global__ void k_sum(const double *__restrict__ a, size_t n, double *partials, unsigned *cnt, double *out) {
   double v[1] = {0.0};
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) v[0] += a[i];
-  block_sums<1>(v, partials);
+  if (block_reduce_last<1>(v, partials, cnt) && threadIdx.x == 0) out[0] = v[0];
 }
 
-int dot(const double *a, const double *b, size_t n, double *partials, double *out, cudaStream_t s) {
-  k_dot<<<RED_BLOCKS, RED_THREADS, 0, s>>>(a, b, n, partials); count_launch();
-  k_finish<1><<<1, 1024, 0, s>>>(partials, RED_BLOCKS, out); count_launch();
+int dot(const double *a, const double *b, size_t n, double *partials, unsigned *cnt, double *out, cudaStream_t s) {
+  k_dot<<<red_blocks(n), RED_THREADS, 0, s>>>(a, b, n, partials, cnt, out); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
-int dot2(const double *a, const double *c, const double *b, size_t n, double *partials, double *out, cudaStream_t s) {
-  k_dot2<<<RED_BLOCKS, RED_THREADS, 0, s>>>(a, c, b, n, partials); count_launch();
-  k_finish<2><<<1, 1024, 0, s>>>(partials, RED_BLOCKS, out); count_launch();
+template <typename T>
+int dot2(const double *a, const double *c, const T *b, size_t n, double *partials, unsigned *cnt, double *out, cudaStream_t s) {
+  k_dot2<T><<<red_blocks(n), RED_THREADS, 0, s>>>(a, c, b, n, partials, cnt, out); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
-int vsum(const double *a, size_t n, double *partials, double *out, cudaStream_t s) {
-  k_sum<<<RED_BLOCKS, RED_THREADS, 0, s>>>(a, n, partials); count_launch();
-  k_finish<1><<<1, 1024, 0, s>>>(partials, RED_BLOCKS, out); count_launch();
+template int dot2<double>(const double *, const double *, const double *, size_t, double *, unsigned *, double *, cudaStream_t);
+template int dot2<float>(const double *, const double *, const float *, size_t, double *, unsigned *, double *, cudaStream_t);
+int vsum(const double *a, size_t n, double *partials, unsigned *cnt, double *out, cudaStream_t s) {
+  k_sum<<<red_blocks(n), RED_THREADS, 0, s>>>(a, n, partials, cnt, out); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
 
 // ---------------------------------------------------------------------------------------
 // flexible PCG updates with device-resident scalars
-// scal layout used by the CG: [0] rd, [1] Kqprev.d, [2] qKq, [3] rr, [4] rdlast, [5] alpha_prev
+// scal layout used by the CG: [0] rd, [1] Kqprev.d, [2] qKq, [3] rr, [4] rdlast, [5] alpha_prev,
+// [6] first iteration. The V-cycle's result is read in its own precision and the residual is handed to it
+// the same way, and a reduction's last block finishes it (and the scalars), so that an iteration's vector
+// work is three launches beside the outer product (it was eleven, 3-6 us each at 130,662 dofs).
 // ---------------------------------------------------------------------------------------
 // q = d + beta q, beta = -alpha_prev * (Kq_prev . d) / rdlast (Polak-Ribiere: (r - rlast).d / rdlast)
-__global__ void k_cg_dir(const double *__restrict__ d, double *__restrict__ q, size_t n, const double *scal, int first) {
-  if (first < 0) first = scal[6] != 0.0;   // flag kept on the device (graph replay)
+template <typename T>
+__global__ void k_cg_dir(const T *__restrict__ d, double *__restrict__ q, size_t n, const double *scal) {
+  const bool first = scal[6] != 0.0;
   double beta = 0.0;
   if (!first) beta = -scal[5] * scal[1] / scal[4];
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    q[i] = first ? d[i] : d[i] + beta * q[i];
+    q[i] = first ? (double)d[i] : (double)d[i] + beta * q[i];
 }
-// alpha = rd / qKq ; x += alpha q ; r -= alpha Kq ; partial r.r
+// alpha = rd / qKq ; x += alpha q ; r -= alpha Kq (and its FP32 copy) ; rr, rdlast, alpha_prev, first = 0
 __global__ void k_cg_update(double *__restrict__ x, double *__restrict__ r, const double *__restrict__ q,
-                            const double *__restrict__ Kq, size_t n, const double *scal, double *partials) {
-  const double alpha = scal[0] / scal[2];
+                            const double *__restrict__ Kq, float *__restrict__ r32, size_t n, double *scal,
+                            double *partials, unsigned *cnt) {
+  const double rd = scal[0], alpha = rd / scal[2];
   double v[1] = {0.0};
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     x[i] += alpha * q[i];
     const double ri = r[i] - alpha * Kq[i];
     r[i] = ri;
+    if (r32) r32[i] = (float)ri;
     v[0] += ri * ri;
   }
-  block_sums<1>(v, partials);
-}
-// scal[4] = scal[0] (rdlast = rd); scal[5] = alpha
-__global__ void k_cg_roll(double *scal) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    scal[5] = scal[0] / scal[2];
-    scal[4] = scal[0];
+  if (block_reduce_last<1>(v, partials, cnt) && threadIdx.x == 0) {
+    scal[3] = v[0];
+    scal[4] = rd;
+    scal[5] = alpha;
+    scal[6] = 0.0;
   }
 }
 
-int cg_dir(const double *d, double *q, size_t n, const double *scal, int first, cudaStream_t s) {
-  k_cg_dir<<<RED_BLOCKS, RED_THREADS, 0, s>>>(d, q, n, scal, first); count_launch();
+template <typename T>
+int cg_dir(const T *d, double *q, size_t n, const double *scal, cudaStream_t s) {
+  k_cg_dir<T><<<red_blocks(n), RED_THREADS, 0, s>>>(d, q, n, scal); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
-int cg_update(double *x, double *r, const double *q, const double *Kq, size_t n, double *scal, double *partials,
-              cudaStream_t s) {
-  k_cg_update<<<RED_BLOCKS, RED_THREADS, 0, s>>>(x, r, q, Kq, n, scal, partials); count_launch();
-  k_finish<1><<<1, 1024, 0, s>>>(partials, RED_BLOCKS, scal + 3); count_launch();
-  k_cg_roll<<<1, 1, 0, s>>>(scal); count_launch();
+template int cg_dir<double>(const double *, double *, size_t, const double *, cudaStream_t);
+template int cg_dir<float>(const float *, double *, size_t, const double *, cudaStream_t);
+int cg_update(double *x, double *r, const double *q, const double *Kq, float *r32, size_t n, double *scal,
+              double *partials, unsigned *cnt, cudaStream_t s) {
+  k_cg_update<<<red_blocks(n), RED_THREADS, 0, s>>>(x, r, q, Kq, r32, n, scal, partials, cnt); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
@@ -164,14 +125,21 @@ int axpby(double a, const double *x, double b, double *y, size_t n, cudaStream_t
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
-// y = (x - y) masked: residual r = b - Kx on free dofs
-__global__ void k_sub_mask(const double *__restrict__ b, double *__restrict__ y, const uint8_t *__restrict__ mask,
-                           size_t n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    y[i] = mask[i] ? b[i] - y[i] : 0.0;
+// y = (b - y) masked: residual r = b - Kx on free dofs, its FP32 copy and out[0] = r.r
+__global__ void k_residual(const double *__restrict__ b, double *__restrict__ y, const uint8_t *__restrict__ mask,
+                           float *__restrict__ y32, size_t n, double *partials, unsigned *cnt, double *out) {
+  double v[1] = {0.0};
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const double r = mask[i] ? b[i] - y[i] : 0.0;
+    y[i] = r;
+    if (y32) y32[i] = (float)r;
+    v[0] += r * r;
+  }
+  if (block_reduce_last<1>(v, partials, cnt) && threadIdx.x == 0) out[0] = v[0];
 }
-int sub_mask(const double *b, double *y, const uint8_t *mask, size_t n, cudaStream_t s) {
-  k_sub_mask<<<RED_BLOCKS, RED_THREADS, 0, s>>>(b, y, mask, n); count_launch();
+int residual(const double *b, double *y, const uint8_t *mask, float *y32, size_t n, double *partials, unsigned *cnt,
+             double *out, cudaStream_t s) {
+  k_residual<<<red_blocks(n), RED_THREADS, 0, s>>>(b, y, mask, y32, n, partials, cnt, out); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
@@ -238,12 +206,15 @@ template int jac<float>(float, const float *, const float *, const float *, floa
 // d_f += Ic2f d_c (gather over fine rows); both masked to free dofs
 // ---------------------------------------------------------------------------------------
 // one warp per coarse row: lane l takes fine entries ptr[i] + l, + 32, ... (coarse rows gather ~40
-// fine nodes), then a shuffle sum
+// fine nodes), then a shuffle sum. On the way down the coarse residual is also handed to what comes
+// next: the first Jacobi sweep from zero, d = w Di r (Di, d), or the operand of the coarsest-level solve
+// on its free dofs (cmap, xfree).
 template <typename T>
 __global__ void __launch_bounds__(256) k_restrict(const int *__restrict__ ptr, const int *__restrict__ col,
                                                   const float *__restrict__ w, int nrow, const T *__restrict__ a,
                                                   const T *__restrict__ b, const uint8_t *__restrict__ mask,
-                                                  T *__restrict__ out) {
+                                                  T *__restrict__ out, T wj, const T *__restrict__ Di, T *__restrict__ d,
+                                                  const int *__restrict__ cmap, T *__restrict__ xfree) {
   const int i = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (i >= nrow) return;
@@ -268,8 +239,14 @@ __global__ void __launch_bounds__(256) k_restrict(const int *__restrict__ ptr, c
     s2 += __shfl_xor_sync(0xffffffffu, s2, o);
   }
   if (lane < 3) {
-    const T v = lane == 0 ? s0 : lane == 1 ? s1 : s2;
-    out[3 * (size_t)i + lane] = mask[3 * (size_t)i + lane] ? v : T(0);
+    const size_t q = 3 * (size_t)i + lane;
+    const T v = mask[q] ? (lane == 0 ? s0 : lane == 1 ? s1 : s2) : T(0);
+    out[q] = v;
+    if (d) d[q] = wj * v * Di[q];
+    if (cmap) {
+      const int f = cmap[q];
+      if (f >= 0) xfree[f] = v;
+    }
   }
 }
 // out = add + P xc (masked); add may alias out; pc: also the Cartesian copy of out
@@ -295,9 +272,10 @@ __global__ void k_prolong(const int *__restrict__ ptr, const int *__restrict__ c
   if (pc.xc) pc.xc[i] = pa_to_cart(pc.trig[i], (float)t[0], (float)t[1], (float)t[2]);
 }
 template <typename T>
-int restrict_(const Level &F, const Level &C, const T *a, const T *b, T *out, cudaStream_t s) {
+int restrict_(const Level &F, const Level &C, const T *a, const T *b, T *out, cudaStream_t s, T wj, const T *Di, T *d,
+              const int *cmap, T *xfree) {
   k_restrict<T><<<(unsigned)(((size_t)C.nnod * 32 + 255) / 256), 256, 0, s>>>(F.R_ptr, F.R_col, F.R_w, C.nnod, a, b,
-                                                                             C.freemask, out);
+                                                                             C.freemask, out, wj, Di, d, cmap, xfree);
   count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
@@ -309,8 +287,10 @@ int prolong(const Level &F, const Level &C, const T *xc, const T *add, T *out, c
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
-template int restrict_<double>(const Level &, const Level &, const double *, const double *, double *, cudaStream_t);
-template int restrict_<float>(const Level &, const Level &, const float *, const float *, float *, cudaStream_t);
+template int restrict_<double>(const Level &, const Level &, const double *, const double *, double *, cudaStream_t,
+                               double, const double *, double *, const int *, double *);
+template int restrict_<float>(const Level &, const Level &, const float *, const float *, float *, cudaStream_t, float,
+                              const float *, float *, const int *, float *);
 template int prolong<double>(const Level &, const Level &, const double *, const double *, double *, const PaCart &,
                              cudaStream_t);
 template int prolong<float>(const Level &, const Level &, const float *, const float *, float *, const PaCart &,
@@ -704,50 +684,55 @@ template int dense_inverse_blocked<double>(const Level &, const double *, double
 template int dense_inverse_blocked<float>(const Level &, const float *, float *, float *, const int *, int,
                                           cudaStream_t);
 
-// y[fidx[row]] = sum_j A[row][j] x[fidx[j]] over the nf free dofs (one warp per row); the fixed
-// entries of y are zeroed beforehand
-template <typename T>
-__global__ void k_dense_gemv(const T *__restrict__ A, int ld, int nf, const int *__restrict__ fidx, const T *__restrict__ x,
-                             T *__restrict__ y) {
-  const int row = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+// y[i] (+)= sum_j A[cmap[i]][j] x[j], x compact on the free dofs (zero padded to the row stride), 0 on fixed
+// dofs: one warp per dof, 16-byte loads of both (the rows are 16-byte aligned), so a row of 2,430 values is
+// 19 independent loads a lane. (Scalar loads with the operand read through the dof list, after a
+// memset of y: 9.0 us at 2.3k free dofs; now 4.6.)
+template <typename T, typename X>
+__global__ void __launch_bounds__(256) k_dense_gemv(const T *__restrict__ A, int ld, int n, const int *__restrict__ cmap,
+                                                    const X *__restrict__ x, X *__restrict__ y, int accumulate) {
+  const int i = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (row >= nf) return;
-  T s = 0;
-  for (int j = lane; j < nf; j += 32) s += A[(size_t)row * ld + j] * x[fidx[j]];
+  if (i >= n) return;
+  const int row = cmap[i];
+  if (row < 0) {
+    if (lane == 0) y[i] = X(0);
+    return;
+  }
+  const T *a = A + (size_t)row * ld;
+  X s = 0;
+#pragma unroll 4
+  for (int j = 4 * lane; j < ld; j += 128) {
+    T av[4];
+    X xv[4];
+    gj_ld4(a + j, av);
+    gj_ld4(x + j, xv);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) s += (X)av[k] * xv[k];
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) y[fidx[row]] = s;
+  if (lane == 0) y[i] = accumulate ? y[i] + s : s;
 }
-// the same with A in FP32 and x, y in FP64 (FP64 accumulation): the refined FP64 coarse solve
-__global__ void k_dense_gemv_mixed(const float *__restrict__ A, int ld, int nf, const int *__restrict__ fidx,
-                                   const double *__restrict__ x, double *__restrict__ y, int accumulate) {
-  const int row = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= nf) return;
-  double s = 0.0;
-  for (int j = lane; j < nf; j += 32) s += (double)A[(size_t)row * ld + j] * x[fidx[j]];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) y[fidx[row]] = accumulate ? y[fidx[row]] + s : s;
-}
-__global__ void k_sub_masked(const double *a, const double *b, const uint8_t *mask, double *out, int n) {
+// a - b on the free dofs, compact
+__global__ void k_sub_compact(const double *a, const double *b, const int *cmap, double *out, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = mask[i] ? a[i] - b[i] : 0.0;
+  if (i < n && cmap[i] >= 0) out[cmap[i]] = a[i] - b[i];
 }
 template <typename T> int bsr_apply(const Level &L, const T *B, const T *x, T *y, cudaStream_t s);
 
 // FP64 coarse solve d = A^-1 r from the FP32 inverse A32 and the FP64 operator B64 of the coarsest
-// level: d = A32 r, then `sweeps` steps of iterative refinement d += A32 (r - A d)
+// level: d = A32 r, then `sweeps` steps of iterative refinement d += A32 (r - A d); xfree holds r on the
+// free dofs (compact) and is overwritten
 int coarse_refined(const Level &L, const float *A32, const double *B64, const double *r, double *d, double *t,
-                   int sweeps, const int *fidx, int nf, cudaStream_t s) {
-  const int n = L.ndof;
-  const unsigned g = (unsigned)((nf + 7) / 8);
-  M3_CUDA(cudaMemsetAsync(d, 0, sizeof(double) * n, s));
-  k_dense_gemv_mixed<<<g, 256, 0, s>>>(A32, dense_ld(nf), nf, fidx, r, d, 0); count_launch();
+                   int sweeps, const int *cmap, double *xfree, int nf, cudaStream_t s) {
+  const int n = L.ndof, ld = dense_ld(nf);
+  const unsigned g = (unsigned)((n + 7) / 8);
+  k_dense_gemv<float, double><<<g, 256, 0, s>>>(A32, ld, n, cmap, xfree, d, 0); count_launch();
   for (int k = 0; k < sweeps; ++k) {
     M3_TRY(bsr_apply<double>(L, B64, d, t, s));
-    k_sub_masked<<<(n + 255) / 256, 256, 0, s>>>(r, t, L.freemask, t, n); count_launch();
-    k_dense_gemv_mixed<<<g, 256, 0, s>>>(A32, dense_ld(nf), nf, fidx, t, d, 1); count_launch();
+    k_sub_compact<<<(n + 255) / 256, 256, 0, s>>>(r, t, cmap, xfree, n); count_launch();
+    k_dense_gemv<float, double><<<g, 256, 0, s>>>(A32, ld, n, cmap, xfree, d, 1); count_launch();
   }
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
@@ -765,14 +750,11 @@ int dense_inverse_from64(const Level &L, const double *B64, float *B32tmp, float
   return dense_inverse_blocked<float>(L, B32tmp, A, work, cmap, nf, s);
 }
 
-// d = A^-1 r on the free dofs, 0 on the fixed ones
+// d = A^-1 r on the free dofs (r compact in xfree), 0 on the fixed ones
 template <typename T>
-int dense_gemv(const T *A, int n, int nf, const int *fidx, const T *x, T *y, cudaStream_t s) {
-  M3_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * n, s));
-  if (nf > 0) {
-    k_dense_gemv<T><<<(nf + 7) / 8, 256, 0, s>>>(A, dense_ld(nf), nf, fidx, x, y);
-    count_launch();
-  }
+int dense_gemv(const T *A, int n, int nf, const int *cmap, const T *xfree, T *y, cudaStream_t s) {
+  k_dense_gemv<T, T><<<(n + 7) / 8, 256, 0, s>>>(A, dense_ld(nf), n, cmap, xfree, y, 0);
+  count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }

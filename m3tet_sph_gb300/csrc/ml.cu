@@ -583,32 +583,40 @@ __global__ void __launch_bounds__(tc::THREADS, 2) k_ml_sweep_tc(FeatLevel L, Mlp
   }
 }
 
-// gather of row-layout corrections C[e][30]: code entries e * 10 + a, element order (same sums as
-// k_ml_gather); each (element, node) triple is read with one 8-byte and one 4-byte load
+// gather of row-layout corrections C[e][30]: code entries e * 10 + a (the sums of k_ml_gather); each
+// (element, node) triple is read with one 8-byte and one 4-byte load.
+// Four lanes share a vertex, as in the node sums of the FP64-accurate operators
 template <typename T>
-__global__ void k_ml_gather_rows(int nnod, const int *__restrict__ ptr, const int *__restrict__ code,
-                                 const float *__restrict__ C, const uint8_t *__restrict__ mask, float omega,
-                                 T *__restrict__ d, PaCart pc) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= nnod) return;
-  const int b = ptr[n], e = ptr[n + 1];
-  if (e <= b) return;
+__global__ void __launch_bounds__(128) k_ml_gather_rows(int nnod, int nv, const int *__restrict__ ptr,
+                                                        const int *__restrict__ code, const float *__restrict__ C,
+                                                        const uint8_t *__restrict__ mask, float omega,
+                                                        T *__restrict__ d, PaCart pc) {
+  const int t = blockIdx.x * 128 + threadIdx.x, nt4 = gather_threads4(nv);
+  const bool quad = t < nt4;
+  const int n = quad ? t >> 2 : nv + t - nt4, sub = quad ? t & 3 : 0, step = quad ? 4 : 1;
+  const bool live = quad ? n < nv : n < nnod;
+  const int b = live ? ptr[n] : 0, e = live ? ptr[n + 1] : 0;
   float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-  for (int k = b; k < e; ++k) {
+#pragma unroll 2
+  for (int k = b + sub; k < e; k += step) {
     const int el = code[k] / 10, a = code[k] - 10 * el;
     const float *c = C + (size_t)el * OUT + 3 * a;
-    if ((a & 1) == 0) {
-      const float2 v = *reinterpret_cast<const float2 *>(c);
-      s0 += v.x;
-      s1 += v.y;
-      s2 += c[2];
-    } else {
-      const float2 v = *reinterpret_cast<const float2 *>(c + 1);
-      s0 += c[0];
-      s1 += v.x;
-      s2 += v.y;
+    const int odd = a & 1;                      // 8-byte aligned pair for even local nodes
+    const float2 v2 = *reinterpret_cast<const float2 *>(c + odd);
+    const float v1 = c[2 * (1 - odd)];
+    s0 += odd ? v1 : v2.x;
+    s1 += odd ? v2.x : v2.y;
+    s2 += odd ? v2.y : v1;
+  }
+  if (quad) {                                   // warps are of one kind
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+      s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+      s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+      s2 += __shfl_xor_sync(0xffffffffu, s2, o);
     }
   }
+  if (sub || e <= b) return;
   const float w = omega / (float)(e - b);
   ml_add_node<T>(n, w * s0, w * s1, w * s2, mask, d, pc);
 }
@@ -1026,7 +1034,7 @@ int ml_sweep(m3sph_mesh *M, int j, const T *r0, const T *kd, const T *Dinv, T *t
     const int grid = std::min(ntile, 2 * g_nsm);
     k_ml_scale<T><<<(unsigned)((L.ndof + 255) / 256), 256, 0, s>>>(r0, kd, Dinv, S->lev[j].z, L.ndof); count_launch();
     k_ml_sweep_tc<<<grid, tc::THREADS, tc::SMEM_ALLOC, s>>>(f, w, S->lev[j].z, S->lev[j].C, S->err); count_launch();
-    k_ml_gather_rows<T><<<(L.nnod + 127) / 128, 128, 0, s>>>(L.nnod, S->lev[j].n2e_ptr, S->lev[j].n2e_code,
+    k_ml_gather_rows<T><<<(gather_threads4(L.nvnod) + L.nnod - L.nvnod + 127) / 128, 128, 0, s>>>(L.nnod, L.nvnod, S->lev[j].n2e_ptr, S->lev[j].n2e_code,
                                                               S->lev[j].C, L.freemask, M->ml_omega, d, pc); count_launch();
     M3_CUDA(cudaGetLastError());
     return M3SPH_OK;

@@ -33,8 +33,12 @@ int stream_build(Level &L, cudaStream_t s);
 int stream_apply_f32(const Level &L, const float *K, const float *x, float *y, cudaStream_t s);
 int stream_apply_jac_f32(const Level &L, const float *K, float w, const float *r, const float *Di, float *d,
                          cudaStream_t s);
-int stream_apply_df(const Level &L, const float *Kh, const float *Kl, const double *x, double *y, cudaStream_t s);
-int stream_apply_f64(const Level &L, const double *K, const double *x, double *y, cudaStream_t s);
+int stream_apply_df(const Level &L, const float *Kh, const float *Kl, const double *x, double *y, const Reduction *red,
+                    double *out, cudaStream_t s);
+int stream_apply_f64(const Level &L, const double *K, const double *x, double *y, const Reduction *red, double *out,
+                     cudaStream_t s);
+int stream_apply_jac_f64(const Level &L, const double *K, double w, const double *r, const double *Di, double *d,
+                         cudaStream_t s);
 int stream_check(const Level &L, cudaStream_t s);
 int pa_upload_tables();
 int ml_feature_rows(m3sph_mesh *M, int j, const float *z, float *X, float *Sn);
@@ -56,20 +60,26 @@ int mass_precondition(const Level &L, const double *M, const double *r, const do
 template <typename T> int galerkin(const Level &F, const T *Kf, Level &C, T *Kc, cudaStream_t s);
 template <typename T> int bsr_assemble(const Level &L, const T *K, T *B, cudaStream_t s);
 template <typename T> int bsr_apply(const Level &L, const T *B, const T *x, T *y, cudaStream_t s);
-int dot(const double *a, const double *b, size_t n, double *partials, double *out, cudaStream_t s);
-int dot2(const double *a, const double *c, const double *b, size_t n, double *partials, double *out, cudaStream_t s);
-int vsum(const double *a, size_t n, double *partials, double *out, cudaStream_t s);
-int cg_dir(const double *d, double *q, size_t n, const double *scal, int first, cudaStream_t s);
-int cg_update(double *x, double *r, const double *q, const double *Kq, size_t n, double *scal, double *partials,
-              cudaStream_t s);
+template <typename T>
+int bsr_apply_jac(const Level &L, const T *B, T w, const T *r, const T *Di, const T *x, T *y, cudaStream_t s);
+int dot(const double *a, const double *b, size_t n, double *partials, unsigned *cnt, double *out, cudaStream_t s);
+template <typename T>
+int dot2(const double *a, const double *c, const T *b, size_t n, double *partials, unsigned *cnt, double *out, cudaStream_t s);
+int vsum(const double *a, size_t n, double *partials, unsigned *cnt, double *out, cudaStream_t s);
+template <typename T> int cg_dir(const T *d, double *q, size_t n, const double *scal, cudaStream_t s);
+int cg_update(double *x, double *r, const double *q, const double *Kq, float *r32, size_t n, double *scal,
+              double *partials, unsigned *cnt, cudaStream_t s);
+int residual(const double *b, double *y, const uint8_t *mask, float *y32, size_t n, double *partials, unsigned *cnt,
+             double *out, cudaStream_t s);
 int axpby(double a, const double *x, double b, double *y, size_t n, cudaStream_t s);
-int sub_mask(const double *b, double *y, const uint8_t *mask, size_t n, cudaStream_t s);
 int apply_mask(double *y, const uint8_t *mask, size_t n, cudaStream_t s);
 int d2f(const double *a, float *b, size_t n, cudaStream_t s);
 int f2d(const float *a, double *b, size_t n, cudaStream_t s);
 template <typename T> int jac_first(T w, const T *r0, const T *Di, T *d, size_t n, cudaStream_t s);
 template <typename T> int jac(T w, const T *r0, const T *Kd, const T *Di, T *d, size_t n, cudaStream_t s);
-template <typename T> int restrict_(const Level &F, const Level &C, const T *a, const T *b, T *out, cudaStream_t s);
+template <typename T>
+int restrict_(const Level &F, const Level &C, const T *a, const T *b, T *out, cudaStream_t s, T wj, const T *Di, T *d,
+              const int *cmap, T *xfree);
 template <typename T>
 int prolong(const Level &F, const Level &C, const T *xc, const T *add, T *out, const PaCart &pc, cudaStream_t s);
 template <typename T>
@@ -77,8 +87,8 @@ int dense_inverse_blocked(const Level &L, const T *B, T *A, T *work, const int *
 int dense_inverse_from64(const Level &L, const double *B64, float *B32tmp, float *A, float *work, const int *cmap,
                          int nf, cudaStream_t s);
 int coarse_refined(const Level &L, const float *A32, const double *B64, const double *r, double *d, double *t,
-                   int sweeps, const int *fidx, int nf, cudaStream_t s);
-template <typename T> int dense_gemv(const T *A, int n, int nf, const int *fidx, const T *x, T *y, cudaStream_t s);
+                   int sweeps, const int *cmap, double *xfree, int nf, cudaStream_t s);
+template <typename T> int dense_gemv(const T *A, int n, int nf, const int *cmap, const T *xfree, T *y, cudaStream_t s);
 size_t dense_inverse_work64(int n);
 size_t dense_inverse_work32(int n);
 int dense_ld(int n);
@@ -449,12 +459,14 @@ extern "C" int m3sph_mesh_destroy(m3sph_mesh *M) {
   dfree(M->coarse.A64);
   dfree(M->coarse.A32);
   dfree(M->coarse.cmap);
-  dfree(M->coarse.fidx);
+  dfree(M->coarse.x64);
+  dfree(M->coarse.x32);
   dfree(M->coarse.B32tmp);
   dfree(M->coarse.t64);
   dfree(M->Ufix);
   dfree(M->bc_rhs);
   dfree(M->red);
+  dfree(M->red_cnt);
   dfree(M->scal);
   dfree(M->T);
   dfree(M->Usoa);
@@ -571,9 +583,11 @@ extern "C" int m3sph_mesh_create(int32_t nmg, const m3sph_level *levels, int32_t
       (st = dalloc(&F.Fb, L0.ndof)) || (st = dalloc(&F.LiMM, L0.nvnod)) || (st = dalloc(&F.err, 4)) ||
       (st = dalloc(&L0.K64, (size_t)kpad<double>() * nel)) || (st = dalloc(&L0.K32, (size_t)kpad<float>() * nel)) ||
       (st = dalloc(&L0.KL32, (size_t)kpad<float>() * nel)) ||
-      (st = dalloc(&M->Ufix, L0.ndof)) || (st = dalloc(&M->bc_rhs, L0.ndof)) || (st = dalloc(&M->red, 4096)) ||
+      (st = dalloc(&M->Ufix, L0.ndof)) || (st = dalloc(&M->bc_rhs, L0.ndof)) || (st = dalloc(&M->red, 4096)) || (st = dalloc(&M->red_cnt, 4)) ||
       (st = dalloc(&M->scal, 64)))
     return fail(st);
+  if (cudaMemsetAsync(M->red_cnt, 0, 4 * sizeof(unsigned), s) != cudaSuccess)
+    return fail(cuda_fail(cudaGetLastError(), "reduction counters"));
   if (cudaMallocHost((void **)&M->h_scal, 64 * sizeof(double)) != cudaSuccess) return fail(M3SPH_ERR_CUDA);
   if (cudaStreamSynchronize(s) != cudaSuccess) return fail(cuda_fail(cudaGetLastError(), "mesh upload"));
   st = slm_build(M, f0);
@@ -785,19 +799,18 @@ static int rebuild_operator(m3sph_mesh *M) {
     std::vector<uint8_t> fm(nc);
     M3_CUDA(cudaMemcpyAsync(fm.data(), Lc.freemask, nc, cudaMemcpyDeviceToHost, s));
     M3_CUDA(cudaStreamSynchronize(s));
-    std::vector<int> cmap(nc, -1), fidx;
-    fidx.reserve(nc);
+    std::vector<int> cmap(nc, -1);
+    int nf = 0;
     for (int i = 0; i < nc; ++i)
-      if (fm[i]) {
-        cmap[i] = (int)fidx.size();
-        fidx.push_back(i);
-      }
+      if (fm[i]) cmap[i] = nf++;
     if (!M->coarse.cmap) M3_TRY(dalloc(&M->coarse.cmap, (size_t)nc));
-    if (!M->coarse.fidx) M3_TRY(dalloc(&M->coarse.fidx, (size_t)nc));
-    M->coarse.nf = (int)fidx.size();
+    if (!M->coarse.x64) M3_TRY(dalloc(&M->coarse.x64, (size_t)dense_ld(nc)));
+    if (!M->coarse.x32) M3_TRY(dalloc(&M->coarse.x32, (size_t)dense_ld(nc)));
+    M->coarse.nf = nf;
     M3_CUDA(cudaMemcpyAsync(M->coarse.cmap, cmap.data(), sizeof(int) * nc, cudaMemcpyHostToDevice, s));
-    if (!fidx.empty())
-      M3_CUDA(cudaMemcpyAsync(M->coarse.fidx, fidx.data(), sizeof(int) * fidx.size(), cudaMemcpyHostToDevice, s));
+    // zero padding past the free dofs
+    M3_CUDA(cudaMemsetAsync(M->coarse.x64, 0, sizeof(double) * dense_ld(nc), s));
+    M3_CUDA(cudaMemsetAsync(M->coarse.x32, 0, sizeof(float) * dense_ld(nc), s));
     M3_CUDA(cudaStreamSynchronize(s));
   }
   const int nf = M->coarse.nf;
@@ -950,14 +963,23 @@ extern "C" int m3sph_stokes_set_vel_bc(m3sph_mesh *M, const int32_t *ifix, const
 static bool g_stream_apply = true;
 static bool g_stream_outer = true;
 
-static int outer_apply(m3sph_mesh *M, const double *x, double *y) {
+// y = K x; qKq: also scal[2] = x.y (in the node sums where the operator is the streamed one)
+static int outer_apply(m3sph_mesh *M, const double *x, double *y, bool qKq = false) {
   Level &L0 = M->lev[0];
+  const Reduction red{M->red, M->red_cnt}, *rp = qKq ? &red : nullptr;
+  double *out = M->scal + 2;
+  if (g_stream_outer && L0.nchunk) {
+    if (M->precision == 1 && M->df_outer) return stream_apply_df(L0, L0.K32, L0.KL32, x, y, rp, out, M->stream);
+    return stream_apply_f64(L0, L0.K64, x, y, rp, out, M->stream);
+  }
+  if (qKq) {
+    M3_TRY(outer_apply(M, x, y));
+    return dot(x, y, L0.ndof, M->red, M->red_cnt, out, M->stream);
+  }
   if (M->precision == 1 && M->df_outer) {
-    if (g_stream_outer && L0.nchunk) return stream_apply_df(L0, L0.K32, L0.KL32, x, y, M->stream);
     return M->split_apply ? ebe_apply_split_df(L0, L0.K32, L0.KL32, x, y, M->stream)
                           : ebe_apply_df(L0, L0.K32, L0.KL32, x, y, M->stream);
   }
-  if (g_stream_outer && L0.nchunk) return stream_apply_f64(L0, L0.K64, x, y, M->stream);
   return M->split_apply ? ebe_apply_split_f64(L0, L0.K64, x, y, M->stream)
                         : ebe_apply<double>(L0, L0.K64, x, y, M->stream);
 }
@@ -987,7 +1009,7 @@ static int stream_apply_T(const Level &L, const float *K, const float *x, float 
   return stream_apply_f32(L, K, x, y, s);
 }
 static int stream_apply_T(const Level &L, const double *K, const double *x, double *y, cudaStream_t s) {
-  return stream_apply_f64(L, K, x, y, s);
+  return stream_apply_f64(L, K, x, y, nullptr, nullptr, s);
 }
 // the level whose FP32 operator is the partially assembled one
 template <typename T>
@@ -1019,6 +1041,8 @@ static int level_op_jac(const Level &L, int img, T w, const T *r, T *d, T *kd, c
   if constexpr (std::is_same<T, float>::value) {
     if (pa_level<T>(L, img)) return pa_apply_jac_f32(L, w, r, L.Dinv32, d, have_cart, s);
     if (img == 0 && g_stream_apply && L.nchunk && L.K32) return stream_apply_jac_f32(L, L.K32, w, r, L.Dinv32, d, s);
+  } else {
+    if (img == 0 && g_stream_outer && L.nchunk && L.K64) return stream_apply_jac_f64(L, L.K64, w, r, L.Dinv64, d, s);
   }
   M3_TRY(level_op<T>(L, img, d, kd, s));
   return jac<T>(w, r, kd, levDi<T>(L), d, L.ndof, s);
@@ -1035,15 +1059,19 @@ static int level_jac_first(const Level &L, int img, T w, const T *r, T *d, cudaS
 
 // the coarsest-level solve of the V-cycle: one GEMV with the dense inverse, or on the plain FP64
 // path with a large coarsest level the FP32 inverse refined against the FP64 operator
+template <typename T> static T *coarse_x(m3sph_mesh *M);
+template <> double *coarse_x<double>(m3sph_mesh *M) { return M->coarse.x64; }
+template <> float *coarse_x<float>(m3sph_mesh *M) { return M->coarse.x32; }
+// r's free dofs are in coarse_x (written by the restriction)
 template <typename T>
 static int coarse_solve(m3sph_mesh *M, const T *Ainv, const T *r, T *d) {
   const Level &Lc = M->lev[M->nmg - 1];
   if constexpr (std::is_same<T, double>::value) {
     if (M->coarse.refine64)
-      return coarse_refined(Lc, M->coarse.A32, Lc.B64, r, d, M->coarse.t64, g_coarse_refine_sweeps, M->coarse.fidx,
-                            M->coarse.nf, M->stream);
+      return coarse_refined(Lc, M->coarse.A32, Lc.B64, r, d, M->coarse.t64, g_coarse_refine_sweeps, M->coarse.cmap,
+                            M->coarse.x64, M->coarse.nf, M->stream);
   }
-  return dense_gemv<T>(Ainv, M->coarse.n, M->coarse.nf, M->coarse.fidx, r, d, M->stream);
+  return dense_gemv<T>(Ainv, M->coarse.n, M->coarse.nf, M->coarse.cmap, coarse_x<T>(M), d, M->stream);
 }
 
 template <typename T>
@@ -1052,8 +1080,8 @@ static int vcycle_T(m3sph_mesh *M, std::vector<T *> &r, std::vector<T *> &d, std
   cudaStream_t s = M->stream;
   const int nm = M->nmg;
   if (nm == 1) {
-    M3_TRY(dense_gemv<T>(Ainv, M->coarse.n, M->coarse.nf, M->coarse.fidx, r[0], d[0], s));
-    return M3SPH_OK;
+    set_error("a single multigrid level has no V-cycle (the coarsest level needs a finer one)");
+    return M3SPH_ERR_BAD_INPUT;
   }
   const bool ml = M->smoother_active;
   // learned levels: the two finest (schedules 0, 1, 3) or the finest only (schedule 2)
@@ -1070,7 +1098,12 @@ static int vcycle_T(m3sph_mesh *M, std::vector<T *> &r, std::vector<T *> &d, std
     auto sweep = [&](const T *k) { return ml_sweep<T>(M, j, r[j], k, levDi<T>(L), tmp[j], d[j], pc); };
     auto op = [&]() { return level_op<T>(L, j, d[j], kd[j], s, true); };
     auto op_jac = [&](double wk) { return level_op_jac<T>(L, j, (T)wk, r[j], d[j], kd[j], s, true); };
-    if (ml && j < nml) {
+    auto sweep_to = [&](double wk, const T *x, T *y) { return bsr_apply_jac<T>(L, levB<T>(L), (T)wk, r[j], levDi<T>(L), x, y, s); };
+    if (!(ml && j < nml) && j > 0) {
+      // assembled level: the restriction left the first sweep in d, sweeps alternate between two vectors
+      M3_TRY(sweep_to(w[1], d[j], tmp[j]));
+      M3_TRY(sweep_to(w[2], tmp[j], d[j]));
+    } else if (ml && j < nml) {
       M3_CUDA(cudaMemsetAsync(d[j], 0, sizeof(T) * n, s));
       M3_TRY(sweep(nullptr));
       if (!one && M->ml_schedule == 3) {
@@ -1087,7 +1120,9 @@ static int vcycle_T(m3sph_mesh *M, std::vector<T *> &r, std::vector<T *> &d, std
       for (int k = 1; k < 3; ++k) M3_TRY(op_jac(w[k]));
     }
     M3_TRY(op());                        // the residual for the restriction
-    M3_TRY(restrict_<T>(L, M->lev[j + 1], r[j], kd[j], r[j + 1], s));
+    const bool last = j + 1 == nm - 1, sweep1 = !last && !(ml && j + 1 < nml);
+    M3_TRY(restrict_<T>(L, M->lev[j + 1], r[j], kd[j], r[j + 1], s, (T)WDc[0], levDi<T>(M->lev[j + 1]),
+                        sweep1 ? d[j + 1] : nullptr, last ? M->coarse.cmap : nullptr, coarse_x<T>(M)));
   }
   M3_TRY(coarse_solve<T>(M, Ainv, r[nm - 1], d[nm - 1]));
   for (int j = nm - 2; j >= 0; --j) {
@@ -1097,6 +1132,14 @@ static int vcycle_T(m3sph_mesh *M, std::vector<T *> &r, std::vector<T *> &d, std
     auto sweep = [&](const T *k) { return ml_sweep<T>(M, j, r[j], k, levDi<T>(L), tmp[j], d[j], pc); };
     auto op = [&]() { return level_op<T>(L, j, d[j], kd[j], s, true); };
     auto op_jac = [&](double wk) { return level_op_jac<T>(L, j, (T)wk, r[j], d[j], kd[j], s, true); };
+    if (!(ml && j < nml) && j > 0) {
+      auto sweep_to = [&](double wk, const T *x, T *y) { return bsr_apply_jac<T>(L, levB<T>(L), (T)wk, r[j], levDi<T>(L), x, y, s); };
+      M3_TRY(prolong<T>(L, M->lev[j + 1], d[j + 1], d[j], tmp[j], pc, s));
+      M3_TRY(sweep_to(w[0], tmp[j], d[j]));
+      M3_TRY(sweep_to(w[1], d[j], tmp[j]));
+      M3_TRY(sweep_to(w[2], tmp[j], d[j]));
+      continue;
+    }
     M3_TRY(prolong<T>(L, M->lev[j + 1], d[j + 1], d[j], d[j], pc, s));
     if (ml && j < nml && one) {
       M3_TRY(op());
@@ -1118,21 +1161,17 @@ static int vcycle_T(m3sph_mesh *M, std::vector<T *> &r, std::vector<T *> &d, std
   return M3SPH_OK;
 }
 
-// d (fp64) = B r (fp64) in the set-up precision
+// d = B r in the set-up precision: FP64 vectors on the plain path, W->r32[0] -> W->d32[0] (whose FP32
+// residual the caller has formed) on the mixed path
 static int vcycle(m3sph_mesh *M, const double *r, double *dout) {
   Work *W = get_work(M);
-  cudaStream_t s = M->stream;
-  const size_t n0 = M->lev[0].ndof;
   if (M->precision == 0) {
     std::vector<double *> rr = W->r64, dd = W->d64;
     rr[0] = const_cast<double *>(r);
     dd[0] = dout;
     return vcycle_T<double>(M, rr, dd, W->kd64, W->t64, M->coarse.A64);
   }
-  M3_TRY(d2f(r, W->r32[0], n0, s));
-  M3_TRY(vcycle_T<float>(M, W->r32, W->d32, W->kd32, W->t32, M->coarse.A32));
-  M3_TRY(f2d(W->d32[0], dout, n0, s));
-  return M3SPH_OK;
+  return vcycle_T<float>(M, W->r32, W->d32, W->kd32, W->t32, M->coarse.A32);
 }
 
 // ======================================================================================
@@ -1168,13 +1207,16 @@ static int cg_iteration(m3sph_mesh *M, double *x) {
   Level &L0 = M->lev[0];
   const size_t n = L0.ndof;
   M3_TRY(vcycle(M, W->r, W->d));
-  M3_TRY(dot2(W->r, W->Kq, W->d, n, M->red, M->scal + 0, s));   // scal[0]=r.d, scal[1]=Kq_prev.d
-  M3_TRY(cg_dir(W->d, W->q, n, M->scal, -1, s));                // first-iteration flag in scal[6]
-  M3_TRY(outer_apply(M, W->q, W->Kq));
-  M3_TRY(dot(W->q, W->Kq, n, M->red, M->scal + 2, s));
-  M3_TRY(cg_update(x, W->r, W->q, W->Kq, n, M->scal, M->red, s));
-  M3_TRY(set_first_flag(M, 0.0));
-  return M3SPH_OK;
+  // scal[0] = r.d, scal[1] = Kq_prev.d; q (first-iteration flag in scal[6])
+  if (M->precision == 0) {
+    M3_TRY(dot2<double>(W->r, W->Kq, W->d, n, M->red, M->red_cnt, M->scal, s));
+    M3_TRY(cg_dir<double>(W->d, W->q, n, M->scal, s));
+  } else {
+    M3_TRY(dot2<float>(W->r, W->Kq, W->d32[0], n, M->red, M->red_cnt, M->scal, s));
+    M3_TRY(cg_dir<float>(W->d32[0], W->q, n, M->scal, s));
+  }
+  M3_TRY(outer_apply(M, W->q, W->Kq, true));
+  return cg_update(x, W->r, W->q, W->Kq, M->precision ? W->r32[0] : nullptr, n, M->scal, M->red, M->red_cnt, s);
 }
 
 // the iteration captured once per solution-vector pointer as a CUDA graph and replayed
@@ -1219,8 +1261,7 @@ static int mgpcg(m3sph_mesh *M, const double *b, double *x, double tol, bool abs
   const size_t n = L0.ndof;
   const double sq = std::sqrt((double)std::max(1, L0.nfree));
   M3_TRY(outer_apply(M, x, W->r));
-  M3_TRY(sub_mask(b, W->r, L0.freemask, n, s));
-  M3_TRY(dot(W->r, W->r, n, M->red, M->scal + 3, s));
+  M3_TRY(residual(b, W->r, L0.freemask, M->precision ? W->r32[0] : nullptr, n, M->red, M->red_cnt, M->scal + 3, s));
   double rr;
   M3_TRY(read_scal(M, 3, rr));
   if (std::isnan(rr)) {
@@ -1275,7 +1316,7 @@ static int mgpcg(m3sph_mesh *M, const double *b, double *x, double tol, bool abs
 // Patera pressure CG (flow3d_patera_mg_sph_p.m:386-632)
 // ======================================================================================
 static int pdot(m3sph_mesh *M, const double *a, const double *b, double &v) {
-  M3_TRY(dot(a, b, M->lev[0].nvnod, M->red, M->scal + 8, M->stream));
+  M3_TRY(dot(a, b, M->lev[0].nvnod, M->red, M->red_cnt, M->scal + 8, M->stream));
   return read_scal(M, 8, v);
 }
 __global__ void k_shift(double *a, double c, int n) {
@@ -1313,7 +1354,7 @@ __global__ void k_absmax_xyz(const double *U, const double *RR, int nnod, unsign
 
 static int remove_mean(m3sph_mesh *M, double *a) {
   const int np = M->lev[0].nvnod;
-  M3_TRY(vsum(a, np, M->red, M->scal + 9, M->stream));
+  M3_TRY(vsum(a, np, M->red, M->red_cnt, M->scal + 9, M->stream));
   double sm;
   M3_TRY(read_scal(M, 9, sm));
   k_shift<<<(np + 255) / 256, 256, 0, M->stream>>>(a, -sm / np, np); count_launch();
@@ -1338,20 +1379,19 @@ static int coupled_residual(m3sph_mesh *M, const double *U, const double *P, dou
   M3_CUDA(cudaMemsetAsync(W->tmp, 0, sizeof(double) * n, s));
   k_rhs<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(M->fin.Fb, W->tmp, M->bc_rhs, L0.freemask, W->Rhs, n); count_launch();
   double ff;
-  M3_TRY(dot(W->Rhs, W->Rhs, n, M->red, M->scal + 10, s));
+  M3_TRY(dot(W->Rhs, W->Rhs, n, M->red, M->red_cnt, M->scal + 10, s));
   M3_TRY(read_scal(M, 10, ff));
   // ru = mask(Fb + G P - bc - K U)
   M3_TRY(build_rhs(M, P, W->Rhs));
   M3_TRY(outer_apply(M, U, W->tmp));
-  M3_TRY(sub_mask(W->Rhs, W->tmp, L0.freemask, n, s));
   double ru;
-  M3_TRY(dot(W->tmp, W->tmp, n, M->red, M->scal + 10, s));
+  M3_TRY(residual(W->Rhs, W->tmp, L0.freemask, nullptr, n, M->red, M->red_cnt, M->scal + 10, s));
   M3_TRY(read_scal(M, 10, ru));
   // rp = -G' U, mean removed
   M3_TRY(div_apply(L0, M->fin.G64, U, 1.0, W->pt, s));
   M3_TRY(remove_mean(M, W->pt));
   double rp;
-  M3_TRY(dot(W->pt, W->pt, np, M->red, M->scal + 10, s));
+  M3_TRY(dot(W->pt, W->pt, np, M->red, M->red_cnt, M->scal + 10, s));
   M3_TRY(read_scal(M, 10, rp));
   rel = std::sqrt(ru + rp) / std::sqrt(std::max(ff, 1e-300));
   return M3SPH_OK;
@@ -1966,7 +2006,7 @@ extern "C" int m3sph_restrict(m3sph_mesh *M, int32_t img, const double *rf, doub
   Level &F = M->lev[img], &C = M->lev[img + 1];
   cudaStream_t s = M->stream;
   M3_CUDA(cudaMemcpyAsync(W->r64[img], rf, sizeof(double) * F.ndof, cudaMemcpyHostToDevice, s));
-  M3_TRY(restrict_<double>(F, C, W->r64[img], nullptr, W->d64[img + 1], s));
+  M3_TRY(restrict_<double>(F, C, W->r64[img], nullptr, W->d64[img + 1], s, 0.0, nullptr, nullptr, nullptr, nullptr));
   M3_CUDA(cudaMemcpyAsync(rc, W->d64[img + 1], sizeof(double) * C.ndof, cudaMemcpyDeviceToHost, s));
   M3_CUDA(cudaStreamSynchronize(s));
   return M3SPH_OK;
@@ -1978,7 +2018,9 @@ extern "C" int m3sph_vcycle(m3sph_mesh *M, const double *r, double *d) {
   cudaStream_t s = M->stream;
   const size_t n = M->lev[0].ndof;
   M3_CUDA(cudaMemcpyAsync(W->tmp, r, sizeof(double) * n, cudaMemcpyHostToDevice, s));
+  if (M->precision) M3_TRY(d2f(W->tmp, W->r32[0], n, s));
   M3_TRY(vcycle(M, W->tmp, W->d));
+  if (M->precision) M3_TRY(f2d(W->d32[0], W->d, n, s));
   M3_CUDA(cudaMemcpyAsync(d, W->d, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
   M3_CUDA(cudaStreamSynchronize(s));
   return M3SPH_OK;

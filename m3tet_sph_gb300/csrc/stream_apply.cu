@@ -565,23 +565,59 @@ __global__ void k_node_gather_jac_f32(const int *__restrict__ ptr, const int *__
   d[i + 2] += w * (r[i + 2] - s2) * Di[i + 2];
 }
 
-__global__ void k_node_gather_f64(const int *__restrict__ ptr, const int *__restrict__ idx, int nnod,
-                                  const double *__restrict__ ye, double *__restrict__ y) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= nnod) return;
-  double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-  const int b = ptr[n], e = ptr[n + 1];
-  for (int j = b; j < e; ++j) {
-    const int o = idx[j], odd = o & 1;   // 16-byte aligned pair for even n, as in the FP32 gather
-    const double2 v2 = *reinterpret_cast<const double2 *>(ye + o + odd);
-    const double v1 = ye[o + 2 * (1 - odd)];
-    s0 += odd ? v1 : v2.x;
-    s1 += odd ? v2.x : v2.y;
-    s2 += odd ? v2.y : v1;
+// phase 2 of the FP64-accurate operators. Four lanes share a vertex (entries in turn, partial sums combined in a
+// fixed order), one lane takes an edge node: with one lane each, the 24 entries of a vertex were 24 dependent
+// index-and-value loads, which set the time on small meshes (15.9 us at 30,720 elements; now 9.0; four
+// lanes for every node took 97.9 us at 491,520 elements against 51.4).
+// What follows the product goes into the same pass: out = x.y of the CG step (DOT), or one weighted Jacobi
+// sweep d += w (r - y) / diag (JAC; d is read only by its own node here).
+enum { GATHER_Y = 0, GATHER_DOT = 1, GATHER_JAC = 2 };
+constexpr int GT = 256;
+template <int MODE>
+__global__ void __launch_bounds__(GT) k_node_gather_f64(const int *__restrict__ ptr, const int *__restrict__ idx, int nnod,
+                                                        int nv, const double *__restrict__ ye, double *__restrict__ y,
+                                                        const double *__restrict__ x, double w,
+                                                        const double *__restrict__ r, const double *__restrict__ Di,
+                                                        double *partials, unsigned *cnt, double *out) {
+  double v[1] = {0.0};
+  const int nt4 = gather_threads4(nv), nt = nt4 + nnod - nv;
+  // whole warps stay in the loop: the shuffles need all lanes of a vertex
+  for (int t0 = blockIdx.x * GT; t0 < nt; t0 += gridDim.x * GT) {
+    const int t = t0 + threadIdx.x;
+    const bool quad = t < nt4;
+    const int n = quad ? t >> 2 : nv + t - nt4, sub = quad ? t & 3 : 0, step = quad ? 4 : 1;
+    const bool live = quad ? n < nv : n < nnod;
+    double s[3] = {0.0, 0.0, 0.0};
+    const int e = live ? ptr[n + 1] : 0;
+#pragma unroll 2
+    for (int j = live ? ptr[n] + sub : 0; j < e; j += step) {
+      const int o = idx[j], odd = o & 1;   // 16-byte aligned pair for even local nodes
+      const double2 v2 = *reinterpret_cast<const double2 *>(ye + o + odd);
+      const double v1 = ye[o + 2 * (1 - odd)];
+      s[0] += odd ? v1 : v2.x;
+      s[1] += odd ? v2.x : v2.y;
+      s[2] += odd ? v2.y : v1;
+    }
+    if (quad) {                            // warps are of one kind
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
+    }
+    if (!live || sub) continue;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const size_t i = 3 * (size_t)n + c;
+      if (MODE == GATHER_JAC) {
+        y[i] += w * (r[i] - s[c]) * Di[i];
+      } else {
+        y[i] = s[c];
+        if (MODE == GATHER_DOT) v[0] += x[i] * s[c];
+      }
+    }
   }
-  y[3 * (size_t)n] = s0;
-  y[3 * (size_t)n + 1] = s1;
-  y[3 * (size_t)n + 2] = s2;
+  if (MODE == GATHER_DOT)
+    if (block_reduce_last<1>(v, partials, cnt) && threadIdx.x == 0) out[0] = v[0];
 }
 
 // ---------------------------------------------------------------------------------------
@@ -778,9 +814,13 @@ static void rowlane_launch(const Level &L, const CUtensorMap &ma, const CUtensor
       ma, mb, L.chunk_conn8, L.nchunk8, L.nel, L.sa_err + 1, L.sa_err, x, L.ye64);
 }
 
+static unsigned gather_grid(const Level &L) {
+  return (unsigned)((gather_threads4(L.nvnod) + L.nnod - L.nvnod + GT - 1) / GT);
+}
+
+// element outputs (phase 1)
 template <class Op>
-static int rowlane_apply(const Level &L, const CUtensorMap &ma, const CUtensorMap &mb, const double *x, double *y,
-                         cudaStream_t s) {
+static int rowlane_elements(const Level &L, const CUtensorMap &ma, const CUtensorMap &mb, const double *x, cudaStream_t s) {
   M3_CUDA(cudaMemsetAsync(L.sa_err + 1, 0, sizeof(int), s));
   if constexpr (std::is_same<Op, RlF64>::value) {
     rowlane_launch<RlF64, 6, 1>(L, ma, mb, x, s);
@@ -798,7 +838,17 @@ static int rowlane_apply(const Level &L, const CUtensorMap &ma, const CUtensorMa
     }
   }
   count_launch();
-  k_node_gather_f64<<<(L.nnod + 255) / 256, 256, 0, s>>>(L.g_ptr, L.g_idx, L.nnod, L.ye64, y);
+  return M3SPH_OK;
+}
+// node sums (phase 2): y = K x, with red also out[0] = x.y
+static int rowlane_sums(const Level &L, double *y, const double *x, const Reduction *red, double *out, cudaStream_t s) {
+  const unsigned g = gather_grid(L);
+  if (red)
+    k_node_gather_f64<GATHER_DOT><<<std::min(g, 2048u), GT, 0, s>>>(   // one partial sum per block
+        L.g_ptr, L.g_idx, L.nnod, L.nvnod, L.ye64, y, x, 0.0, nullptr, nullptr, red->partials, red->cnt, out);
+  else
+    k_node_gather_f64<GATHER_Y><<<g, GT, 0, s>>>(L.g_ptr, L.g_idx, L.nnod, L.nvnod, L.ye64, y, nullptr, 0.0, nullptr,
+                                                 nullptr, nullptr, nullptr, nullptr);
   count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
@@ -819,22 +869,40 @@ int stream_apply_jac_f32(const Level &L, const float *K, float w, const float *r
   return M3SPH_OK;
 }
 
-// y = (K_hi + K_lo) x with FP64 accuracy (double-float arithmetic)
-int stream_apply_df(const Level &L, const float *Kh, const float *Kl, const double *x, double *y, cudaStream_t s) {
+// y = (K_hi + K_lo) x with FP64 accuracy (double-float arithmetic); red: also out[0] = x.y
+int stream_apply_df(const Level &L, const float *Kh, const float *Kl, const double *x, double *y, const Reduction *red,
+                    double *out, cudaStream_t s) {
   M3_TRY(stream_ready(L, Kh));
   M3_TRY(stream_ready(L, Kl));
   CUtensorMap ma, mb;
   M3_TRY(encode_k(L, Kh, false, RlDF::ROWS, sr::E, &ma, true));
   M3_TRY(encode_k(L, Kl, false, RlDF::ROWS, sr::E, &mb, true));
-  return rowlane_apply<RlDF>(L, ma, mb, x, y, s);
+  M3_TRY(rowlane_elements<RlDF>(L, ma, mb, x, s));
+  return rowlane_sums(L, y, x, red, out, s);
 }
 
-// y = K x in FP64 from the FP64 element matrices
-int stream_apply_f64(const Level &L, const double *K, const double *x, double *y, cudaStream_t s) {
+// y = K x in FP64 from the FP64 element matrices; red: also out[0] = x.y
+int stream_apply_f64(const Level &L, const double *K, const double *x, double *y, const Reduction *red, double *out,
+                     cudaStream_t s) {
   M3_TRY(stream_ready(L, K));
   CUtensorMap ma;
   M3_TRY(encode_k(L, K, true, RlF64::ROWS, sr::E, &ma, true));
-  return rowlane_apply<RlF64>(L, ma, ma, x, y, s);
+  M3_TRY(rowlane_elements<RlF64>(L, ma, ma, x, s));
+  return rowlane_sums(L, y, x, red, out, s);
+}
+
+// d += w (r - K d) / diag in FP64 (one weighted Jacobi sweep)
+int stream_apply_jac_f64(const Level &L, const double *K, double w, const double *r, const double *Di, double *d,
+                         cudaStream_t s) {
+  M3_TRY(stream_ready(L, K));
+  CUtensorMap ma;
+  M3_TRY(encode_k(L, K, true, RlF64::ROWS, sr::E, &ma, true));
+  M3_TRY(rowlane_elements<RlF64>(L, ma, ma, d, s));
+  k_node_gather_f64<GATHER_JAC><<<gather_grid(L), GT, 0, s>>>(L.g_ptr, L.g_idx, L.nnod, L.nvnod, L.ye64, d, nullptr, w, r, Di,
+                                                              nullptr, nullptr, nullptr);
+  count_launch();
+  M3_CUDA(cudaGetLastError());
+  return M3SPH_OK;
 }
 
 // reads (and clears) the error word of the streamed apply
