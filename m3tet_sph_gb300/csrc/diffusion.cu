@@ -2,11 +2,17 @@
 // elements on the 8-child split of every P2 tetrahedron, double-Jacobian element integrals,
 // lumped capacity, theta scheme, Dirichlet temperatures, Jacobi-preconditioned Polak-Ribiere CG.
 //
-// Layout: split elements `sub` [4][nsub] (node ids), packed conductivity C [10][nsub] (entries
-// (i,j), i >= j, in the order 00 10 11 20 21 22 30 31 32 33), element products ye [4][nsub], and a
-// node -> (local, element) list in element order for the fixed-order node sums (no atomics). One
-// operator application reads 80 B of C, 16 B of ids and 32 B of gathered T per element and writes /
-// re-reads 32 B of ye: HBM-bound.
+// Layout: split elements `sub` [4][nsub] (node ids), packed conductivity C [10][nsub] (entries (i,j), i >= j,
+// in the order 00 10 11 20 21 22 30 31 32 33) and a node -> (local, element) list in element order. The
+// conductivity is assembled into rows (node -> neighbour columns, values) once per set-up: a product then
+// reads 12 B per nonzero, about 15 a node, where the element form read and wrote 160 B per split element,
+// about 6 a node (98 us per product at 338k nodes; now 29 us). Sums run in a fixed order, no atomics.
+//
+// The CG keeps its scalars on the device: three launches per iteration (direction; product and q.Aq; step
+// with r.r and the dots of the next direction), whose kernels do nothing once a flag says that the
+// iteration has ended, so the host looks at it every DIFF_CHECK iterations only (it read four scalars per
+// iteration, each a wait).
+#include <algorithm>
 #include <cmath>
 #include <string>
 #include <vector>
@@ -15,7 +21,8 @@
 
 namespace m3sph {
 
-int dot(const double *a, const double *b, size_t n, double *partials, unsigned *cnt, double *out, cudaStream_t s);
+unsigned red_blocks(size_t n);
+const double *slm_x90(m3sph_mesh *M);
 
 // children of a P2 tetrahedron (local node numbers 0..9) for the three interior diagonals, and the
 // diagonals' end nodes (tetmesh_p2_to_p1.m): the table that the reference's split follows
@@ -32,13 +39,18 @@ struct DiffState {
   int *sub = nullptr;                  // [4][nsub]
   uint8_t *cls = nullptr;              // [nsub]
   double *C = nullptr;                 // [10][nsub]
-  double *ye = nullptr;                // [4][nsub]
+  double *Me = nullptr;                // [4][nsub] lumped element capacities
   int *gptr = nullptr, *gidx = nullptr;  // [nnod+1], [4 nsub]: local * nsub + element
-  double *ML = nullptr, *Cdiag = nullptr;  // [nnod]
+  // rows of the assembled conductivity, columns sorted: entry k of row n is at sptr[n / 32] + 32 k + n % 32
+  int *sptr = nullptr, *rlen = nullptr, *rcol = nullptr;  // [slices of 32 rows], [nnod], [padded nonzeros]
+  double *rval = nullptr;              // [padded nonzeros]
+  double *ML = nullptr, *Cdiag = nullptr, *Mi = nullptr;  // [nnod]; Mi: inverse diagonal, 0 on fixed nodes
   uint8_t *fixmask = nullptr;          // [nnod]
   int *ifix = nullptr;                 // [nfix]
   double *vfix = nullptr;              // [nfix]
-  double *rhs = nullptr, *x = nullptr, *r = nullptr, *d = nullptr, *q = nullptr, *Aq = nullptr, *rl = nullptr;
+  double *rhs = nullptr, *r = nullptr, *q = nullptr, *Aq = nullptr, *T = nullptr;
+  int fixcap = 0;
+  double *scal = nullptr;              // CG scalars (DS_*)
   int *err = nullptr;
 };
 
@@ -46,24 +58,21 @@ static DiffState *diff_state(m3sph_mesh *M) { return reinterpret_cast<DiffState 
 
 static void diff_free(void *p) {
   DiffState *D = reinterpret_cast<DiffState *>(p);
-  for (void *q : {(void *)D->sub, (void *)D->cls, (void *)D->C, (void *)D->ye, (void *)D->gptr, (void *)D->gidx,
-                  (void *)D->ML, (void *)D->Cdiag, (void *)D->fixmask, (void *)D->ifix, (void *)D->vfix, (void *)D->rhs,
-                  (void *)D->x, (void *)D->r, (void *)D->d, (void *)D->q, (void *)D->Aq, (void *)D->rl, (void *)D->err})
+  for (void *q : {(void *)D->sub, (void *)D->cls, (void *)D->C, (void *)D->Me, (void *)D->gptr, (void *)D->gidx,
+                  (void *)D->sptr, (void *)D->rlen, (void *)D->rcol, (void *)D->rval, (void *)D->ML, (void *)D->Mi, (void *)D->Cdiag, (void *)D->fixmask,
+                  (void *)D->ifix, (void *)D->vfix, (void *)D->rhs, (void *)D->r, (void *)D->q, (void *)D->Aq,
+                  (void *)D->T, (void *)D->scal, (void *)D->err})
     if (q) cudaFree(q);
   delete D;
 }
 
-__device__ __forceinline__ void c2s_d(double x, double y, double z, double &th, double &ph, double &r) {
-  r = sqrt(x * x + y * y + z * z);
-  th = atan2(sqrt(x * x + y * y), z);
-  ph = atan2(y, x);
-  if (ph < 0.0) ph += 2.0 * M_PI;
-}
-
 // element integrals of one split element (assembly_diffusion_els_*_opt.m): vertex (theta, phi, r)
-// in the element's frame, J_SL from them, J_CS at each of the 4 points of ip_tetrahedron(4)
+// in the element's frame (X-90 coordinates from the location tables), J_SL from them, J_CS at each of the 4
+// points of ip_tetrahedron(4). FP64 issue bounds it, so the gradients are multiplied in the spherical basis,
+// where the metric is diagonal and the linear element's derivatives are constant: 3.7 ms at 2.0M split elements
+// with Cartesian gradients at every point and the X-90 frame formed per element; now 0.82 ms.
 __global__ void k_diff_setup(int nsub, const int *__restrict__ sub, const uint8_t *__restrict__ cls,
-                             const double *__restrict__ X, const double *__restrict__ S, int nnod, double kappa,
+                             const double *__restrict__ SX, const double *__restrict__ S, int nnod, double kappa,
                              double *__restrict__ C, double *__restrict__ Me, int *err) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= nsub) return;
@@ -80,7 +89,9 @@ __global__ void k_diff_setup(int nsub, const int *__restrict__ sub, const uint8_
         if (V[1][i] > 2.0 * M_PI) V[1][i] -= 2.0 * M_PI;
       }
     } else {   // X-90-rotated frame: (x, -z, y)
-      c2s_d(X[n], -X[2 * (size_t)nnod + n], X[nnod + n], V[0][i], V[1][i], V[2][i]);
+      V[0][i] = SX[n];
+      V[1][i] = SX[nnod + n];
+      V[2][i] = SX[2 * (size_t)nnod + n];
     }
   }
   // J_SL[j][k] = d sph_k / d loc_j with dN4 = [I; -1 -1 -1]
@@ -90,48 +101,44 @@ __global__ void k_diff_setup(int nsub, const int *__restrict__ sub, const uint8_
   const double det = J[0][0] * (J[1][1] * J[2][2] - J[1][2] * J[2][1]) - J[0][1] * (J[1][0] * J[2][2] - J[1][2] * J[2][0]) +
                      J[0][2] * (J[1][0] * J[2][1] - J[1][1] * J[2][0]);
   if (det < 0.0) atomicOr(err, 1);
-  const double id = 1.0 / det;
-  double Li[3][3];   // inverse of J_SL: Li[k][j] = d loc_j / d sph_k
-  Li[0][0] = (J[1][1] * J[2][2] - J[1][2] * J[2][1]) * id;
-  Li[0][1] = (J[0][2] * J[2][1] - J[0][1] * J[2][2]) * id;
-  Li[0][2] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) * id;
-  Li[1][0] = (J[1][2] * J[2][0] - J[1][0] * J[2][2]) * id;
-  Li[1][1] = (J[0][0] * J[2][2] - J[0][2] * J[2][0]) * id;
-  Li[1][2] = (J[0][2] * J[1][0] - J[0][0] * J[1][2]) * id;
-  Li[2][0] = (J[1][0] * J[2][1] - J[1][1] * J[2][0]) * id;
-  Li[2][1] = (J[0][1] * J[2][0] - J[0][0] * J[2][1]) * id;
-  Li[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * id;
+  // cofactors: d N_i / d sph_k = cf[k][i] / det, constant over the element (sum_i = 0)
+  double cf[3][4];
+  cf[0][0] = J[1][1] * J[2][2] - J[1][2] * J[2][1];
+  cf[0][1] = J[0][2] * J[2][1] - J[0][1] * J[2][2];
+  cf[0][2] = J[0][1] * J[1][2] - J[0][2] * J[1][1];
+  cf[1][0] = J[1][2] * J[2][0] - J[1][0] * J[2][2];
+  cf[1][1] = J[0][0] * J[2][2] - J[0][2] * J[2][0];
+  cf[1][2] = J[0][2] * J[1][0] - J[0][0] * J[1][2];
+  cf[2][0] = J[1][0] * J[2][1] - J[1][1] * J[2][0];
+  cf[2][1] = J[0][1] * J[2][0] - J[0][0] * J[2][1];
+  cf[2][2] = J[0][0] * J[1][1] - J[0][1] * J[1][0];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) cf[k][3] = -(cf[k][0] + cf[k][1] + cf[k][2]);
+  // det J_CS = r^2 sin(theta) and grad N_i . grad N_j = d_r d_r + d_th d_th / r^2 + d_ph d_ph / (r sin(theta))^2:
+  // the points enter through three sums only
   const double a = (5.0 + 3.0 * sqrt(5.0)) / 20.0, b = (5.0 - sqrt(5.0)) / 20.0;
-  double Cp[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0}, Ml[4] = {0, 0, 0, 0};
+  const double bt = b * (V[0][0] + V[0][1] + V[0][2] + V[0][3]), br = b * (V[2][0] + V[2][1] + V[2][2] + V[2][3]);
+  double st[4], wp[4];
+#pragma unroll
   for (int ip = 0; ip < 4; ++ip) {
-    const double N[4] = {ip == 0 ? a : b, ip == 1 ? a : b, ip == 2 ? a : b, ip == 3 ? a : b};
-    double sp[3];
-    for (int k = 0; k < 3; ++k) sp[k] = V[k][0] * N[0] + V[k][1] * N[1] + V[k][2] * N[2] + V[k][3] * N[3];
-    const double th = sp[0], ph = sp[1], rr = sp[2];
+    const double th = bt + (a - b) * V[0][ip], rr = br + (a - b) * V[2][ip];
     if (th == 0.0) atomicOr(err, 2);
-    double st, ct, sph, cph;
-    sincos(th, &st, &ct);
-    sincos(ph, &sph, &cph);
-    const double dCS = rr * rr * st;
-    const double SC[3][3] = {{rr * st * ct * cph / dCS, -rr * sph / dCS, rr * rr * st * st * cph / dCS},
-                             {rr * st * ct * sph / dCS, rr * cph / dCS, rr * rr * st * st * sph / dCS},
-                             {-rr * st * st / dCS, 0.0, rr * rr * st * ct / dCS}};
-    double Jd[3][3];   // Jd[x][j] = d loc_j / d cart_x
-    for (int x = 0; x < 3; ++x)
-      for (int j = 0; j < 3; ++j) Jd[x][j] = SC[x][0] * Li[0][j] + SC[x][1] * Li[1][j] + SC[x][2] * Li[2][j];
-    double g[4][3];
-    for (int x = 0; x < 3; ++x) {
-      g[0][x] = Jd[x][0];
-      g[1][x] = Jd[x][1];
-      g[2][x] = Jd[x][2];
-      g[3][x] = -Jd[x][0] - Jd[x][1] - Jd[x][2];
-    }
-    const double w = dCS * det * 0.25;
-    int k = 0;
-    for (int i = 0; i < 4; ++i) {
-      for (int j = 0; j <= i; ++j, ++k) Cp[k] += kappa * w * (g[i][0] * g[j][0] + g[i][1] * g[j][1] + g[i][2] * g[j][2]);
-      Ml[i] += w * N[i];   // row sum of w N_i N_j (sum_j N_j = 1)
-    }
+    st[ip] = sin(th);
+    wp[ip] = rr * rr * st[ip];
+  }
+  const double hr = wp[0] + wp[1] + wp[2] + wp[3], ht = st[0] + st[1] + st[2] + st[3];
+  const double s01 = st[0] * st[1], s23 = st[2] * st[3];
+  const double hp = ((st[0] + st[1]) * s23 + (st[2] + st[3]) * s01) / (s01 * s23);   // sum of 1 / sin(theta)
+  const double f = 0.25 * kappa / det;
+  const double h[3] = {f * ht, f * hp, f * hr};
+  double Cp[10], Ml[4];
+  int k = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const double a0 = h[0] * cf[0][i], a1 = h[1] * cf[1][i], a2 = h[2] * cf[2][i];
+#pragma unroll
+    for (int j = 0; j <= i; ++j, ++k) Cp[k] = a0 * cf[0][j] + a1 * cf[1][j] + a2 * cf[2][j];
+    Ml[i] = 0.25 * det * (b * hr + (a - b) * wp[i]);   // row sum of w N_i N_j (sum_j N_j = 1)
   }
   for (int k = 0; k < 10; ++k) C[(size_t)k * nsub + e] = Cp[k];
   for (int i = 0; i < 4; ++i) Me[(size_t)i * nsub + e] = Ml[i];
@@ -139,63 +146,188 @@ __global__ void k_diff_setup(int nsub, const int *__restrict__ sub, const uint8_
 
 __device__ __forceinline__ int pk(int i, int j) { return i >= j ? i * (i + 1) / 2 + j : j * (j + 1) / 2 + i; }
 
-// ye_e = C_e x_e
-__global__ void k_diff_elem(int nsub, const int *__restrict__ sub, const double *__restrict__ C,
-                            const double *__restrict__ x, double *__restrict__ ye) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nsub) return;
-  double xe[4], c[10];
-  for (int i = 0; i < 4; ++i) xe[i] = x[sub[(size_t)i * nsub + e]];
-  for (int k = 0; k < 10; ++k) c[k] = C[(size_t)k * nsub + e];
-  for (int i = 0; i < 4; ++i) {
-    double s = 0.0;
-    for (int j = 0; j < 4; ++j) s += c[pk(i, j)] * xe[j];
-    ye[(size_t)i * nsub + e] = s;
-  }
-}
-
-// y_n = a ML_n x_n + c sum(ye) over the node's entries in element order; fixed rows 0 if masked
-__global__ void k_diff_gather(int nnod, const int *__restrict__ gptr, const int *__restrict__ gidx,
-                              const double *__restrict__ ye, const double *__restrict__ ML, const double *__restrict__ x,
-                              double a, double c, const uint8_t *__restrict__ fixmask, double *__restrict__ y) {
+// lumped capacity: per node the sum of its elements' values in element order
+__global__ void k_diff_lump(int nnod, const int *__restrict__ gptr, const int *__restrict__ gidx,
+                            const double *__restrict__ Me, double *__restrict__ ML) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= nnod) return;
   double s = 0.0;
-  for (int k = gptr[n]; k < gptr[n + 1]; ++k) s += ye[gidx[k]];
-  const double v = (a != 0.0 ? a * ML[n] * x[n] : 0.0) + c * s;
-  y[n] = (fixmask && fixmask[n]) ? 0.0 : v;
+  for (int k = gptr[n]; k < gptr[n + 1]; ++k) s += Me[gidx[k]];
+  ML[n] = s;
 }
 
-__global__ void k_diff_jacobi(int n, const double *ML, const double *Cdiag, double c, const uint8_t *fixmask,
-                              const double *r, double *d) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) d[i] = fixmask[i] ? 0.0 : r[i] / (ML[i] + c * Cdiag[i]);
+// Row pattern, one warp per node: its neighbours (itself included) through a hash table in shared memory.
+// With rcol null the row lengths; then the columns, sorted. At most 128 elements share a vertex (the mesh
+// set-up's colour limit), so a node of the split has fewer than 400 neighbours.
+constexpr int DP_WARPS = 4, DP_TAB = 1024;
+__global__ void __launch_bounds__(DP_WARPS * 32) k_diff_pattern(int nnod, int nsub, const int *__restrict__ sub,
+                                                                const int *__restrict__ gptr, const int *__restrict__ gidx,
+                                                                int *__restrict__ rlen, const int *__restrict__ sptr,
+                                                                int *__restrict__ rcol) {
+  __shared__ int tab[DP_WARPS][DP_TAB];
+  __shared__ int list[DP_WARPS][DP_TAB];
+  const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n = blockIdx.x * DP_WARPS + wl;
+  if (n >= nnod) return;
+  int *h = tab[wl], *out = list[wl];
+  for (int i = lane; i < DP_TAB; i += 32) h[i] = -1;
+  __syncwarp();
+  const int b = gptr[n], m = 4 * (gptr[n + 1] - b);
+  for (int t = lane; t < m; t += 32) {
+    const int e = gidx[b + (t >> 2)] % nsub, v = sub[(size_t)(t & 3) * nsub + e];
+    int s = (int)(((unsigned)v * 2654435761u) >> 22);
+    for (int probe = 0; probe < DP_TAB; ++probe) {
+      const int old = atomicCAS(&h[s], -1, v);
+      if (old == -1 || old == v) break;
+      s = (s + 1) & (DP_TAB - 1);
+    }
+  }
+  __syncwarp();
+  int cnt = 0;
+  for (int i = lane; i < DP_TAB; i += 32) {
+    const int v = h[i];
+    const unsigned mask = __ballot_sync(0xffffffffu, v >= 0);
+    if (v >= 0) out[cnt + __popc(mask & ((1u << lane) - 1u))] = v;
+    cnt += __popc(mask);
+  }
+  __syncwarp();
+  if (!rcol) {
+    if (lane == 0) rlen[n] = cnt;
+    return;
+  }
+  for (int i = lane; i < cnt; i += 32) {
+    const int v = out[i];
+    int rank = 0;
+    for (int k = 0; k < cnt; ++k) rank += out[k] < v;
+    rcol[(size_t)sptr[n >> 5] + 32 * rank + (n & 31)] = v;
+  }
 }
-__global__ void k_diff_sub(int n, const double *a, const double *b, double *out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = a[i] - b[i];
+// Row values, 16 lanes per node: a lane sums its column's entries over the node's elements in element order
+__global__ void __launch_bounds__(256) k_diff_rows(int nnod, int nsub, const int *__restrict__ sub,
+                                                   const double *__restrict__ C, const int *__restrict__ gptr,
+                                                   const int *__restrict__ gidx, const int *__restrict__ sptr,
+                                                   const int *__restrict__ rlen, const int *__restrict__ rcol,
+                                                   double *__restrict__ rval,
+                                                   double *__restrict__ Cdiag) {
+  const int n = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 4), lane = threadIdx.x & 15;
+  if (n >= nnod) return;
+  const int b = gptr[n], f = gptr[n + 1];
+  const size_t r0 = (size_t)sptr[n >> 5] + (n & 31);
+  const int len = rlen[n];
+  for (int k = lane; k < len; k += 16) {
+    const int col = rcol[r0 + 32 * k];
+    double v = 0.0;
+    for (int g = b; g < f; ++g) {
+      const int o = gidx[g], i = o / nsub, e = o - i * nsub;
+      int j = -1;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (sub[(size_t)q * nsub + e] == col) j = q;
+      if (j >= 0) v += C[(size_t)pk(i, j) * nsub + e];
+    }
+    rval[r0 + 32 * k] = v;
+    if (col == n) Cdiag[n] = v;
+  }
 }
-// r = rhs - Ax on the free rows, 0 on the fixed ones
-__global__ void k_diff_resid(int n, const double *rhs, const double *Ax, const uint8_t *fixmask, double *r) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) r[i] = fixmask[i] ? 0.0 : rhs[i] - Ax[i];
+
+// CG scalars on the device
+enum { DS_RD = 0, DS_BETA, DS_ALPHA, DS_TOL2, DS_RR, DS_DONE, DS_IT, DS_BAD, DS_N };
+
+// Row products, a thread per row on slices of 32 rows: s_n = sum C_nm x_m, and with it
+//   DP_RHS    y = ML x + c s                                (right-hand side)
+//   DP_RESID  y = rhs - (ML x + c s) on free nodes, 0 on fixed ones, q = 0, Mi = 1 / diag; r.r and the dots
+//             of the first direction: the scalars of a CG from this residual
+//   DP_CG     y = ML x + c s on free nodes, 0 on fixed ones; alpha = rd / x.y
+// With 8 lanes per row the shuffles' additions and the one lane that finishes a row were most of the FP64
+// issue: 61 us at 338k rows, 5.2M nonzeros; now 29 us.
+enum { DP_RHS = 0, DP_RESID = 1, DP_CG = 2 };
+template <int MODE>
+__global__ void __launch_bounds__(256) k_diff_rowprod(int nnod, const int *__restrict__ sptr, const int *__restrict__ rlen,
+                                                      const int *__restrict__ rcol, const double *__restrict__ rval,
+                                                      const double *__restrict__ ML, const double *__restrict__ x, double c,
+                                                      const uint8_t *__restrict__ fixmask, double *__restrict__ y,
+                                                      const double *__restrict__ rhs, const double *__restrict__ Cdiag,
+                                                      double *__restrict__ Mi, double *__restrict__ q, double tol,
+                                                      double *scal, double *partials, unsigned *cnt) {
+  if (MODE == DP_CG && scal[DS_DONE] != 0.0) return;
+  double v[2] = {0.0, 0.0};
+  for (int n = blockIdx.x * 256 + threadIdx.x; n < nnod; n += gridDim.x * 256) {
+    const int len = rlen[n];
+    const size_t r0 = (size_t)sptr[n >> 5] + (n & 31);
+    double s = 0.0;
+#pragma unroll 4
+    for (int k = 0; k < len; ++k) s += rval[r0 + 32 * k] * x[rcol[r0 + 32 * k]];
+    const double m = ML[n], a = m * x[n] + c * s;
+    const bool fixed = MODE != DP_RHS && fixmask[n];
+    if (MODE == DP_RHS) {
+      y[n] = a;
+    } else if (MODE == DP_RESID) {
+      const double r = fixed ? 0.0 : rhs[n] - a, mi = fixed ? 0.0 : 1.0 / (m + c * Cdiag[n]);
+      y[n] = r;
+      Mi[n] = mi;
+      q[n] = 0.0;
+      v[0] += r * r;
+      v[1] += r * (r * mi);
+    } else {
+      const double t = fixed ? 0.0 : a;
+      y[n] = t;
+      v[0] += x[n] * t;
+    }
+  }
+  if (MODE == DP_RHS) return;
+  if (!block_reduce_last<2>(v, partials, cnt) || threadIdx.x) return;
+  if (MODE == DP_RESID) {
+    // pcg_solver_p.m: the tolerance is relative to the initial residual. A residual that is exactly zero
+    // (a field the step leaves unchanged) or below it is converged
+    scal[DS_RR] = v[0];
+    scal[DS_TOL2] = tol * tol * v[0];
+    scal[DS_RD] = v[1];
+    scal[DS_BETA] = 0.0;
+    scal[DS_DONE] = (v[0] < tol * tol * v[0] || v[0] == 0.0) ? 1.0 : 0.0;
+    scal[DS_IT] = 0.0;
+    scal[DS_BAD] = 0.0;
+  } else {
+    scal[DS_ALPHA] = scal[DS_RD] / v[0];
+  }
+}
+// q = d + beta q, d = r / diag on free nodes
+__global__ void k_diff_dir(int n, const double *__restrict__ r, const double *__restrict__ Mi, double *__restrict__ q,
+                           const double *__restrict__ scal) {
+  if (scal[DS_DONE] != 0.0) return;
+  const double beta = scal[DS_BETA];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    q[i] = r[i] * Mi[i] + beta * q[i];
+}
+// x += alpha q ; r -= alpha Aq ; then r.r and for the next direction d = r / diag: r.d and Aq.d, which give
+// beta = (r - rlast).d / rdlast = -alpha Aq.d / rdlast (Polak-Ribiere)
+__global__ void __launch_bounds__(256) k_diff_step(int n, const double *__restrict__ q, const double *__restrict__ Aq,
+                                                   double *__restrict__ x, double *__restrict__ r,
+                                                   const double *__restrict__ Mi, double *scal, int itmax,
+                                                   double *partials, unsigned *cnt) {
+  if (scal[DS_DONE] != 0.0) return;
+  const double alpha = scal[DS_ALPHA];
+  double v[3] = {0.0, 0.0, 0.0};
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const double a = Aq[i], ri = r[i] - alpha * a, d = ri * Mi[i];
+    x[i] += alpha * q[i];
+    r[i] = ri;
+    v[0] += ri * ri;
+    v[1] += ri * d;
+    v[2] += a * d;
+  }
+  if (!block_reduce_last<3>(v, partials, cnt) || threadIdx.x) return;
+  const double it = scal[DS_IT] + 1.0;
+  scal[DS_IT] = it;
+  scal[DS_RR] = v[0];
+  scal[DS_BETA] = -alpha * v[2] / scal[DS_RD];
+  scal[DS_RD] = v[1];
+  if (isnan(v[0])) scal[DS_BAD] = 1.0;
+  if (isnan(v[0]) || v[0] < scal[DS_TOL2] || it >= itmax) scal[DS_DONE] = 1.0;
 }
 __global__ void k_diff_setfix(const int *ifix, const double *vfix, int nfix, double *x) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < nfix) x[ifix[i]] = vfix[i];
 }
-__global__ void k_diff_dir(int n, const double *d, double beta, double *q, int first) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) q[i] = first ? d[i] : d[i] + beta * q[i];
-}
-__global__ void k_diff_step(int n, double alpha, const double *q, const double *Aq, double *x, double *r) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    x[i] += alpha * q[i];
-    r[i] -= alpha * Aq[i];
-  }
-}
-
 static int dalloc_d(void **p, size_t bytes) {
   M3_CUDA(cudaMalloc(p, bytes ? bytes : 1));
   return M3SPH_OK;
@@ -267,18 +399,42 @@ static int diff_build(m3sph_mesh *M, DiffState *D, double theta_cone) {
   int st;
   if ((st = dalloc_d((void **)&D->sub, sub.size() * sizeof(int))) ||
       (st = dalloc_d((void **)&D->cls, cls.size())) || (st = dalloc_d((void **)&D->C, 10 * nsub * sizeof(double))) ||
-      (st = dalloc_d((void **)&D->ye, 4 * nsub * sizeof(double))) ||
+      (st = dalloc_d((void **)&D->Me, 4 * nsub * sizeof(double))) ||
+      (st = dalloc_d((void **)&D->scal, DS_N * sizeof(double))) ||
+      (st = dalloc_d((void **)&D->rlen, (size_t)nnod * sizeof(int))) ||
+      (st = dalloc_d((void **)&D->sptr, ((size_t)nnod + 31) / 32 * sizeof(int))) ||
       (st = dalloc_d((void **)&D->gptr, ptr.size() * sizeof(int))) ||
       (st = dalloc_d((void **)&D->gidx, idx.size() * sizeof(int))) ||
       (st = dalloc_d((void **)&D->ML, nnod * sizeof(double))) || (st = dalloc_d((void **)&D->Cdiag, nnod * sizeof(double))) ||
       (st = dalloc_d((void **)&D->fixmask, nnod)) || (st = dalloc_d((void **)&D->err, sizeof(int))))
     return st;
-  for (double **p : {&D->rhs, &D->x, &D->r, &D->d, &D->q, &D->Aq, &D->rl})
+  for (double **p : {&D->Mi, &D->rhs, &D->r, &D->q, &D->Aq, &D->T})
     if ((st = dalloc_d((void **)p, nnod * sizeof(double)))) return st;
   M3_CUDA(cudaMemcpyAsync(D->sub, sub.data(), sub.size() * sizeof(int), cudaMemcpyHostToDevice, s));
   M3_CUDA(cudaMemcpyAsync(D->cls, cls.data(), cls.size(), cudaMemcpyHostToDevice, s));
   M3_CUDA(cudaMemcpyAsync(D->gptr, ptr.data(), ptr.size() * sizeof(int), cudaMemcpyHostToDevice, s));
   M3_CUDA(cudaMemcpyAsync(D->gidx, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+  // row pattern: lengths, starts of the slices (on the host), columns
+  const unsigned g = (unsigned)((nnod + DP_WARPS - 1) / DP_WARPS);
+  k_diff_pattern<<<g, DP_WARPS * 32, 0, s>>>(nnod, D->nsub, D->sub, D->gptr, D->gidx, D->rlen, nullptr, nullptr); count_launch();
+  M3_CUDA(cudaGetLastError());
+  std::vector<int> rlen(nnod), sptr((nnod + 31) / 32);
+  M3_CUDA(cudaMemcpyAsync(rlen.data(), D->rlen, nnod * sizeof(int), cudaMemcpyDeviceToHost, s));
+  M3_CUDA(cudaStreamSynchronize(s));
+  size_t nnz = 0;
+  for (size_t b = 0; b < sptr.size(); ++b) {
+    sptr[b] = (int)nnz;
+    nnz += 32 * (size_t)*std::max_element(rlen.begin() + 32 * b, rlen.begin() + std::min<size_t>(nnod, 32 * b + 32));
+    if (nnz > 2147483647ull) {
+      set_error("mesh too large for the diffusion rows");
+      return M3SPH_ERR_BAD_INPUT;
+    }
+  }
+  if ((st = dalloc_d((void **)&D->rcol, nnz * sizeof(int))) || (st = dalloc_d((void **)&D->rval, nnz * sizeof(double))))
+    return st;
+  M3_CUDA(cudaMemcpyAsync(D->sptr, sptr.data(), sptr.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+  k_diff_pattern<<<g, DP_WARPS * 32, 0, s>>>(nnod, D->nsub, D->sub, D->gptr, D->gidx, nullptr, D->sptr, D->rcol); count_launch();
+  M3_CUDA(cudaGetLastError());
   M3_CUDA(cudaStreamSynchronize(s));
   return M3SPH_OK;
 }
@@ -288,11 +444,11 @@ static int diff_integrate(m3sph_mesh *M, DiffState *D) {
   cudaStream_t s = M->stream;
   const int nsub = D->nsub, nnod = D->nnod;
   M3_CUDA(cudaMemsetAsync(D->err, 0, sizeof(int), s));
-  // the lumped element capacities go through ye, then the fixed-order node sums
-  k_diff_setup<<<(nsub + 127) / 128, 128, 0, s>>>(nsub, D->sub, D->cls, M->fin.gcoord, M->fin.gcoord_sph, nnod, D->kappa,
-                                                  D->C, D->ye, D->err); count_launch();
-  k_diff_gather<<<(nnod + 255) / 256, 256, 0, s>>>(nnod, D->gptr, D->gidx, D->ye, nullptr, nullptr, 0.0, 1.0, nullptr,
-                                                   D->ML); count_launch();
+  k_diff_setup<<<(nsub + 127) / 128, 128, 0, s>>>(nsub, D->sub, D->cls, slm_x90(M), M->fin.gcoord_sph, nnod, D->kappa, D->C,
+                                                  D->Me, D->err); count_launch();
+  k_diff_lump<<<(nnod + 127) / 128, 128, 0, s>>>(nnod, D->gptr, D->gidx, D->Me, D->ML); count_launch();
+  k_diff_rows<<<(unsigned)(((size_t)nnod * 16 + 255) / 256), 256, 0, s>>>(nnod, nsub, D->sub, D->C, D->gptr, D->gidx, D->sptr,
+                                                                         D->rlen, D->rcol, D->rval, D->Cdiag); count_launch();
   M3_CUDA(cudaGetLastError());
   int herr = 0;
   M3_CUDA(cudaMemcpyAsync(&herr, D->err, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -308,40 +464,6 @@ static int diff_integrate(m3sph_mesh *M, DiffState *D) {
   return M3SPH_OK;
 }
 
-__global__ void k_diff_diag_elem(int nsub, const double *__restrict__ C, double *__restrict__ ye) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nsub) return;
-  const int dk[4] = {0, 2, 5, 9};
-  for (int i = 0; i < 4; ++i) ye[(size_t)i * nsub + e] = C[(size_t)dk[i] * nsub + e];
-}
-
-// conductivity diagonal: per node the sum of its elements' packed diagonal entries (00 11 22 33)
-static int diff_diag(m3sph_mesh *M, DiffState *D) {
-  cudaStream_t s = M->stream;
-  k_diff_diag_elem<<<(D->nsub + 127) / 128, 128, 0, s>>>(D->nsub, D->C, D->ye); count_launch();
-  k_diff_gather<<<(D->nnod + 255) / 256, 256, 0, s>>>(D->nnod, D->gptr, D->gidx, D->ye, nullptr, nullptr, 0.0, 1.0,
-                                                      nullptr, D->Cdiag); count_launch();
-  M3_CUDA(cudaGetLastError());
-  return M3SPH_OK;
-}
-
-// y = a ML x + c C x (fixed rows zeroed when masked)
-static int diff_apply(m3sph_mesh *M, DiffState *D, const double *x, double a, double c, bool masked, double *y) {
-  cudaStream_t s = M->stream;
-  k_diff_elem<<<(D->nsub + 127) / 128, 128, 0, s>>>(D->nsub, D->sub, D->C, x, D->ye); count_launch();
-  k_diff_gather<<<(D->nnod + 255) / 256, 256, 0, s>>>(D->nnod, D->gptr, D->gidx, D->ye, D->ML, x, a, c,
-                                                      masked ? D->fixmask : nullptr, y); count_launch();
-  M3_CUDA(cudaGetLastError());
-  return M3SPH_OK;
-}
-
-static int read2(m3sph_mesh *M, int idx, double &v) {
-  M3_CUDA(cudaMemcpyAsync(M->h_scal + idx, M->scal + idx, sizeof(double), cudaMemcpyDeviceToHost, M->stream));
-  M3_CUDA(cudaStreamSynchronize(M->stream));
-  v = M->h_scal[idx];
-  return M3SPH_OK;
-}
-
 // one diffusion3d_p step on the device-resident T (nnod) over dt; *nit = PCG iterations
 int diffusion_resident(m3sph_mesh *M, double *T, double dt, int *nit) {
   DiffState *D = diff_state(M);
@@ -351,62 +473,40 @@ int diffusion_resident(m3sph_mesh *M, double *T, double dt, int *nit) {
   }
   cudaStream_t s = M->stream;
   const int n = D->nnod;
-  const unsigned g = (unsigned)((n + 255) / 256);
   const double c = dt * D->theta;
+  const unsigned gr = (unsigned)std::min((n + 255) / 256, 2048);   // two partial sums per block
   // rhs = M T - dt (1 - theta) C T (diffusion3d_p.m:96-97)
-  M3_TRY(diff_apply(M, D, T, 1.0, -dt * (1.0 - D->theta), false, D->rhs));
+  k_diff_rowprod<DP_RHS><<<gr, 256, 0, s>>>(n, D->sptr, D->rlen, D->rcol, D->rval, D->ML, T, -dt * (1.0 - D->theta), nullptr,
+                                            D->rhs, nullptr, nullptr, nullptr, nullptr, 0.0, nullptr, nullptr,
+                                            nullptr); count_launch();
   // T(ifix) = vfix; r = rhs - A T on the free rows (A(:,ifix) vfix moves to the rhs through T)
-  if (D->nfix) k_diff_setfix<<<(D->nfix + 255) / 256, 256, 0, s>>>(D->ifix, D->vfix, D->nfix, T); count_launch();
-  M3_TRY(diff_apply(M, D, T, 1.0, c, true, D->Aq));
-  k_diff_resid<<<g, 256, 0, s>>>(n, D->rhs, D->Aq, D->fixmask, D->r); count_launch();
-  M3_CUDA(cudaMemsetAsync(D->q, 0, n * sizeof(double), s));
-  // pcg_solver_p.m: tol relative to normdf of the initial residual over the free rows
-  const int nfree = n - D->nfix;
-  const double sq = std::sqrt((double)std::max(1, nfree));
-  double rr = 0.0;
-  M3_TRY(dot(D->r, D->r, n, M->red, M->red_cnt, M->scal + 20, s));
-  M3_TRY(read2(M, 20, rr));
-  double norm_r = std::sqrt(rr) / sq;
-  const double tol = D->tol * norm_r;
-  int it = 0;
-  double rd = 0.0;
-  // an exactly zero initial residual (a field the step leaves unchanged, e.g. a constant one) is
-  // converged: pcg_solver_p.m would test 0 < 0 and go on to alpha = 0/0
-  if (!(norm_r < tol) && norm_r > 0.0) {
-    for (it = 1; it <= D->itmax; ++it) {
-      k_diff_jacobi<<<g, 256, 0, s>>>(n, D->ML, D->Cdiag, c, D->fixmask, D->r, D->d); count_launch();
-      double beta = 0.0;
-      if (it > 1) {
-        // beta = (r - rlast) . d / rdlast (Polak-Ribiere)
-        k_diff_sub<<<g, 256, 0, s>>>(n, D->r, D->rl, D->Aq); count_launch();
-        double num;
-        M3_TRY(dot(D->Aq, D->d, n, M->red, M->red_cnt, M->scal + 21, s));
-        M3_TRY(read2(M, 21, num));
-        beta = num / rd;
-      }
-      k_diff_dir<<<g, 256, 0, s>>>(n, D->d, beta, D->q, it == 1); count_launch();
-      M3_TRY(dot(D->r, D->d, n, M->red, M->red_cnt, M->scal + 22, s));
-      M3_TRY(read2(M, 22, rd));
-      M3_TRY(diff_apply(M, D, D->q, 1.0, c, true, D->Aq));
-      double qAq;
-      M3_TRY(dot(D->q, D->Aq, n, M->red, M->red_cnt, M->scal + 23, s));
-      M3_TRY(read2(M, 23, qAq));
-      M3_CUDA(cudaMemcpyAsync(D->rl, D->r, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-      const double alpha = rd / qAq;
-      k_diff_step<<<g, 256, 0, s>>>(n, alpha, D->q, D->Aq, T, D->r); count_launch();
-      M3_TRY(dot(D->r, D->r, n, M->red, M->red_cnt, M->scal + 20, s));
-      M3_TRY(read2(M, 20, rr));
-      norm_r = std::sqrt(rr) / sq;
-      if (std::isnan(norm_r)) {
-        set_error("NaN in the diffusion solve");
-        return M3SPH_ERR_NAN;
-      }
-      if (norm_r < tol) break;
-    }
-    it = std::min(it, D->itmax);
+  if (D->nfix) {
+    k_diff_setfix<<<(D->nfix + 255) / 256, 256, 0, s>>>(D->ifix, D->vfix, D->nfix, T); count_launch();
   }
-  M3_CUDA(cudaGetLastError());
-  if (nit) *nit = it;
+  k_diff_rowprod<DP_RESID><<<gr, 256, 0, s>>>(n, D->sptr, D->rlen, D->rcol, D->rval, D->ML, T, c, D->fixmask, D->r, D->rhs,
+                                              D->Cdiag, D->Mi, D->q, D->tol, D->scal, M->red, M->red_cnt); count_launch();
+  // iterations are launched DIFF_CHECK at a time; those past the end do nothing
+  constexpr int DIFF_CHECK = 6;
+  double h[DS_N];
+  for (int it = 0;; it += DIFF_CHECK) {
+    M3_CUDA(cudaGetLastError());
+    M3_CUDA(cudaMemcpyAsync(h, D->scal, sizeof(h), cudaMemcpyDeviceToHost, s));
+    M3_CUDA(cudaStreamSynchronize(s));
+    if (h[DS_DONE] != 0.0 || std::isnan(h[DS_RR])) break;
+    for (int k = 0; k < DIFF_CHECK; ++k) {
+      k_diff_dir<<<red_blocks(n), 256, 0, s>>>(n, D->r, D->Mi, D->q, D->scal); count_launch();
+      k_diff_rowprod<DP_CG><<<gr, 256, 0, s>>>(n, D->sptr, D->rlen, D->rcol, D->rval, D->ML, D->q, c, D->fixmask, D->Aq,
+                                               nullptr, nullptr, nullptr, nullptr, 0.0, D->scal, M->red,
+                                               M->red_cnt); count_launch();
+      k_diff_step<<<red_blocks(n), 256, 0, s>>>(n, D->q, D->Aq, T, D->r, D->Mi, D->scal, D->itmax, M->red,
+                                                M->red_cnt); count_launch();
+    }
+  }
+  if (h[DS_BAD] != 0.0) {
+    set_error("NaN in the diffusion solve");
+    return M3SPH_ERR_NAN;
+  }
+  if (nit) *nit = (int)h[DS_IT];
   return M3SPH_OK;
 }
 
@@ -443,20 +543,22 @@ extern "C" int m3sph_diffusion_setup(m3sph_mesh *M, const m3sph_diffusion_opts *
     fx[i] = ifix[i] - 1;
     mask[fx[i]] = 1;
   }
-  if (D->ifix) cudaFree(D->ifix);
-  if (D->vfix) cudaFree(D->vfix);
-  D->ifix = nullptr;
-  D->vfix = nullptr;
   D->nfix = nfix;
-  M3_TRY(dalloc_d((void **)&D->ifix, std::max(1, nfix) * sizeof(int)));
-  M3_TRY(dalloc_d((void **)&D->vfix, std::max(1, nfix) * sizeof(double)));
+  if (nfix > D->fixcap || !D->ifix) {
+    if (D->ifix) cudaFree(D->ifix);
+    if (D->vfix) cudaFree(D->vfix);
+    D->ifix = nullptr;
+    D->vfix = nullptr;
+    D->fixcap = std::max(1, nfix);
+    M3_TRY(dalloc_d((void **)&D->ifix, D->fixcap * sizeof(int)));
+    M3_TRY(dalloc_d((void **)&D->vfix, D->fixcap * sizeof(double)));
+  }
   if (nfix) {
     M3_CUDA(cudaMemcpyAsync(D->ifix, fx.data(), nfix * sizeof(int), cudaMemcpyHostToDevice, s));
     M3_CUDA(cudaMemcpyAsync(D->vfix, vfix, nfix * sizeof(double), cudaMemcpyHostToDevice, s));
   }
   M3_CUDA(cudaMemcpyAsync(D->fixmask, mask.data(), D->nnod, cudaMemcpyHostToDevice, s));
   M3_TRY(diff_integrate(M, D));
-  M3_TRY(diff_diag(M, D));
   M3_CUDA(cudaStreamSynchronize(s));
   return M3SPH_OK;
 }
@@ -473,8 +575,7 @@ extern "C" int m3sph_diffusion3d(m3sph_mesh *M, double *T, double dt, int32_t *n
     return M3SPH_ERR_BAD_INPUT;
   }
   cudaStream_t s = M->stream;
-  double *Td = nullptr;
-  M3_CUDA(cudaMalloc(&Td, D->nnod * sizeof(double)));
+  double *Td = D->T;
   int st = M3SPH_OK, it = 0;
   if (cudaMemcpyAsync(Td, T, D->nnod * sizeof(double), cudaMemcpyHostToDevice, s) != cudaSuccess)
     st = cuda_fail(cudaGetLastError(), "m3sph_diffusion3d upload");
@@ -482,7 +583,6 @@ extern "C" int m3sph_diffusion3d(m3sph_mesh *M, double *T, double dt, int32_t *n
   if (!st && (cudaMemcpyAsync(T, Td, D->nnod * sizeof(double), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
               cudaStreamSynchronize(s) != cudaSuccess))
     st = cuda_fail(cudaGetLastError(), "m3sph_diffusion3d download");
-  cudaFree(Td);
   if (nit) *nit = it;
   return st;
 }

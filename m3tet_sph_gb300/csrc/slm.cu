@@ -1374,6 +1374,8 @@ static int slm_cubic_gradients(m3sph_mesh *M, SlmState *S, const double *B, int 
 }
 
 static SlmState *slm_state(m3sph_mesh *M) { return reinterpret_cast<SlmState *>(M->slm); }
+// X-90-frame (theta, phi, r) of every node, [3][nnod]
+const double *slm_x90(m3sph_mesh *M) { return slm_state(M)->SX; }
 
 }  // namespace m3sph
 

@@ -79,3 +79,20 @@ def test_time_step_with_diffusion_half_steps(built_lib, tiny_plates):
     finally:
         dm.close()
         dm2.close()
+
+
+@pytest.mark.parametrize("itmax", [1, 5, 6, 7, 12])
+def test_diffusion_iteration_limit(case, itmax):
+    """The iterations are launched a few at a time and end on the device: with a tolerance that is never
+    met exactly itmax of them count, around the edges of a batch. The iterates then differ from the
+    oracle's by rounding alone: 1e-10 of the field, as for the converged ones."""
+    w, dm = case
+    f = w['levels'][0]
+    T0 = 2500.0 * w['T']
+    fix = np.nonzero(f['PointID'] > 0)[0]
+    dm.diffusion_setup(KAPPA, fix, T0[fix], tol=1e-300, itmax=itmax)
+    T, nit = dm.diffusion(T0, 5000.0)
+    D = TO.Diffusion(f['GCOORD'], f['GCOORD_SPH'], _split(f), KAPPA, fix)
+    Tr, nitr = D.step(T0, 5000.0, T0[fix], tol=1e-300, itmax=itmax)
+    assert nit == nitr == itmax
+    assert np.max(np.abs(T - Tr)) <= 1e-10 * np.max(np.abs(T0))
