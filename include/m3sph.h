@@ -309,6 +309,10 @@ M3SPH_API int m3sph_apply_timing(m3sph_mesh *mesh, int32_t img, int32_t precisio
  * (theta,phi,r) triplets (npt x 3). els_guess (1-based, may be NULL) seeds the neighbour walk. */
 M3SPH_API int m3sph_tsearch_sph(m3sph_mesh *mesh, const double *thphr, int32_t npt, const int32_t *els_guess,
                                 int32_t *els_out, double *lc_out, m3sph_locate_info *info);
+/* The same with component-major arrays: thphr and lc_out are 3 x npt (all theta, all phi, all r), the layout
+ * the kernels use, so nothing is transposed. m3sph_interp3d_tet_soa and m3sph_interp3d_cubic_soa take lc so. */
+M3SPH_API int m3sph_tsearch_sph_soa(m3sph_mesh *mesh, const double *thphr, int32_t npt, const int32_t *els_guess,
+                                    int32_t *els_out, double *lc_out, m3sph_locate_info *info);
 /* Location benchmark: the points (npt x 3, as for m3sph_tsearch_sph) are uploaded once, then nrep
  * device-resident locations (walk, ring resolution, brute force, counts) are timed with CUDA events;
  * *ms = mean time per location, info = counts of the last one. */
@@ -319,9 +323,13 @@ M3SPH_API int m3sph_locate_timing(m3sph_mesh *mesh, const double *thphr, int32_t
  * reference's indexing error). npt = 0 does nothing. The same holds for m3sph_interp3d_cubic. */
 M3SPH_API int m3sph_interp3d_tet(m3sph_mesh *mesh, const int32_t *els, const double *lc, int32_t npt,
                                  const double *V, int32_t nvar, int32_t monotonic, double *Vi);
+M3SPH_API int m3sph_interp3d_tet_soa(m3sph_mesh *mesh, const int32_t *els, const double *lc, int32_t npt,
+                                     const double *V, int32_t nvar, int32_t monotonic, double *Vi);
 /* Replaces interp3d_cubic_p (interp3d_cubic_p.m:80-382) for one nodal field V (nnod). */
 M3SPH_API int m3sph_interp3d_cubic(m3sph_mesh *mesh, const int32_t *els, const double *lc, int32_t npt,
                                    const double *V, int32_t monotonic, int32_t method_wght, double *Vi);
+M3SPH_API int m3sph_interp3d_cubic_soa(m3sph_mesh *mesh, const int32_t *els, const double *lc, int32_t npt,
+                                       const double *V, int32_t monotonic, int32_t method_wght, double *Vi);
 /* Allocation-free variant of m3sph_interp3d_cubic (no counterpart in the reference). For callers
  * that cannot allocate device memory while they run: a host that owns all device memory through
  * its own pool, a time loop with a fixed memory footprint, or a host with work in flight on other

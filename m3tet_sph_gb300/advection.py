@@ -23,17 +23,25 @@ def _dm(MESH):
     return dm
 
 
+def _points(x, npt=None):
+    """A (3,npt) array of points for the C ABI: (contiguous array, component-major). Arrays of another shape
+    are handed over point by point."""
+    x = np.asarray(x)
+    soa = x.ndim == 2 and x.shape[0] == 3 and npt in (None, x.shape[1])
+    return np.ascontiguousarray(x if soa else x.T), soa
+
+
 def tsearch2_sph(dm, gTH_PT, els_guess=None):
     """Locate points (3,npt) given in (theta,phi,r): returns (els 1-based, lc (3,npt), info)."""
-    P = np.ascontiguousarray(np.asarray(gTH_PT, dtype=np.float64).T)
-    npt = P.shape[0]
-    els = np.zeros(npt, np.int32)
-    lc = np.zeros((npt, 3))
+    P, soa = _points(np.asarray(gTH_PT, dtype=np.float64))
+    npt = P.shape[1] if soa else P.shape[0]
+    els = np.empty(npt, np.int32)
+    lc = np.empty((3, npt) if soa else (npt, 3))
     info = L.LocateInfo()
     g = None if els_guess is None else np.ascontiguousarray(els_guess, dtype=np.int32)
-    L.check(L.lib().m3sph_tsearch_sph(dm.h, L.dptr(P), npt, L.iptr(g) if g is not None else None, L.iptr(els),
-                                       L.dptr(lc), C.byref(info)))
-    return els, lc.T.copy(), info.as_dict()
+    fn = L.lib().m3sph_tsearch_sph_soa if soa else L.lib().m3sph_tsearch_sph
+    L.check(fn(dm.h, L.dptr(P), npt, L.iptr(g) if g is not None else None, L.iptr(els), L.dptr(lc), C.byref(info)))
+    return els, lc if soa else lc.T.copy(), info.as_dict()
 
 
 def locate_timing(dm, gTH_PT, nrep=5):
@@ -50,20 +58,22 @@ def interp3d_tet(dm, els, lc, V, monotonic=False):
     V = np.asarray(V, dtype=np.float64)
     V2 = V[:, None] if V.ndim == 1 else V
     npt = len(els)
-    out = np.zeros((npt, V2.shape[1]))
-    L.check(L.lib().m3sph_interp3d_tet(dm.h, L.iptr(np.ascontiguousarray(els, dtype=np.int32)),
-                                        L.dptr(np.ascontiguousarray(np.asarray(lc).T)), npt,
-                                        L.dptr(np.ascontiguousarray(V2)), V2.shape[1], int(monotonic), L.dptr(out)))
+    out = np.empty((npt, V2.shape[1]))
+    lc, soa = _points(lc, npt)
+    fn = L.lib().m3sph_interp3d_tet_soa if soa else L.lib().m3sph_interp3d_tet
+    L.check(fn(dm.h, L.iptr(np.ascontiguousarray(els, dtype=np.int32)), L.dptr(lc), npt,
+               L.dptr(np.ascontiguousarray(V2)), V2.shape[1], int(monotonic), L.dptr(out)))
     return out[:, 0] if V.ndim == 1 else out
 
 
 def interp3d_cubic_p(dm, els, lc, V, monotonic=True, method_wght='dist'):
     npt = len(els)
-    out = np.zeros(npt)
-    L.check(L.lib().m3sph_interp3d_cubic(dm.h, L.iptr(np.ascontiguousarray(els, dtype=np.int32)),
-                                          L.dptr(np.ascontiguousarray(np.asarray(lc).T)), npt,
-                                          L.dptr(np.ascontiguousarray(V, dtype=np.float64)), int(monotonic),
-                                          1 if method_wght == 'dist' else 0, L.dptr(out)))
+    out = np.empty(npt)
+    lc, soa = _points(lc, npt)
+    fn = L.lib().m3sph_interp3d_cubic_soa if soa else L.lib().m3sph_interp3d_cubic
+    L.check(fn(dm.h, L.iptr(np.ascontiguousarray(els, dtype=np.int32)), L.dptr(lc), npt,
+               L.dptr(np.ascontiguousarray(V, dtype=np.float64)), int(monotonic), 1 if method_wght == 'dist' else 0,
+               L.dptr(out)))
     return out
 
 

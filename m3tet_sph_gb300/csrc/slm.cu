@@ -1384,6 +1384,12 @@ using namespace m3sph;
 // element ids of interp3d_tet / interp3d_cubic_p callers: 1-based, within the mesh (the reference
 // indexes EL2NOD with them, so any other value is an error there too)
 static int check_element_ids(const int32_t *els, int npt, int nel, const char *fn) {
+  int32_t lo = els[0], hi = els[0];
+  for (int i = 1; i < npt; ++i) {
+    lo = std::min(lo, els[i]);
+    hi = std::max(hi, els[i]);
+  }
+  if (lo >= 1 && hi <= nel) return M3SPH_OK;
   for (int i = 0; i < npt; ++i)
     if (els[i] < 1 || els[i] > nel) {
       set_error(std::string(fn) + ": element id " + std::to_string(els[i]) + " at point " + std::to_string(i + 1) +
@@ -1402,8 +1408,20 @@ static int slm_check(m3sph_mesh *M) {
   return M3SPH_OK;
 }
 
-extern "C" int m3sph_tsearch_sph(m3sph_mesh *M, const double *thphr, int32_t npt, const int32_t *els_guess,
-                                 int32_t *els_out, double *lc_out, m3sph_locate_info *info) {
+// The host arrays of the calls below are point-major (3 values per point, the C and MATLAB layout) or, in the
+// *_soa entry points, component-major (3 x npt, the Python mirrors' layout), which the kernels use: those are
+// copied as they are. Point-major ones are transposed on the device through a free buffer: 1.5M points took
+// 12 ms in two host transposes, 200k interpolation points 0.4 ms in host loops over points and ids.
+static int points_to_device(const double *h, int npt, bool soa, double *stage, double *dst, cudaStream_t s) {
+  M3_CUDA(cudaMemcpyAsync(soa ? dst : stage, h, sizeof(double) * 3 * (size_t)npt, cudaMemcpyHostToDevice, s));
+  if (!soa) {
+    k_aos3_to_soa<<<(npt + 255) / 256, 256, 0, s>>>(stage, npt, dst); count_launch();
+  }
+  return M3SPH_OK;
+}
+
+static int tsearch_host(m3sph_mesh *M, const double *thphr, int32_t npt, const int32_t *els_guess, int32_t *els_out,
+                        double *lc_out, m3sph_locate_info *info, bool soa) {
   int st = slm_check(M);
   if (st) return st;
   if (npt < 0 || (npt > 0 && (!thphr || !els_out))) {
@@ -1415,24 +1433,33 @@ extern "C" int m3sph_tsearch_sph(m3sph_mesh *M, const double *thphr, int32_t npt
   Level &L0 = M->lev[0];
   if ((st = slm_reserve(S, npt, L0.nel, L0.nnod, L0.nvnod))) return st;
   cudaStream_t s = M->stream;
-  // points arrive point-major (th ph r per point); S->lc stages them for the transpose to S->P
-  M3_CUDA(cudaMemcpyAsync(S->lc, thphr, sizeof(double) * 3 * (size_t)npt, cudaMemcpyHostToDevice, s));
-  k_aos3_to_soa<<<(npt + 255) / 256, 256, 0, s>>>(S->lc, npt, S->P); count_launch();
+  M3_TRY(points_to_device(thphr, npt, soa, S->lc, S->P, s));
   if (els_guess) {
     M3_CUDA(cudaMemcpyAsync(S->guess, els_guess, sizeof(int) * npt, cudaMemcpyHostToDevice, s));
     k_add_int<<<(npt + 255) / 256, 256, 0, s>>>(S->guess, npt, -1); count_launch();
   }
   st = slm_locate(M, S, npt, els_guess != nullptr, npt == L0.nnod, false, info);
   if (st && st != M3SPH_ERR_POINT_NOT_FOUND) return st;
-  // 1-based ids; local coordinates back to point-major order (S->P is free now)
+  // 1-based ids; point-major local coordinates through S->P, which is free now
   k_add_int<<<(npt + 255) / 256, 256, 0, s>>>(S->els, npt, 1); count_launch();
   M3_CUDA(cudaMemcpyAsync(els_out, S->els, sizeof(int) * npt, cudaMemcpyDeviceToHost, s));
   if (lc_out) {
-    k_soa3_to_aos<<<(npt + 255) / 256, 256, 0, s>>>(S->lc, npt, S->P); count_launch();
-    M3_CUDA(cudaMemcpyAsync(lc_out, S->P, sizeof(double) * 3 * (size_t)npt, cudaMemcpyDeviceToHost, s));
+    if (!soa) {
+      k_soa3_to_aos<<<(npt + 255) / 256, 256, 0, s>>>(S->lc, npt, S->P); count_launch();
+    }
+    M3_CUDA(cudaMemcpyAsync(lc_out, soa ? S->lc : S->P, sizeof(double) * 3 * (size_t)npt, cudaMemcpyDeviceToHost, s));
   }
   M3_CUDA(cudaStreamSynchronize(s));
   return st;
+}
+
+extern "C" int m3sph_tsearch_sph(m3sph_mesh *M, const double *thphr, int32_t npt, const int32_t *els_guess,
+                                 int32_t *els_out, double *lc_out, m3sph_locate_info *info) {
+  return tsearch_host(M, thphr, npt, els_guess, els_out, lc_out, info, false);
+}
+extern "C" int m3sph_tsearch_sph_soa(m3sph_mesh *M, const double *thphr, int32_t npt, const int32_t *els_guess,
+                                     int32_t *els_out, double *lc_out, m3sph_locate_info *info) {
+  return tsearch_host(M, thphr, npt, els_guess, els_out, lc_out, info, true);
 }
 
 extern "C" int m3sph_locate_timing(m3sph_mesh *M, const double *thphr, int32_t npt, int32_t nrep, double *ms,
@@ -1466,8 +1493,15 @@ extern "C" int m3sph_locate_timing(m3sph_mesh *M, const double *thphr, int32_t n
   return st;
 }
 
-extern "C" int m3sph_interp3d_tet(m3sph_mesh *M, const int32_t *els, const double *lc, int32_t npt, const double *V,
-                                  int32_t nvar, int32_t monotonic, double *Vi) {
+// ids (1-based on the host, checked) and local coordinates of interpolation points
+static int interp_points(SlmState *S, const int32_t *els, const double *lc, int npt, bool soa, cudaStream_t s) {
+  M3_CUDA(cudaMemcpyAsync(S->els, els, sizeof(int) * npt, cudaMemcpyHostToDevice, s));
+  k_add_int<<<(npt + 255) / 256, 256, 0, s>>>(S->els, npt, -1); count_launch();
+  return points_to_device(lc, npt, soa, S->P, S->lc, s);
+}
+
+static int interp_tet_host(m3sph_mesh *M, const int32_t *els, const double *lc, int32_t npt, const double *V, int32_t nvar,
+                           int32_t monotonic, double *Vi, bool soa) {
   int st = slm_check(M);
   if (st) return st;
   if (npt < 0 || nvar < 1 || nvar > 3 || (npt > 0 && (!els || !lc || !V || !Vi))) {
@@ -1480,29 +1514,37 @@ extern "C" int m3sph_interp3d_tet(m3sph_mesh *M, const int32_t *els, const doubl
   if ((st = check_element_ids(els, npt, L0.nel, "m3sph_interp3d_tet"))) return st;
   if ((st = slm_reserve(S, npt, L0.nel, L0.nnod, L0.nvnod))) return st;
   cudaStream_t s = M->stream;
-  std::vector<int> e(npt);
-  std::vector<double> l(3 * (size_t)npt), v((size_t)nvar * L0.nnod);
-  for (int i = 0; i < npt; ++i) {
-    e[i] = els[i] - 1;
-    for (int k = 0; k < 3; ++k) l[(size_t)k * npt + i] = lc[3 * (size_t)i + k];
+  M3_TRY(interp_points(S, els, lc, npt, soa, s));
+  const double *v = V;
+  std::vector<double> vt, o;
+  if (nvar > 1) {   // fields one after the other
+    vt.resize((size_t)nvar * L0.nnod);
+    for (int n = 0; n < L0.nnod; ++n)
+      for (int k = 0; k < nvar; ++k) vt[(size_t)k * L0.nnod + n] = V[(size_t)n * nvar + k];
+    v = vt.data();
+    o.resize((size_t)nvar * npt);
   }
-  for (int n = 0; n < L0.nnod; ++n)
-    for (int k = 0; k < nvar; ++k) v[(size_t)k * L0.nnod + n] = V[(size_t)n * nvar + k];
-  M3_CUDA(cudaMemcpyAsync(S->els, e.data(), sizeof(int) * npt, cudaMemcpyHostToDevice, s));
-  M3_CUDA(cudaMemcpyAsync(S->lc, l.data(), sizeof(double) * l.size(), cudaMemcpyHostToDevice, s));
-  M3_CUDA(cudaMemcpyAsync(S->V, v.data(), sizeof(double) * v.size(), cudaMemcpyHostToDevice, s));
+  M3_CUDA(cudaMemcpyAsync(S->V, v, sizeof(double) * nvar * L0.nnod, cudaMemcpyHostToDevice, s));
   k_interp_p2<<<(npt + 127) / 128, 128, 0, s>>>(S->view, S->els, S->lc, npt, S->V, nvar, monotonic, S->out); count_launch();
   M3_CUDA(cudaGetLastError());
-  std::vector<double> o((size_t)nvar * npt);
-  M3_CUDA(cudaMemcpyAsync(o.data(), S->out, sizeof(double) * o.size(), cudaMemcpyDeviceToHost, s));
+  M3_CUDA(cudaMemcpyAsync(nvar > 1 ? o.data() : Vi, S->out, sizeof(double) * nvar * (size_t)npt, cudaMemcpyDeviceToHost, s));
   M3_CUDA(cudaStreamSynchronize(s));
-  for (int i = 0; i < npt; ++i)
+  for (int i = 0; i < npt && nvar > 1; ++i)
     for (int k = 0; k < nvar; ++k) Vi[(size_t)i * nvar + k] = o[(size_t)k * npt + i];
   return M3SPH_OK;
 }
 
-extern "C" int m3sph_interp3d_cubic(m3sph_mesh *M, const int32_t *els, const double *lc, int32_t npt, const double *V,
-                                    int32_t monotonic, int32_t method_wght, double *Vi) {
+extern "C" int m3sph_interp3d_tet(m3sph_mesh *M, const int32_t *els, const double *lc, int32_t npt, const double *V,
+                                  int32_t nvar, int32_t monotonic, double *Vi) {
+  return interp_tet_host(M, els, lc, npt, V, nvar, monotonic, Vi, false);
+}
+extern "C" int m3sph_interp3d_tet_soa(m3sph_mesh *M, const int32_t *els, const double *lc, int32_t npt, const double *V,
+                                      int32_t nvar, int32_t monotonic, double *Vi) {
+  return interp_tet_host(M, els, lc, npt, V, nvar, monotonic, Vi, true);
+}
+
+static int interp_cubic_host(m3sph_mesh *M, const int32_t *els, const double *lc, int32_t npt, const double *V,
+                             int32_t monotonic, int32_t method_wght, double *Vi, bool soa) {
   int st = slm_check(M);
   if (st) return st;
   if (npt < 0 || (npt > 0 && (!els || !lc || !V || !Vi))) {
@@ -1515,14 +1557,7 @@ extern "C" int m3sph_interp3d_cubic(m3sph_mesh *M, const int32_t *els, const dou
   if ((st = check_element_ids(els, npt, L0.nel, "m3sph_interp3d_cubic"))) return st;
   if ((st = slm_reserve(S, npt, L0.nel, L0.nnod, L0.nvnod))) return st;
   cudaStream_t s = M->stream;
-  std::vector<int> e(npt);
-  std::vector<double> l(3 * (size_t)npt);
-  for (int i = 0; i < npt; ++i) {
-    e[i] = els[i] - 1;
-    for (int k = 0; k < 3; ++k) l[(size_t)k * npt + i] = lc[3 * (size_t)i + k];
-  }
-  M3_CUDA(cudaMemcpyAsync(S->els, e.data(), sizeof(int) * npt, cudaMemcpyHostToDevice, s));
-  M3_CUDA(cudaMemcpyAsync(S->lc, l.data(), sizeof(double) * l.size(), cudaMemcpyHostToDevice, s));
+  M3_TRY(interp_points(S, els, lc, npt, soa, s));
   M3_CUDA(cudaMemcpyAsync(S->V, V, sizeof(double) * L0.nnod, cudaMemcpyHostToDevice, s));
   if ((st = slm_cubic_gradients(M, S, S->V, method_wght))) return st;
   k_cubic_interp<<<(npt + 127) / 128, 128, 0, s>>>(S->view, M->fin.gcoord, S->els, S->lc, npt, S->V, S->gn, S->wn,
@@ -1531,6 +1566,15 @@ extern "C" int m3sph_interp3d_cubic(m3sph_mesh *M, const int32_t *els, const dou
   M3_CUDA(cudaMemcpyAsync(Vi, S->out, sizeof(double) * npt, cudaMemcpyDeviceToHost, s));
   M3_CUDA(cudaStreamSynchronize(s));
   return M3SPH_OK;
+}
+
+extern "C" int m3sph_interp3d_cubic(m3sph_mesh *M, const int32_t *els, const double *lc, int32_t npt, const double *V,
+                                    int32_t monotonic, int32_t method_wght, double *Vi) {
+  return interp_cubic_host(M, els, lc, npt, V, monotonic, method_wght, Vi, false);
+}
+extern "C" int m3sph_interp3d_cubic_soa(m3sph_mesh *M, const int32_t *els, const double *lc, int32_t npt, const double *V,
+                                        int32_t monotonic, int32_t method_wght, double *Vi) {
+  return interp_cubic_host(M, els, lc, npt, V, monotonic, method_wght, Vi, true);
 }
 
 // advect3d_slm_p_sph with PC2 backtracking: T (nnod) updated in place; els_BT / els_INTERP

@@ -213,3 +213,26 @@ def test_empty_inputs_and_element_id_range(tiny):
         assert np.allclose(v, 1.0, rtol=0, atol=1e-14)
     finally:
         dm.close()
+
+
+@pytest.mark.parametrize("npt,nvar", [(1, 1), (257, 3)])
+def test_point_major_and_component_major_arrays_agree(mesh_case, npt, nvar):
+    """The C entry points that take npt x 3 arrays and those that take 3 x npt ones give the same bits."""
+    import ctypes as C
+    from m3tet_sph_gb300 import _lib as L
+    w, dm, _ = mesh_case
+    P = random_shell_points(npt, 5)
+    V = np.ascontiguousarray(np.random.default_rng(6).normal(size=(dm.nnod, nvar)))
+    got = []
+    for suf, lay in (("", np.transpose), ("_soa", np.array)):
+        fn = lambda name: getattr(L.lib(), name + suf)
+        pts = np.ascontiguousarray(lay(P))
+        els, lc, info = np.zeros(npt, np.int32), np.zeros_like(pts), L.LocateInfo()
+        L.check(fn("m3sph_tsearch_sph")(dm.h, L.dptr(pts), npt, None, L.iptr(els), L.dptr(lc), C.byref(info)))
+        vt, vc = np.zeros((npt, nvar)), np.zeros(npt)
+        L.check(fn("m3sph_interp3d_tet")(dm.h, L.iptr(els), L.dptr(lc), npt, L.dptr(V), nvar, 1, L.dptr(vt)))
+        v0 = np.ascontiguousarray(V[:, 0])
+        L.check(fn("m3sph_interp3d_cubic")(dm.h, L.iptr(els), L.dptr(lc), npt, L.dptr(v0), 1, 1, L.dptr(vc)))
+        got.append((els, np.ascontiguousarray(lay(lc)) if suf == "" else lc, vt, vc))
+    for a, b in zip(*got):
+        assert a.shape == b.shape and np.array_equal(a, b)
