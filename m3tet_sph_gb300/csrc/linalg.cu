@@ -2,6 +2,7 @@
 // (intermesh_transfer_matrix / Ic2f' restriction), Jacobi smoothing and the dense coarse
 // solve that stands in for cholesky_factorization / cholesky_solve.
 #include "common.cuh"
+#include "tc.cuh"
 
 namespace m3sph {
 
@@ -336,12 +337,12 @@ __global__ void k_dense_from_bsr(const int *__restrict__ ptr, const int *__restr
 //    16-wide sub-panels: the 16 x 16 pivot block by one warp through shuffles, the rest as rank-16
 //    updates. (One pivot at a time in shared memory took 975 us per panel in FP32 and 3,941 us in FP64;
 //    now 74 us, and 129 us for the 64-wide FP64 block.)
-//  * k_gjb_panels saves C (transposed) and forms R;
-//  * k_gjb_update is a tile GEMM: NB x NB tiles, 256 threads, an RT x RT register block per thread read
-//    from shared memory as 16-byte vectors, chunks of the inner dimension brought in by 16-byte
-//    asynchronous copies two chunks ahead (panels are padded to whole tiles with zeros, so the copies
-//    need no bounds). FP32 issue bounds it: 588 us per panel at 14.8k free dofs = 48 TFLOP/s (the full
-//    form with 4-byte copies: 1,886 us).
+//  * k_gjb_panels saves C (transposed), forms R and writes panel k of the matrix (its products summed by
+//    chunks of 16: 2 to 3 % less error of the inverse);
+//  * FP32: k_gjb_update_tc, on the tensor cores. FP64: k_gjb_update, a tile GEMM of NB x NB tiles, 256
+//    threads, an RT x RT register block per thread read from shared memory as 16-byte vectors, chunks of the
+//    inner dimension brought in by 16-byte asynchronous copies two chunks ahead (panels are padded to whole
+//    tiles with zeros, so the copies need no bounds); FP64 issue bounds it.
 // NB is 64 in FP64: the diagonal block is inverted on one SM, whose FP64 rate (2 FMA a cycle) makes a
 // 128-wide block cost 0.5 ms.
 // ---------------------------------------------------------------------------------------
@@ -349,12 +350,29 @@ template <typename T> struct Gj;
 template <> struct Gj<float> { static constexpr int NB = 128, KC = 16; using V = float4; static constexpr int VN = 4; };
 template <> struct Gj<double> { static constexpr int NB = 64, KC = 8; using V = double2; static constexpr int VN = 2; };
 constexpr int GJ_ST = 3;             // chunk stages
+// tensor-core update (FP32): operand images of a 128 x 128 panel block, three BF16 parts whose sum is the FP32
+// value, K-major and 128-byte swizzled: [half of K][part][128 rows][64 K]
+namespace gu {
+constexpr int NB = 128, ATOM = NB * 128, HALF = 3 * ATOM, IMAGE = 2 * HALF;
+constexpr int WARPS = 16, THREADS = (WARPS + 2) * 32;     // two groups of 8 epilogue warps, a copy warp, an MMA warp
+constexpr int STAGE_LD = 20;                               // floats per row of a warp's staging tile of 16 rows
+constexpr int OFF_A = 0, OFF_B = IMAGE, OFF_ST = OFF_B + 2 * HALF;
+constexpr int OFF_BAR = OFF_ST + WARPS * 16 * STAGE_LD * 4;  // a_full, b_full[2], b_empty[2], acc_full[4], acc_empty[2], drain
+// The accumulators round towards zero: sums of the magnitude of the result are cut four times per half of K, by
+// half a unit in the last place on average (a unit is 2^-24 to 2^-23 of the value). The third part of C gives
+// this back.
+constexpr float ROUNDING = 1e-7f;
+constexpr int OFF_TM = OFF_BAR + 12 * 8;
+constexpr int SMEM = OFF_TM + 8, SMEM_ALLOC = SMEM + 1024;
+static_assert(OFF_BAR % 8 == 0 && OFF_ST % 16 == 0 && SMEM_ALLOC <= 232448, "one CTA per SM");
+}  // namespace gu
 constexpr int GJ_SB = 16;            // sub-panel width of the diagonal block
 
 // values of the work array: D^-1, its transpose, the saved column panel and the row panel
+// FP32: also the operand images of the two panels and an error word
 template <typename T> size_t gj_work(int n) {
   const size_t NB = Gj<T>::NB, npad = (n + NB - 1) / NB * NB;
-  return 2 * NB * NB + 2 * NB * npad;
+  return 2 * NB * NB + 2 * NB * npad + (sizeof(T) == 4 ? 2 * (npad / NB) * (gu::IMAGE / 4) + 4 : 0);
 }
 size_t dense_inverse_work64(int n) { return gj_work<double>(n); }
 size_t dense_inverse_work32(int n) { return gj_work<float>(n); }
@@ -510,6 +528,11 @@ __device__ __forceinline__ void gj_tile(T (&acc)[RT][RT], const T *__restrict__ 
     __syncthreads();                     // chunk ch has landed, everyone is done with chunk ch - 1
     issue(ch + GJ_ST - 1);
     const T(*xs)[NB] = sm[ch % GJ_ST][0], (*ys)[NB] = sm[ch % GJ_ST][1];
+    T part[RT][RT];                      // a chunk's sum by itself: shorter chains of roundings
+#pragma unroll
+    for (int a = 0; a < RT; ++a)
+#pragma unroll
+      for (int b = 0; b < RT; ++b) part[a][b] = T(0);
 #pragma unroll
     for (int m = 0; m < KC; ++m) {
       T xv[RT], yv[RT];
@@ -521,21 +544,65 @@ __device__ __forceinline__ void gj_tile(T (&acc)[RT][RT], const T *__restrict__ 
 #pragma unroll
       for (int a = 0; a < RT; ++a)
 #pragma unroll
-        for (int b = 0; b < RT; ++b) acc[a][b] += xv[a] * yv[b];
+        for (int b = 0; b < RT; ++b) (sizeof(T) == 4 ? part : acc)[a][b] += xv[a] * yv[b];
     }
+    if (sizeof(T) == 4)
+#pragma unroll
+      for (int a = 0; a < RT; ++a)
+#pragma unroll
+        for (int b = 0; b < RT; ++b) acc[a][b] += part[a][b];
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
+// operand image of block column j0 of a panel S (128 K-rows of npad values): row c = column j0 + c of S, times
+// 1 + up
+__device__ __forceinline__ void gj_image(const float *S, size_t npad, int j0, float up, unsigned char *img) {
+  for (int q = threadIdx.x; q < 128 * 16; q += 256) {
+    const int c = q & 127, ch = q >> 7;
+    uint32_t w[3][4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      float v[2], p[3][2];
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const float x = S[(size_t)(8 * ch + 2 * h + t) * npad + j0 + c];
+        v[t] = x;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          if (k == 2) v[t] += up * x;
+          p[k][t] = __bfloat162float(__float2bfloat16_rn(v[t]));
+          v[t] -= p[k][t];               // exact: 8 of the 24 bits each time
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k) w[k][h] = tc_pack(p[k][0], p[k][1]);
+    }
+    unsigned char *o = img + (ch >> 3) * gu::HALF + tc_sw(c, ch & 7);
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      *reinterpret_cast<uint4 *>(o + k * gu::ATOM) = make_uint4(w[k][0], w[k][1], w[k][2], w[k][3]);
+  }
+}
+
 // block j: saved column panel Ct[m][i] = C_i[m] for its rows i and row panel R = +-D^-1 C_j' for its
-// columns (minus for panels already swept, j < kblk); zero padding past n
+// columns (minus for panels already swept, j < kblk), zero padding past n; then panel k of the matrix itself:
+// its row R, its column -C D^-1 = -R' and its diagonal block D^-1. FP32: the operand images of C and R as well.
 template <typename T>
-__global__ void __launch_bounds__(256) k_gjb_panels(const T *__restrict__ A, int ld, int n, int kblk, int nb,
-                                                    const T *__restrict__ DinvT, size_t npad, T *__restrict__ R, T *Ct) {
+__global__ void __launch_bounds__(256) k_gjb_panels(T *__restrict__ A, int ld, int n, int kblk, int nb,
+                                                    const T *__restrict__ Dinv, const T *__restrict__ DinvT, size_t npad,
+                                                    T *R, T *Ct, unsigned char *imgC, unsigned char *imgR) {
   constexpr int NB = Gj<T>::NB, RT = NB / 16;
   __shared__ T tr[32][33];
   const int j = blockIdx.x, j0 = j * NB, kb = kblk * NB;
   const bool swept = j < kblk;
+  if (j == kblk) {
+    for (int q = threadIdx.x; q < NB * NB; q += 256) {
+      const int r = q / NB, c = q % NB;
+      if (r < nb && c < nb) A[(size_t)(kb + r) * ld + kb + c] = Dinv[q];
+    }
+    return;
+  }
   if (swept) {
     // C_i = -A_ki' : row m of tile (k, j) is column m of C
     for (int q = threadIdx.x; q < NB * NB; q += 256) {
@@ -567,49 +634,48 @@ __global__ void __launch_bounds__(256) k_gjb_panels(const T *__restrict__ A, int
       T v[4];
 #pragma unroll
       for (int b = 0; b < 4; ++b) v[b] = swept ? -acc[a][g + b] : acc[a][g + b];
-      gj_st4(&R[gj_idx<T>(ty, a) * npad + j0 + gj_idx<T>(tx, g)], v);
+      const int m = gj_idx<T>(ty, a), c = j0 + gj_idx<T>(tx, g);
+      gj_st4(&R[m * npad + c], v);
+      if (swept && m < nb) gj_st4(&A[(size_t)(kb + m) * ld + c], v);
     }
-}
-
-// tile (bi, bj), bj <= bi, of the update: A - C R outside panel k; the panel's row R; its column
-// -C D^-1 = -R'; the diagonal block D^-1
-template <typename T>
-__global__ void __launch_bounds__(256, 2) k_gjb_update(T *__restrict__ A, int ld, int n, int kblk, int nb,
-                                                       const T *__restrict__ Dinv, size_t npad, const T *__restrict__ R,
-                                                       const T *__restrict__ Ct) {
-  constexpr int NB = Gj<T>::NB, RT = NB / 16;
-  __shared__ T tr[32][33];
-  int bi = (int)((sqrtf(8.f * blockIdx.x + 1.f) - 1.f) * 0.5f);
-  while ((size_t)bi * (bi + 1) / 2 > blockIdx.x) --bi;
-  while ((size_t)(bi + 1) * (bi + 2) / 2 <= blockIdx.x) ++bi;
-  const int bj = (int)(blockIdx.x - (size_t)bi * (bi + 1) / 2);
-  const int i0 = bi * NB, j0 = bj * NB, kb = kblk * NB;
-  if (bi == kblk) {
-    for (int q = threadIdx.x; q < NB * NB; q += 256) {
-      const int r = q / NB, c = q % NB;
-      if (r >= nb) break;
-      if (bj == kblk) {
-        if (c < nb) A[(size_t)(kb + r) * ld + kb + c] = Dinv[q];
-      } else {
-        A[(size_t)(kb + r) * ld + j0 + c] = R[r * npad + j0 + c];
-      }
-    }
-    return;
-  }
-  if (bj == kblk) {
+  __syncthreads();
+  if (!swept) {
     const int lx = threadIdx.x % 32, ly = threadIdx.x / 32;
     for (int b = 0; b < (NB / 32) * (NB / 32); ++b) {
       const int r0 = (b / (NB / 32)) * 32, m0 = (b % (NB / 32)) * 32;
       __syncthreads();
-      for (int y = ly; y < 32; y += 8) tr[y][lx] = R[(size_t)(m0 + y) * npad + i0 + r0 + lx];
+      for (int y = ly; y < 32; y += 8) tr[y][lx] = R[(size_t)(m0 + y) * npad + j0 + r0 + lx];
       __syncthreads();
       for (int y = ly; y < 32; y += 8) {
-        const int i = i0 + r0 + y, m = m0 + lx;
+        const int i = j0 + r0 + y, m = m0 + lx;
         if (i < n && m < nb) A[(size_t)i * ld + kb + m] = -tr[lx][y];
       }
     }
-    return;
   }
+  if constexpr (sizeof(T) == 4) {
+    gj_image(Ct, npad, j0, gu::ROUNDING, imgC + (size_t)j * gu::IMAGE);
+    gj_image(R, npad, j0, 0.f, imgR + (size_t)j * gu::IMAGE);
+  }
+}
+
+// tile t of the lower triangle without panel k: block row and column
+__device__ __forceinline__ void gj_tile_of(size_t t, int kblk, int &bi, int &bj) {
+  bi = (int)((sqrtf(8.f * t + 1.f) - 1.f) * 0.5f);
+  while ((size_t)bi * (bi + 1) / 2 > t) --bi;
+  while ((size_t)(bi + 1) * (bi + 2) / 2 <= t) ++bi;
+  bj = (int)(t - (size_t)bi * (bi + 1) / 2);
+  bi += bi >= kblk;
+  bj += bj >= kblk;
+}
+
+// A - C R on a tile outside panel k (FP64)
+template <typename T>
+__global__ void __launch_bounds__(256, 2) k_gjb_update(T *__restrict__ A, int ld, int n, int kblk, size_t npad,
+                                                       const T *__restrict__ R, const T *__restrict__ Ct) {
+  constexpr int NB = Gj<T>::NB, RT = NB / 16;
+  int bi, bj;
+  gj_tile_of(blockIdx.x, kblk, bi, bj);
+  const int i0 = bi * NB, j0 = bj * NB;
   T acc[RT][RT];
   gj_tile<T, RT>(acc, Ct + i0, npad, R + j0, npad);
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
@@ -627,6 +693,214 @@ __global__ void __launch_bounds__(256, 2) k_gjb_update(T *__restrict__ A, int ld
       for (int b = 0; b < 4; ++b) v[b] -= acc[a][g + b];
       gj_st4(p, v);
     }
+  }
+}
+
+// The same for FP32 on the tensor cores. A product of two FP32 values is the six largest of the nine products of
+// their BF16 parts (the rest is below 2^-26 of it); the accumulators are FP32. An accumulator takes a half of K,
+// first the five small products and then the large one, so that the roundings of the former are 2^-8 smaller,
+// the two halves are added in FP32, and what rounding towards zero takes is given back (gu::ROUNDING). Against
+// FP64 inverses of difference matrices of 129 to 14,801 unknowns and contrasts of 1e2 to 1e4 the error of the
+// whole inverse is 0 to 10 % below that of FP32 multiply-adds (without ROUNDING 1 to 4 % above).
+// A persistent CTA takes a run of tiles of the triangle, row by row: the row's operand stays in shared memory
+// (96 KB), the column's comes in halves of 48 KB through a ring of two, and the accumulators of two tiles
+// alternate in TMEM between two groups of epilogue warps, which subtract through a staging tile. At 14.8k free
+// dofs 223 us per panel, FP32 multiply-adds 589 us; the triangle read and written at the copy rate would be
+// 130 us, the MMAs alone are 82 us: what is left is the latency of the A accesses (272 us with chunks fetched when
+// they were needed, 255 us without the prefetch of the next tile into L2).
+__global__ void __launch_bounds__(gu::THREADS, 1) k_gjb_update_tc(float *__restrict__ A, int ld, int n, int kblk,
+                                                                  size_t ntile, const unsigned char *__restrict__ imgC,
+                                                                  const unsigned char *__restrict__ imgR, int *err) {
+  using namespace gu;
+  extern __shared__ __align__(16) unsigned char gj_raw[];
+  unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(gj_raw) + 1023) & ~uintptr_t(1023));
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t sbase = tc_smem_u32(sm);
+  const uint32_t a_full = sbase + OFF_BAR, b_full = a_full + 8, b_empty = a_full + 24, acc_full = a_full + 40,
+                 acc_empty = a_full + 72, drain = a_full + 88;
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + OFF_TM);
+  if (tid == 0) {
+    tc_bar_init(a_full, 1);
+    tc_bar_init(drain, 1);
+    for (int b = 0; b < 2; ++b) {
+      tc_bar_init(b_full + 8 * b, 1);
+      tc_bar_init(b_empty + 8 * b, 1);
+    }
+    for (int b = 0; b < 4; ++b) tc_bar_init(acc_full + 8 * b, 1);
+    for (int b = 0; b < 2; ++b) tc_bar_init(acc_empty + 8 * b, WARPS / 2);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem_u32(tslot)), "r"(512)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tslot;
+  const size_t t0 = ntile * blockIdx.x / gridDim.x, t1 = ntile * (blockIdx.x + 1) / gridDim.x;
+  int bi, bj;
+  if (warp == WARPS) {
+    // ---------------- copies ----------------
+    if (lane == 0) {
+      int row = -1, na = 0, nbt[2] = {0, 0};        // copies issued per barrier
+      bool ok = true;
+      uint32_t it = 0;
+      for (size_t t = t0; t < t1 && ok; ++t, ++it) {
+        gj_tile_of(t, kblk, bi, bj);
+        for (int h = 0; h < 2 && ok; ++h) {
+          if (it) ok = tc_bar_wait(b_empty + 8 * h, (it - 1) & 1);
+          // a new row: its operand goes where the last tile's MMAs read, so both halves must be done
+          if (h == 0 && bi != row) {
+            if (it) ok = ok && tc_bar_wait(b_empty + 8, (it - 1) & 1);
+            if (ok) {
+              tc_bulk_load(sbase + OFF_A, imgC + (size_t)bi * IMAGE, IMAGE, a_full);
+              ++na;
+              row = bi;
+            }
+          }
+          if (!ok) break;
+          tc_bulk_load(sbase + OFF_B + h * HALF, imgR + (size_t)bj * IMAGE + h * HALF, HALF, b_full + 8 * h);
+          ++nbt[h];
+        }
+      }
+      if (!ok) {
+        atomicOr(err, 1);
+        if (na) tc_bar_wait(a_full, (na - 1) & 1);          // copies still in flight
+        for (int h = 0; h < 2; ++h)
+          if (nbt[h]) tc_bar_wait(b_full + 8 * h, (nbt[h] - 1) & 1);
+      }
+    }
+    __syncwarp();
+  } else if (warp == WARPS + 1) {
+    // ---------------- MMAs ----------------
+    if (lane == 0) {
+      // products of parts (A, B), smallest first
+      constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
+      int row = -1, na = 0;
+      bool ok = true;
+      uint32_t it = 0;
+      for (size_t t = t0; t < t1 && ok; ++t, ++it) {
+        gj_tile_of(t, kblk, bi, bj);
+        const int buf = it & 1;
+        if (it >= 2) ok = tc_bar_wait(acc_empty + 8 * buf, ((it >> 1) - 1) & 1);
+        if (ok && bi != row) {
+          ok = tc_bar_wait(a_full, na & 1);
+          ++na;
+          row = bi;
+        }
+        for (int h = 0; h < 2 && ok; ++h) {
+          ok = tc_bar_wait(b_full + 8 * h, it & 1);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t sa = sbase + OFF_A + h * HALF, sb = sbase + OFF_B + h * HALF, d = tmem + 256 * buf + 128 * h;
+#pragma unroll
+          for (int p = 0; p < 6; ++p)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              tc_mma(d, tc_sdesc(sa + PA[p] * ATOM + 32 * k), tc_sdesc(sb + PB[p] * ATOM + 32 * k), tc_idesc(NB, NB),
+                     p > 0 || k > 0);
+          tc_commit(b_empty + 8 * h);
+          tc_commit(acc_full + 8 * (2 * buf + h));
+        }
+      }
+      if (!ok) {
+        atomicOr(err, 2);
+        tc_commit(drain);                    // MMAs still in flight
+        tc_bar_wait(drain, 0);
+      }
+    }
+    __syncwarp();
+  } else {
+    // ---------------- epilogue: groups take every other tile; in a group warp w has rows 32 (w % 4) .. + 31 and
+    // columns 64 (w / 4) .. + 63, 16 at a time ----------------
+    const int grp = warp >> 3, r0 = 32 * (warp & 3), c0 = 64 * ((warp >> 2) & 1), lr = lane >> 2, lc = 4 * (lane & 3);
+    float *st = reinterpret_cast<float *>(sm + OFF_ST) + warp * 16 * STAGE_LD;
+    const uint32_t trow = tmem + ((uint32_t)r0 << 16) + c0 + 256 * grp;
+    // a tile's part into L2, half a row of 256 bytes at a time (a load's own prefetch would bring 32)
+    auto prefetch = [&](size_t t) {
+      if (t >= t1) return;
+      gj_tile_of(t, kblk, bi, bj);
+      const int i = bi * NB + r0 + lane, j = bj * NB + c0;
+      if (i < n && j < ld)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(A + (size_t)i * ld + j),
+                     "r"(4 * min(64, ld - j)));
+    };
+    // 16 columns of A ahead: while a chunk is worked on, the next one (of the group's next tile after the last) is
+    // on its way
+    int i0 = 0, j0 = 0;
+    float *p = nullptr;
+    auto locate = [&](size_t t) {
+      gj_tile_of(t, kblk, bi, bj);
+      i0 = bi * NB + r0 + lr;
+      j0 = bj * NB + c0 + lc;
+      p = A + (size_t)i0 * ld + j0;
+    };
+    auto fetch = [&](float4(&v)[4], int q) {   // rows lr + 8 a
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+        if (j0 + 16 * q < ld && i0 + 8 * a < n) v[a] = *reinterpret_cast<const float4 *>(p + (size_t)(8 * a) * ld + 16 * q);
+    };
+    uint32_t use = 0;
+    float4 v[2][4];
+    prefetch(t0 + grp);
+    if (t0 + grp < t1) {
+      locate(t0 + grp);
+      fetch(v[0], 0);
+    }
+    for (size_t t = t0 + grp; t < t1; t += 2, ++use) {
+      prefetch(t + 2);
+      bool ok = tc_bar_wait(acc_full + 8 * (2 * grp), use & 1) && tc_bar_wait(acc_full + 8 * (2 * grp + 1), use & 1);
+      if (!__all_sync(0xffffffffu, ok)) {
+        if (lane == 0) atomicOr(err, 4);
+        break;
+      }
+      tc_fence_after();
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int ic = i0;
+        const bool jin = j0 + 16 * q < ld;
+        float *pc = p + 16 * q;
+        if (q < 3) {
+          fetch(v[(q + 1) & 1], q + 1);
+        } else if (t + 2 < t1) {
+          locate(t + 2);
+          fetch(v[0], 0);
+        }
+        float x[16], y[16];
+        tc_ld16(trow + 16 * q, x);
+        tc_ld16(trow + 128 + 16 * q, y);
+        if (q == 3) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) tc_arrive(acc_empty + 8 * grp);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {          // 16 rows at a time through the staging tile
+          __syncwarp();
+          if ((lane >> 4) == h)
+#pragma unroll
+            for (int c = 0; c < 16; c += 4)
+              *reinterpret_cast<float4 *>(st + (lane & 15) * STAGE_LD + c) =
+                  make_float4(x[c] + y[c], x[c + 1] + y[c + 1], x[c + 2] + y[c + 2], x[c + 3] + y[c + 3]);
+          __syncwarp();
+#pragma unroll
+          for (int a = 2 * h; a < 2 * h + 2; ++a) {
+            const float4 u = *reinterpret_cast<const float4 *>(st + (lr + 8 * (a & 1)) * STAGE_LD + lc), w = v[q & 1][a];
+            if (jin && ic + 8 * a < n)
+              *reinterpret_cast<float4 *>(pc + (size_t)(8 * a) * ld) =
+                  make_float4(w.x - u.x, w.y - u.y, w.z - u.z, w.w - u.w);
+          }
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
   }
 }
 
@@ -655,18 +929,44 @@ int gj_blocked_inverse(T *A, int ld, int n, T *work, cudaStream_t s) {
   const int nbk = (n + NB - 1) / NB;
   const size_t npad = (size_t)nbk * NB;
   T *Dinv = work, *DinvT = Dinv + NB * NB, *R = DinvT + NB * NB, *Ct = R + NB * npad;
+  const size_t ntile = (size_t)nbk * (nbk - 1) / 2;        // lower tiles outside a panel
+  unsigned char *imgC = nullptr, *imgR = nullptr;
+  int *err = nullptr;
   M3_CUDA(cudaFuncSetAttribute(k_gjb_panels<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gj_smem<T>()));
-  M3_CUDA(cudaFuncSetAttribute(k_gjb_update<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gj_smem<T>()));
+  if constexpr (sizeof(T) == 4) {
+    imgC = reinterpret_cast<unsigned char *>(Ct + NB * npad);
+    imgR = imgC + (size_t)nbk * gu::IMAGE;
+    err = reinterpret_cast<int *>(imgR + (size_t)nbk * gu::IMAGE);
+    M3_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
+    M3_CUDA(cudaFuncSetAttribute(k_gjb_update_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, gu::SMEM_ALLOC));
+  } else {
+    M3_CUDA(cudaFuncSetAttribute(k_gjb_update<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gj_smem<T>()));
+  }
   for (int k = 0; k < nbk; ++k) {
     const int kb = k * NB, nb = std::min(NB, n - kb);
     k_gjb_diag<T><<<1, 256, 0, s>>>(A, ld, kb, nb, Dinv, DinvT); count_launch();
-    k_gjb_panels<T><<<nbk, 256, gj_smem<T>(), s>>>(A, ld, n, k, nb, DinvT, npad, R, Ct); count_launch();
-    k_gjb_update<T><<<(unsigned)((size_t)nbk * (nbk + 1) / 2), 256, gj_smem<T>(), s>>>(A, ld, n, k, nb, Dinv, npad, R, Ct);
+    k_gjb_panels<T><<<nbk, 256, gj_smem<T>(), s>>>(A, ld, n, k, nb, Dinv, DinvT, npad, R, Ct, imgC, imgR); count_launch();
+    if (nbk == 1) break;
+    if constexpr (sizeof(T) == 4) {
+      k_gjb_update_tc<<<(unsigned)std::min<size_t>(ntile, 152), gu::THREADS, gu::SMEM_ALLOC, s>>>(A, ld, n, k, ntile, imgC,
+                                                                                                  imgR, err);
+    } else {
+      k_gjb_update<T><<<(unsigned)ntile, 256, gj_smem<T>(), s>>>(A, ld, n, k, npad, R, Ct);
+    }
     count_launch();
   }
   const unsigned g = (unsigned)((n + 31) / 32);
   k_gjb_mirror<T><<<dim3(g, g), 256, 0, s>>>(A, ld, n); count_launch();
   M3_CUDA(cudaGetLastError());
+  if (err) {
+    int h = 0;
+    M3_CUDA(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    M3_CUDA(cudaStreamSynchronize(s));
+    if (h) {
+      set_error("coarse inverse: a bounded wait gave up (code " + std::to_string(h) + ")");
+      return M3SPH_ERR_CUDA;
+    }
+  }
   return M3SPH_OK;
 }
 

@@ -12,6 +12,7 @@
 #include <mma.h>
 
 #include "common.cuh"
+#include "tc.cuh"
 
 namespace m3sph {
 
@@ -259,76 +260,10 @@ constexpr int OFF_TM = OFF_BAR + 5 * 8;
 constexpr int SMEM = OFF_TM + 8;
 constexpr int SMEM_ALLOC = SMEM + 1024;         // room to align the base to 1024 B
 constexpr int TMEM_COLS = 128;                  // H uses 128 columns, Y reuses the first 32
-constexpr unsigned long long TIMEOUT_NS = 1000000000ull;
 static_assert(OFF_W2 % 1024 == 0 && W2_ATOM % 1024 == 0 && OFF_F % 1024 == 0 && OFF_G % 1024 == 0,
               "swizzle atoms start on 1024 B");
 static_assert(OFF_BAR % 8 == 0 && 2 * (SMEM_ALLOC + 1024) <= 233472, "two CTAs per SM");
-// instruction descriptor of tcgen05.mma kind::f16: D f32 (bits 4-5 = 1), A and B BF16 (bits 7-9,
-// 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 in bits 17-22, M >> 4 in bits 24-28
-constexpr uint32_t idesc(int m, int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
 }  // namespace tc
-
-__device__ __forceinline__ uint32_t tc_smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-// shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups 1024 B apart
-__device__ __forceinline__ uint64_t tc_sdesc(uint32_t saddr) {
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
-         ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
-}
-// byte offset of 16-byte chunk c of row r in a 128-byte-swizzled K-major atom
-__device__ __forceinline__ uint32_t tc_sw(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
-__device__ __forceinline__ void tc_st16(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-__device__ __forceinline__ uint32_t tc_pack(float lo, float hi) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t *>(&v);
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tc_mma(uint32_t tmem, uint64_t a, uint64_t b, uint32_t id, uint32_t acc) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem),
-      "l"(a), "l"(b), "r"(id), "r"(acc)
-      : "memory");
-}
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
-      "[%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-__device__ __forceinline__ bool tc_bar_test(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool tc_bar_wait(uint32_t bar, uint32_t parity) {
-  if (tc_bar_test(bar, parity)) return true;
-  unsigned long long t0, t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-  for (;;) {
-    for (int i = 0; i < 32; ++i)
-      if (tc_bar_test(bar, parity)) return true;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    if (t - t0 > tc::TIMEOUT_NS) return false;
-  }
-}
 
 // the 52 FP32 features of element e from the Jacobi-scaled residual z = (r0 - kd) Dinv: the 30
 // local values divided by their norm s, the 10 standardised log-viscosities, the 12 geometry
@@ -392,20 +327,6 @@ __global__ void k_ml_scale(const T *__restrict__ r0, const T *__restrict__ kd, c
   z[i] = (float)(rv * Dinv[i]);
 }
 
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
 // barrier of the 128 compute threads (named barrier 1) that ANDs a predicate over them
 __device__ __forceinline__ bool tc_group_and(bool v) {
   uint32_t out;
@@ -416,10 +337,6 @@ __device__ __forceinline__ bool tc_group_and(bool v) {
                : "memory");
   return out != 0;
 }
-__device__ __forceinline__ void tc_arrive(uint32_t bar) {
-  asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.shared::cta.b64 st, [%0];\n}" ::"r"(bar) : "memory");
-}
-
 __global__ void __launch_bounds__(tc::THREADS, 2) k_ml_sweep_tc(FeatLevel L, MlpDev w, const float *__restrict__ z,
                                                                 float *__restrict__ C, int *__restrict__ err) {
   using namespace tc;
@@ -515,7 +432,7 @@ __global__ void __launch_bounds__(tc::THREADS, 2) k_ml_sweep_tc(FeatLevel L, Mlp
 #pragma unroll
         for (int k = 0; k < 4; ++k)
           tc_mma(tmem, tc_sdesc(sbase + OFF_F + b * ATOM + 32 * k), tc_sdesc(sbase + tc::OFF_W1 + 32 * k),
-                 idesc(ROWS, HID), k > 0);
+                 tc_idesc(ROWS, HID), k > 0);
         tc_commit(f_empty + 8 * b);      // the feature buffer is free once these MMAs are done
         tc_commit(mma_done);
       }
@@ -551,7 +468,7 @@ __global__ void __launch_bounds__(tc::THREADS, 2) k_ml_sweep_tc(FeatLevel L, Mlp
 #pragma unroll
         for (int k = 0; k < 8; ++k)
           tc_mma(tmem, tc_sdesc(sbase + OFF_G + (k >> 2) * ATOM + 32 * (k & 3)),
-                 tc_sdesc(sbase + tc::OFF_W2 + (k >> 2) * W2_ATOM + 32 * (k & 3)), idesc(ROWS, OUTP), k > 0);
+                 tc_sdesc(sbase + tc::OFF_W2 + (k >> 2) * W2_ATOM + 32 * (k & 3)), tc_idesc(ROWS, OUTP), k > 0);
         tc_commit(mma_done);
       }
       pending = true;
