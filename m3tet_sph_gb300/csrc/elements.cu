@@ -759,6 +759,7 @@ int level_inverse_diag(Level &L, const float *K, cudaStream_t s) {
 constexpr int GR_T = 64;
 __global__ void __launch_bounds__(GR_T) k_grad_elem(const double *__restrict__ G, const int *__restrict__ el2nod, int nel,
                                                     const double *__restrict__ q, double *__restrict__ ye) {
+  grid_dep();
   __shared__ double sy[GR_T * 31];
   const int e0 = blockIdx.x * GR_T, e = e0 + threadIdx.x;
   if (e < nel) {
@@ -781,6 +782,7 @@ __global__ void __launch_bounds__(GR_T) k_grad_elem(const double *__restrict__ G
 // element outputs of G' z: 4 consecutive values per element
 __global__ void __launch_bounds__(128) k_div_elem(const double *__restrict__ G, const int *__restrict__ el2nod, int nel,
                                                   const double *__restrict__ z, double *__restrict__ se) {
+  grid_dep();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= nel) return;
   double v[4] = {0.0, 0.0, 0.0, 0.0};
@@ -802,6 +804,7 @@ __global__ void __launch_bounds__(128) k_div_elem(const double *__restrict__ G, 
 __global__ void __launch_bounds__(128) k_mass_elem(const double *__restrict__ M, const int *__restrict__ el2nod, int nel,
                                                    const double *__restrict__ r, const double *__restrict__ w,
                                                    double *__restrict__ se) {
+  grid_dep();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= nel) return;
   double de[4], ye[4] = {0, 0, 0, 0};
@@ -836,6 +839,7 @@ __device__ __forceinline__ double vertex_sum(const int *__restrict__ ptr, const 
 }
 __global__ void k_vertex_gather(const int *__restrict__ ptr, const int *__restrict__ idx, int nv,
                                 const double *__restrict__ se, double scale, double *__restrict__ out) {
+  grid_dep();
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v < nv) out[v] = scale * vertex_sum(ptr, idx, v, se);
 }
@@ -843,6 +847,7 @@ __global__ void k_vertex_gather(const int *__restrict__ ptr, const int *__restri
 __global__ void k_vertex_precond(const int *__restrict__ ptr, const int *__restrict__ idx, int nv,
                                  const double *__restrict__ se, const double *__restrict__ r,
                                  const double *__restrict__ w, double *__restrict__ d) {
+  grid_dep();
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= nv) return;
   const double rv = r[v], wv = w[v];
@@ -853,6 +858,7 @@ __global__ void k_vertex_precond(const int *__restrict__ ptr, const int *__restr
 __global__ void k_node_gather_rhs(const int *__restrict__ ptr, const int *__restrict__ idx, int nnod,
                                   const double *__restrict__ ye, const uint8_t *__restrict__ mask,
                                   const double *__restrict__ Fb, const double *__restrict__ bc, double *__restrict__ y) {
+  grid_dep();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= nnod) return;
   double t[3] = {0.0, 0.0, 0.0};
@@ -871,35 +877,40 @@ __global__ void k_node_gather_rhs(const int *__restrict__ ptr, const int *__rest
 // y = G q; with a mask: on free dofs only; with Fb, bc: y = Fb + G q - bc on free dofs
 int grad_apply(const Level &L, const double *G, const double *q, const uint8_t *mask, const double *Fb, const double *bc,
                double *y, cudaStream_t s) {
-  k_grad_elem<<<(L.nel + GR_T - 1) / GR_T, GR_T, 0, s>>>(G, L.el2nod, L.nel, q, L.ye64); count_launch();
-  k_node_gather_rhs<<<(L.nnod + 127) / 128, 128, 0, s>>>(L.g_ptr, L.g_idx, L.nnod, L.ye64, mask, Fb, bc, y); count_launch();
+  launch_pdl(k_grad_elem, (L.nel + GR_T - 1) / GR_T, GR_T, 0, s, G, L.el2nod, L.nel, q, L.ye64); count_launch();
+  launch_pdl(k_node_gather_rhs, (L.nnod + 127) / 128, 128, 0, s, L.g_ptr, L.g_idx, L.nnod, L.ye64, mask, Fb, bc,
+             y); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
 // out = scale G' z
 int div_apply(const Level &L, const double *G, const double *z, double scale, double *out, cudaStream_t s) {
-  k_div_elem<<<(L.nel + 127) / 128, 128, 0, s>>>(G, L.el2nod, L.nel, z, L.ye64); count_launch();
-  k_vertex_gather<<<(L.nvnod + 127) / 128, 128, 0, s>>>(L.g_ptr, L.g_idx, L.nvnod, L.ye64, scale, out); count_launch();
+  launch_pdl(k_div_elem, (L.nel + 127) / 128, 128, 0, s, G, L.el2nod, L.nel, z, L.ye64); count_launch();
+  launch_pdl(k_vertex_gather, (L.nvnod + 127) / 128, 128, 0, s, L.g_ptr, L.g_idx, L.nvnod, L.ye64, scale,
+             out); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
 // row sums of the pressure mass matrix
 int mass_lump(const Level &L, const double *M, double *out, cudaStream_t s) {
-  k_mass_elem<<<(L.nel + 127) / 128, 128, 0, s>>>(M, L.el2nod, L.nel, nullptr, nullptr, L.ye64); count_launch();
-  k_vertex_gather<<<(L.nvnod + 127) / 128, 128, 0, s>>>(L.g_ptr, L.g_idx, L.nvnod, L.ye64, 1.0, out); count_launch();
+  launch_pdl(k_mass_elem, (L.nel + 127) / 128, 128, 0, s, M, L.el2nod, L.nel, nullptr, nullptr, L.ye64); count_launch();
+  launch_pdl(k_vertex_gather, (L.nvnod + 127) / 128, 128, 0, s, L.g_ptr, L.g_idx, L.nvnod, L.ye64, 1.0,
+             out); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
 // d = w r + w (r - M (w r)) with w the inverse lumped mass
 int mass_precondition(const Level &L, const double *M, const double *r, const double *w, double *d, cudaStream_t s) {
-  k_mass_elem<<<(L.nel + 127) / 128, 128, 0, s>>>(M, L.el2nod, L.nel, r, w, L.ye64); count_launch();
-  k_vertex_precond<<<(L.nvnod + 127) / 128, 128, 0, s>>>(L.g_ptr, L.g_idx, L.nvnod, L.ye64, r, w, d); count_launch();
+  launch_pdl(k_mass_elem, (L.nel + 127) / 128, 128, 0, s, M, L.el2nod, L.nel, r, w, L.ye64); count_launch();
+  launch_pdl(k_vertex_precond, (L.nvnod + 127) / 128, 128, 0, s, L.g_ptr, L.g_idx, L.nvnod, L.ye64, r, w,
+             d); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
 // node sums of element vectors V [nel][30]
 int gather_elvec(const Level &L, const double *V, double *out, cudaStream_t s) {
-  k_node_gather_rhs<<<(L.nnod + 127) / 128, 128, 0, s>>>(L.g_ptr, L.g_idx, L.nnod, V, nullptr, nullptr, nullptr, out);
+  launch_pdl(k_node_gather_rhs, (L.nnod + 127) / 128, 128, 0, s, L.g_ptr, L.g_idx, L.nnod, V, nullptr, nullptr,
+             nullptr, out);
   count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
@@ -1037,15 +1048,31 @@ __global__ void __launch_bounds__(256) k_bsr_spmv(const int *__restrict__ ptr, c
                                                   const T *__restrict__ r, const T *__restrict__ Di) {
   const int i = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
-  if (i >= nrow) return;
+  // the lane's first block is fetched before the operand is ready
+  const bool row = i < nrow;
+  int k = row ? ptr[i] + lane : 0;
+  const int ke = row ? ptr[i + 1] : 0;
+  int j = 0;
+  T b[9] = {};
+  if (k < ke) {
+    j = col[k];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) b[q] = B[q * nnzb + k];
+  }
+  grid_dep();
+  if (!row) return;
   T s0 = 0, s1 = 0, s2 = 0;
-  const int kb = ptr[i], ke = ptr[i + 1];
-  for (int k = kb + lane; k < ke; k += 32) {
-    const int j = col[k];
+  while (k < ke) {
     const T x0 = x[3 * j], x1 = x[3 * j + 1], x2 = x[3 * j + 2];
-    s0 += B[k] * x0 + B[nnzb + k] * x1 + B[2 * nnzb + k] * x2;
-    s1 += B[3 * nnzb + k] * x0 + B[4 * nnzb + k] * x1 + B[5 * nnzb + k] * x2;
-    s2 += B[6 * nnzb + k] * x0 + B[7 * nnzb + k] * x1 + B[8 * nnzb + k] * x2;
+    s0 += b[0] * x0 + b[1] * x1 + b[2] * x2;
+    s1 += b[3] * x0 + b[4] * x1 + b[5] * x2;
+    s2 += b[6] * x0 + b[7] * x1 + b[8] * x2;
+    k += 32;
+    if (k < ke) {
+      j = col[k];
+#pragma unroll
+      for (int q = 0; q < 9; ++q) b[q] = B[q * nnzb + k];
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -1069,8 +1096,8 @@ int bsr_assemble(const Level &L, const T *K, T *B, cudaStream_t s) {
 }
 template <typename T>
 int bsr_apply(const Level &L, const T *B, const T *x, T *y, cudaStream_t s) {
-  k_bsr_spmv<T, false><<<(unsigned)(((size_t)L.nnod * 32 + 255) / 256), 256, 0, s>>>(
-      L.bsr_ptr, L.bsr_col, B, L.nnod, (size_t)L.nnzb, x, y, T(0), nullptr, nullptr);
+  launch_pdl(k_bsr_spmv<T, false>, (unsigned)(((size_t)L.nnod * 32 + 255) / 256), 256, 0, s, L.bsr_ptr, L.bsr_col, B,
+             L.nnod, (size_t)L.nnzb, x, y, T(0), nullptr, nullptr);
   count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
@@ -1078,7 +1105,8 @@ int bsr_apply(const Level &L, const T *B, const T *x, T *y, cudaStream_t s) {
 // y = x + w (r - B x) Di
 template <typename T>
 int bsr_apply_jac(const Level &L, const T *B, T w, const T *r, const T *Di, const T *x, T *y, cudaStream_t s) {
-  k_bsr_spmv<T, true><<<(unsigned)(((size_t)L.nnod * 32 + 255) / 256), 256, 0, s>>>(L.bsr_ptr, L.bsr_col, B, L.nnod,
+  launch_pdl(k_bsr_spmv<T, true>, (unsigned)(((size_t)L.nnod * 32 + 255) / 256), 256, 0, s, L.bsr_ptr, L.bsr_col, B,
+             L.nnod,
                                                                                    (size_t)L.nnzb, x, y, w, r, Di);
   count_launch();
   M3_CUDA(cudaGetLastError());

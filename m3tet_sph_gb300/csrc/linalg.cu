@@ -16,6 +16,7 @@ unsigned red_blocks(size_t n) {
 // out[0] = a.b
 __global__ void k_dot(const double *__restrict__ a, const double *__restrict__ b, size_t n, double *partials,
                       unsigned *cnt, double *out) {
+  grid_dep();
   double v[1] = {0.0};
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     v[0] += a[i] * b[i];
@@ -25,6 +26,7 @@ __global__ void k_dot(const double *__restrict__ a, const double *__restrict__ b
 template <typename T>
 __global__ void k_dot2(const double *__restrict__ a, const double *__restrict__ c, const T *__restrict__ b, size_t n,
                        double *partials, unsigned *cnt, double *out) {
+  grid_dep();
   double v[2] = {0.0, 0.0};
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const double bi = (double)b[i];
@@ -38,26 +40,27 @@ __global__ void k_dot2(const double *__restrict__ a, const double *__restrict__ 
 }
 // out[0] = sum(a)
 __global__ void k_sum(const double *__restrict__ a, size_t n, double *partials, unsigned *cnt, double *out) {
+  grid_dep();
   double v[1] = {0.0};
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) v[0] += a[i];
   if (block_reduce_last<1>(v, partials, cnt) && threadIdx.x == 0) out[0] = v[0];
 }
 
 int dot(const double *a, const double *b, size_t n, double *partials, unsigned *cnt, double *out, cudaStream_t s) {
-  k_dot<<<red_blocks(n), RED_THREADS, 0, s>>>(a, b, n, partials, cnt, out); count_launch();
+  launch_pdl(k_dot, red_blocks(n), RED_THREADS, 0, s, a, b, n, partials, cnt, out); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
 template <typename T>
 int dot2(const double *a, const double *c, const T *b, size_t n, double *partials, unsigned *cnt, double *out, cudaStream_t s) {
-  k_dot2<T><<<red_blocks(n), RED_THREADS, 0, s>>>(a, c, b, n, partials, cnt, out); count_launch();
+  launch_pdl(k_dot2<T>, red_blocks(n), RED_THREADS, 0, s, a, c, b, n, partials, cnt, out); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
 template int dot2<double>(const double *, const double *, const double *, size_t, double *, unsigned *, double *, cudaStream_t);
 template int dot2<float>(const double *, const double *, const float *, size_t, double *, unsigned *, double *, cudaStream_t);
 int vsum(const double *a, size_t n, double *partials, unsigned *cnt, double *out, cudaStream_t s) {
-  k_sum<<<red_blocks(n), RED_THREADS, 0, s>>>(a, n, partials, cnt, out); count_launch();
+  launch_pdl(k_sum, red_blocks(n), RED_THREADS, 0, s, a, n, partials, cnt, out); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
@@ -72,6 +75,7 @@ int vsum(const double *a, size_t n, double *partials, unsigned *cnt, double *out
 // q = d + beta q, beta = -alpha_prev * (Kq_prev . d) / rdlast (Polak-Ribiere: (r - rlast).d / rdlast)
 template <typename T>
 __global__ void k_cg_dir(const T *__restrict__ d, double *__restrict__ q, size_t n, const double *scal) {
+  grid_dep();
   const bool first = scal[6] != 0.0;
   double beta = 0.0;
   if (!first) beta = -scal[5] * scal[1] / scal[4];
@@ -82,6 +86,7 @@ __global__ void k_cg_dir(const T *__restrict__ d, double *__restrict__ q, size_t
 __global__ void k_cg_update(double *__restrict__ x, double *__restrict__ r, const double *__restrict__ q,
                             const double *__restrict__ Kq, float *__restrict__ r32, size_t n, double *scal,
                             double *partials, unsigned *cnt) {
+  grid_dep();
   const double rd = scal[0], alpha = rd / scal[2];
   double v[1] = {0.0};
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -101,7 +106,7 @@ __global__ void k_cg_update(double *__restrict__ x, double *__restrict__ r, cons
 
 template <typename T>
 int cg_dir(const T *d, double *q, size_t n, const double *scal, cudaStream_t s) {
-  k_cg_dir<T><<<red_blocks(n), RED_THREADS, 0, s>>>(d, q, n, scal); count_launch();
+  launch_pdl(k_cg_dir<T>, red_blocks(n), RED_THREADS, 0, s, d, q, n, scal); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
@@ -109,7 +114,7 @@ template int cg_dir<double>(const double *, double *, size_t, const double *, cu
 template int cg_dir<float>(const float *, double *, size_t, const double *, cudaStream_t);
 int cg_update(double *x, double *r, const double *q, const double *Kq, float *r32, size_t n, double *scal,
               double *partials, unsigned *cnt, cudaStream_t s) {
-  k_cg_update<<<red_blocks(n), RED_THREADS, 0, s>>>(x, r, q, Kq, r32, n, scal, partials, cnt); count_launch();
+  launch_pdl(k_cg_update, red_blocks(n), RED_THREADS, 0, s, x, r, q, Kq, r32, n, scal, partials, cnt); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
@@ -118,17 +123,19 @@ int cg_update(double *x, double *r, const double *q, const double *Kq, float *r3
 // generic elementwise kernels
 // ---------------------------------------------------------------------------------------
 __global__ void k_axpby(double a, const double *__restrict__ x, double b, double *__restrict__ y, size_t n) {
+  grid_dep();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     y[i] = a * x[i] + b * y[i];
 }
 int axpby(double a, const double *x, double b, double *y, size_t n, cudaStream_t s) {
-  k_axpby<<<RED_BLOCKS, RED_THREADS, 0, s>>>(a, x, b, y, n); count_launch();
+  launch_pdl(k_axpby, RED_BLOCKS, RED_THREADS, 0, s, a, x, b, y, n); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
 // y = (b - y) masked: residual r = b - Kx on free dofs, its FP32 copy and out[0] = r.r
 __global__ void k_residual(const double *__restrict__ b, double *__restrict__ y, const uint8_t *__restrict__ mask,
                            float *__restrict__ y32, size_t n, double *partials, unsigned *cnt, double *out) {
+  grid_dep();
   double v[1] = {0.0};
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const double r = mask[i] ? b[i] - y[i] : 0.0;
@@ -140,7 +147,7 @@ __global__ void k_residual(const double *__restrict__ b, double *__restrict__ y,
 }
 int residual(const double *b, double *y, const uint8_t *mask, float *y32, size_t n, double *partials, unsigned *cnt,
              double *out, cudaStream_t s) {
-  k_residual<<<red_blocks(n), RED_THREADS, 0, s>>>(b, y, mask, y32, n, partials, cnt, out); count_launch();
+  launch_pdl(k_residual, red_blocks(n), RED_THREADS, 0, s, b, y, mask, y32, n, partials, cnt, out); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
@@ -175,6 +182,7 @@ int f2d(const float *a, double *b, size_t n, cudaStream_t s) {
 // first down sweep: d = w * r0 * Dinv
 template <typename T>
 __global__ void k_jac_first(T w, const T *__restrict__ r0, const T *__restrict__ Di, T *__restrict__ d, size_t n) {
+  grid_dep();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     d[i] = w * r0[i] * Di[i];
 }
@@ -182,18 +190,19 @@ __global__ void k_jac_first(T w, const T *__restrict__ r0, const T *__restrict__
 template <typename T>
 __global__ void k_jac(T w, const T *__restrict__ r0, const T *__restrict__ Kd, const T *__restrict__ Di,
                       T *__restrict__ d, size_t n) {
+  grid_dep();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     d[i] += w * (r0[i] - Kd[i]) * Di[i];
 }
 template <typename T>
 int jac_first(T w, const T *r0, const T *Di, T *d, size_t n, cudaStream_t s) {
-  k_jac_first<T><<<RED_BLOCKS, RED_THREADS, 0, s>>>(w, r0, Di, d, n); count_launch();
+  launch_pdl(k_jac_first<T>, RED_BLOCKS, RED_THREADS, 0, s, w, r0, Di, d, n); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
 template <typename T>
 int jac(T w, const T *r0, const T *Kd, const T *Di, T *d, size_t n, cudaStream_t s) {
-  k_jac<T><<<RED_BLOCKS, RED_THREADS, 0, s>>>(w, r0, Kd, Di, d, n); count_launch();
+  launch_pdl(k_jac<T>, RED_BLOCKS, RED_THREADS, 0, s, w, r0, Kd, Di, d, n); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
@@ -218,11 +227,18 @@ __global__ void __launch_bounds__(256) k_restrict(const int *__restrict__ ptr, c
                                                   const int *__restrict__ cmap, T *__restrict__ xfree) {
   const int i = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
-  if (i >= nrow) return;
+  const bool row = i < nrow;
+  const int kb = row ? ptr[i] + lane : 0, ke = row ? ptr[i + 1] : 0;
+  int j = kb < ke ? col[kb] : 0;
+  T wk = kb < ke ? (T)w[kb] : T(0);
+  grid_dep();
+  if (!row) return;
   T s0 = 0, s1 = 0, s2 = 0;
-  for (int k = ptr[i] + lane; k < ptr[i + 1]; k += 32) {
-    const int j = col[k];
-    const T wk = (T)w[k];
+  for (int k = kb; k < ke; k += 32) {
+    if (k != kb) {
+      j = col[k];
+      wk = (T)w[k];
+    }
     if (b) {
       s0 += wk * (a[3 * j] - b[3 * j]);
       s1 += wk * (a[3 * j + 1] - b[3 * j + 1]);
@@ -255,6 +271,7 @@ template <typename T>
 __global__ void k_prolong(const int *__restrict__ ptr, const int *__restrict__ col, const float *__restrict__ w,
                           int nrow, const T *__restrict__ xc, const T *add, const uint8_t *__restrict__ mask, T *out,
                           PaCart pc) {
+  grid_dep();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nrow) return;
   T t[3] = {0, 0, 0};
@@ -275,7 +292,8 @@ __global__ void k_prolong(const int *__restrict__ ptr, const int *__restrict__ c
 template <typename T>
 int restrict_(const Level &F, const Level &C, const T *a, const T *b, T *out, cudaStream_t s, T wj, const T *Di, T *d,
               const int *cmap, T *xfree) {
-  k_restrict<T><<<(unsigned)(((size_t)C.nnod * 32 + 255) / 256), 256, 0, s>>>(F.R_ptr, F.R_col, F.R_w, C.nnod, a, b,
+  launch_pdl(k_restrict<T>, (unsigned)(((size_t)C.nnod * 32 + 255) / 256), 256, 0, s, F.R_ptr, F.R_col, F.R_w, C.nnod,
+             a, b,
                                                                              C.freemask, out, wj, Di, d, cmap, xfree);
   count_launch();
   M3_CUDA(cudaGetLastError());
@@ -283,7 +301,8 @@ int restrict_(const Level &F, const Level &C, const T *a, const T *b, T *out, cu
 }
 template <typename T>
 int prolong(const Level &F, const Level &C, const T *xc, const T *add, T *out, const PaCart &pc, cudaStream_t s) {
-  k_prolong<T><<<(F.nnod + 255) / 256, 256, 0, s>>>(F.P_ptr, F.P_col, F.P_w, F.nnod, xc, add, F.freemask, out, pc);
+  launch_pdl(k_prolong<T>, (F.nnod + 255) / 256, 256, 0, s, F.P_ptr, F.P_col, F.P_w, F.nnod, xc, add, F.freemask, out,
+             pc);
   count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
@@ -991,6 +1010,7 @@ template int dense_inverse_blocked<float>(const Level &, const float *, float *,
 template <typename T, typename X>
 __global__ void __launch_bounds__(256) k_dense_gemv(const T *__restrict__ A, int ld, int n, const int *__restrict__ cmap,
                                                     const X *__restrict__ x, X *__restrict__ y, int accumulate) {
+  grid_dep();
   const int i = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (i >= n) return;
@@ -1028,11 +1048,11 @@ int coarse_refined(const Level &L, const float *A32, const double *B64, const do
                    int sweeps, const int *cmap, double *xfree, int nf, cudaStream_t s) {
   const int n = L.ndof, ld = dense_ld(nf);
   const unsigned g = (unsigned)((n + 7) / 8);
-  k_dense_gemv<float, double><<<g, 256, 0, s>>>(A32, ld, n, cmap, xfree, d, 0); count_launch();
+  launch_pdl(k_dense_gemv<float, double>, g, 256, 0, s, A32, ld, n, cmap, xfree, d, 0); count_launch();
   for (int k = 0; k < sweeps; ++k) {
     M3_TRY(bsr_apply<double>(L, B64, d, t, s));
     k_sub_compact<<<(n + 255) / 256, 256, 0, s>>>(r, t, cmap, xfree, n); count_launch();
-    k_dense_gemv<float, double><<<g, 256, 0, s>>>(A32, ld, n, cmap, xfree, d, 1); count_launch();
+    launch_pdl(k_dense_gemv<float, double>, g, 256, 0, s, A32, ld, n, cmap, xfree, d, 1); count_launch();
   }
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
@@ -1053,7 +1073,7 @@ int dense_inverse_from64(const Level &L, const double *B64, float *B32tmp, float
 // d = A^-1 r on the free dofs (r compact in xfree), 0 on the fixed ones
 template <typename T>
 int dense_gemv(const T *A, int n, int nf, const int *cmap, const T *xfree, T *y, cudaStream_t s) {
-  k_dense_gemv<T, T><<<(n + 7) / 8, 256, 0, s>>>(A, dense_ld(nf), n, cmap, xfree, y, 0);
+  launch_pdl(k_dense_gemv<T, T>, (n + 7) / 8, 256, 0, s, A, dense_ld(nf), n, cmap, xfree, y, 0);
   count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;

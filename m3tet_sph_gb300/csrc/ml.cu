@@ -321,6 +321,7 @@ __global__ void k_ml_feature_rows(FeatLevel L, const float *__restrict__ z,
 template <typename T>
 __global__ void k_ml_scale(const T *__restrict__ r0, const T *__restrict__ kd, const T *__restrict__ Dinv,
                            float *__restrict__ z, size_t n) {
+  grid_dep();
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const T rv = kd ? (T)(r0[i] - kd[i]) : r0[i];
@@ -383,6 +384,7 @@ __global__ void __launch_bounds__(tc::THREADS, 2) k_ml_sweep_tc(FeatLevel L, Mlp
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_dep();                          // the kernel before this one writes z, not the weights
   const uint32_t tmem = *tslot;
   const int ntile = (L.nel + ROWS - 1) / ROWS;
 
@@ -508,6 +510,7 @@ __global__ void __launch_bounds__(128) k_ml_gather_rows(int nnod, int nv, const 
                                                         const int *__restrict__ code, const float *__restrict__ C,
                                                         const uint8_t *__restrict__ mask, float omega,
                                                         T *__restrict__ d, PaCart pc) {
+  grid_dep();
   const int t = blockIdx.x * 128 + threadIdx.x, nt4 = gather_threads4(nv);
   const bool quad = t < nt4;
   const int n = quad ? t >> 2 : nv + t - nt4, sub = quad ? t & 3 : 0, step = quad ? 4 : 1;
@@ -949,9 +952,12 @@ int ml_sweep(m3sph_mesh *M, int j, const T *r0, const T *kd, const T *Dinv, T *t
   if (g_ml_infer == 1) {
     const int ntile = (L.nel + tc::ROWS - 1) / tc::ROWS;
     const int grid = std::min(ntile, 2 * g_nsm);
-    k_ml_scale<T><<<(unsigned)((L.ndof + 255) / 256), 256, 0, s>>>(r0, kd, Dinv, S->lev[j].z, L.ndof); count_launch();
-    k_ml_sweep_tc<<<grid, tc::THREADS, tc::SMEM_ALLOC, s>>>(f, w, S->lev[j].z, S->lev[j].C, S->err); count_launch();
-    k_ml_gather_rows<T><<<(gather_threads4(L.nvnod) + L.nnod - L.nvnod + 127) / 128, 128, 0, s>>>(L.nnod, L.nvnod, S->lev[j].n2e_ptr, S->lev[j].n2e_code,
+    launch_pdl(k_ml_scale<T>, (unsigned)((L.ndof + 255) / 256), 256, 0, s, r0, kd, Dinv, S->lev[j].z,
+               L.ndof); count_launch();
+    launch_pdl(k_ml_sweep_tc, grid, tc::THREADS, tc::SMEM_ALLOC, s, f, w, S->lev[j].z, S->lev[j].C,
+               S->err); count_launch();
+    launch_pdl(k_ml_gather_rows<T>, (gather_threads4(L.nvnod) + L.nnod - L.nvnod + 127) / 128, 128, 0, s, L.nnod,
+               L.nvnod, S->lev[j].n2e_ptr, S->lev[j].n2e_code,
                                                               S->lev[j].C, L.freemask, M->ml_omega, d, pc); count_launch();
     M3_CUDA(cudaGetLastError());
     return M3SPH_OK;

@@ -256,6 +256,7 @@ k_pa_tile(const float *__restrict__ pa, const int *__restrict__ el2nod, int nel,
                    : "memory");
     for (int i = lane; i < ns; i += 32)
       asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(pa_smem_u32(s_slot + i)), "l"(slot + s0 + i) : "memory");
+    grid_dep();                        // factors, connectivity and tables are constants, the operand is not
     uint64_t v[10][3];
 #pragma unroll
     for (int n = 0; n < 10; ++n) {
@@ -403,6 +404,7 @@ __device__ __forceinline__ void pa_node_sum(const int *__restrict__ nptr, const 
 }
 __global__ void k_pa_cart(int nnod, const float4 *__restrict__ trig, const uint8_t *__restrict__ mask,
                           const float *__restrict__ x, float4 *__restrict__ xc) {
+  grid_dep();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= nnod) return;
   const size_t i = 3 * (size_t)n;
@@ -411,6 +413,7 @@ __global__ void k_pa_cart(int nnod, const float4 *__restrict__ trig, const uint8
 __global__ void k_pa_gather(int nnod, const int *__restrict__ nptr, const float4 *__restrict__ yb,
                             const float4 *__restrict__ trig,
                             const uint8_t *__restrict__ mask, float *__restrict__ y) {
+  grid_dep();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= nnod) return;
   float v[3];
@@ -423,6 +426,7 @@ __global__ void k_pa_gather_jac(int nnod, const int *__restrict__ nptr, const fl
                                 const float4 *__restrict__ trig,
                                 const uint8_t *__restrict__ mask, float w, const float *__restrict__ r,
                                 const float *__restrict__ Di, float *__restrict__ d, float4 *__restrict__ xc) {
+  grid_dep();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= nnod) return;
   const float4 tr = trig[n];
@@ -441,6 +445,7 @@ __global__ void k_pa_gather_jac(int nnod, const int *__restrict__ nptr, const fl
 __global__ void k_pa_jac_first(int nnod, const float4 *__restrict__ trig, const uint8_t *__restrict__ mask, float w,
                                const float *__restrict__ r, const float *__restrict__ Di, float *__restrict__ d,
                                float4 *__restrict__ xc) {
+  grid_dep();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= nnod) return;
   float dn[3];
@@ -455,7 +460,8 @@ __global__ void k_pa_jac_first(int nnod, const float4 *__restrict__ trig, const 
 }
 
 static void pa_tiles(const Level &L, cudaStream_t s) {
-  k_pa_tile<<<(L.nel + PA_E - 1) / PA_E, 32, 0, s>>>(L.pa32, L.el2nod, L.nel, L.pa_xc, L.pa_tptr, L.pa_slot, L.pa_ent,
+  launch_pdl(k_pa_tile, (L.nel + PA_E - 1) / PA_E, 32, 0, s, L.pa32, L.el2nod, L.nel, L.pa_xc, L.pa_tptr, L.pa_slot,
+             L.pa_ent,
                                                        L.pa_yb, L.sa_err);
   count_launch();
 }
@@ -463,7 +469,7 @@ constexpr int PA_NT = 128;                           // node passes: threads per
 static unsigned pa_ngrid(const Level &L) { return (unsigned)((L.nnod + PA_NT - 1) / PA_NT); }
 
 int pa_jac_first_f32(const Level &L, float w, const float *r, const float *Di, float *d, cudaStream_t s) {
-  k_pa_jac_first<<<pa_ngrid(L), PA_NT, 0, s>>>(L.nnod, L.pa_trig, L.freemask, w, r, Di, d, L.pa_xc);
+  launch_pdl(k_pa_jac_first, pa_ngrid(L), PA_NT, 0, s, L.nnod, L.pa_trig, L.freemask, w, r, Di, d, L.pa_xc);
   count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
@@ -472,11 +478,11 @@ int pa_jac_first_f32(const Level &L, float w, const float *r, const float *Di, f
 // y = K x; have_cart: xc already holds x (written by the pass that made x)
 int pa_apply_f32(const Level &L, const float *x, float *y, bool have_cart, cudaStream_t s) {
   if (!have_cart) {
-    k_pa_cart<<<pa_ngrid(L), PA_NT, 0, s>>>(L.nnod, L.pa_trig, L.freemask, x, L.pa_xc);
+    launch_pdl(k_pa_cart, pa_ngrid(L), PA_NT, 0, s, L.nnod, L.pa_trig, L.freemask, x, L.pa_xc);
     count_launch();
   }
   pa_tiles(L, s);
-  k_pa_gather<<<pa_ngrid(L), PA_NT, 0, s>>>(L.nnod, L.pa_nptr, L.pa_yb, L.pa_trig, L.freemask, y);
+  launch_pdl(k_pa_gather, pa_ngrid(L), PA_NT, 0, s, L.nnod, L.pa_nptr, L.pa_yb, L.pa_trig, L.freemask, y);
   count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
@@ -485,11 +491,11 @@ int pa_apply_f32(const Level &L, const float *x, float *y, bool have_cart, cudaS
 // d += w (r - K d) / diag (one weighted Jacobi sweep); leaves the new d in xc
 int pa_apply_jac_f32(const Level &L, float w, const float *r, const float *Di, float *d, bool have_cart, cudaStream_t s) {
   if (!have_cart) {
-    k_pa_cart<<<pa_ngrid(L), PA_NT, 0, s>>>(L.nnod, L.pa_trig, L.freemask, d, L.pa_xc);
+    launch_pdl(k_pa_cart, pa_ngrid(L), PA_NT, 0, s, L.nnod, L.pa_trig, L.freemask, d, L.pa_xc);
     count_launch();
   }
   pa_tiles(L, s);
-  k_pa_gather_jac<<<pa_ngrid(L), PA_NT, 0, s>>>(L.nnod, L.pa_nptr, L.pa_yb, L.pa_trig, L.freemask, w, r, Di, d,
+  launch_pdl(k_pa_gather_jac, pa_ngrid(L), PA_NT, 0, s, L.nnod, L.pa_nptr, L.pa_yb, L.pa_trig, L.freemask, w, r, Di, d,
                                                 L.pa_xc);
   count_launch();
   M3_CUDA(cudaGetLastError());

@@ -1320,6 +1320,7 @@ static int pdot(m3sph_mesh *M, const double *a, const double *b, double &v) {
   return read_scal(M, 8, v);
 }
 __global__ void k_shift(double *a, double c, int n) {
+  grid_dep();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) a[i] += c;
 }
@@ -1357,7 +1358,7 @@ static int remove_mean(m3sph_mesh *M, double *a) {
   M3_TRY(vsum(a, np, M->red, M->red_cnt, M->scal + 9, M->stream));
   double sm;
   M3_TRY(read_scal(M, 9, sm));
-  k_shift<<<(np + 255) / 256, 256, 0, M->stream>>>(a, -sm / np, np); count_launch();
+  launch_pdl(k_shift, (np + 255) / 256, 256, 0, M->stream, a, -sm / np, np); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }

@@ -333,7 +333,8 @@ __global__ void __launch_bounds__(sa::Lay<NCX, NGW>::THREADS, 1)
 
 // phase 2: y at node n = sum over the node's (element, local node) entries in element order
 __global__ void k_node_gather_f32(const int *__restrict__ ptr, const int *__restrict__ idx, int nnod,
-                                  const float *__restrict__ ye, float *__restrict__ y) {
+                                  const float *__restrict__ ye, float *__restrict__ y, int *ticket) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *ticket = 0;     // for the next product
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= nnod) return;
   float s0 = 0.f, s1 = 0.f, s2 = 0.f;
@@ -454,13 +455,16 @@ __global__ void __launch_bounds__(32 * (NCW * SPLIT + 1), 1)
     const uint64_t pol = evict_first_policy();
     int it = 0;
     bool ok = true;
+    // the first NST chunks of a CTA are fixed: their matrices and connectivity are on their way before the
+    // kernel that writes x has finished (it may also be the one that sets the ticket back)
     for (;; ++it) {
       const int s = it % NST;
+      if (it == NST) grid_dep();
       if (it >= NST && !mbar_wait(empty(s), ((it / NST) & 1) ^ 1)) {
         ok = false;
         break;
       }
-      const int t = atomicAdd(ticket, 1);
+      const int t = it < NST ? (int)(blockIdx.x + it * gridDim.x) : (int)(NST * gridDim.x) + atomicAdd(ticket, 1);
       if (t >= nchunk) break;
       const int e0 = t * E;
       hdr[s] = make_int4(e0, min(E, nel - e0), t, it);
@@ -490,6 +494,7 @@ __global__ void __launch_bounds__(32 * (NCW * SPLIT + 1), 1)
   }
 
   // ---------------- consumers: SPLIT warps per stage, each with E / SPLIT elements ----------------
+  grid_dep();
   constexpr int EW = E / SPLIT;
   constexpr int EGI = EG < EW ? EG : EW;   // elements interleaved per pass
   const int owner = warp / SPLIT, part = warp % SPLIT, eb = part * EW;
@@ -544,7 +549,8 @@ __global__ void __launch_bounds__(32 * (NCW * SPLIT + 1), 1)
 // d_n += w (r_n - (K d)_n) / diag_n follows in the same pass (d_n is read only by its own node)
 __global__ void k_node_gather_jac_f32(const int *__restrict__ ptr, const int *__restrict__ idx, int nnod,
                                       const float *__restrict__ ye, float w, const float *__restrict__ r,
-                                      const float *__restrict__ Di, float *__restrict__ d) {
+                                      const float *__restrict__ Di, float *__restrict__ d, int *ticket) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *ticket = 0;     // for the next product
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= nnod) return;
   float s0 = 0.f, s1 = 0.f, s2 = 0.f;
@@ -578,7 +584,10 @@ __global__ void __launch_bounds__(GT) k_node_gather_f64(const int *__restrict__ 
                                                         int nv, const double *__restrict__ ye, double *__restrict__ y,
                                                         const double *__restrict__ x, double w,
                                                         const double *__restrict__ r, const double *__restrict__ Di,
-                                                        double *partials, unsigned *cnt, double *out) {
+                                                        double *partials, unsigned *cnt, double *out,
+                                                        int *ticket) {
+  grid_dep();
+  if (blockIdx.x == 0 && threadIdx.x == 0) *ticket = 0;     // for the next product
   double v[1] = {0.0};
   const int nt4 = gather_threads4(nv), nt = nt4 + nnod - nv;
   // whole warps stay in the loop: the shuffles need all lanes of a vertex
@@ -760,10 +769,9 @@ int stream_apply_f32(const Level &L, const float *K, const float *x, float *y, c
   M3_TRY(stream_ready(L, K));
   CUtensorMap map;
   M3_TRY(encode_k32(L, K, &map));
-  M3_CUDA(cudaMemsetAsync(L.sa_err + 1, 0, sizeof(int), s));
   f32_phase1(L, map, x, s);
   count_launch();
-  k_node_gather_f32<<<(L.nnod + 255) / 256, 256, 0, s>>>(L.g_ptr, L.g_idx, L.nnod, L.ye32, y);
+  k_node_gather_f32<<<(L.nnod + 255) / 256, 256, 0, s>>>(L.g_ptr, L.g_idx, L.nnod, L.ye32, y, L.sa_err + 1);
   count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
@@ -810,8 +818,8 @@ static int rowlane_attrs() {
 
 template <class Op, int NCW, int SPLIT>
 static void rowlane_launch(const Level &L, const CUtensorMap &ma, const CUtensorMap &mb, const double *x, cudaStream_t s) {
-  k_stream_rowlane<Op, NCW, 2, SPLIT><<<L.sa_grid, 32 * (NCW * SPLIT + 1), sr::Map<NCW>::SMEM_ALLOC, s>>>(
-      ma, mb, L.chunk_conn8, L.nchunk8, L.nel, L.sa_err + 1, L.sa_err, x, L.ye64);
+  launch_pdl(k_stream_rowlane<Op, NCW, 2, SPLIT>, L.sa_grid, 32 * (NCW * SPLIT + 1), sr::Map<NCW>::SMEM_ALLOC, s, ma,
+             mb, L.chunk_conn8, L.nchunk8, L.nel, L.sa_err + 1, L.sa_err, x, L.ye64);
 }
 
 static unsigned gather_grid(const Level &L) {
@@ -821,7 +829,6 @@ static unsigned gather_grid(const Level &L) {
 // element outputs (phase 1)
 template <class Op>
 static int rowlane_elements(const Level &L, const CUtensorMap &ma, const CUtensorMap &mb, const double *x, cudaStream_t s) {
-  M3_CUDA(cudaMemsetAsync(L.sa_err + 1, 0, sizeof(int), s));
   if constexpr (std::is_same<Op, RlF64>::value) {
     rowlane_launch<RlF64, 6, 1>(L, ma, mb, x, s);
   } else {
@@ -844,11 +851,13 @@ static int rowlane_elements(const Level &L, const CUtensorMap &ma, const CUtenso
 static int rowlane_sums(const Level &L, double *y, const double *x, const Reduction *red, double *out, cudaStream_t s) {
   const unsigned g = gather_grid(L);
   if (red)
-    k_node_gather_f64<GATHER_DOT><<<std::min(g, 2048u), GT, 0, s>>>(   // one partial sum per block
-        L.g_ptr, L.g_idx, L.nnod, L.nvnod, L.ye64, y, x, 0.0, nullptr, nullptr, red->partials, red->cnt, out);
+    launch_pdl(k_node_gather_f64<GATHER_DOT>, std::min(g, 2048u), GT, 0, s, // one partial sum per block
+        L.g_ptr, L.g_idx, L.nnod, L.nvnod, L.ye64, y, x, 0.0, nullptr, nullptr, red->partials, red->cnt, out,
+        L.sa_err + 1);
   else
-    k_node_gather_f64<GATHER_Y><<<g, GT, 0, s>>>(L.g_ptr, L.g_idx, L.nnod, L.nvnod, L.ye64, y, nullptr, 0.0, nullptr,
-                                                 nullptr, nullptr, nullptr, nullptr);
+    launch_pdl(k_node_gather_f64<GATHER_Y>, g, GT, 0, s, L.g_ptr, L.g_idx, L.nnod, L.nvnod, L.ye64, y, nullptr, 0.0,
+               nullptr,
+               nullptr, nullptr, nullptr, nullptr, L.sa_err + 1);
   count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
@@ -860,10 +869,9 @@ int stream_apply_jac_f32(const Level &L, const float *K, float w, const float *r
   M3_TRY(stream_ready(L, K));
   CUtensorMap map;
   M3_TRY(encode_k32(L, K, &map));
-  M3_CUDA(cudaMemsetAsync(L.sa_err + 1, 0, sizeof(int), s));
   f32_phase1(L, map, d, s);
   count_launch();
-  k_node_gather_jac_f32<<<(L.nnod + 255) / 256, 256, 0, s>>>(L.g_ptr, L.g_idx, L.nnod, L.ye32, w, r, Di, d);
+  k_node_gather_jac_f32<<<(L.nnod + 255) / 256, 256, 0, s>>>(L.g_ptr, L.g_idx, L.nnod, L.ye32, w, r, Di, d, L.sa_err + 1);
   count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
@@ -898,8 +906,9 @@ int stream_apply_jac_f64(const Level &L, const double *K, double w, const double
   CUtensorMap ma;
   M3_TRY(encode_k(L, K, true, RlF64::ROWS, sr::E, &ma, true));
   M3_TRY(rowlane_elements<RlF64>(L, ma, ma, d, s));
-  k_node_gather_f64<GATHER_JAC><<<gather_grid(L), GT, 0, s>>>(L.g_ptr, L.g_idx, L.nnod, L.nvnod, L.ye64, d, nullptr, w, r, Di,
-                                                              nullptr, nullptr, nullptr);
+  launch_pdl(k_node_gather_f64<GATHER_JAC>, gather_grid(L), GT, 0, s, L.g_ptr, L.g_idx, L.nnod, L.nvnod, L.ye64, d,
+             nullptr, w, r, Di,
+             nullptr, nullptr, nullptr, L.sa_err + 1);
   count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
