@@ -240,6 +240,11 @@ struct Finest {
   int *err = nullptr;                 // device error flags
 };
 
+// state of a velocity solve's CG, at scal + CG_STATE: the host sets it, the step kernel ends the loop
+enum { CG_STATE = 24, CG_TOL = 24, CG_SQ, CG_PREV, CG_IT, CG_LIMIT, CG_LEARNED, CG_STATUS, CG_STATE_END };
+enum { CG_RUN = 0, CG_CONVERGED, CG_NAN, CG_STALLED, CG_LIMIT_REACHED };
+constexpr int CG_LOOP_MAX = 256;    // iterations of a captured loop before the host looks at it
+
 struct Coarse {
   int n = 0;                          // dofs of the coarsest level
   int nf = 0;                         // its free dofs: the dense inverse is nf rows of dense_ld(nf) values
@@ -344,13 +349,13 @@ struct m3sph_mesh {
   std::vector<void *> work;           // device buffers owned by the workspace
   void *wk = nullptr;                 // host-side workspace descriptor
   void (*wk_free)(void *) = nullptr;
-  std::vector<std::pair<double *, cudaGraphExec_t>> graphs;   // captured MG-PCG iterations
+  struct CgGraph { double *key; cudaGraphExec_t exec; unsigned long long kernels; };
+  std::vector<CgGraph> graphs;        // captured MG-PCG loops and their kernels per iteration
   bool use_graphs = true;
   bool df_outer = true;               // double-float outer operator on the mixed path
   bool split_apply = true;            // 4-warp split element-by-element kernels on the finest level
   int ml_schedule = 1;                // learned smoothing per side: 0 learned-Jacobi-learned, 1 one learned sweep
   float ml_omega = 1.0f;              // relaxation weight of the learned correction
-  unsigned long long graph_kernels = 0;   // kernel launches per captured iteration
   void *ml = nullptr;                 // learned smoother state
   void (*ml_free)(void *) = nullptr;
   int smoother = 0;                   // 0 Jacobi, 1 learned smoother on the two finest levels

@@ -82,10 +82,13 @@ __global__ void k_cg_dir(const T *__restrict__ d, double *__restrict__ q, size_t
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     q[i] = first ? (double)d[i] : (double)d[i] + beta * q[i];
 }
-// alpha = rd / qKq ; x += alpha q ; r -= alpha Kq (and its FP32 copy) ; rr, rdlast, alpha_prev, first = 0
+// alpha = rd / qKq ; x += alpha q ; r -= alpha Kq (and its FP32 copy) ; rr, rdlast, alpha_prev, first = 0.
+// Then whether the loop goes on: it ends when the residual is below the tolerance or NaN, at the iteration
+// limit, or, with the learned smoother, at a contraction factor above 0.95 (or growth). `loop` is the condition of
+// the captured loop around the iteration (0: the host runs it).
 __global__ void k_cg_update(double *__restrict__ x, double *__restrict__ r, const double *__restrict__ q,
                             const double *__restrict__ Kq, float *__restrict__ r32, size_t n, double *scal,
-                            double *partials, unsigned *cnt) {
+                            double *partials, unsigned *cnt, cudaGraphConditionalHandle loop) {
   grid_dep();
   const double rd = scal[0], alpha = rd / scal[2];
   double v[1] = {0.0};
@@ -101,6 +104,16 @@ __global__ void k_cg_update(double *__restrict__ x, double *__restrict__ r, cons
     scal[4] = rd;
     scal[5] = alpha;
     scal[6] = 0.0;
+    const double rrms = sqrt(v[0]) / scal[CG_SQ], it = scal[CG_IT] + 1.0, prev = scal[CG_PREV];
+    const bool last = it >= scal[CG_LIMIT], stalled = it > 1.0 && rrms > 0.95 * prev;
+    const int status = isnan(rrms) ? CG_NAN
+                       : rrms < scal[CG_TOL] ? CG_CONVERGED
+                       : scal[CG_LEARNED] != 0.0 && (stalled || last) ? CG_STALLED
+                       : last ? CG_LIMIT_REACHED : CG_RUN;
+    scal[CG_PREV] = rrms;
+    scal[CG_IT] = it;
+    scal[CG_STATUS] = (double)status;
+    if (loop) cudaGraphSetConditional(loop, status == CG_RUN && (long long)it % CG_LOOP_MAX != 0);
   }
 }
 
@@ -113,8 +126,9 @@ int cg_dir(const T *d, double *q, size_t n, const double *scal, cudaStream_t s) 
 template int cg_dir<double>(const double *, double *, size_t, const double *, cudaStream_t);
 template int cg_dir<float>(const float *, double *, size_t, const double *, cudaStream_t);
 int cg_update(double *x, double *r, const double *q, const double *Kq, float *r32, size_t n, double *scal,
-              double *partials, unsigned *cnt, cudaStream_t s) {
-  launch_pdl(k_cg_update, red_blocks(n), RED_THREADS, 0, s, x, r, q, Kq, r32, n, scal, partials, cnt); count_launch();
+              double *partials, unsigned *cnt, cudaGraphConditionalHandle loop, cudaStream_t s) {
+  launch_pdl(k_cg_update, red_blocks(n), RED_THREADS, 0, s, x, r, q, Kq, r32, n, scal, partials, cnt, loop);
+  count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
