@@ -60,6 +60,24 @@ __device__ __forceinline__ void df_mac(float vh, float vl, float xh, float xl, f
   sl += err + e;
 }
 
+#ifdef __CUDACC__
+// Sums of three values over groups of W lanes (all lanes of a warp call it): the lanes that start quarter c of a
+// group get sum c. Two exchanges split the values over the quarters, so it takes 2 + 1 + log2(W / 4) additions
+// and not 3 log2(W).
+template <int W, typename T>
+__device__ __forceinline__ T lane_sum3(T s0, T s1, T s2) {
+  const int lane = threadIdx.x % W;
+  const bool h = lane & (W / 2), q = lane & (W / 4);
+  T a = (h ? s2 : s0) + __shfl_xor_sync(0xffffffffu, h ? s0 : s2, W / 2);
+  const T t = __shfl_xor_sync(0xffffffffu, h ? s1 : T(0), W / 2);
+  const T b = (h ? T(0) : s1) + t;
+  a = (q ? b : a) + __shfl_xor_sync(0xffffffffu, q ? a : b, W / 4);
+#pragma unroll
+  for (int o = W / 8; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  return a;
+}
+#endif
+
 // Block reduction whose last block finishes it: v[k] summed over the grid in a fixed order (threads of a
 // block by shuffles, then blocks in order), so the result does not depend on scheduling. `cnt` is 0 before
 // and after. Returns true in the last block, whose thread 0 holds the sums. Blocks of up to 256 threads.

@@ -1038,16 +1038,17 @@ __global__ void k_bsr_assemble(const T *__restrict__ K, int nel, int nnzb, const
   for (int q = 0; q < 9; ++q) B[(size_t)q * nnzb + k] = acc[q];   // [9][nnzb]
 }
 
-// y = B x for a 3x3-block CSR matrix with blocks stored [9][nnzb]: one warp per block row, lane l
-// takes blocks ptr[i] + l, ptr[i] + l + 32, ... (all loads of a warp coalesced), then a shuffle sum.
+// y = B x for a 3x3-block CSR matrix with blocks stored [9][nnzb]: LPR lanes per block row, lane l takes blocks
+// ptr[i] + l, ptr[i] + l + LPR, ... (neighbouring rows' blocks follow each other, so the loads stay whole
+// sectors), then a shuffle sum.
 // JAC: one weighted Jacobi sweep y = x + w (r - B x) Di (y another vector than x)
-template <typename T, bool JAC>
+template <typename T, bool JAC, int LPR>
 __global__ void __launch_bounds__(256) k_bsr_spmv(const int *__restrict__ ptr, const int *__restrict__ col,
                                                   const T *__restrict__ B, int nrow, size_t nnzb,
                                                   const T *__restrict__ x, T *__restrict__ y, T w,
                                                   const T *__restrict__ r, const T *__restrict__ Di) {
-  const int i = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
+  const int i = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) / LPR);
+  const int lane = threadIdx.x % LPR;
   // the lane's first block is fetched before the operand is ready
   const bool row = i < nrow;
   int k = row ? ptr[i] + lane : 0;
@@ -1060,32 +1061,36 @@ __global__ void __launch_bounds__(256) k_bsr_spmv(const int *__restrict__ ptr, c
     for (int q = 0; q < 9; ++q) b[q] = B[q * nnzb + k];
   }
   grid_dep();
-  if (!row) return;
   T s0 = 0, s1 = 0, s2 = 0;
   while (k < ke) {
     const T x0 = x[3 * j], x1 = x[3 * j + 1], x2 = x[3 * j + 2];
     s0 += b[0] * x0 + b[1] * x1 + b[2] * x2;
     s1 += b[3] * x0 + b[4] * x1 + b[5] * x2;
     s2 += b[6] * x0 + b[7] * x1 + b[8] * x2;
-    k += 32;
+    k += LPR;
     if (k < ke) {
       j = col[k];
 #pragma unroll
       for (int q = 0; q < 9; ++q) b[q] = B[q * nnzb + k];
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-  }
-  if (lane < 3) {
-    const size_t q = 3 * (size_t)i + lane;
-    const T v = lane == 0 ? s0 : lane == 1 ? s1 : s2;
+  const T v = lane_sum3<LPR>(s0, s1, s2);
+  if (row && lane % (LPR / 4) == 0 && lane < 3 * (LPR / 4)) {
+    const size_t q = 3 * (size_t)i + lane / (LPR / 4);
     if constexpr (JAC) y[q] = x[q] + w * (r[q] - v) * Di[q];
     else y[q] = v;
   }
+}
+// Lanes per row. While two warps' rounds of the chip (64 warps on each of 152 SMs) hold a warp per row, that is
+// quickest (latency); above, eight lanes (fewer additions and instructions per row). FP32, 32 and 8 lanes: 3.3 and
+// 5.7 us at 5,778 rows, 4.7 and 6.2 at 12,810, 11.7 and 10.5 at 43,554, 33.9 and 22.5 at 92,178. FP64 at 5,778
+// rows: 10.0 and 15.8 us, and 14.1 with three separate sums over the warp.
+static int bsr_lanes(const Level &L) { return L.nnod > 2 * 152 * 64 ? 8 : 32; }
+template <typename T, bool JAC, int LPR, typename... A>
+static void bsr_launch(const Level &L, cudaStream_t s, const T *B, A... a) {
+  launch_pdl(k_bsr_spmv<T, JAC, LPR>, (unsigned)(((size_t)L.nnod * LPR + 255) / 256), 256, 0, s, L.bsr_ptr, L.bsr_col, B,
+             L.nnod, (size_t)L.nnzb, a...);
+  count_launch();
 }
 
 template <typename T>
@@ -1096,19 +1101,17 @@ int bsr_assemble(const Level &L, const T *K, T *B, cudaStream_t s) {
 }
 template <typename T>
 int bsr_apply(const Level &L, const T *B, const T *x, T *y, cudaStream_t s) {
-  launch_pdl(k_bsr_spmv<T, false>, (unsigned)(((size_t)L.nnod * 32 + 255) / 256), 256, 0, s, L.bsr_ptr, L.bsr_col, B,
-             L.nnod, (size_t)L.nnzb, x, y, T(0), nullptr, nullptr);
-  count_launch();
+  const T *none = nullptr;
+  if (bsr_lanes(L) == 8) bsr_launch<T, false, 8>(L, s, B, x, y, T(0), none, none);
+  else bsr_launch<T, false, 32>(L, s, B, x, y, T(0), none, none);
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
 // y = x + w (r - B x) Di
 template <typename T>
 int bsr_apply_jac(const Level &L, const T *B, T w, const T *r, const T *Di, const T *x, T *y, cudaStream_t s) {
-  launch_pdl(k_bsr_spmv<T, true>, (unsigned)(((size_t)L.nnod * 32 + 255) / 256), 256, 0, s, L.bsr_ptr, L.bsr_col, B,
-             L.nnod,
-                                                                                   (size_t)L.nnzb, x, y, w, r, Di);
-  count_launch();
+  if (bsr_lanes(L) == 8) bsr_launch<T, true, 8>(L, s, B, x, y, w, r, Di);
+  else bsr_launch<T, true, 32>(L, s, B, x, y, w, r, Di);
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }

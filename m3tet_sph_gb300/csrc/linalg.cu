@@ -263,15 +263,10 @@ __global__ void __launch_bounds__(256) k_restrict(const int *__restrict__ ptr, c
       s2 += wk * a[3 * j + 2];
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-  }
-  if (lane < 3) {
-    const size_t q = 3 * (size_t)i + lane;
-    const T v = mask[q] ? (lane == 0 ? s0 : lane == 1 ? s1 : s2) : T(0);
+  const T t = lane_sum3<32>(s0, s1, s2);
+  if (lane % 8 == 0 && lane < 24) {
+    const size_t q = 3 * (size_t)i + lane / 8;
+    const T v = mask[q] ? t : T(0);
     out[q] = v;
     if (d) d[q] = wj * v * Di[q];
     if (cmap) {
