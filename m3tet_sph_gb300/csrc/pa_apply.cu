@@ -191,33 +191,6 @@ __device__ __forceinline__ void pa_bulk_load(uint32_t dst, const float *src, uin
       : "memory");
 }
 
-// two FP32 values in one 64-bit register
-__device__ __forceinline__ uint64_t pk(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 unpk(uint64_t v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
 __global__ void __launch_bounds__(32, 8)
 k_pa_tile(const float *__restrict__ pa, const int *__restrict__ el2nod, int nel, const float4 *__restrict__ xc,
           const int *__restrict__ tptr, const int2 *__restrict__ slot, const uint16_t *__restrict__ ent,
@@ -261,11 +234,11 @@ k_pa_tile(const float *__restrict__ pa, const int *__restrict__ el2nod, int nel,
 #pragma unroll
     for (int n = 0; n < 10; ++n) {
       const float4 a = xc[n0[n]], b = xc[n1[n]];
-      v[n][0] = pk(a.x, b.x);
-      v[n][1] = pk(a.y, b.y);
-      v[n][2] = pk(a.z, b.z);
+      v[n][0] = f2_pack(a.x, b.x);
+      v[n][1] = f2_pack(a.y, b.y);
+      v[n][2] = f2_pack(a.z, b.z);
     }
-    const uint64_t m1 = pk(-1.f, -1.f), c4 = pk(4.f, 4.f);
+    const uint64_t m1 = f2_pack(-1.f, -1.f), c4 = f2_pack(4.f, 4.f);
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
       const uint64_t z3[4] = {v[7][p], v[9][p], v[6][p], v[3][p]};      // Z_3m
@@ -274,9 +247,9 @@ k_pa_tile(const float *__restrict__ pa, const int *__restrict__ el2nod, int nel,
                                 {v[8][p], v[5][p], v[2][p], v[6][p]}};
 #pragma unroll
       for (int j = 0; j < 3; ++j) {
-        const uint64_t d = fma2(m1, v[j][p], v[3][p]);                  // u_3 - u_j
+        const uint64_t d = f2_fma(m1, v[j][p], v[3][p]);                  // u_3 - u_j
 #pragma unroll
-        for (int m = 0; m < 4; ++m) E[p][j][m] = fma2(c4, fma2(m1, z3[m], z[j][m]), d);
+        for (int m = 0; m < 4; ++m) E[p][j][m] = f2_fma(c4, f2_fma(m1, z3[m], z[j][m]), d);
       }
     }
   }
@@ -312,27 +285,27 @@ k_pa_tile(const float *__restrict__ pa, const int *__restrict__ el2nod, int nel,
         uint64_t g[3];
 #pragma unroll
         for (int j = 0; j < 3; ++j)
-          g[j] = fma2(lam[0], E[p][j][0], fma2(lam[1], E[p][j][1], fma2(lam[2], E[p][j][2], mul2(lam[3], E[p][j][3]))));
+          g[j] = f2_fma(lam[0], E[p][j][0], f2_fma(lam[1], E[p][j][1], f2_fma(lam[2], E[p][j][2], f2_mul(lam[3], E[p][j][3]))));
 #pragma unroll
-        for (int k = 0; k < 3; ++k) L[p][k] = fma2(g[0], a[3 * k], fma2(g[1], a[3 * k + 1], mul2(g[2], a[3 * k + 2])));
+        for (int k = 0; k < 3; ++k) L[p][k] = f2_fma(g[0], a[3 * k], f2_fma(g[1], a[3 * k + 1], f2_mul(g[2], a[3 * k + 2])));
       }
-      const uint64_t two = pk(2.f, 2.f), mt = pk(-2.f / 3.f, -2.f / 3.f);
-      const uint64_t tr = mul2(mt, add2(add2(L[0][0], L[1][1]), L[2][2]));
+      const uint64_t two = f2_pack(2.f, 2.f), mt = f2_pack(-2.f / 3.f, -2.f / 3.f);
+      const uint64_t tr = f2_mul(mt, f2_add(f2_add(L[0][0], L[1][1]), L[2][2]));
       uint64_t S[3][3];
 #pragma unroll
       for (int p = 0; p < 3; ++p) {
-        S[p][p] = fma2(two, L[p][p], tr);
+        S[p][p] = f2_fma(two, L[p][p], tr);
 #pragma unroll
-        for (int k = 0; k < p; ++k) S[p][k] = S[k][p] = add2(L[p][k], L[k][p]);
+        for (int k = 0; k < p; ++k) S[p][k] = S[k][p] = f2_add(L[p][k], L[k][p]);
       }
       // back to the reference directions: T[p][j] = sum_c S[p][c] A[c][j], and its moments
 #pragma unroll
       for (int p = 0; p < 3; ++p)
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-          const uint64_t t = fma2(S[p][0], a[j], fma2(S[p][1], a[3 + j], mul2(S[p][2], a[6 + j])));
+          const uint64_t t = f2_fma(S[p][0], a[j], f2_fma(S[p][1], a[3 + j], f2_mul(S[p][2], a[6 + j])));
 #pragma unroll
-          for (int m = 0; m < 4; ++m) F[p][j][m] = fma2(lam[m], t, F[p][j][m]);
+          for (int m = 0; m < 4; ++m) F[p][j][m] = f2_fma(lam[m], t, F[p][j][m]);
         }
     }
     __syncwarp();                                    // every lane done with the stage
@@ -341,7 +314,7 @@ k_pa_tile(const float *__restrict__ pa, const int *__restrict__ el2nod, int nel,
   }
   // element outputs over the ring (every copy has landed), then the sums of the tile's nodes. With
   // W_jm = sum lam_m T_j (T_3 = -sum_j T_j): vertex v: 4 W_vv - sum_m W_vm; edge (j, m): 4 (W_jm + W_mj)
-  const uint64_t m1 = pk(-1.f, -1.f), c4 = pk(4.f, 4.f);
+  const uint64_t m1 = f2_pack(-1.f, -1.f), c4 = f2_pack(4.f, 4.f);
 #pragma unroll
   for (int p = 0; p < 3; ++p) {
     uint64_t W[4][4];
@@ -349,18 +322,18 @@ k_pa_tile(const float *__restrict__ pa, const int *__restrict__ el2nod, int nel,
     for (int m = 0; m < 4; ++m) {
 #pragma unroll
       for (int j = 0; j < 3; ++j) W[j][m] = F[p][j][m];
-      W[3][m] = mul2(m1, add2(add2(W[0][m], W[1][m]), W[2][m]));
+      W[3][m] = f2_mul(m1, f2_add(f2_add(W[0][m], W[1][m]), W[2][m]));
     }
     float *o = ring + p * PA_LD + lane;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const float2 r = unpk(fma2(c4, W[k][k], mul2(m1, add2(add2(W[k][0], W[k][1]), add2(W[k][2], W[k][3])))));
+      const float2 r = f2_unpack(f2_fma(c4, W[k][k], f2_mul(m1, f2_add(f2_add(W[k][0], W[k][1]), f2_add(W[k][2], W[k][3])))));
       o[3 * k * PA_LD] = r.x;
       o[3 * k * PA_LD + 32] = r.y;
     }
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
-      const float2 r = unpk(mul2(c4, add2(W[pa_ea(k)][pa_eb(k)], W[pa_eb(k)][pa_ea(k)])));
+      const float2 r = f2_unpack(f2_mul(c4, f2_add(W[pa_ea(k)][pa_eb(k)], W[pa_eb(k)][pa_ea(k)])));
       o[3 * (4 + k) * PA_LD] = r.x;
       o[3 * (4 + k) * PA_LD + 32] = r.y;
     }
