@@ -285,7 +285,7 @@ struct Finest {
 };
 
 // state of a velocity solve's CG, at scal + CG_STATE: the host sets it, the step kernel ends the loop
-enum { CG_STATE = 24, CG_TOL = 24, CG_SQ, CG_PREV, CG_IT, CG_LIMIT, CG_LEARNED, CG_STATUS, CG_STATE_END };
+enum { CG_STATE = 24, CG_TOL = 24, CG_SQ, CG_PREV, CG_IT, CG_LIMIT, CG_LEARNED, CG_STATUS, CG_RR0, CG_STATE_END };
 enum { CG_RUN = 0, CG_CONVERGED, CG_NAN, CG_STALLED, CG_LIMIT_REACHED };
 constexpr int CG_LOOP_MAX = 256;    // iterations of a captured loop before the host looks at it
 

@@ -136,16 +136,6 @@ int cg_update(double *x, double *r, const double *q, const double *Kq, float *r3
 // ---------------------------------------------------------------------------------------
 // generic elementwise kernels
 // ---------------------------------------------------------------------------------------
-__global__ void k_axpby(double a, const double *__restrict__ x, double b, double *__restrict__ y, size_t n) {
-  grid_dep();
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    y[i] = a * x[i] + b * y[i];
-}
-int axpby(double a, const double *x, double b, double *y, size_t n, cudaStream_t s) {
-  launch_pdl(k_axpby, RED_BLOCKS, RED_THREADS, 0, s, a, x, b, y, n); count_launch();
-  M3_CUDA(cudaGetLastError());
-  return M3SPH_OK;
-}
 // y = (b - y) masked: residual r = b - Kx on free dofs, its FP32 copy and out[0] = r.r
 __global__ void k_residual(const double *__restrict__ b, double *__restrict__ y, const uint8_t *__restrict__ mask,
                            float *__restrict__ y32, size_t n, double *partials, unsigned *cnt, double *out) {

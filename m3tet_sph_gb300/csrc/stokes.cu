@@ -71,7 +71,6 @@ int cg_update(double *x, double *r, const double *q, const double *Kq, float *r3
               double *partials, unsigned *cnt, cudaGraphConditionalHandle loop, cudaStream_t s);
 int residual(const double *b, double *y, const uint8_t *mask, float *y32, size_t n, double *partials, unsigned *cnt,
              double *out, cudaStream_t s);
-int axpby(double a, const double *x, double b, double *y, size_t n, cudaStream_t s);
 int apply_mask(double *y, const uint8_t *mask, size_t n, cudaStream_t s);
 int d2f(const double *a, float *b, size_t n, cudaStream_t s);
 int f2d(const float *a, double *b, size_t n, cudaStream_t s);
@@ -1191,9 +1190,12 @@ static int read_scal(m3sph_mesh *M, int idx, double &v) {
 }
 
 struct CgState { double v[CG_STATE_END - CG_STATE]; };
+// CG_RR0 is kept at the first call of a solve from the initial residual (scal[3])
 __global__ void k_cg_state(double *scal, CgState st, double first) {
-  if (threadIdx.x < CG_STATE_END - CG_STATE) scal[CG_STATE + threadIdx.x] = st.v[threadIdx.x];
+  const int k = CG_STATE + threadIdx.x;
+  if (k < CG_STATE_END && k != CG_RR0) scal[k] = st.v[threadIdx.x];
   if (threadIdx.x == 0) scal[6] = first;
+  if (k == CG_RR0 && first != 0.0) scal[k] = scal[3];
 }
 
 // one flexible-PCG iteration on device-resident data (no host synchronisation): V-cycle,
@@ -1277,15 +1279,21 @@ static int mgpcg(m3sph_mesh *M, const double *b, double *x, double tol, bool abs
   const double sq = std::sqrt((double)std::max(1, L0.nfree));
   M3_TRY(outer_apply(M, x, W->r));
   M3_TRY(residual(b, W->r, L0.freemask, M->precision ? W->r32[0] : nullptr, n, M->red, M->red_cnt, M->scal + 3, s));
-  double rr;
-  M3_TRY(read_scal(M, 3, rr));
-  if (std::isnan(rr)) {
+  // a tolerance relative to the initial residual needs it on the host; an absolute one does not, and a NaN is
+  // then found by the first iteration
+  auto rhs_nan = []() {
     set_error("RHS vector contains NaNs");
     return M3SPH_ERR_NAN;
+  };
+  double rrms = 0.0;
+  if (!abs_tol || itmax <= 0) {
+    double rr;
+    M3_TRY(read_scal(M, 3, rr));
+    if (std::isnan(rr)) return rhs_nan();
+    rrms = std::sqrt(rr) / sq;
+    if (!abs_tol) tol = tol * rrms;
   }
-  double rrms = std::sqrt(rr) / sq;
-  if (!abs_tol) tol = tol * rrms;
-  CgState cg{{tol, sq, rrms, 0.0, (double)itmax, M->smoother_active ? 1.0 : 0.0, (double)CG_RUN}};
+  CgState cg{{tol, sq, rrms, 0.0, (double)itmax, M->smoother_active ? 1.0 : 0.0, (double)CG_RUN, 0.0}};
   auto val = [&](int k) -> double & { return cg.v[k - CG_STATE]; };
   double first = 1.0;
   while (itmax > 0) {
@@ -1309,6 +1317,7 @@ static int mgpcg(m3sph_mesh *M, const double *b, double *x, double tol, bool abs
       st.nvc += (int)(it - it0);
     } while (status == CG_RUN);
     if (status == CG_NAN) {
+      if (std::isnan(val(CG_RR0))) return rhs_nan();
       set_error("NaN in MG-PCG residual");
       return M3SPH_ERR_NAN;
     }
@@ -1332,14 +1341,43 @@ static int mgpcg(m3sph_mesh *M, const double *b, double *x, double tol, bool abs
 // ======================================================================================
 // Patera pressure CG (flow3d_patera_mg_sph_p.m:386-632)
 // ======================================================================================
+static int pdot_to(m3sph_mesh *M, const double *a, const double *b, int slot) {
+  return dot(a, b, M->lev[0].nvnod, M->red, M->red_cnt, M->scal + slot, M->stream);
+}
 static int pdot(m3sph_mesh *M, const double *a, const double *b, double &v) {
   M3_TRY(dot(a, b, M->lev[0].nvnod, M->red, M->red_cnt, M->scal + 8, M->stream));
   return read_scal(M, 8, v);
 }
-__global__ void k_shift(double *a, double c, int n) {
+// a - mean(a) from the sum in sum[0]
+__global__ void k_remove_mean(double *a, const double *sum, int n) {
   grid_dep();
+  const double c = -sum[0] / n;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) a[i] += c;
+}
+// scalars of the pressure CG on the device: r.d of the last and of this direction, rlast.d, q.Sq
+enum { PT_RDLAST = 18, PT_RD, PT_RLD, PT_QSQ };
+// q = d + beta q, beta = (r - rlast).d / rdlast
+__global__ void k_patera_dir(const double *__restrict__ d, double *__restrict__ q, int n, const double *scal) {
+  grid_dep();
+  const double beta = (scal[PT_RD] - scal[PT_RLD]) / scal[PT_RDLAST];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) q[i] = d[i] + beta * q[i];
+}
+// alpha = r.d / q.Sq ; P += alpha q ; U += alpha z ; rlast = r ; r -= alpha Sq
+__global__ void k_patera_step(double *__restrict__ P, const double *__restrict__ q, double *__restrict__ U,
+                              const double *__restrict__ z, double *__restrict__ r, double *__restrict__ rlast,
+                              const double *__restrict__ Sq, int np, int n, const double *scal) {
+  grid_dep();
+  const double alpha = scal[PT_RDLAST] / scal[PT_QSQ];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) U[i] += alpha * z[i];
+  if (i < np) {
+    P[i] += alpha * q[i];
+    const double ri = r[i];
+    rlast[i] = ri;
+    r[i] = ri - alpha * Sq[i];
+  }
 }
 __global__ void k_rhs(const double *Fb, const double *GP, const double *bc, const uint8_t *mask, double *out, size_t n) {
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -1373,9 +1411,7 @@ __global__ void k_absmax_xyz(const double *U, const double *RR, int nnod, unsign
 static int remove_mean(m3sph_mesh *M, double *a) {
   const int np = M->lev[0].nvnod;
   M3_TRY(vsum(a, np, M->red, M->red_cnt, M->scal + 9, M->stream));
-  double sm;
-  M3_TRY(read_scal(M, 9, sm));
-  launch_pdl(k_shift, (np + 255) / 256, 256, 0, M->stream, a, -sm / np, np); count_launch();
+  launch_pdl(k_remove_mean, (np + 255) / 256, 256, 0, M->stream, a, M->scal + 9, np); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
@@ -1454,7 +1490,7 @@ static int solve_core(m3sph_mesh *M, const m3sph_opts *opts, m3sph_info &inf) {
   inf.nitU += cs.it;
   double tol_U_restart = rtol_U * tol_Pat;
   bool restart = true, conv_problem = false;
-  double norm_rP0 = norm_rP, rd = 0.0, rdlast = 0.0, tol_Z = 0.0;
+  double norm_rP0 = norm_rP, tol_Z = 0.0;
   int itPat = 0;
   const double target = opts->target_rel_residual;
   bool converged = false;
@@ -1466,28 +1502,22 @@ static int solve_core(m3sph_mesh *M, const m3sph_opts *opts, m3sph_info &inf) {
       norm_rP0 = norm_rP;
       tol_Z = rtol_U * std::max(rtol_restart * norm_rP0, tol_Pat);
     } else {
-      // beta = (r - rlast).d / rdlast
-      double rd_new, rld;
-      M3_TRY(pdot(M, r, d, rd_new));
-      M3_TRY(pdot(M, W->prl, d, rld));
-      const double beta = (rd_new - rld) / rdlast;
-      M3_TRY(axpby(1.0, d, beta, q, np, s));
+      M3_TRY(pdot_to(M, r, d, PT_RD));
+      M3_TRY(pdot_to(M, W->prl, d, PT_RLD));
+      launch_pdl(k_patera_dir, (np + 255) / 256, 256, 0, s, d, q, np, M->scal); count_launch();
+      M3_CUDA(cudaGetLastError());
     }
     M3_TRY(remove_mean(M, q));
-    M3_TRY(pdot(M, r, d, rd));
-    rdlast = rd;
+    M3_TRY(pdot_to(M, r, d, PT_RDLAST));
     M3_TRY(grad_apply(L0, M->fin.G64, q, L0.freemask, nullptr, nullptr, y, s));
     M3_CUDA(cudaMemsetAsync(z, 0, sizeof(double) * n, s));
     M3_TRY(mgpcg(M, y, z, tol_Z, true, itmax_U, cs));
     inf.nitZ += cs.it;
     M3_TRY(div_apply(L0, M->fin.G64, z, 1.0, Sq, s));
-    double qSq;
-    M3_TRY(pdot(M, q, Sq, qSq));
-    M3_CUDA(cudaMemcpyAsync(W->prl, r, sizeof(double) * np, cudaMemcpyDeviceToDevice, s));
-    const double alpha = rd / qSq;
-    M3_TRY(axpby(alpha, q, 1.0, Pd, np, s));
-    M3_TRY(axpby(alpha, z, 1.0, U, n, s));
-    M3_TRY(axpby(-alpha, Sq, 1.0, r, np, s));
+    M3_TRY(pdot_to(M, q, Sq, PT_QSQ));
+    launch_pdl(k_patera_step, (unsigned)((n + 255) / 256), 256, 0, s, Pd, q, U, z, r, W->prl, Sq, np, (int)n, M->scal);
+    count_launch();
+    M3_CUDA(cudaGetLastError());
     M3_TRY(remove_mean(M, r));
     const double norm_rP_last = norm_rP;
     M3_TRY(pdot(M, r, r, rr));
