@@ -354,7 +354,7 @@ int stokes_set_pressure(m3sph_mesh *M, const double *P);
 int ml_build(m3sph_mesh *M);
 int ml_features(m3sph_mesh *M, const double *h_visc);
 template <typename T>
-int ml_sweep(m3sph_mesh *M, int j, const T *r0, const T *kd, const T *Dinv, T *tmp, T *d, const PaCart &pc);
+int ml_sweep(m3sph_mesh *M, int j, const T *r0, const T *kd, const T *Dinv, T *tmp, T *d, const PaCart &pc, bool first);
 int ml_init_kernels();
 int ml_set_infer(int v);
 int ml_check(m3sph_mesh *M);

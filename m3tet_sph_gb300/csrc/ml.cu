@@ -188,20 +188,19 @@ __global__ void __launch_bounds__(256) k_ml_infer(FeatLevel L, MlpDev w, const T
   }
 }
 
-// d_n += v on free dofs (a non-finite value is dropped); pc: also the Cartesian copy of d
+// d_n += v on free dofs (a non-finite value is dropped), from zero if `first`; pc: also the Cartesian copy of d
 template <typename T>
 __device__ __forceinline__ void ml_add_node(int n, float v0, float v1, float v2, const uint8_t *__restrict__ mask,
-                                            T *__restrict__ d, const PaCart &pc) {
+                                            bool first, T *__restrict__ d, const PaCart &pc) {
   const float v[3] = {v0, v1, v2};
   float x[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const size_t i = 3 * (size_t)n + c;
-    T t = d[i];
-    if (mask[i] && isfinite(v[c])) {
-      t += (T)v[c];
-      d[i] = t;
-    }
+    T t = first ? T(0) : d[i];
+    const bool add = mask[i] && isfinite(v[c]);
+    if (add) t += (T)v[c];
+    if (add || first) d[i] = t;
     x[c] = mask[i] ? (float)t : 0.f;
   }
   if (pc.xc) pc.xc[n] = pa_to_cart(pc.trig[n], x[0], x[1], x[2]);
@@ -210,7 +209,7 @@ __device__ __forceinline__ void ml_add_node(int n, float v0, float v1, float v2,
 // d[3n+c] += omega * sum over (element, local node) of node n of C[3a+c][e] / multiplicity(n)
 template <typename T>
 __global__ void k_ml_gather(int nnod, int nel, const int *__restrict__ ptr, const int *__restrict__ code,
-                            const float *__restrict__ C, const uint8_t *__restrict__ mask, float omega,
+                            const float *__restrict__ C, const uint8_t *__restrict__ mask, float omega, bool first,
                             T *__restrict__ d, PaCart pc) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= nnod) return;
@@ -226,7 +225,7 @@ __global__ void k_ml_gather(int nnod, int nel, const int *__restrict__ ptr, cons
   // a non-finite correction (an unusable network) is dropped; the outer CG's rate check then
   // switches the smoother off
   const float w = omega / (float)(e - b);
-  ml_add_node<T>(n, w * s0, w * s1, w * s2, mask, d, pc);
+  ml_add_node<T>(n, w * s0, w * s1, w * s2, mask, first, d, pc);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -508,18 +507,20 @@ __global__ void __launch_bounds__(tc::THREADS, 2) k_ml_sweep_tc(FeatLevel L, Mlp
 template <typename T>
 __global__ void __launch_bounds__(128) k_ml_gather_rows(int nnod, int nv, const int *__restrict__ ptr,
                                                         const int *__restrict__ code, const float *__restrict__ C,
-                                                        const uint8_t *__restrict__ mask, float omega,
+                                                        const uint8_t *__restrict__ mask, float omega, bool first,
                                                         T *__restrict__ d, PaCart pc) {
-  grid_dep();
   const int t = blockIdx.x * 128 + threadIdx.x, nt4 = gather_threads4(nv);
   const bool quad = t < nt4;
   const int n = quad ? t >> 2 : nv + t - nt4, sub = quad ? t & 3 : 0, step = quad ? 4 : 1;
   const bool live = quad ? n < nv : n < nnod;
   const int b = live ? ptr[n] : 0, e = live ? ptr[n + 1] : 0;
+  int next = b + sub < e ? code[b + sub] : 0;   // connectivity, ahead of the wait and of the values
+  grid_dep();
   float s0 = 0.f, s1 = 0.f, s2 = 0.f;
 #pragma unroll 2
   for (int k = b + sub; k < e; k += step) {
-    const int el = code[k] / 10, a = code[k] - 10 * el;
+    const int el = next / 10, a = next - 10 * el;
+    if (k + step < e) next = code[k + step];
     const float *c = C + (size_t)el * OUT + 3 * a;
     const int odd = a & 1;                      // 8-byte aligned pair for even local nodes
     const float2 v2 = *reinterpret_cast<const float2 *>(c + odd);
@@ -538,7 +539,7 @@ __global__ void __launch_bounds__(128) k_ml_gather_rows(int nnod, int nv, const 
   }
   if (sub || e <= b) return;
   const float w = omega / (float)(e - b);
-  ml_add_node<T>(n, w * s0, w * s1, w * s2, mask, d, pc);
+  ml_add_node<T>(n, w * s0, w * s1, w * s2, mask, first, d, pc);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -943,7 +944,7 @@ int ml_check(m3sph_mesh *M) {
 
 // d += PoU(MLP(features(r0 - kd))) on level j (kd may be null: residual r0)
 template <typename T>
-int ml_sweep(m3sph_mesh *M, int j, const T *r0, const T *kd, const T *Dinv, T *tmp, T *d, const PaCart &pc) {
+int ml_sweep(m3sph_mesh *M, int j, const T *r0, const T *kd, const T *Dinv, T *tmp, T *d, const PaCart &pc, bool first) {
   MlState *S = mls(M);
   Level &L = M->lev[j];
   cudaStream_t s = M->stream;
@@ -957,8 +958,8 @@ int ml_sweep(m3sph_mesh *M, int j, const T *r0, const T *kd, const T *Dinv, T *t
     launch_pdl(k_ml_sweep_tc, grid, tc::THREADS, tc::SMEM_ALLOC, s, f, w, S->lev[j].z, S->lev[j].C,
                S->err); count_launch();
     launch_pdl(k_ml_gather_rows<T>, (gather_threads4(L.nvnod) + L.nnod - L.nvnod + 127) / 128, 128, 0, s, L.nnod,
-               L.nvnod, S->lev[j].n2e_ptr, S->lev[j].n2e_code,
-                                                              S->lev[j].C, L.freemask, M->ml_omega, d, pc); count_launch();
+               L.nvnod, S->lev[j].n2e_ptr, S->lev[j].n2e_code, S->lev[j].C, L.freemask, M->ml_omega, first, d, pc);
+    count_launch();
     M3_CUDA(cudaGetLastError());
     return M3SPH_OK;
   }
@@ -969,14 +970,14 @@ int ml_sweep(m3sph_mesh *M, int j, const T *r0, const T *kd, const T *Dinv, T *t
   }
   k_ml_infer<T><<<(L.nel + INF_ROWS - 1) / INF_ROWS, 256, INF_SMEM, s>>>(f, w, r, Dinv, S->lev[j].C); count_launch();
   k_ml_gather<T><<<(L.nnod + 127) / 128, 128, 0, s>>>(L.nnod, L.nel, S->lev[j].n2e_ptr, S->lev[j].n2e_code,
-                                                       S->lev[j].C, L.freemask, M->ml_omega, d, pc); count_launch();
+                                                       S->lev[j].C, L.freemask, M->ml_omega, first, d, pc); count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
 template int ml_sweep<float>(m3sph_mesh *, int, const float *, const float *, const float *, float *, float *,
-                             const PaCart &);
+                             const PaCart &, bool);
 template int ml_sweep<double>(m3sph_mesh *, int, const double *, const double *, const double *, double *, double *,
-                              const PaCart &);
+                              const PaCart &, bool);
 
 int ml_init_kernels() {
   M3_CUDA(cudaFuncSetAttribute(k_ml_infer<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)INF_SMEM));

@@ -1092,9 +1092,8 @@ static int vcycle_T(m3sph_mesh *M, std::vector<T *> &r, std::vector<T *> &d, std
   for (int j = 0; j < nm - 1; ++j) {
     const Level &L = M->lev[j];
     const double *w = j == 0 ? WD0 : WDc;
-    const size_t n = L.ndof;
     const PaCart pc = pa_level<T>(L, j) ? PaCart{L.pa_trig, L.pa_xc} : PaCart{};
-    auto sweep = [&](const T *k) { return ml_sweep<T>(M, j, r[j], k, levDi<T>(L), tmp[j], d[j], pc); };
+    auto sweep = [&](const T *k, bool first) { return ml_sweep<T>(M, j, r[j], k, levDi<T>(L), tmp[j], d[j], pc, first); };
     auto op = [&]() { return level_op<T>(L, j, d[j], kd[j], s, true); };
     auto op_jac = [&](double wk) { return level_op_jac<T>(L, j, (T)wk, r[j], d[j], kd[j], s, true); };
     auto sweep_to = [&](double wk, const T *x, T *y) { return bsr_apply_jac<T>(L, levB<T>(L), (T)wk, r[j], levDi<T>(L), x, y, s); };
@@ -1103,8 +1102,7 @@ static int vcycle_T(m3sph_mesh *M, std::vector<T *> &r, std::vector<T *> &d, std
       M3_TRY(sweep_to(w[1], d[j], tmp[j]));
       M3_TRY(sweep_to(w[2], tmp[j], d[j]));
     } else if (ml && j < nml) {
-      M3_CUDA(cudaMemsetAsync(d[j], 0, sizeof(T) * n, s));
-      M3_TRY(sweep(nullptr));
+      M3_TRY(sweep(nullptr, true));
       if (!one && M->ml_schedule == 3) {
         // learned sweep from zero, one weighted Jacobi sweep
         M3_TRY(op_jac(w[2]));
@@ -1112,7 +1110,7 @@ static int vcycle_T(m3sph_mesh *M, std::vector<T *> &r, std::vector<T *> &d, std
         // learned sweep, weighted Jacobi sweep, learned sweep
         M3_TRY(op_jac(w[1]));
         M3_TRY(op());
-        M3_TRY(sweep(kd[j]));
+        M3_TRY(sweep(kd[j], false));
       }
     } else {
       M3_TRY(level_jac_first<T>(L, j, (T)w[0], r[j], d[j], s));
@@ -1128,7 +1126,7 @@ static int vcycle_T(m3sph_mesh *M, std::vector<T *> &r, std::vector<T *> &d, std
     const Level &L = M->lev[j];
     const double *w = j == 0 ? WU0 : WUc;
     const PaCart pc = pa_level<T>(L, j) ? PaCart{L.pa_trig, L.pa_xc} : PaCart{};
-    auto sweep = [&](const T *k) { return ml_sweep<T>(M, j, r[j], k, levDi<T>(L), tmp[j], d[j], pc); };
+    auto sweep = [&](const T *k) { return ml_sweep<T>(M, j, r[j], k, levDi<T>(L), tmp[j], d[j], pc, false); };
     auto op = [&]() { return level_op<T>(L, j, d[j], kd[j], s, true); };
     auto op_jac = [&](double wk) { return level_op_jac<T>(L, j, (T)wk, r[j], d[j], kd[j], s, true); };
     if (!(ml && j < nml) && j > 0) {
@@ -1945,7 +1943,7 @@ extern "C" int m3sph_ml_sweep32(m3sph_mesh *M, int32_t img, const float *r, cons
   if (kd) M3_CUDA(cudaMemcpyAsync(W->kd32[img], kd, sizeof(float) * n, cudaMemcpyHostToDevice, s));
   M3_CUDA(cudaMemcpyAsync(W->d32[img], d, sizeof(float) * n, cudaMemcpyHostToDevice, s));
   M3_TRY(ml_sweep<float>(M, img, W->r32[img], kd ? W->kd32[img] : nullptr, L.Dinv32, W->t32[img], W->d32[img],
-                         PaCart{}));
+                         PaCart{}, false));
   M3_CUDA(cudaMemcpyAsync(d, W->d32[img], sizeof(float) * n, cudaMemcpyDeviceToHost, s));
   M3_CUDA(cudaStreamSynchronize(s));
   return ml_check(M);
