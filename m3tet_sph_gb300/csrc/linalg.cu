@@ -397,9 +397,89 @@ size_t dense_inverse_work32(int n) { return gj_work<float>(n); }
 // row stride of the dense inverse: whole 16-byte vectors
 int dense_ld(int n) { return (n + 3) & ~3; }
 
+
+// acc = sum_m X[m][row] Y[m][col] over m < NB, X and Y with row strides ldx, ldy (16-byte aligned).
+// Thread (ty, tx) owns rows and columns in groups of four consecutive indices: gj_idx
+template <typename T>
+__device__ __forceinline__ int gj_idx(int t, int a) {
+  constexpr int NG = Gj<T>::NB / 64;                 // groups per thread
+  return (a >> 2) * (Gj<T>::NB / NG) + 4 * t + (a & 3);
+}
+__device__ __forceinline__ void gj_ld4(const float *p, float *v) {
+  const float4 q = *reinterpret_cast<const float4 *>(p);
+  v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+}
+__device__ __forceinline__ void gj_ld4(const double *p, double *v) {
+  const double2 a = *reinterpret_cast<const double2 *>(p), b = *reinterpret_cast<const double2 *>(p + 2);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ void gj_st4(float *p, const float *v) {
+  *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void gj_st4(double *p, const double *v) {
+  *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
+  *reinterpret_cast<double2 *>(p + 2) = make_double2(v[2], v[3]);
+}
+template <typename T> constexpr size_t gj_smem() { return sizeof(T) * GJ_ST * 2 * Gj<T>::KC * Gj<T>::NB; }
+template <typename T, int RT, int CT>
+__device__ __forceinline__ void gj_tile(T (&acc)[RT][CT], const T *X, size_t ldx, const T *Y, size_t ldy) {
+  constexpr int NB = Gj<T>::NB, KC = Gj<T>::KC, NCH = NB / KC, VN = 16 / sizeof(T), PR = NB / VN, PY = 16 * CT / VN;
+  extern __shared__ __align__(16) unsigned char gj_raw[];
+  T(*sm)[2][KC][NB] = reinterpret_cast<T(*)[2][KC][NB]>(gj_raw);
+  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+#pragma unroll
+  for (int a = 0; a < RT; ++a)
+#pragma unroll
+    for (int b = 0; b < CT; ++b) acc[a][b] = T(0);
+  auto issue = [&](int ch) {
+    if (ch < NCH) {
+      for (int q = threadIdx.x; q < KC * PR; q += 256) {
+        const int m = q / PR, v = (q % PR) * VN, k = ch * KC + m;
+        const uint32_t dx = (uint32_t)__cvta_generic_to_shared(&sm[ch % GJ_ST][0][m][v]);
+        const uint32_t dy = (uint32_t)__cvta_generic_to_shared(&sm[ch % GJ_ST][1][m][v]);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dx), "l"(X + k * ldx + v) : "memory");
+        if (PY == PR || q % PR < PY)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dy), "l"(Y + k * ldy + v) : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int ch = 0; ch < GJ_ST - 1; ++ch) issue(ch);
+  for (int ch = 0; ch < NCH; ++ch) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(GJ_ST - 2) : "memory");
+    __syncthreads();                     // chunk ch has landed, everyone is done with chunk ch - 1
+    issue(ch + GJ_ST - 1);
+    const T(*xs)[NB] = sm[ch % GJ_ST][0], (*ys)[NB] = sm[ch % GJ_ST][1];
+    T part[RT][CT];                      // a chunk's sum by itself: shorter chains of roundings
+#pragma unroll
+    for (int a = 0; a < RT; ++a)
+#pragma unroll
+      for (int b = 0; b < CT; ++b) part[a][b] = T(0);
+#pragma unroll
+    for (int m = 0; m < KC; ++m) {
+      T xv[RT], yv[CT];
+#pragma unroll
+      for (int g = 0; g < RT; g += 4) gj_ld4(&xs[m][gj_idx<T>(ty, g)], xv + g);
+#pragma unroll
+      for (int g = 0; g < CT; g += 4) gj_ld4(&ys[m][gj_idx<T>(tx, g)], yv + g);
+#pragma unroll
+      for (int a = 0; a < RT; ++a)
+#pragma unroll
+        for (int b = 0; b < CT; ++b) (sizeof(T) == 4 ? part : acc)[a][b] += xv[a] * yv[b];
+    }
+    if (sizeof(T) == 4)
+#pragma unroll
+      for (int a = 0; a < RT; ++a)
+#pragma unroll
+        for (int b = 0; b < CT; ++b) acc[a][b] += part[a][b];
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) k_gjb_diag(const T *__restrict__ A, int ld, int kb, int nb, T *__restrict__ Dinv,
-                                                  T *__restrict__ DinvT) {
+                                                  T *__restrict__ DinvT, const T *Ct, const T *R, size_t npad) {
   constexpr int NB = Gj<T>::NB, RT = NB / 16, SB = GJ_SB;
   __shared__ T sC[NB][SB + 1], sK[SB][NB], sR[SB][NB], sD[SB][SB + 1];
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16, r0 = ty * RT, c0 = tx * RT;
@@ -411,6 +491,28 @@ __global__ void __launch_bounds__(256) k_gjb_diag(const T *__restrict__ A, int l
       const int r = r0 + i, c = c0 + j;
       a[i][j] = (r < nb && c < nb) ? A[(size_t)(kb + r) * ld + kb + c] : (r == c ? T(1) : T(0));
     }
+  if (sizeof(T) == 4 && Ct) {            // A - C R of the panel before, padded rows and columns are zero
+    T u[RT][RT];
+    gj_tile<T, RT, RT>(u, Ct + kb, npad, R + kb, npad);
+    // its threads hold groups of four rows and columns 64 apart: through shared memory to whole pieces
+    extern __shared__ __align__(16) unsigned char gj_raw[];
+    T(*su)[NB] = reinterpret_cast<T(*)[NB]>(gj_raw);
+    for (int h = 0; h < NB / 16; ++h) {
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < RT; ++i)
+#pragma unroll
+        for (int j = 0; j < RT; ++j)
+          if (gj_idx<T>(ty, i) / 16 == h) su[gj_idx<T>(ty, i) % 16][gj_idx<T>(tx, j)] = u[i][j];
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < RT; ++i)
+#pragma unroll
+        for (int j = 0; j < RT; ++j)
+          if ((r0 + i) / 16 == h) a[i][j] -= su[(r0 + i) % 16][c0 + j];
+    }
+    __syncthreads();
+  }
   for (int p0 = 0; p0 < NB; p0 += SB) {
     const bool inr = r0 >= p0 && r0 < p0 + SB, inc = c0 >= p0 && c0 < p0 + SB;    // RT divides SB
 #pragma unroll
@@ -493,91 +595,11 @@ __global__ void __launch_bounds__(256) k_gjb_diag(const T *__restrict__ A, int l
     }
 }
 
-// acc = sum_m X[m][row] Y[m][col] over m < NB, X and Y with row strides ldx, ldy (16-byte aligned).
-// Thread (ty, tx) owns rows and columns in groups of four consecutive indices: gj_idx
-template <typename T>
-__device__ __forceinline__ int gj_idx(int t, int a) {
-  constexpr int NG = Gj<T>::NB / 64;                 // groups per thread
-  return (a >> 2) * (Gj<T>::NB / NG) + 4 * t + (a & 3);
-}
-__device__ __forceinline__ void gj_ld4(const float *p, float *v) {
-  const float4 q = *reinterpret_cast<const float4 *>(p);
-  v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-}
-__device__ __forceinline__ void gj_ld4(const double *p, double *v) {
-  const double2 a = *reinterpret_cast<const double2 *>(p), b = *reinterpret_cast<const double2 *>(p + 2);
-  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
-__device__ __forceinline__ void gj_st4(float *p, const float *v) {
-  *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
-}
-__device__ __forceinline__ void gj_st4(double *p, const double *v) {
-  *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
-  *reinterpret_cast<double2 *>(p + 2) = make_double2(v[2], v[3]);
-}
-template <typename T> constexpr size_t gj_smem() { return sizeof(T) * GJ_ST * 2 * Gj<T>::KC * Gj<T>::NB; }
-template <typename T, int RT>
-__device__ __forceinline__ void gj_tile(T (&acc)[RT][RT], const T *__restrict__ X, size_t ldx, const T *__restrict__ Y,
-                                        size_t ldy) {
-  constexpr int NB = Gj<T>::NB, KC = Gj<T>::KC, NCH = NB / KC, VN = 16 / sizeof(T), PR = NB / VN;
-  extern __shared__ __align__(16) unsigned char gj_raw[];
-  T(*sm)[2][KC][NB] = reinterpret_cast<T(*)[2][KC][NB]>(gj_raw);
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-#pragma unroll
-  for (int a = 0; a < RT; ++a)
-#pragma unroll
-    for (int b = 0; b < RT; ++b) acc[a][b] = T(0);
-  auto issue = [&](int ch) {
-    if (ch < NCH) {
-      for (int q = threadIdx.x; q < KC * PR; q += 256) {
-        const int m = q / PR, v = (q % PR) * VN, k = ch * KC + m;
-        const uint32_t dx = (uint32_t)__cvta_generic_to_shared(&sm[ch % GJ_ST][0][m][v]);
-        const uint32_t dy = (uint32_t)__cvta_generic_to_shared(&sm[ch % GJ_ST][1][m][v]);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dx), "l"(X + k * ldx + v) : "memory");
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dy), "l"(Y + k * ldy + v) : "memory");
-      }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-#pragma unroll
-  for (int ch = 0; ch < GJ_ST - 1; ++ch) issue(ch);
-  for (int ch = 0; ch < NCH; ++ch) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(GJ_ST - 2) : "memory");
-    __syncthreads();                     // chunk ch has landed, everyone is done with chunk ch - 1
-    issue(ch + GJ_ST - 1);
-    const T(*xs)[NB] = sm[ch % GJ_ST][0], (*ys)[NB] = sm[ch % GJ_ST][1];
-    T part[RT][RT];                      // a chunk's sum by itself: shorter chains of roundings
-#pragma unroll
-    for (int a = 0; a < RT; ++a)
-#pragma unroll
-      for (int b = 0; b < RT; ++b) part[a][b] = T(0);
-#pragma unroll
-    for (int m = 0; m < KC; ++m) {
-      T xv[RT], yv[RT];
-#pragma unroll
-      for (int g = 0; g < RT; g += 4) {
-        gj_ld4(&xs[m][gj_idx<T>(ty, g)], xv + g);
-        gj_ld4(&ys[m][gj_idx<T>(tx, g)], yv + g);
-      }
-#pragma unroll
-      for (int a = 0; a < RT; ++a)
-#pragma unroll
-        for (int b = 0; b < RT; ++b) (sizeof(T) == 4 ? part : acc)[a][b] += xv[a] * yv[b];
-    }
-    if (sizeof(T) == 4)
-#pragma unroll
-      for (int a = 0; a < RT; ++a)
-#pragma unroll
-        for (int b = 0; b < RT; ++b) acc[a][b] += part[a][b];
-  }
-  asm volatile("cp.async.wait_all;" ::: "memory");
-}
-
-// operand image of block column j0 of a panel S (128 K-rows of npad values): row c = column j0 + c of S, times
-// 1 + up
-__device__ __forceinline__ void gj_image(const float *S, size_t npad, int j0, float up, unsigned char *img) {
-  for (int q = threadIdx.x; q < 128 * 16; q += 256) {
-    const int c = q & 127, ch = q >> 7;
+// rows c0 .. c0 + 63 of the operand image of block column j0 of a panel S (128 K-rows of npad values): row c =
+// column j0 + c of S, times 1 + up
+__device__ __forceinline__ void gj_image(const float *S, size_t npad, int j0, int c0, float up, unsigned char *img) {
+  for (int q = threadIdx.x; q < 64 * 16; q += 256) {
+    const int c = c0 + (q & 63), ch = q >> 6;
     uint32_t w[3][4];
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
@@ -603,34 +625,37 @@ __device__ __forceinline__ void gj_image(const float *S, size_t npad, int j0, fl
   }
 }
 
-// block j: saved column panel Ct[m][i] = C_i[m] for its rows i and row panel R = +-D^-1 C_j' for its
-// columns (minus for panels already swept, j < kblk), zero padding past n; then panel k of the matrix itself:
-// its row R, its column -C D^-1 = -R' and its diagonal block D^-1. FP32: the operand images of C and R as well.
+// block j, columns c0 .. c0 + NW - 1 of it: saved column panel Ct[m][i] = C_i[m] for its rows i and row panel
+// R = +-D^-1 C_j' for its columns (minus for panels already swept, j < kblk), zero padding past n; then panel k of
+// the matrix itself: its row R, its column -C D^-1 = -R' and its diagonal block D^-1. FP32: the operand images of
+// C and R as well, and two CTAs per block (70 -> 50 us at 14.8k free dofs: a CTA's share is a serial chain of loads,
+// product and stores).
+template <typename T> constexpr int GJ_PANEL_CTAS = sizeof(T) == 4 ? 2 : 1;
 template <typename T>
 __global__ void __launch_bounds__(256) k_gjb_panels(T *__restrict__ A, int ld, int n, int kblk, int nb,
                                                     const T *__restrict__ Dinv, const T *__restrict__ DinvT, size_t npad,
                                                     T *R, T *Ct, unsigned char *imgC, unsigned char *imgR) {
-  constexpr int NB = Gj<T>::NB, RT = NB / 16;
+  constexpr int NB = Gj<T>::NB, RT = NB / 16, NW = NB / GJ_PANEL_CTAS<T>, CT = NW / 16;
   __shared__ T tr[32][33];
-  const int j = blockIdx.x, j0 = j * NB, kb = kblk * NB;
+  const int j = blockIdx.x, c0 = blockIdx.y * NW, j0 = j * NB + c0, kb = kblk * NB;
   const bool swept = j < kblk;
   if (j == kblk) {
-    for (int q = threadIdx.x; q < NB * NB; q += 256) {
-      const int r = q / NB, c = q % NB;
-      if (r < nb && c < nb) A[(size_t)(kb + r) * ld + kb + c] = Dinv[q];
+    for (int q = threadIdx.x; q < NB * NW; q += 256) {
+      const int r = q / NW, c = c0 + q % NW;
+      if (r < nb && c < nb) A[(size_t)(kb + r) * ld + kb + c] = Dinv[r * NB + c];
     }
     return;
   }
   if (swept) {
     // C_i = -A_ki' : row m of tile (k, j) is column m of C
-    for (int q = threadIdx.x; q < NB * NB; q += 256) {
-      const int m = q / NB, c = q % NB;
+    for (int q = threadIdx.x; q < NB * NW; q += 256) {
+      const int m = q / NW, c = q % NW;
       Ct[m * npad + j0 + c] = (m < nb) ? -A[(size_t)(kb + m) * ld + j0 + c] : T(0);
     }
   } else {
     // tile (j, k), transposed 32 x 32 at a time
     const int lx = threadIdx.x % 32, ly = threadIdx.x / 32;
-    for (int b = 0; b < (NB / 32) * (NB / 32); ++b) {
+    for (int b = 0; b < (NW / 32) * (NB / 32); ++b) {
       const int i0 = (b / (NB / 32)) * 32, m0 = (b % (NB / 32)) * 32;
       __syncthreads();
       for (int y = ly; y < 32; y += 8) {
@@ -642,13 +667,13 @@ __global__ void __launch_bounds__(256) k_gjb_panels(T *__restrict__ A, int ld, i
     }
   }
   __syncthreads();
-  T acc[RT][RT];
-  gj_tile<T, RT>(acc, DinvT, NB, Ct + j0, npad);
+  T acc[RT][CT];
+  gj_tile<T, RT, CT>(acc, DinvT, NB, Ct + j0, npad);
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
 #pragma unroll
   for (int a = 0; a < RT; ++a)
 #pragma unroll
-    for (int g = 0; g < RT; g += 4) {
+    for (int g = 0; g < CT; g += 4) {
       T v[4];
 #pragma unroll
       for (int b = 0; b < 4; ++b) v[b] = swept ? -acc[a][g + b] : acc[a][g + b];
@@ -659,7 +684,7 @@ __global__ void __launch_bounds__(256) k_gjb_panels(T *__restrict__ A, int ld, i
   __syncthreads();
   if (!swept) {
     const int lx = threadIdx.x % 32, ly = threadIdx.x / 32;
-    for (int b = 0; b < (NB / 32) * (NB / 32); ++b) {
+    for (int b = 0; b < (NW / 32) * (NB / 32); ++b) {
       const int r0 = (b / (NB / 32)) * 32, m0 = (b % (NB / 32)) * 32;
       __syncthreads();
       for (int y = ly; y < 32; y += 8) tr[y][lx] = R[(size_t)(m0 + y) * npad + j0 + r0 + lx];
@@ -671,8 +696,8 @@ __global__ void __launch_bounds__(256) k_gjb_panels(T *__restrict__ A, int ld, i
     }
   }
   if constexpr (sizeof(T) == 4) {
-    gj_image(Ct, npad, j0, gu::ROUNDING, imgC + (size_t)j * gu::IMAGE);
-    gj_image(R, npad, j0, 0.f, imgR + (size_t)j * gu::IMAGE);
+    gj_image(Ct, npad, j * NB, c0, gu::ROUNDING, imgC + (size_t)j * gu::IMAGE);
+    gj_image(R, npad, j * NB, c0, 0.f, imgR + (size_t)j * gu::IMAGE);
   }
 }
 
@@ -695,7 +720,7 @@ __global__ void __launch_bounds__(256, 2) k_gjb_update(T *__restrict__ A, int ld
   gj_tile_of(blockIdx.x, kblk, bi, bj);
   const int i0 = bi * NB, j0 = bj * NB;
   T acc[RT][RT];
-  gj_tile<T, RT>(acc, Ct + i0, npad, R + j0, npad);
+  gj_tile<T, RT, RT>(acc, Ct + i0, npad, R + j0, npad);
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
 #pragma unroll
   for (int a = 0; a < RT; ++a) {
@@ -719,7 +744,8 @@ __global__ void __launch_bounds__(256, 2) k_gjb_update(T *__restrict__ A, int ld
 // first the five small products and then the large one, so that the roundings of the former are 2^-8 smaller,
 // the two halves are added in FP32, and what rounding towards zero takes is given back (gu::ROUNDING). Against
 // FP64 inverses of difference matrices of 129 to 14,801 unknowns and contrasts of 1e2 to 1e4 the error of the
-// whole inverse is 0 to 10 % below that of FP32 multiply-adds (without ROUNDING 1 to 4 % above).
+// whole inverse is 0 to 10 % below that of FP32 multiply-adds (without ROUNDING 1 to 4 % above); on the coarsest
+// levels of shells, 630 to 17,334 dofs, a V-cycle's error from the inverse is 8 to 40 % below.
 // A persistent CTA takes a run of tiles of the triangle, row by row: the row's operand stays in shared memory
 // (96 KB), the column's comes in halves of 48 KB through a ring of two, and the accumulators of two tiles
 // alternate in TMEM between two groups of epilogue warps, which subtract through a staging tile. At 14.8k free
@@ -727,7 +753,7 @@ __global__ void __launch_bounds__(256, 2) k_gjb_update(T *__restrict__ A, int ld
 // 130 us, the MMAs alone are 82 us: what is left is the latency of the A accesses (272 us with chunks fetched when
 // they were needed, 255 us without the prefetch of the next tile into L2).
 __global__ void __launch_bounds__(gu::THREADS, 1) k_gjb_update_tc(float *__restrict__ A, int ld, int n, int kblk,
-                                                                  size_t ntile, const unsigned char *__restrict__ imgC,
+                                                                  int done, size_t ntile, const unsigned char *__restrict__ imgC,
                                                                   const unsigned char *__restrict__ imgR, int *err) {
   using namespace gu;
   extern __shared__ __align__(16) unsigned char gj_raw[];
@@ -839,8 +865,9 @@ __global__ void __launch_bounds__(gu::THREADS, 1) k_gjb_update_tc(float *__restr
     // a tile's part into L2, half a row of 256 bytes at a time (a load's own prefetch would bring 32)
     auto prefetch = [&](size_t t) {
       if (t >= t1) return;
-      gj_tile_of(t, kblk, bi, bj);
-      const int i = bi * NB + r0 + lane, j = bj * NB + c0;
+      int pi, pj;
+      gj_tile_of(t, kblk, pi, pj);
+      const int i = pi * NB + r0 + lane, j = pj * NB + c0;
       if (i < n && j < ld)
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(A + (size_t)i * ld + j),
                      "r"(4 * min(64, ld - j)));
@@ -875,10 +902,11 @@ __global__ void __launch_bounds__(gu::THREADS, 1) k_gjb_update_tc(float *__restr
         break;
       }
       tc_fence_after();
+      const bool skip = bi == done && bj == done;      // the block k_gjb_diag updates itself
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int ic = i0;
-        const bool jin = j0 + 16 * q < ld;
+        const bool jin = j0 + 16 * q < ld && !skip;
         float *pc = p + 16 * q;
         if (q < 3) {
           fetch(v[(q + 1) & 1], q + 1);
@@ -940,6 +968,26 @@ __global__ void __launch_bounds__(256) k_gjb_mirror(T *__restrict__ A, int ld, i
   }
 }
 
+// second stream of an inversion and its two events
+struct GjSide {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t panel = nullptr, inverted = nullptr;
+  int open() {
+    M3_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    M3_CUDA(cudaEventCreateWithFlags(&panel, cudaEventDisableTiming));
+    M3_CUDA(cudaEventCreateWithFlags(&inverted, cudaEventDisableTiming));
+    return M3SPH_OK;
+  }
+  ~GjSide() {
+    if (stream) {
+      cudaStreamSynchronize(stream);
+      cudaStreamDestroy(stream);
+    }
+    if (panel) cudaEventDestroy(panel);
+    if (inverted) cudaEventDestroy(inverted);
+  }
+};
+
 // in-place inverse of the n x n SPD matrix A with row stride ld; work holds gj_work(n) values
 template <typename T>
 int gj_blocked_inverse(T *A, int ld, int n, T *work, cudaStream_t s) {
@@ -950,6 +998,7 @@ int gj_blocked_inverse(T *A, int ld, int n, T *work, cudaStream_t s) {
   const size_t ntile = (size_t)nbk * (nbk - 1) / 2;        // lower tiles outside a panel
   unsigned char *imgC = nullptr, *imgR = nullptr;
   int *err = nullptr;
+  M3_CUDA(cudaFuncSetAttribute(k_gjb_diag<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gj_smem<T>()));
   M3_CUDA(cudaFuncSetAttribute(k_gjb_panels<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gj_smem<T>()));
   if constexpr (sizeof(T) == 4) {
     imgC = reinterpret_cast<unsigned char *>(Ct + NB * npad);
@@ -960,14 +1009,32 @@ int gj_blocked_inverse(T *A, int ld, int n, T *work, cudaStream_t s) {
   } else {
     M3_CUDA(cudaFuncSetAttribute(k_gjb_update<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gj_smem<T>()));
   }
+  // Large matrices: the next diagonal block is updated and inverted on a second stream while the other tiles are
+  // updated on all SMs but one. That pays when the update (223 us at 116 blocks, with their square) is longer than the
+  // extra product of the diagonal block's CTA (35 us): from 48 blocks on.
+  GjSide side;
+  const bool ahead = sizeof(T) == 4 && nbk >= 48;
+  if (ahead) M3_TRY(side.open());
   for (int k = 0; k < nbk; ++k) {
     const int kb = k * NB, nb = std::min(NB, n - kb);
-    k_gjb_diag<T><<<1, 256, 0, s>>>(A, ld, kb, nb, Dinv, DinvT); count_launch();
-    k_gjb_panels<T><<<nbk, 256, gj_smem<T>(), s>>>(A, ld, n, k, nb, Dinv, DinvT, npad, R, Ct, imgC, imgR); count_launch();
+    if (!ahead || k == 0) {
+      k_gjb_diag<T><<<1, 256, 0, s>>>(A, ld, kb, nb, Dinv, DinvT, nullptr, nullptr, npad); count_launch();
+    } else {
+      M3_CUDA(cudaStreamWaitEvent(s, side.inverted, 0));
+    }
+    k_gjb_panels<T><<<dim3(nbk, GJ_PANEL_CTAS<T>), 256, gj_smem<T>(), s>>>(A, ld, n, k, nb, Dinv, DinvT, npad, R, Ct, imgC,
+                                                                            imgR); count_launch();
     if (nbk == 1) break;
+    if (ahead && k + 1 < nbk) {
+      const int kb1 = kb + NB, nb1 = std::min(NB, n - kb1);
+      M3_CUDA(cudaEventRecord(side.panel, s));
+      M3_CUDA(cudaStreamWaitEvent(side.stream, side.panel, 0));
+      k_gjb_diag<T><<<1, 256, gj_smem<T>(), side.stream>>>(A, ld, kb1, nb1, Dinv, DinvT, Ct, R, npad); count_launch();
+      M3_CUDA(cudaEventRecord(side.inverted, side.stream));
+    }
     if constexpr (sizeof(T) == 4) {
-      k_gjb_update_tc<<<(unsigned)std::min<size_t>(ntile, 152), gu::THREADS, gu::SMEM_ALLOC, s>>>(A, ld, n, k, ntile, imgC,
-                                                                                                  imgR, err);
+      k_gjb_update_tc<<<(unsigned)std::min<size_t>(ntile, ahead ? 151 : 152), gu::THREADS, gu::SMEM_ALLOC, s>>>(
+          A, ld, n, k, ahead ? k + 1 : -1, ntile, imgC, imgR, err);
     } else {
       k_gjb_update<T><<<(unsigned)ntile, 256, gj_smem<T>(), s>>>(A, ld, n, k, npad, R, Ct);
     }

@@ -67,3 +67,22 @@ def test_coarse_inverse_panel_edges(level, layers, built_lib):
     finally:
         d.set_option("coarse_f64_direct_max", 6000)
         d.close()
+
+
+def test_coarse_inverse_diagonal_block_ahead(built_lib):
+    """A coarsest level of 9,630 dofs, whose FP32 inverse updates and inverts each diagonal block beside the
+    other tiles, against the FP64 inverse, as above."""
+    from m3tet_sph_gb300 import stokes, workloads
+    w = workloads.make_workload('c2', level=3, nlayer=4, nmg=2)
+    d = stokes.DeviceMesh(w['levels'])
+    try:
+        r = np.random.default_rng(4).standard_normal(d.ndof)
+        out = []
+        for direct_max in (20000, 0):
+            d.set_option("coarse_f64_direct_max", direct_max)
+            d.setup(w['visc'], w['dens'], w['ifix'], w['vfix'], w['phys'], precision=0)
+            out.append(d.vcycle(r))
+        assert np.linalg.norm(out[1] - out[0]) < 1e-11 * np.linalg.norm(out[0])
+    finally:
+        d.set_option("coarse_f64_direct_max", 6000)
+        d.close()
