@@ -142,10 +142,10 @@ def peaks():
 # DRAM bytes per element of one streamed FP32 apply (both kernels), from the ncu capture of the
 # 491,520-element shell: (948.76 + 20.05 + 83.85 + 4.28) MB / 491,520
 TRAFFIC_PER_ELEMENT_F32 = (948.76e6 + 20.05e6 + 83.85e6 + 4.28e6) / 491520
-# the same for the partially assembled FP32 apply (k_pa_elem_f32 + k_node_gather_f32)
-TRAFFIC_PER_ELEMENT_PA = (289.01e6 + 19.20e6 + 83.85e6 + 4.28e6) / 491520
+# the same for the partially assembled FP32 apply (k_pa_tile + k_pa_gather)
+TRAFFIC_PER_ELEMENT_PA = (298.76e6 + 3.92e6 + 36.30e6) / 491520
 # the same for the double-float outer apply (k_stream_rowlane<RlDF> + k_node_gather_f64)
-TRAFFIC_PER_ELEMENT_DF = (1.900e9 + 72.74e6 + 190.52e6 + 10.03e6) / 491520
+TRAFFIC_PER_ELEMENT_DF = (1.892e9 + 68.02e6 + 233.59e6 + 9.67e6) / 491520
 
 
 def algorithmic_apply_bytes(nel, ndof, nvnod, s):
@@ -162,9 +162,10 @@ def apply_bytes_df(nel, ndof):
 
 
 def apply_bytes_pa(nel, ndof, nnod):
-    """Bytes one partially assembled FP32 apply streams: 14 x 9 FP32 factors, a free-dof word and
-    10 int32 connectivity entries per element, 16 B of rotation angles per node, x and y in FP32."""
-    return nel * (504 + 4 + 40) + 16 * nnod + 2 * 4 * ndof
+    """Bytes one partially assembled FP32 apply streams: per element 14 x 9 FP32 factors, 10 int32
+    connectivity entries, 10 2-byte table entries and about 3 tile nodes (8 B of table, 16 B written
+    and read back); per node 16 B of operand and 16 B of rotation; y in FP32."""
+    return nel * (504 + 40 + 20 + 3 * (8 + 16 + 16)) + 32 * nnod + 4 * ndof
 
 
 def apply_bytes(nel, ndof, s):
@@ -248,7 +249,7 @@ def run_gb300(args, rank, ws, td):
     bdf = apply_bytes_df(nel, ndof)
     if args.fp32_operator:
         b32 = apply_bytes_pa(nel, ndof, ndof // 3)
-        fp32 = {"kernel": "finest-level FP32 apply, partially assembled: k_pa_elem_f32 + k_node_gather_f32",
+        fp32 = {"kernel": "finest-level FP32 apply, partially assembled: k_pa_tile + k_pa_gather",
                 "traffic": TRAFFIC_PER_ELEMENT_PA * nel, "streamed_basis": "per-point geometric factors"}
     else:
         b32 = apply_bytes(nel, ndof, 4)
