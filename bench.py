@@ -162,10 +162,10 @@ def apply_bytes_df(nel, ndof):
 
 
 def apply_bytes_pa(nel, ndof, nnod):
-    """Bytes one partially assembled FP32 apply streams: per element 14 x 9 FP32 factors, 10 int32
-    connectivity entries, 10 2-byte table entries and about 3 tile nodes (8 B of table, 16 B written
-    and read back); per node 16 B of operand and 16 B of rotation; y in FP32."""
-    return nel * (504 + 40 + 20 + 3 * (8 + 16 + 16)) + 32 * nnod + 4 * ndof
+    """Bytes one partially assembled FP32 apply streams, the tile tables and tile sums left out: 14 x 9
+    FP32 factors, a 4-byte word and 10 int32 connectivity entries per element, 16 B of rotation angles
+    per node, x and y in FP32."""
+    return nel * (504 + 4 + 40) + 16 * nnod + 2 * 4 * ndof
 
 
 def apply_bytes(nel, ndof, s):
