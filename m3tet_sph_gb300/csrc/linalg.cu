@@ -991,6 +991,7 @@ struct GjSide {
 // in-place inverse of the n x n SPD matrix A with row stride ld; work holds gj_work(n) values
 template <typename T>
 int gj_blocked_inverse(T *A, int ld, int n, T *work, cudaStream_t s) {
+  if (n == 0) return M3SPH_OK;         // every dof prescribed: nothing to invert, and no grid to launch
   constexpr int NB = Gj<T>::NB;
   const int nbk = (n + NB - 1) / NB;
   const size_t npad = (size_t)nbk * NB;

@@ -61,3 +61,28 @@ def test_17k_coarsest_level(built_lib):
         assert np.linalg.norm(U - U0) < 1e-8 * np.linalg.norm(U0), name
         assert np.linalg.norm(P - P0) < 1e-8 * np.linalg.norm(P0), name
     assert abs(its["fp64 refined"] - its["fp64 inverse"]) <= 2
+
+
+@pytest.mark.parametrize("precision,direct_max", [(0, 6000), (0, 0), (1, 6000)])
+def test_coarsest_level_without_free_dofs(built_lib, tiny_plates, precision, direct_max):
+    """Every velocity dof prescribed: the set-up succeeds, the force vector is the one of a set-up with
+    free dofs (it does not depend on them) and a V-cycle gives zero."""
+    from m3tet_sph_gb300 import stokes
+    w = tiny_plates
+    dm = stokes.DeviceMesh(w['levels'])
+    try:
+        dm.setup(w['visc'], w['dens'], w['ifix'], w['vfix'], w['phys'], precision=precision)
+        f = dm.force()
+        rng = np.random.default_rng(8)
+        dm.set_option("coarse_f64_direct_max", direct_max)
+        dm.setup(w['visc'], w['dens'], np.arange(dm.ndof), rng.standard_normal(dm.ndof), w['phys'],
+                 precision=precision)
+        assert np.array_equal(dm.force(), f)
+        assert not dm.element_matrices()[0].any()
+        assert not dm.vcycle(rng.standard_normal(dm.ndof)).any()
+        # the next set-up has free dofs again
+        dm.setup(w['visc'], w['dens'], w['ifix'], w['vfix'], w['phys'], precision=precision)
+        assert dm.vcycle(rng.standard_normal(dm.ndof)).any()
+    finally:
+        dm.set_option("coarse_f64_direct_max", 6000)
+        dm.close()
