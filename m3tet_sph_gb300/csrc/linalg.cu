@@ -83,6 +83,7 @@ __global__ void k_cg_dir(const T *__restrict__ d, double *__restrict__ q, size_t
     q[i] = first ? (double)d[i] : (double)d[i] + beta * q[i];
 }
 // alpha = rd / qKq ; x += alpha q ; r -= alpha Kq (and its FP32 copy) ; rr, rdlast, alpha_prev, first = 0.
+// A NaN step (a NaN right-hand side, or a breakdown) leaves x as it is; the NaN residual then ends the loop.
 // Then whether the loop goes on: it ends when the residual is below the tolerance or NaN, at the iteration
 // limit, or, with the learned smoother, at a contraction factor above 0.95 (or growth). `loop` is the condition of
 // the captured loop around the iteration (0: the host runs it).
@@ -91,9 +92,10 @@ __global__ void k_cg_update(double *__restrict__ x, double *__restrict__ r, cons
                             double *partials, unsigned *cnt, cudaGraphConditionalHandle loop) {
   grid_dep();
   const double rd = scal[0], alpha = rd / scal[2];
+  const bool step = !isnan(alpha);
   double v[1] = {0.0};
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    x[i] += alpha * q[i];
+    if (step) x[i] += alpha * q[i];
     const double ri = r[i] - alpha * Kq[i];
     r[i] = ri;
     if (r32) r32[i] = (float)ri;

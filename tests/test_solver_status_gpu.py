@@ -92,3 +92,23 @@ def test_calculate_dt_matches_oracle(dm_plates):
         dt, adv = dm.calculate_dt(limit, dtmax)
         dt_r, adv_r = O.calculate_dt(X, U[0::3], U[1::3], U[2::3], limit, dtmax)
         assert dt == dt_r and adv == adv_r, (limit, dtmax, dt, dt_r)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("is_abs_tol", [False, True])
+def test_nan_right_hand_side_leaves_the_iterate(dm_plates, precision, is_abs_tol):
+    """A NaN right-hand side is an error with either kind of tolerance, and the resident velocity is
+    the initial guess afterwards, bit for bit."""
+    from m3tet_sph_gb300 import _lib as L
+    w, dm = dm_plates
+    dm.setup(w['visc'], w['dens'], w['ifix'], w['vfix'], w['phys'], precision=precision)
+    rng = np.random.default_rng(12)
+    x0, b = rng.standard_normal(dm.ndof), rng.standard_normal(dm.ndof)
+    dm.mgpcg(b, x0, 1e-3, is_abs_tol, itmax=0)          # x0 is the resident velocity now
+    U0, _ = dm.solution()
+    free = np.setdiff1d(np.arange(dm.ndof), w['ifix'])
+    b[free[len(free) // 2]] = np.nan
+    with pytest.raises(L.M3SphError, match='RHS vector contains NaNs') as ei:
+        dm.mgpcg(b, x0, 1e-3, is_abs_tol, itmax=7)
+    assert ei.value.code == 3
+    assert np.array_equal(dm.solution()[0], U0)
