@@ -295,7 +295,9 @@ M3SPH_API int m3sph_ml_sweep32(m3sph_mesh *mesh, int32_t img, const float *r, co
  * kernel, 0-3, default 0), "coarse_f64_direct_max" (plain FP64 path: coarsest levels up to this many
  * dofs get an FP64 dense inverse, larger ones the FP32 inverse refined against the FP64 coarsest
  * operator in every coarse solve; default 6000; takes effect at the next set-up), "coarse_refine_sweeps"
- * (refinement steps of that solve, default 3). */
+ * (refinement steps of that solve, default 3), "wait_error" (sets the error words that bounded waits of the
+ * kernels set when they give up, 1 the streamed products', 2 the learned sweep's: the next call that uses them
+ * reports M3SPH_ERR_CUDA and clears them; for checks of the error handling). */
 M3SPH_API int m3sph_set_option(m3sph_mesh *mesh, const char *name, int32_t value);
 /* Cumulative number of CUDA kernels this library has launched (all handles). */
 M3SPH_API int m3sph_launch_count(unsigned long long *count);

@@ -286,7 +286,7 @@ struct Finest {
 
 // state of a velocity solve's CG, at scal + CG_STATE: the host sets it, the step kernel ends the loop
 enum { CG_STATE = 24, CG_TOL = 24, CG_SQ, CG_PREV, CG_IT, CG_LIMIT, CG_LEARNED, CG_STATUS, CG_RR0, CG_STATE_END };
-enum { CG_RUN = 0, CG_CONVERGED, CG_NAN, CG_STALLED, CG_LIMIT_REACHED };
+enum { CG_RUN = 0, CG_CONVERGED, CG_NAN, CG_STALLED, CG_LIMIT_REACHED, CG_WAIT_ERROR };
 constexpr int CG_LOOP_MAX = 256;    // iterations of a captured loop before the host looks at it
 
 struct Coarse {
@@ -317,6 +317,11 @@ __device__ __forceinline__ float4 pa_to_cart(const float4 tr, float x0, float x1
 // threads of a node-sum pass that go to the nv vertices, four each, in whole warps; edge nodes follow, one
 // thread each
 __host__ __device__ __forceinline__ int gather_threads4(int nv) { return (4 * nv + 31) & ~31; }
+
+// error words that bounded waits set when they give up (either may be null)
+struct WaitWords {
+  const int *w[2];
+};
 
 // scratch of a grid reduction
 struct Reduction {
@@ -358,6 +363,7 @@ int ml_sweep(m3sph_mesh *M, int j, const T *r0, const T *kd, const T *Dinv, T *t
 int ml_init_kernels();
 int ml_set_infer(int v);
 int ml_check(m3sph_mesh *M);
+int *ml_error_word(m3sph_mesh *M);
 bool ml_ready(m3sph_mesh *M);
 int ml_add_samples(m3sph_mesh *M, const double *r, const double *err, int stride, int offset);
 int ml_reserve(m3sph_mesh *M, long cap);

@@ -84,12 +84,13 @@ __global__ void k_cg_dir(const T *__restrict__ d, double *__restrict__ q, size_t
 }
 // alpha = rd / qKq ; x += alpha q ; r -= alpha Kq (and its FP32 copy) ; rr, rdlast, alpha_prev, first = 0.
 // A NaN step (a NaN right-hand side, or a breakdown) leaves x as it is; the NaN residual then ends the loop.
-// Then whether the loop goes on: it ends when the residual is below the tolerance or NaN, at the iteration
-// limit, or, with the learned smoother, at a contraction factor above 0.95 (or growth). `loop` is the condition of
-// the captured loop around the iteration (0: the host runs it).
+// Then whether the loop goes on: it ends when a bounded wait of the iteration's kernels gave up (their error
+// words, wait_err; the products are then wrong), when the residual is below the tolerance or NaN, at the
+// iteration limit, or, with the learned smoother, at a contraction factor above 0.95 (or growth). `loop` is the
+// condition of the captured loop around the iteration (0: the host runs it).
 __global__ void k_cg_update(double *__restrict__ x, double *__restrict__ r, const double *__restrict__ q,
                             const double *__restrict__ Kq, float *__restrict__ r32, size_t n, double *scal,
-                            double *partials, unsigned *cnt, cudaGraphConditionalHandle loop) {
+                            double *partials, unsigned *cnt, WaitWords wait_err, cudaGraphConditionalHandle loop) {
   grid_dep();
   const double rd = scal[0], alpha = rd / scal[2];
   const bool step = !isnan(alpha);
@@ -108,7 +109,10 @@ __global__ void k_cg_update(double *__restrict__ x, double *__restrict__ r, cons
     scal[6] = 0.0;
     const double rrms = sqrt(v[0]) / scal[CG_SQ], it = scal[CG_IT] + 1.0, prev = scal[CG_PREV];
     const bool last = it >= scal[CG_LIMIT], stalled = it > 1.0 && rrms > 0.95 * prev;
-    const int status = isnan(rrms) ? CG_NAN
+    bool gave_up = false;
+    for (const int *w : wait_err.w) gave_up |= w && __ldcg(w) != 0;
+    const int status = gave_up ? CG_WAIT_ERROR
+                       : isnan(rrms) ? CG_NAN
                        : rrms < scal[CG_TOL] ? CG_CONVERGED
                        : scal[CG_LEARNED] != 0.0 && (stalled || last) ? CG_STALLED
                        : last ? CG_LIMIT_REACHED : CG_RUN;
@@ -128,8 +132,8 @@ int cg_dir(const T *d, double *q, size_t n, const double *scal, cudaStream_t s) 
 template int cg_dir<double>(const double *, double *, size_t, const double *, cudaStream_t);
 template int cg_dir<float>(const float *, double *, size_t, const double *, cudaStream_t);
 int cg_update(double *x, double *r, const double *q, const double *Kq, float *r32, size_t n, double *scal,
-              double *partials, unsigned *cnt, cudaGraphConditionalHandle loop, cudaStream_t s) {
-  launch_pdl(k_cg_update, red_blocks(n), RED_THREADS, 0, s, x, r, q, Kq, r32, n, scal, partials, cnt, loop);
+              double *partials, unsigned *cnt, WaitWords wait_err, cudaGraphConditionalHandle loop, cudaStream_t s) {
+  launch_pdl(k_cg_update, red_blocks(n), RED_THREADS, 0, s, x, r, q, Kq, r32, n, scal, partials, cnt, wait_err, loop);
   count_launch();
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;

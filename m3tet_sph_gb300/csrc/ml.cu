@@ -928,6 +928,8 @@ int ml_set_infer(int v) {
   return M3SPH_OK;
 }
 
+int *ml_error_word(m3sph_mesh *M) { return mls(M) ? mls(M)->err : nullptr; }
+
 int ml_check(m3sph_mesh *M) {
   MlState *S = mls(M);
   if (!S || !S->err) return M3SPH_OK;

@@ -68,7 +68,7 @@ int dot2(const double *a, const double *c, const T *b, size_t n, double *partial
 int vsum(const double *a, size_t n, double *partials, unsigned *cnt, double *out, cudaStream_t s);
 template <typename T> int cg_dir(const T *d, double *q, size_t n, const double *scal, cudaStream_t s);
 int cg_update(double *x, double *r, const double *q, const double *Kq, float *r32, size_t n, double *scal,
-              double *partials, unsigned *cnt, cudaGraphConditionalHandle loop, cudaStream_t s);
+              double *partials, unsigned *cnt, WaitWords wait_err, cudaGraphConditionalHandle loop, cudaStream_t s);
 int residual(const double *b, double *y, const uint8_t *mask, float *y32, size_t n, double *partials, unsigned *cnt,
              double *out, cudaStream_t s);
 int apply_mask(double *y, const uint8_t *mask, size_t n, cudaStream_t s);
@@ -1187,6 +1187,12 @@ static int read_scal(m3sph_mesh *M, int idx, double &v) {
   return M3SPH_OK;
 }
 
+// reads and clears the error words of the bounded waits behind the V-cycle and the outer product
+static int check_waits(m3sph_mesh *M) {
+  const int a = stream_check(M->lev[0], M->stream), b = ml_check(M);
+  return a ? a : b;
+}
+
 struct CgState { double v[CG_STATE_END - CG_STATE]; };
 // CG_RR0 is kept at the first call of a solve from the initial residual (scal[3])
 __global__ void k_cg_state(double *scal, CgState st, double first) {
@@ -1213,7 +1219,8 @@ static int cg_iteration(m3sph_mesh *M, double *x, cudaGraphConditionalHandle loo
     M3_TRY(cg_dir<float>(W->d32[0], W->q, n, M->scal, s));
   }
   M3_TRY(outer_apply(M, W->q, W->Kq, true));
-  return cg_update(x, W->r, W->q, W->Kq, M->precision ? W->r32[0] : nullptr, n, M->scal, M->red, M->red_cnt, loop, s);
+  return cg_update(x, W->r, W->q, W->Kq, M->precision ? W->r32[0] : nullptr, n, M->scal, M->red, M->red_cnt,
+                   WaitWords{{L0.sa_err, ml_error_word(M)}}, loop, s);
 }
 
 // The loop over iterations, captured once per solution-vector pointer: a graph of one conditional node whose body
@@ -1314,6 +1321,11 @@ static int mgpcg(m3sph_mesh *M, const double *b, double *x, double tol, bool abs
       if (M->use_graphs) add_launches(g.kernels * (unsigned long long)(it - it0));
       st.nvc += (int)(it - it0);
     } while (status == CG_RUN);
+    if (status == CG_WAIT_ERROR) {
+      M3_TRY(check_waits(M));
+      set_error("velocity CG: a bounded wait gave up");
+      return M3SPH_ERR_CUDA;
+    }
     if (status == CG_NAN) {
       if (std::isnan(val(CG_RR0))) return rhs_nan();
       set_error("NaN in MG-PCG residual");
@@ -1583,8 +1595,7 @@ static int solve_core(m3sph_mesh *M, const m3sph_opts *opts, m3sph_info &inf) {
   double rel = 0.0;
   M3_TRY(coupled_residual(M, U, Pd, rel));
   inf.rel_residual = rel;
-  M3_TRY(stream_check(L0, s));
-  M3_TRY(ml_check(M));
+  M3_TRY(check_waits(M));
   // The reference returns its last iterate silently when itmax_Pat runs out or after the second
   // convergence problem (flow3d_patera_mg_sph_p.m:580-606); here the iterate is still returned, but
   // with M3SPH_ERR_NOT_CONVERGED. With a target the final coupled residual decides.
@@ -2067,6 +2078,7 @@ extern "C" int m3sph_vcycle(m3sph_mesh *M, const double *r, double *d) {
   if (M->precision) M3_TRY(d2f(W->tmp, W->r32[0], n, s));
   M3_TRY(vcycle(M, W->tmp, W->d));
   if (M->precision) M3_TRY(f2d(W->d32[0], W->d, n, s));
+  M3_TRY(check_waits(M));
   M3_CUDA(cudaMemcpyAsync(d, W->d, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
   M3_CUDA(cudaStreamSynchronize(s));
   return M3SPH_OK;
@@ -2084,6 +2096,7 @@ extern "C" int m3sph_mgpcg(m3sph_mesh *M, const double *b, double *x, double tol
   M3_CUDA(cudaMemcpyAsync(W->U, x, sizeof(double) * n, cudaMemcpyHostToDevice, s));
   CGStats cs;
   M3_TRY(mgpcg(M, W->Rhs, W->U, tol, is_abs_tol != 0, itmax, cs));
+  M3_TRY(check_waits(M));
   M3_CUDA(cudaMemcpyAsync(x, W->U, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
   M3_CUDA(cudaStreamSynchronize(s));
   if (itCG) *itCG = cs.it;
@@ -2185,6 +2198,17 @@ extern "C" int m3sph_set_option(m3sph_mesh *M, const char *name, int32_t value) 
     g_split_apply = value != 0;
   } else if (n == "graphs") {
     M->use_graphs = value != 0;
+  } else if (n == "wait_error") {
+    // the words as a wait that gave up leaves them: 1 the streamed products', 2 the learned sweep's
+    if (value < 1 || value > 3 || ((value & 2) && !ml_error_word(M))) {
+      set_error("wait_error must be 1 (streamed products), 2 (learned sweep) or 3 (both)");
+      return M3SPH_ERR_BAD_INPUT;
+    }
+    M3_CUDA(cudaSetDevice(M->device));
+    M3_CUDA(cudaStreamSynchronize(M->stream));
+    const int one = 1;
+    if (value & 1) M3_CUDA(cudaMemcpy(M->lev[0].sa_err, &one, sizeof(int), cudaMemcpyHostToDevice));
+    if (value & 2) M3_CUDA(cudaMemcpy(ml_error_word(M), &one, sizeof(int), cudaMemcpyHostToDevice));
   } else if (n == "df_outer") {
     M->df_outer = value != 0;
   } else if (n == "coarse_f64_direct_max") {

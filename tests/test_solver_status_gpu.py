@@ -112,3 +112,44 @@ def test_nan_right_hand_side_leaves_the_iterate(dm_plates, precision, is_abs_tol
         dm.mgpcg(b, x0, 1e-3, is_abs_tol, itmax=7)
     assert ei.value.code == 3
     assert np.array_equal(dm.solution()[0], U0)
+
+
+@pytest.mark.parametrize("word", [1, 2, 3])
+@pytest.mark.parametrize("graphs", [0, 1])
+def test_a_wait_that_gave_up_is_reported(dm_plates, graphs, word):
+    """With the error word of a bounded wait set (as a kernel sets it whose wait gives up, so that its
+    products are wrong), the V-cycle, the velocity CG and the solve fail instead of returning a result,
+    the CG ends with the iteration that saw it, and the call after is clean."""
+    import ctypes as C
+    from m3tet_sph_gb300 import _lib as L, learned
+    w, dm = dm_plates
+    dm.setup(w['visc'], w['dens'], w['ifix'], w['vfix'], w['phys'], precision=1)
+    learned.set_params(dm, np.load(Path(learned.__file__).with_name('smoother_c1.npy')), trained=True)
+
+    def launches():
+        n = C.c_ulonglong()
+        L.check(L.lib().m3sph_launch_count(C.byref(n)))
+        return n.value
+
+    rng = np.random.default_rng(9)
+    b, x0 = rng.standard_normal(dm.ndof), np.zeros(dm.ndof)
+    calls = (lambda: dm.vcycle(b), lambda: dm.mgpcg(b, x0, 0.0, True, 60)[0],
+             lambda: dm.mgpcg(b, x0, 0.0, True, 0)[0], lambda: dm.solve(rtol_Pat=1e-4, allow_not_converged=True)[0])
+    try:
+        dm.set_option("graphs", graphs)
+        dm.mgpcg(b, x0, 0.0, True, 1)                    # captures the loop
+        n0 = launches()
+        dm.mgpcg(b, x0, 0.0, True, 1)
+        n1 = launches()
+        for k, call in enumerate(calls):
+            want = call()
+            dm.set_option("wait_error", word)
+            n2 = launches()
+            with pytest.raises(L.M3SphError, match='bounded wait') as ei:
+                call()
+            assert ei.value.code == L.ERR_CUDA
+            if k == 1:
+                assert launches() - n2 == n1 - n0
+            assert np.array_equal(call(), want)
+    finally:
+        dm.set_option("graphs", 1)
