@@ -281,14 +281,14 @@ __global__ void __launch_bounds__(256) k_diff_rowprod(int nnod, const int *__res
   if (!block_reduce_last<2>(v, partials, cnt) || threadIdx.x) return;
   if (MODE == DP_RESID) {
     // pcg_solver_p.m: the tolerance is relative to the initial residual. A residual that is exactly zero
-    // (a field the step leaves unchanged) or below it is converged
+    // (a field the step leaves unchanged) or below it is converged; a NaN one is an error
     scal[DS_RR] = v[0];
     scal[DS_TOL2] = tol * tol * v[0];
     scal[DS_RD] = v[1];
     scal[DS_BETA] = 0.0;
-    scal[DS_DONE] = (v[0] < tol * tol * v[0] || v[0] == 0.0) ? 1.0 : 0.0;
+    scal[DS_DONE] = (v[0] < tol * tol * v[0] || v[0] == 0.0 || isnan(v[0])) ? 1.0 : 0.0;
     scal[DS_IT] = 0.0;
-    scal[DS_BAD] = 0.0;
+    scal[DS_BAD] = isnan(v[0]) ? 1.0 : 0.0;
   } else {
     scal[DS_ALPHA] = scal[DS_RD] / v[0];
   }
@@ -495,7 +495,7 @@ int diffusion_resident(m3sph_mesh *M, double *T, double dt, int *nit) {
     M3_CUDA(cudaGetLastError());
     M3_CUDA(cudaMemcpyAsync(h, D->scal, sizeof(h), cudaMemcpyDeviceToHost, s));
     M3_CUDA(cudaStreamSynchronize(s));
-    if (h[DS_DONE] != 0.0 || std::isnan(h[DS_RR])) break;
+    if (h[DS_DONE] != 0.0) break;
     for (int k = 0; k < DIFF_CHECK; ++k) {
       k_diff_dir<<<red_blocks(n), 256, 0, s>>>(n, D->r, D->Mi, D->q, D->scal); count_launch();
       k_diff_rowprod<DP_CG><<<gr, 256, 0, s>>>(n, D->sptr, D->rlen, D->rcol, D->rval, D->ML, D->q, c, D->fixmask, D->Aq,

@@ -96,3 +96,23 @@ def test_diffusion_iteration_limit(case, itmax):
     Tr, nitr = D.step(T0, 5000.0, T0[fix], tol=1e-300, itmax=itmax)
     assert nit == nitr == itmax
     assert np.max(np.abs(T - Tr)) <= 1e-10 * np.max(np.abs(T0))
+
+
+@pytest.mark.parametrize("where", ["free", "fixed value"])
+def test_diffusion_of_a_nan_is_an_error(case, where):
+    """A NaN temperature (or prescribed one) makes the initial residual NaN: an error, as a NaN that
+    comes up in a later iteration is, and not a converged field."""
+    from m3tet_sph_gb300 import _lib as L
+    w, dm = case
+    f = w['levels'][0]
+    T0 = 2500.0 * w['T']
+    fix = np.nonzero(f['PointID'] > 0)[0]
+    v = T0[fix].copy()
+    if where == "free":
+        T0[np.setdiff1d(np.arange(f['nnod']), fix)[11]] = np.nan
+    else:
+        v[5] = np.nan
+    dm.diffusion_setup(KAPPA, fix, v)
+    with pytest.raises(L.M3SphError, match='NaN') as ei:
+        dm.diffusion(T0, 50.0)
+    assert ei.value.code == L.ERR_NAN
