@@ -52,6 +52,7 @@ struct DiffState {
   int fixcap = 0;
   double *scal = nullptr;              // CG scalars (DS_*)
   int *err = nullptr;
+  bool ready = false;                  // a set-up has run to its end
 };
 
 static DiffState *diff_state(m3sph_mesh *M) { return reinterpret_cast<DiffState *>(M->diff); }
@@ -470,7 +471,7 @@ static int diff_integrate(m3sph_mesh *M, DiffState *D) {
 // one diffusion3d_p step on the device-resident T (nnod) over dt; *nit = PCG iterations
 int diffusion_resident(m3sph_mesh *M, double *T, double dt, int *nit) {
   DiffState *D = diff_state(M);
-  if (!D) {
+  if (!D || !D->ready) {
     set_error("diffusion not set up (call m3sph_diffusion_setup)");
     return M3SPH_ERR_BAD_INPUT;
   }
@@ -525,27 +526,35 @@ extern "C" int m3sph_diffusion_setup(m3sph_mesh *M, const m3sph_diffusion_opts *
   }
   M3_CUDA(cudaSetDevice(M->device));
   cudaStream_t s = M->stream;
-  DiffState *D = diff_state(M);
-  if (!D) {
-    D = new DiffState();
-    M->diff = D;
-    M->diff_free = diff_free;
-    M3_TRY(diff_build(M, D, o->theta_cone > 0 ? o->theta_cone : 45.0));
-  }
-  D->kappa = o->kappa;
-  D->theta = o->theta;
-  D->tol = o->tol > 0 ? o->tol : 1e-8;
-  D->itmax = o->itmax > 0 ? o->itmax : 500;
+  // the list is checked first: a set-up refused for it leaves an earlier one as it was
+  const int nnod = M->lev[0].nnod;
   std::vector<int> fx(nfix);
-  std::vector<uint8_t> mask(D->nnod, 0);
+  std::vector<uint8_t> mask(nnod, 0);
   for (int i = 0; i < nfix; ++i) {
-    if (ifix[i] < 1 || ifix[i] > D->nnod) {
+    if (ifix[i] < 1 || ifix[i] > nnod) {
       set_error("m3sph_diffusion_setup: ifix entry out of range");
       return M3SPH_ERR_BAD_INPUT;
     }
     fx[i] = ifix[i] - 1;
     mask[fx[i]] = 1;
   }
+  DiffState *D = diff_state(M);
+  if (!D) {
+    // a state that could not be built is not kept, so that no later call takes it for a set-up
+    D = new DiffState();
+    const int st = diff_build(M, D, o->theta_cone > 0 ? o->theta_cone : 45.0);
+    if (st) {
+      diff_free(D);
+      return st;
+    }
+    M->diff = D;
+    M->diff_free = diff_free;
+  }
+  D->ready = false;                    // until every array below holds this set-up
+  D->kappa = o->kappa;
+  D->theta = o->theta;
+  D->tol = o->tol > 0 ? o->tol : 1e-8;
+  D->itmax = o->itmax > 0 ? o->itmax : 500;
   D->nfix = nfix;
   if (nfix > D->fixcap || !D->ifix) {
     if (D->ifix) cudaFree(D->ifix);
@@ -563,6 +572,7 @@ extern "C" int m3sph_diffusion_setup(m3sph_mesh *M, const m3sph_diffusion_opts *
   M3_CUDA(cudaMemcpyAsync(D->fixmask, mask.data(), D->nnod, cudaMemcpyHostToDevice, s));
   M3_TRY(diff_integrate(M, D));
   M3_CUDA(cudaStreamSynchronize(s));
+  D->ready = true;
   return M3SPH_OK;
 }
 
@@ -573,7 +583,7 @@ extern "C" int m3sph_diffusion3d(m3sph_mesh *M, double *T, double dt, int32_t *n
   }
   M3_CUDA(cudaSetDevice(M->device));
   DiffState *D = diff_state(M);
-  if (!D) {
+  if (!D || !D->ready) {
     set_error("m3sph_diffusion3d: call m3sph_diffusion_setup first");
     return M3SPH_ERR_BAD_INPUT;
   }

@@ -116,3 +116,28 @@ def test_diffusion_of_a_nan_is_an_error(case, where):
     with pytest.raises(L.M3SphError, match='NaN') as ei:
         dm.diffusion(T0, 50.0)
     assert ei.value.code == L.ERR_NAN
+
+
+def test_refused_diffusion_setup(built_lib, tiny_plates):
+    """A set-up that is refused is not a set-up: without an earlier one the diffusion call says so, and
+    an earlier one stays as it was."""
+    from m3tet_sph_gb300 import _lib as L, stokes
+    w = tiny_plates
+    f = w['levels'][0]
+    T0 = 2500.0 * w['T']
+    fix = np.nonzero(f['PointID'] > 0)[0]
+    dm = stokes.DeviceMesh(w['levels'])
+    try:
+        for round_ in range(2):
+            for bad in (f['nnod'], -1):
+                with pytest.raises(L.M3SphError, match='out of range'):
+                    dm.diffusion_setup(7 * KAPPA, np.append(fix, bad), np.append(T0[fix], 0.0), theta=0.5, itmax=3)
+            if round_ == 0:
+                with pytest.raises(L.M3SphError, match='m3sph_diffusion_setup first'):
+                    dm.diffusion(T0, 50.0)
+                dm.diffusion_setup(KAPPA, fix, T0[fix])
+                T, nit = dm.diffusion(T0, 50.0)
+        T2, nit2 = dm.diffusion(T0, 50.0)
+        assert nit2 == nit and np.array_equal(T2, T)
+    finally:
+        dm.close()
