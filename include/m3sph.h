@@ -280,10 +280,10 @@ M3SPH_API int m3sph_ml_features(m3sph_mesh *mesh, int32_t img, const float *z, f
 M3SPH_API int m3sph_ml_sweep32(m3sph_mesh *mesh, int32_t img, const float *r, const float *kd, float *d);
 
 /* Kernel-variant switches for measurement and tests (per process, results equal to rounding):
- * "stream_apply" (streamed finest-level FP32 operator, default 1; 0: one launch per colour),
+ * "stream_apply" (streamed finest-level FP32 operator, default 1; 0: element products by plain loads),
  * "stream_outer" (streamed double-float / FP64 finest-level operators, default 1),
  * "stream_outer_variant" (warp layout of the double-float kernel, 0-7, default 4),
- * "split_apply" (4-warp per-colour kernels when streaming is off, default 1), "graphs" (CUDA-graph
+ * "split_apply" (when streaming is off: 1 four warps per 32 elements, default; 0 one thread per element), "graphs" (CUDA-graph
  * replay of MG-PCG iterations, default 1), "df_outer" (double-float outer operator on the mixed
  * path, default 1), "ml_schedule" (learned smoothing on the two finest levels: 0 learned-Jacobi-
  * learned, 1 one learned sweep per side (default), 3 learned + one Jacobi sweep per side; 2 one

@@ -403,7 +403,7 @@ struct m3sph_mesh {
   std::vector<CgGraph> graphs;        // captured MG-PCG loops and their kernels per iteration
   bool use_graphs = true;
   bool df_outer = true;               // double-float outer operator on the mixed path
-  bool split_apply = true;            // 4-warp split element-by-element kernels on the finest level
+  bool split_apply = true;            // 4-warp split element products where the streamed ones are off
   int ml_schedule = 1;                // learned smoothing per side: 0 learned-Jacobi-learned, 1 one learned sweep
   float ml_omega = 1.0f;              // relaxation weight of the learned correction
   void *ml = nullptr;                 // learned smoother state

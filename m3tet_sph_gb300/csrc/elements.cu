@@ -1,5 +1,5 @@
 // Element-level kernels: curved P2P1 element matrices (double Jacobian), element-by-element
-// operator application with a coloured, atomic-free scatter, and element-wise Galerkin
+// products with fixed-order node sums (no atomics), and element-wise Galerkin
 // coarse operators.
 //
 // Reference behaviour restated (paths inside the reference project):
@@ -15,6 +15,9 @@
 #include "common.cuh"
 
 namespace m3sph {
+
+int node_sums(const Level &L, float *y, cudaStream_t s);
+int node_sums(const Level &L, double *y, cudaStream_t s);
 
 __constant__ ShapeTables c_sf;
 
@@ -372,8 +375,22 @@ int launch_element_setup(const SetupArgs &a, cudaStream_t s) {
 }
 
 // ----------------------------------------------------------------------------------------
-// element-by-element y += K x over one colour (no two elements of a colour share a node)
+// element products of the finest level without the streamed kernels' rings (options stream_apply and
+// stream_outer 0): element outputs, 30 consecutive values each, which the node passes of the streamed
+// kernels sum. At 245,760 elements, FP32 / double-float / FP64, product and sums: 92 / 329 / 412 us with one
+// thread per element, 147 / 741 / 512 us with four warps per 32 elements. (One launch per colour, adding to the
+// nodes: 0.93 / 2.31 / 2.04 ms and 0.89 / 1.54 / 1.49 ms with elements stored in colour order, 1.20 / 2.48 / 2.47
+// ms and 1.30 / 2.02 / 2.27 ms through a list of the colours' elements.)
+//
+// One thread per element (split_apply 0), outputs staged in shared memory
 // ----------------------------------------------------------------------------------------
+constexpr int EBE_T = 64;
+template <typename T> __device__ __forceinline__ void ebe_store(T (*sy)[31], int e0, int nel, T *__restrict__ out) {
+  __syncthreads();
+  const int nv = min(EBE_T, nel - e0) * 30;
+  T *o = out + (size_t)e0 * 30;
+  for (int i = threadIdx.x; i < nv; i += EBE_T) o[i] = sy[i / 30][i % 30];
+}
 template <typename T> struct Vec;
 template <> struct Vec<float> { using type = float4; };
 template <> struct Vec<double> { using type = double2; };
@@ -386,14 +403,12 @@ template <> __device__ __forceinline__ double lane<double2, double>(const double
 }
 
 template <typename T>
-__global__ void __launch_bounds__(128) k_ebe_apply(const T *__restrict__ K, const int *__restrict__ el2nod, int nel,
-                                                   const int *__restrict__ corder, int e_begin, int e_end,
-                                                   const T *__restrict__ x, T *__restrict__ y) {
+__global__ void __launch_bounds__(EBE_T) k_ebe_apply(const T *__restrict__ K, const int *__restrict__ el2nod, int nel,
+                                                    const T *__restrict__ x, T *__restrict__ out) {
   using VT = typename Vec<T>::type;
   constexpr int V = KVec<T>::V;
-  const int i0 = e_begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i0 >= e_end) return;
-  const int e = corder[i0];
+  __shared__ T sy[EBE_T][31];
+  const int e0 = blockIdx.x * EBE_T, e = min(e0 + (int)threadIdx.x, nel - 1);   // past the end: computed, not stored
   int nod[10];
 #pragma unroll
   for (int n = 0; n < 10; ++n) nod[n] = __ldg(el2nod + (size_t)n * nel + e);
@@ -420,23 +435,20 @@ __global__ void __launch_bounds__(128) k_ebe_apply(const T *__restrict__ K, cons
     }
   }
 #pragma unroll
-  for (int n = 0; n < 10; ++n)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) y[3 * nod[n] + c] += ye[3 * n + c];
+  for (int q = 0; q < 30; ++q) sy[threadIdx.x][q] = ye[q];
+  ebe_store<T>(sy, e0, nel, out);
 }
 
-// y += K x in FP64 accuracy from FP32 arithmetic: K = hi + lo (two FP32 arrays, hi is the FP32
+// K x in FP64 accuracy from FP32 arithmetic: K = hi + lo (two FP32 arrays, hi is the FP32
 // operator of the V-cycle), x split the same way at the gather; each product is formed exactly
 // (FMA error term) and accumulated in double-float (Knuth two-sum). ~10 FP32 operations per
 // multiply-add instead of one FP64 FMA, which GB300 issues at 1/62 of its FP32 rate.
 
-__global__ void __launch_bounds__(128) k_ebe_apply_df(const float *__restrict__ Kh, const float *__restrict__ Kl,
-                                                      const int *__restrict__ el2nod, int nel,
-                                                      const int *__restrict__ corder, int e_begin, int e_end,
-                                                      const double *__restrict__ x, double *__restrict__ y) {
-  const int i0 = e_begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i0 >= e_end) return;
-  const int e = corder[i0];
+__global__ void __launch_bounds__(EBE_T) k_ebe_apply_df(const float *__restrict__ Kh, const float *__restrict__ Kl,
+                                                       const int *__restrict__ el2nod, int nel,
+                                                       const double *__restrict__ x, double *__restrict__ out) {
+  __shared__ double sy[EBE_T][31];
+  const int e0 = blockIdx.x * EBE_T, e = min(e0 + (int)threadIdx.x, nel - 1);
   int nod[10];
 #pragma unroll
   for (int n = 0; n < 10; ++n) nod[n] = __ldg(el2nod + (size_t)n * nel + e);
@@ -471,27 +483,19 @@ __global__ void __launch_bounds__(128) k_ebe_apply_df(const float *__restrict__ 
     }
   }
 #pragma unroll
-  for (int n = 0; n < 10; ++n)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) y[3 * nod[n] + c] += (double)sh[3 * n + c] + (double)sl[3 * n + c];
+  for (int q = 0; q < 30; ++q) sy[threadIdx.x][q] = (double)sh[q] + (double)sl[q];
+  ebe_store<double>(sy, e0, nel, out);
 }
 
 int ebe_apply_df(const Level &L, const float *Kh, const float *Kl, const double *x, double *y, cudaStream_t s) {
-  M3_CUDA(cudaMemsetAsync(y, 0, sizeof(double) * L.ndof, s));
-  const int nc = (int)L.cstart.size() - 1;
-  for (int c = 0; c < nc; ++c) {
-    const int b = L.cstart[c], e = L.cstart[c + 1];
-    if (e <= b) continue;
-    k_ebe_apply_df<<<(e - b + 127) / 128, 128, 0, s>>>(Kh, Kl, L.el2nod, L.nel, L.corder, b, e, x, y); count_launch();
-  }
-  M3_CUDA(cudaGetLastError());
-  return M3SPH_OK;
+  k_ebe_apply_df<<<(L.nel + EBE_T - 1) / EBE_T, EBE_T, 0, s>>>(Kh, Kl, L.el2nod, L.nel, x, L.ye64); count_launch();
+  return node_sums(L, y, s);
 }
 
 // ----------------------------------------------------------------------------------------
-// split element-by-element apply: a CTA of 4 warps handles 32 elements of one colour; warp w
-// reads the w-th quarter of the packed matrix (lanes = elements of the colour), partial results are summed in shared memory and scattered.
-// Packed entry k -> (row, col) is resolved at compile time.
+// split element products (split_apply 1): a CTA of 4 warps handles 32 elements; warp w reads the w-th
+// quarter of the packed matrix (lanes = elements, so every load of a warp is one contiguous 512-byte segment),
+// the partial results are summed in shared memory. Packed entry k -> (row, col) is resolved at compile time.
 // ----------------------------------------------------------------------------------------
 
 struct OpF32 {   // FP32 V-cycle operator
@@ -597,14 +601,13 @@ __device__ __forceinline__ void run_part(const Op &op, int e, size_t nel, const 
 
 template <class Op, typename XT>
 __global__ void __launch_bounds__(128) k_ebe_apply_split(Op op, const int *__restrict__ el2nod, int nel,
-                                                         const int *__restrict__ corder, int e_begin, int e_end, const XT *__restrict__ x, XT *__restrict__ y) {
+                                                         const XT *__restrict__ x, XT *__restrict__ out) {
   using A = typename Op::acc_t;
   __shared__ XT sY[4][30][33];
   __shared__ int sNod[10][32];
   const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
-  const int e0 = e_begin + blockIdx.x * 32;
-  const bool valid = e0 + lane < e_end;
-  const int e = valid ? corder[e0 + lane] : 0;
+  const int e0 = blockIdx.x * 32, e = e0 + lane;
+  const bool valid = e < nel;
   if (part == 0)
 #pragma unroll
     for (int n = 0; n < 10; ++n) sNod[n][lane] = valid ? __ldg(el2nod + (size_t)n * nel + e) : 0;
@@ -636,25 +639,20 @@ __global__ void __launch_bounds__(128) k_ebe_apply_split(Op op, const int *__res
       sY[part][q][lane] = (XT)yh[q];
   }
   __syncthreads();
-  for (int o = threadIdx.x; o < 30 * 32; o += 128) {
-    const int q = o >> 5, el = o & 31;
-    if (e0 + el >= e_end) continue;
-    const XT v = sY[0][q][el] + sY[1][q][el] + sY[2][q][el] + sY[3][q][el];
-    y[3 * sNod[q / 3][el] + q % 3] += v;
+  const int nv = min(32, nel - e0) * 30;
+  for (int o = threadIdx.x; o < nv; o += 128) {
+    const int el = o / 30, q = o - 30 * el;
+    out[(size_t)e0 * 30 + o] = sY[0][q][el] + sY[1][q][el] + sY[2][q][el] + sY[3][q][el];
   }
 }
 
+static float *element_outputs(const Level &L, float *) { return L.ye32; }
+static double *element_outputs(const Level &L, double *) { return L.ye64; }
+
 template <class Op, typename XT>
 static int ebe_apply_split(const Level &L, const Op &op, const XT *x, XT *y, cudaStream_t s) {
-  M3_CUDA(cudaMemsetAsync(y, 0, sizeof(XT) * L.ndof, s));
-  const int nc = (int)L.cstart.size() - 1;
-  for (int c = 0; c < nc; ++c) {
-    const int b = L.cstart[c], e = L.cstart[c + 1];
-    if (e <= b) continue;
-    k_ebe_apply_split<Op, XT><<<(e - b + 31) / 32, 128, 0, s>>>(op, L.el2nod, L.nel, L.corder, b, e, x, y); count_launch();
-  }
-  M3_CUDA(cudaGetLastError());
-  return M3SPH_OK;
+  k_ebe_apply_split<Op, XT><<<(L.nel + 31) / 32, 128, 0, s>>>(op, L.el2nod, L.nel, x, element_outputs(L, y)); count_launch();
+  return node_sums(L, y, s);
 }
 
 int ebe_apply_split_f32(const Level &L, const float *K, const float *x, float *y, cudaStream_t s) {
@@ -669,15 +667,8 @@ int ebe_apply_split_df(const Level &L, const float *Kh, const float *Kl, const d
 
 template <typename T>
 int ebe_apply(const Level &L, const T *K, const T *x, T *y, cudaStream_t s) {
-  M3_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * L.ndof, s));
-  const int nc = (int)L.cstart.size() - 1;
-  for (int c = 0; c < nc; ++c) {
-    const int b = L.cstart[c], e = L.cstart[c + 1];
-    if (e <= b) continue;
-    k_ebe_apply<T><<<(e - b + 127) / 128, 128, 0, s>>>(K, L.el2nod, L.nel, L.corder, b, e, x, y); count_launch();
-  }
-  M3_CUDA(cudaGetLastError());
-  return M3SPH_OK;
+  k_ebe_apply<T><<<(L.nel + EBE_T - 1) / EBE_T, EBE_T, 0, s>>>(K, L.el2nod, L.nel, x, element_outputs(L, y)); count_launch();
+  return node_sums(L, y, s);
 }
 template int ebe_apply<double>(const Level &, const double *, const double *, double *, cudaStream_t);
 template int ebe_apply<float>(const Level &, const float *, const float *, float *, cudaStream_t);

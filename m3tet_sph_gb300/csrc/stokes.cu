@@ -180,7 +180,7 @@ static void dfree(void *p) {
   if (p) cudaFree(p);
 }
 
-// ---- greedy element colouring (per-colour kernels): elements sharing a vertex get different colours ----
+// ---- greedy element colouring: elements sharing a vertex get different colours ----
 static int color_elements(const std::vector<int> &el, int nel, int nvert_ids, std::vector<int> &color, int &ncolor) {
   std::vector<uint64_t> used(2 * (size_t)nvert_ids, 0);
   color.assign(nel, -1);
@@ -317,9 +317,8 @@ static int build_level(m3sph_mesh *M, int img, const m3sph_level &in, Level &L) 
   L.cstart = cnt;
   // Elements keep the caller's order: the 8 children of a parent are consecutive on every level, so
   // neighbours in memory are neighbours in space and the nodes that a warp gathers share cache lines.
-  // (Colour order, which only the per-colour kernels need, spread a warp's nodes over the whole
-  // vector: the partially assembled apply took 104 us at 491,520 elements.) The per-colour kernels go
-  // through the list `corder`.
+  // (Colour order spread a warp's nodes over the whole vector: the partially assembled apply took 104 us
+  // at 491,520 elements.) Training samples are drawn through the colour-ordered list `corder`.
   std::vector<int> corder(in.nel), fill(cnt.begin(), cnt.end() - 1);
   for (int e = 0; e < in.nel; ++e) corder[fill[color[e]]++] = e;
   std::vector<int> el_soa((size_t)in.nel * 10);
@@ -958,7 +957,7 @@ extern "C" int m3sph_stokes_set_vel_bc(m3sph_mesh *M, const int32_t *ifix, const
 // FP64-accurate finest-level operator for the outer iterations: native FP64 on the plain path,
 // double-float FP32 arithmetic on the mixed path
 // streamed finest-level operators (TMA ring + fixed-order node sums) for the FP32 V-cycle operator
-// and, optionally, for the FP64-accurate outer operators; off: per-colour kernels
+// and, optionally, for the FP64-accurate outer operators; off: plain element products, the same sums
 static bool g_stream_apply = true;
 static bool g_stream_outer = true;
 

@@ -806,16 +806,14 @@ static void f32_phase1(const Level &L, const CUtensorMap &map, const float *x, c
   }
 }
 
+int node_sums(const Level &L, float *y, cudaStream_t s);
 int stream_apply_f32(const Level &L, const float *K, const float *x, float *y, cudaStream_t s) {
   M3_TRY(stream_ready(L, K));
   CUtensorMap map;
   M3_TRY(encode_k32(L, K, &map));
   f32_phase1(L, map, x, s);
   count_launch();
-  k_node_gather_f32<<<(L.nnod + 255) / 256, 256, 0, s>>>(L.g_ptr, L.g_idx, L.nnod, L.ye32, y, L.sa_err + 1);
-  count_launch();
-  M3_CUDA(cudaGetLastError());
-  return M3SPH_OK;
+  return node_sums(L, y, s);
 }
 
 // row-per-lane kernels. Double-float: `owners` warps-groups own stages in turn, SPLIT warps share a
@@ -903,6 +901,15 @@ static int rowlane_sums(const Level &L, double *y, const double *x, const Reduct
   M3_CUDA(cudaGetLastError());
   return M3SPH_OK;
 }
+
+// y = node sums of the element outputs (ye32, ye64) that another kernel left
+int node_sums(const Level &L, float *y, cudaStream_t s) {
+  k_node_gather_f32<<<(L.nnod + 255) / 256, 256, 0, s>>>(L.g_ptr, L.g_idx, L.nnod, L.ye32, y, L.sa_err + 1);
+  count_launch();
+  M3_CUDA(cudaGetLastError());
+  return M3SPH_OK;
+}
+int node_sums(const Level &L, double *y, cudaStream_t s) { return rowlane_sums(L, y, nullptr, nullptr, nullptr, s); }
 
 // d += w (r - K d) / diag with K d from the streamed apply (one weighted Jacobi sweep)
 int stream_apply_jac_f32(const Level &L, const float *K, float w, const float *r, const float *Di, float *d,

@@ -86,3 +86,39 @@ def test_coarse_inverse_diagonal_block_ahead(built_lib):
     finally:
         d.set_option("coarse_f64_direct_max", 6000)
         d.close()
+
+
+@pytest.mark.parametrize("split", [0, 1])
+def test_products_without_streaming(dm, split):
+    """The finest-level products with stream_apply and stream_outer off, either form: FP64, double-float
+    and FP32 against the FP64 element matrices summed on the host; one launch for the elements and one for
+    the nodes. Tolerances as above: rounding (6e-8, 1e-14 of double-float, 1e-16) over sums of a few
+    hundred terms."""
+    import ctypes as C
+    from m3tet_sph_gb300 import _lib as L
+
+    def launches():
+        n = C.c_ulonglong()
+        L.check(L.lib().m3sph_launch_count(C.byref(n)))
+        return n.value
+
+    w, d = dm
+    EL, n = w['levels'][0]['EL2NOD'], 3 * w['levels'][0]['nnod']
+    K, _, _ = d.element_matrices()
+    dof = (3 * EL[:, :, None] + np.arange(3)).reshape(len(EL), 30)
+    x = np.random.default_rng(6).standard_normal(n).astype(np.float32).astype(np.float64)
+    y = np.bincount(dof.ravel(), np.einsum('eij,ej->ei', K, x[dof]).ravel(), n)
+    opts = dict(stream_apply=0, stream_outer=0, fp32_operator=0, split_apply=split)
+    try:
+        for k, v in opts.items():
+            d.set_option(k, v)
+        for fn, tol in ((lambda: d.level_apply(0, x), 1e-13), (lambda: d.apply(x), 1e-11),
+                        (lambda: d.level_apply32(0, x.astype(np.float32)), 1e-5)):
+            n0 = launches()
+            got = fn()
+            assert launches() - n0 == 2
+            assert np.linalg.norm(got - y) <= tol * np.linalg.norm(y)
+            assert np.array_equal(fn(), got)
+    finally:
+        for k in opts:
+            d.set_option(k, 1)
