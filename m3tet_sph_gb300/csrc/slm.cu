@@ -114,8 +114,20 @@ __device__ __forceinline__ void point_frames(double th, double ph, double r, Poi
   frame_z180(th, ph, r, f.pz);
   frame_x90(th, ph, r, f.px);
 }
-// the frames in FP32 without FP64 trigonometry (GB300 issues FP64 at 1/64 of its FP32 rate): what the
-// FP32 walk and pre-filter need, both with margins far above FP32 rounding
+// the frames rounded to FP32 once: what the FP32 pre-filter of the rings and of the brute force works on
+__device__ __forceinline__ PointFramesT<float> frames_f32(const PointFrames &f) {
+  PointFramesT<float> g;
+  for (int k = 0; k < 3; ++k) {
+    g.p0[k] = (float)f.p0[k];
+    g.pz[k] = (float)f.pz[k];
+    g.px[k] = (float)f.px[k];
+  }
+  return g;
+}
+// the frames by FP32 trigonometry (GB300 issues FP64 at 1/64 of its FP32 rate), for the FP32 walk only: it ends
+// in a starting element for the FP64 walk, which decides, so its error costs steps at most. Largest errors of
+// the X-90 coordinates of points in the cones: 4.8e-7 (theta), 6.4e-7 (phi), 1.2e-3 km (r); rounded once 1.2e-7,
+// 2.4e-7 and 2.4e-4 km.
 __device__ __forceinline__ void point_frames_f32(double th, double ph, double r, PointFramesT<float> &g) {
   double z[3];
   frame_z180(th, ph, r, z);
@@ -284,8 +296,8 @@ struct GapBest {
   __device__ int pick() const { return non >= 0 ? non : iso; }
 };
 
-// an FP32 pre-filter skips the FP64 evaluation of elements the point is far from: FP32 barycentrics
-// err by ~1e-5 here, so an element whose FP32 need exceeds the largest gap tolerance by PRE_MARGIN
+// an FP32 pre-filter skips the FP64 evaluation of elements the point is far from: FP32 barycentrics of
+// frames and vertices rounded once err by ~1e-5 here, so an element whose FP32 need exceeds the largest gap tolerance by PRE_MARGIN
 // can be neither a tie candidate nor a gap contender in FP64
 constexpr float PRE_MARGIN = 1e-3f;
 __device__ __forceinline__ bool far_f32(const SlmMesh &m, int e, const PointFramesT<float> &g) {
@@ -477,8 +489,8 @@ __device__ __forceinline__ void ring_visit(const SlmMesh &m, int e0, int depth, 
 // (placed points) or with any of those (points the walk could not place).
 //
 // FP64 bounds it: an FP64 instruction takes the SM 16 cycles whatever the number of active lanes. So a
-// block takes 32 points at a time: one warp forms the X-90 frames of all of them, one point per lane,
-// while the warps (4 points each) filter the rings in FP32 and list what is left, about 8 elements a
+// block takes 32 points at a time: one warp forms the X-90 frames of all of them, one point per lane;
+// then the warps (4 points each) filter the rings in FP32 and list what is left, about 8 elements a
 // point; the FP64 coordinates of the 4 points' lists are then formed together by the lanes of a warp,
 // and one lane per point applies the rules. (One warp per point, every lane forming the point's frames
 // and each round of 32 ring elements its FP64 coordinates, took 1,069 us for the 43,554 departure points of
@@ -501,6 +513,14 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 2) k_resolve_ring(SlmMesh m, 
   RingSmem &S = *reinterpret_cast<RingSmem *>(ring_raw);
   const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int total = *ntodo;
+  // frames of point pt of the 32 (its X-90 frame is in S.px)
+  auto frames = [&](int i, int pt, PointFrames &f) {
+    f.p0[0] = P[i];
+    f.p0[1] = P[npt + i];
+    f.p0[2] = P[2 * (size_t)npt + i];
+    frame_z180(f.p0[0], f.p0[1], f.p0[2], f.pz);
+    for (int c = 0; c < 3; ++c) f.px[c] = S.px[c][pt];
+  };
   for (int base = blockIdx.x * RING_PTS; base < total; base += gridDim.x * RING_PTS) {
     const int nloc = min(RING_PTS, total - base);
     if (wl == 0 && lane < nloc) {
@@ -509,13 +529,15 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 2) k_resolve_ring(SlmMesh m, 
       frame_x90(P[i], P[npt + i], P[2 * (size_t)npt + i], x);
       for (int k = 0; k < 3; ++k) S.px[k][lane] = x[k];
     }
+    __syncthreads();
     for (int w = 0; w < RING_PPW; ++w) {
       const int pt = wl * RING_PPW + w;
       int cnt = 0;
       if (pt < nloc) {
         const int i = todo[base + pt];
-        PointFramesT<float> g;
-        point_frames_f32(P[i], P[npt + i], P[2 * (size_t)npt + i], g);
+        PointFrames f;
+        frames(i, pt, f);
+        const PointFramesT<float> g = frames_f32(f);
         ring_visit(m, els[i], (status[i] & 1) ? 1 : 2, lane, S.vt[wl], [&](int e, bool live) {
           const bool keep = live && !far_f32(m, e, g);
           const unsigned mask = __ballot_sync(0xffffffffu, keep);
@@ -536,11 +558,7 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 2) k_resolve_ring(SlmMesh m, 
       while (t >= off[w + 1]) ++w;
       const int pt = wl * RING_PPW + w, k = t - off[w], i = todo[base + pt], e = S.id[pt][k];
       PointFrames f;
-      f.p0[0] = P[i];
-      f.p0[1] = P[npt + i];
-      f.p0[2] = P[2 * (size_t)npt + i];
-      frame_z180(f.p0[0], f.p0[1], f.p0[2], f.pz);
-      for (int c = 0; c < 3; ++c) f.px[c] = S.px[c][pt];
+      frames(i, pt, f);
       double lc[3], mn, mx;
       int am;
       S.step[pt][k] = local_coords(m, e, f, lc);
@@ -601,9 +619,8 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 2) k_resolve_ring(SlmMesh m, 
       if (lane == 0) *n = 0;
       __syncwarp();
       PointFrames f;
-      point_frames(P[i], P[npt + i], P[2 * (size_t)npt + i], f);
-      PointFramesT<float> g;
-      point_frames_f32(P[i], P[npt + i], P[2 * (size_t)npt + i], g);
+      frames(i, pt, f);
+      const PointFramesT<float> g = frames_f32(f);
       GapBest G;
       ring_visit(m, els[i], (status[i] & 1) ? 1 : 2, lane, S.vt[wl], [&](int e, bool live) {
         if (live) eval_shared(m, e, f, g, ids, fl, n, G);
@@ -785,8 +802,7 @@ __global__ void __launch_bounds__(BRUTE_WARPS * 32) k_locate_brute(SlmMesh m, co
     const int i = todo[w];
     PointFrames f;
     point_frames(P[i], P[npt + i], P[2 * (size_t)npt + i], f);
-    PointFramesT<float> g;
-    point_frames_f32(P[i], P[npt + i], P[2 * (size_t)npt + i], g);
+    const PointFramesT<float> g = frames_f32(f);
     GapBest G;
     for (int e = lane; e < m.nel; e += 32) eval_shared(m, e, f, g, s_id[wl], s_fl[wl], &s_n[wl], G);
     __syncwarp();
