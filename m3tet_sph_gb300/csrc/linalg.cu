@@ -815,12 +815,11 @@ __global__ void __launch_bounds__(gu::THREADS, 1) k_gjb_update_tc(float *__restr
           ++nbt[h];
         }
       }
-      if (!ok) {
-        atomicOr(err, 1);
-        if (na) tc_bar_wait(a_full, (na - 1) & 1);          // copies still in flight
-        for (int h = 0; h < 2; ++h)
-          if (nbt[h]) tc_bar_wait(b_full + 8 * h, (nbt[h] - 1) & 1);
-      }
+      if (!ok) atomicOr(err, 1);
+      // no copy may be in flight when the block ends, whichever warp gave up
+      if (na) tc_bar_wait(a_full, (na - 1) & 1);
+      for (int h = 0; h < 2; ++h)
+        if (nbt[h]) tc_bar_wait(b_full + 8 * h, (nbt[h] - 1) & 1);
     }
     __syncwarp();
   } else if (warp == WARPS + 1) {
@@ -855,11 +854,9 @@ __global__ void __launch_bounds__(gu::THREADS, 1) k_gjb_update_tc(float *__restr
           tc_commit(acc_full + 8 * (2 * buf + h));
         }
       }
-      if (!ok) {
-        atomicOr(err, 2);
-        tc_commit(drain);                    // MMAs still in flight
-        tc_bar_wait(drain, 0);
-      }
+      if (!ok) atomicOr(err, 2);
+      tc_commit(drain);                      // nor an MMA when TMEM is given back
+      tc_bar_wait(drain, 0);
     }
     __syncwarp();
   } else {
