@@ -369,7 +369,7 @@ __device__ __forceinline__ void store_point(int i, int npt, int e, double (&lc)[
 
 // rule 1 / rule 2 on the warp's shared candidate list (duplicates removed first), by lane 0;
 // writes the point's element, local coordinates and status (base_status: 1 placed by a ring, 16 by
-// the brute force)
+// the brute force, after which a point without an element is not found: -1 and zeros)
 __device__ void finish_point(const SlmMesh &m, const PointFrames &f, int i, int npt, int *ids, uint8_t *fl, int nc,
                              int gap_e, int q, int base_status, int adjust, int *els, double *lc_out, uint8_t *status) {
   int kind = nc > MAX_CAND ? 64 : 0;
@@ -393,11 +393,12 @@ __device__ void finish_point(const SlmMesh &m, const PointFrames &f, int i, int 
     e = gap_e;
     kind |= (base_status & 16) | 4;
   }
+  double lc[3] = {0.0, 0.0, 0.0};
   if (e < 0) {
+    if (base_status & 16) store_point(i, npt, -1, lc, 0, els, lc_out);
     status[i] = (uint8_t)(8 | (kind & 64));
     return;
   }
-  double lc[3];
   local_coords(m, e, f, lc);
   store_point(i, npt, e, lc, adjust, els, lc_out);
   status[i] = (uint8_t)kind;
@@ -497,7 +498,7 @@ __device__ __forceinline__ void ring_visit(const SlmMesh &m, int e0, int depth, 
 // the 30,720-element shell and 6,464 us for the listed ones of 1.5M random points there; now 316 and
 // 1,287 us.)
 constexpr int RING_WARPS = 8, RING_PTS = 32, RING_PPW = RING_PTS / RING_WARPS;
-constexpr int RING_CAP = 48;     // listed elements per point; more (never on a shell mesh): one by one
+constexpr int RING_CAP = 48;     // listed elements per point; more (a point with NaN coordinates): one by one
 struct RingSmem {
   double px[3][RING_PTS];
   double need[RING_PTS][RING_CAP], step[RING_PTS][RING_CAP], lc[RING_PTS][RING_CAP][3];

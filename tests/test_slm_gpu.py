@@ -236,3 +236,34 @@ def test_point_major_and_component_major_arrays_agree(mesh_case, npt, nvar):
         got.append((els, np.ascontiguousarray(lay(lc)) if suf == "" else lc, vt, vc))
     for a, b in zip(*got):
         assert a.shape == b.shape and np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("npt", [1, 31, 33, 200])
+def test_points_without_coordinates(mesh_case, npt):
+    """A point with a NaN coordinate keeps every ring element in the FP32 filter, more than a point's
+    list holds, so its ring is resolved element by element: it is not found (element 0), and the points beside it
+    (every third is a mesh node, which needs its ring too) are located as without it."""
+    import ctypes as C
+    from m3tet_sph_gb300 import _lib as L
+    w, dm, _ = mesh_case
+    P = random_shell_points(npt, 21)
+    P[:, ::3] = w['levels'][0]['GCOORD_SPH'][:, 40:40 + len(range(0, npt, 3))]
+
+    def locate(P):
+        P = np.ascontiguousarray(P)
+        els, lc, info = np.full(npt, -7, np.int32), np.zeros((3, npt)), L.LocateInfo()
+        code = L.lib().m3sph_tsearch_sph_soa(dm.h, L.dptr(P), npt, None, L.iptr(els), L.dptr(lc), C.byref(info))
+        return code, els, lc, info.as_dict()
+
+    code, els, lc, info = locate(P)
+    assert code == L.OK and info['nlost'] == 0
+    bad = np.arange(npt) % 5 == 0
+    for k, c in ((0, 0), (1, 1), (2, 2)):
+        Q = P.copy()
+        Q[c, np.nonzero(bad)[0][k::3]] = np.nan
+        n = np.isnan(Q).any(0)
+        code, e, l, info = locate(Q)
+        assert code == (L.ERR_NOT_FOUND if n.any() else L.OK)
+        assert info['nlost'] == n.sum()
+        assert np.all(e[n] == 0) and np.all(l[:, n] == 0)
+        assert np.array_equal(e[~n], els[~n]) and np.array_equal(l[:, ~n], lc[:, ~n])
