@@ -86,3 +86,46 @@ def test_coarsest_level_without_free_dofs(built_lib, tiny_plates, precision, dir
     finally:
         dm.set_option("coarse_f64_direct_max", 6000)
         dm.close()
+
+
+# mean relative error of a V-cycle with the unrefined FP32 inverse, when the inverse was formed by FP32
+# multiply-adds throughout: (surface level, layers, free dofs of the coarsest level, seeds of the dofs
+# fixed for that): over 3 x 8 vectors (None: every free dof, 8 vectors)
+FP32_INVERSE = [(2, 2, 100, 1, 3.99e-9), (2, 2, 129, 3, 8.65e-9), (2, 2, 250, 3, 1.81e-8), (2, 2, 500, 3, 5.07e-8),
+                (2, 2, None, 1, 1.94e-7), (2, 4, None, 1, 9.58e-8), (3, 2, None, 1, 3.96e-7), (3, 4, 5996, 1, 9.12e-8),
+                (3, 4, 6094, 1, 1.01e-7)]
+
+
+@pytest.mark.parametrize("level,layers,nfree,seeds,bound", FP32_INVERSE)
+def test_fp32_inverse_is_as_accurate_as_fp32_multiply_adds(built_lib, level, layers, nfree, seeds, bound):
+    """The FP32 inverse by itself (no refinement) against the FP64 inverse, 1 to 48 panels of 128, the last
+    ones partial, either side of the size from which the next diagonal block runs ahead: the error of a
+    V-cycle is that of an inverse formed with FP32 multiply-adds (the figures above), which may differ by
+    20 % with the matrix on small ones. (Without the correction for truncation the errors are 1.1 to 1.3
+    times the figures from 7 panels on.)"""
+    from m3tet_sph_gb300 import stokes, workloads
+    w = workloads.make_workload('c2', level=level, nlayer=layers, nmg=2)
+    nc = 3 * w['levels'][-1]['nnod']
+    rhs_seeds = range(6) if nfree in (100, 5996, 6094) else range(8)
+    d = stokes.DeviceMesh(w['levels'])
+    err = []
+    try:
+        for seed in range(seeds):
+            ifix, vfix = w['ifix'], w['vfix']
+            if nfree is not None:
+                free = np.setdiff1d(np.arange(nc), ifix)
+                seed = 7 if seeds == 1 else seed
+                more = np.random.default_rng(seed).permutation(free)[:len(free) - nfree]
+                ifix, vfix = np.concatenate([ifix, more]), np.concatenate([vfix, np.zeros(len(more))])
+            out = []
+            for direct_max, sweeps in ((20000, 3), (0, 0)):
+                d.set_option("coarse_f64_direct_max", direct_max)
+                d.set_option("coarse_refine_sweeps", sweeps)
+                d.setup(w['visc'], w['dens'], ifix, vfix, w['phys'], precision=0)
+                out.append([d.vcycle(np.random.default_rng(s).standard_normal(d.ndof)) for s in rhs_seeds])
+            err += [np.linalg.norm(b - a) / np.linalg.norm(a) for a, b in zip(*out)]
+    finally:
+        d.set_option("coarse_f64_direct_max", 6000)
+        d.set_option("coarse_refine_sweeps", 3)
+        d.close()
+    assert np.mean(err) <= 1.2 * bound

@@ -153,3 +153,49 @@ def test_a_wait_that_gave_up_is_reported(dm_plates, graphs, word):
             assert np.array_equal(call(), want)
     finally:
         dm.set_option("graphs", 1)
+
+
+@pytest.mark.parametrize("precision,itmax", [(0, 1), (0, 2), (0, 255), (0, 256), (0, 257), (0, 513),
+                                             (1, 1), (1, 255), (1, 256), (1, 257)])
+def test_captured_loop_and_host_loop_agree(dm_plates, precision, itmax):
+    """The captured CG loop runs 256 iterations before the host looks at it; without graphs the host
+    runs every iteration. Both launch the same kernels in the same order: exactly itmax iterations for a
+    tolerance that is never met, and the same bits. Viscosities over 8 decades and a large right-hand side
+    keep the residual of so many iterations above the smallest FP32 (FP64) numbers, where every form breaks
+    down."""
+    w, dm = dm_plates
+    visc = 10.0 ** np.random.default_rng(2).uniform(-4, 4, len(w['visc']))
+    dm.setup(visc, w['dens'], w['ifix'], w['vfix'], w['phys'], precision=precision)
+    rng = np.random.default_rng(14)
+    b, x0 = rng.standard_normal(dm.ndof) * (1e30 if precision else 1e60), rng.standard_normal(dm.ndof)
+    out = []
+    try:
+        for graphs in (1, 0):
+            dm.set_option("graphs", graphs)
+            # the second ends at the same iteration for both, in between
+            out.append(dm.mgpcg(b, x0, 0.0, True, itmax) + dm.mgpcg(b, x0, 1e-3, False, itmax))
+    finally:
+        dm.set_option("graphs", 1)
+    g, h = out
+    assert g[1] == h[1] == itmax and g[4] == h[4] <= itmax
+    for k in (0, 2, 3, 5):
+        assert np.array_equal(g[k], h[k])
+
+
+@pytest.mark.parametrize("graphs", [0, 1])
+def test_solve_with_either_loop(dm_plates, graphs):
+    """The learned solve, whose CG may switch the smoother off, with the captured and the host loop."""
+    from m3tet_sph_gb300 import learned
+    w, dm = dm_plates
+    dm.setup(w['visc'], w['dens'], w['ifix'], w['vfix'], w['phys'], precision=1)
+    learned.set_params(dm, np.load(Path(learned.__file__).with_name('smoother_c1.npy')), trained=True)
+    kw = dict(rtol_Pat=1e-8, rtol_U=5e-3, itmax_Pat=200, itmax_U=40, target_rel_residual=1e-8, smoother=1)
+    ref = dm.solve(**kw)
+    try:
+        dm.set_option("graphs", graphs)
+        got = dm.solve(**kw)
+    finally:
+        dm.set_option("graphs", 1)
+    assert got[2]['itPat'] == ref[2]['itPat'] and got[2]['nvcycle'] == ref[2]['nvcycle']
+    assert got[2]['smoother_fallbacks'] == ref[2]['smoother_fallbacks']
+    assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])
