@@ -1911,6 +1911,7 @@ extern "C" int m3sph_level_apply(m3sph_mesh *M, int32_t img, const double *x, do
     M3_CUDA(cudaMemcpyAsync(y, W->kd64[img], sizeof(double) * n, cudaMemcpyDeviceToHost, s));
   }
   M3_CUDA(cudaStreamSynchronize(s));
+  M3_TRY(stream_check(L, s));
   return M3SPH_OK;
 }
 
@@ -2277,6 +2278,7 @@ extern "C" int m3sph_ml_collect(m3sph_mesh *M, uint64_t seed, int32_t n_iterates
   }
   M3_CUDA(cudaStreamSynchronize(s));
   M->smoother_active = act;
+  M3_TRY(stream_check(L0, s));
   if (count) *count = ml_count(M);
   return M3SPH_OK;
 }

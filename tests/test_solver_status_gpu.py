@@ -199,3 +199,21 @@ def test_solve_with_either_loop(dm_plates, graphs):
     assert got[2]['itPat'] == ref[2]['itPat'] and got[2]['nvcycle'] == ref[2]['nvcycle']
     assert got[2]['smoother_fallbacks'] == ref[2]['smoother_fallbacks']
     assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])
+
+
+def test_operator_calls_report_a_wait_that_gave_up(dm_plates):
+    """The finest-level products and the training pairs made from them do too."""
+    from m3tet_sph_gb300 import _lib as L
+    w, dm = dm_plates
+    dm.setup(w['visc'], w['dens'], w['ifix'], w['vfix'], w['phys'], precision=1)
+    x = np.random.default_rng(10).standard_normal(dm.ndof)
+    L.check(L.lib().m3sph_ml_reserve(dm.h, 1 << 16))
+
+    def collect():
+        L.check(L.lib().m3sph_ml_collect(dm.h, 1, 1, 8, None))
+
+    for call in (lambda: dm.apply(x), lambda: dm.level_apply(0, x), lambda: dm.level_apply32(0, x), collect):
+        dm.set_option("wait_error", 1)
+        with pytest.raises(L.M3SphError, match='bounded wait'):
+            call()
+        call()
