@@ -101,6 +101,7 @@ static void add_launches(unsigned long long k) { g_launches.fetch_add(k, std::me
 void set_error(const std::string &msg) { g_err = msg; }
 int cuda_fail(cudaError_t e, const char *what) {
   g_err = std::string("CUDA error ") + cudaGetErrorString(e) + " in " + what;
+  cudaGetLastError();                  // reported here: the next call's launch checks must not see it again
   return M3SPH_ERR_CUDA;
 }
 

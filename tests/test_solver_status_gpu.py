@@ -217,3 +217,18 @@ def test_operator_calls_report_a_wait_that_gave_up(dm_plates):
         with pytest.raises(L.M3SphError, match='bounded wait'):
             call()
         call()
+
+
+def test_a_failed_allocation_is_reported_once(built_lib, tiny_plates):
+    """An allocation that does not fit fails its call and not the one after it."""
+    from m3tet_sph_gb300 import _lib as L, stokes
+    w = tiny_plates
+    dm = stokes.DeviceMesh(w['levels'])
+    try:
+        dm.setup(w['visc'], w['dens'], w['ifix'], w['vfix'], w['phys'], precision=1)
+        x = np.random.default_rng(11).standard_normal(dm.ndof)
+        y = dm.apply(x)
+        assert L.lib().m3sph_ml_reserve(dm.h, 10 ** 13) == L.ERR_CUDA
+        assert np.array_equal(dm.apply(x), y)
+    finally:
+        dm.close()
