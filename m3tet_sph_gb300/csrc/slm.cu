@@ -1262,9 +1262,14 @@ int slm_build(m3sph_mesh *M, const m3sph_level &f0) {
 
 static int slm_reserve(SlmState *S, size_t npt, int nel, int nnod, int nv) {
   if (npt <= S->cap && S->P) return M3SPH_OK;
-  for (void *q : {(void *)S->P, (void *)S->lc, (void *)S->V, (void *)S->out, (void *)S->upu, (void *)S->rpu,
-                  (void *)S->U, (void *)S->els, (void *)S->guess, (void *)S->todo, (void *)S->list, (void *)S->status})
-    if (q) cudaFree(q);
+  // freed pointers are forgotten: if an allocation below fails, the next call starts from nothing
+  S->cap = 0;
+  auto drop = [](auto *&p) {
+    if (p) cudaFree(p);
+    p = nullptr;
+  };
+  drop(S->P), drop(S->lc), drop(S->V), drop(S->out), drop(S->upu), drop(S->rpu), drop(S->U);
+  drop(S->els), drop(S->guess), drop(S->todo), drop(S->list), drop(S->status);
   const size_t n = std::max(npt, (size_t)nnod);
   int st;
   if ((st = sl_alloc(&S->P, 3 * n)) || (st = sl_alloc(&S->lc, 3 * n)) || (st = sl_alloc(&S->V, 3 * (size_t)nnod)) ||
@@ -1273,7 +1278,8 @@ static int slm_reserve(SlmState *S, size_t npt, int nel, int nnod, int nv) {
       (st = sl_alloc(&S->els, n)) || (st = sl_alloc(&S->guess, n)) || (st = sl_alloc(&S->todo, n)) ||
       (st = sl_alloc(&S->list, 3 * n)) || (st = sl_alloc(&S->status, n)))
     return st;
-  if (!S->gel) {
+  if (!S->acc) {                       // the last of these
+    drop(S->gel), drop(S->wel), drop(S->gn), drop(S->wn), drop(S->Xc), drop(S->kk);
     if ((st = sl_alloc(&S->gel, 3 * (size_t)nel)) || (st = sl_alloc(&S->wel, 4 * (size_t)nel)) ||
         (st = sl_alloc(&S->gn, 3 * (size_t)nv)) || (st = sl_alloc(&S->wn, (size_t)nv)) ||
         (st = sl_alloc(&S->Xc, 3 * (size_t)nnod)) || (st = sl_alloc(&S->kk, 3 * (size_t)nnod)) ||

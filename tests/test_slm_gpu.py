@@ -267,3 +267,40 @@ def test_points_without_coordinates(mesh_case, npt):
         assert info['nlost'] == n.sum()
         assert np.all(e[n] == 0) and np.all(l[:, n] == 0)
         assert np.array_equal(e[~n], els[~n]) and np.array_equal(l[:, ~n], lc[:, ~n])
+
+
+def test_location_after_one_that_did_not_fit(tiny):
+    """A call with more points than device memory holds fails, and the next ones work on memory of their
+    own: no pointer of the failed reservation, or of the one before, is used again."""
+    import ctypes as C
+    import torch
+    from m3tet_sph_gb300 import _lib as L, advection as A, stokes
+    dm = stokes.DeviceMesh(tiny['levels'])
+    hold = None
+    try:
+        P = random_shell_points(3000, 33)
+        T = tiny['T']
+        els, lc, _ = A.tsearch2_sph(dm, P)
+        v = A.interp3d_cubic_p(dm, els, lc, T)
+        free, _ = torch.cuda.mem_get_info()
+        npt = 2 ** 31 - 1024                     # 52 GB for the points alone, 208 GB in all
+        keep = 70 << 30
+        if free < keep + (8 << 30):
+            pytest.skip('less device memory than the call asks for')
+        hold = torch.empty(free - keep, dtype=torch.uint8, device='cuda')
+        out, info = np.zeros(4, np.int32), L.LocateInfo()
+        # refused before any host array is read
+        code = L.lib().m3sph_tsearch_sph(dm.h, L.dptr(P), npt, None, L.iptr(out), None, C.byref(info))
+        assert code == L.ERR_CUDA
+        del hold
+        hold = None
+        torch.cuda.empty_cache()
+        for n in (2000, 3000):
+            e, l, _ = A.tsearch2_sph(dm, P[:, :n])
+            assert np.array_equal(e, els[:n]) and np.array_equal(l, lc[:, :n])
+            assert np.array_equal(A.interp3d_cubic_p(dm, e, l, T), v[:n])
+    finally:
+        if hold is not None:
+            del hold
+            torch.cuda.empty_cache()
+        dm.close()
