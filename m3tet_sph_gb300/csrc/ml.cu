@@ -1052,14 +1052,18 @@ int ml_feature_rows(m3sph_mesh *M, int j, const float *z, float *X, float *Sn) {
 int ml_reserve(m3sph_mesh *M, long cap) {
   MlState *S = mls(M);
   if (S->cap >= cap) return M3SPH_OK;
-  for (void *q : {(void *)S->X, (void *)S->X2, (void *)S->T, (void *)S->T2})
-    if (q) cudaFree(q);
+  // the old samples go with their arrays, also when the new ones do not fit
+  S->cap = S->count = 0;
+  auto drop = [](auto *&p) {
+    if (p) cudaFree(p);
+    p = nullptr;
+  };
+  drop(S->X), drop(S->X2), drop(S->T), drop(S->T2);
   M3_TRY(ml_alloc(&S->X, (size_t)cap * INP));
   M3_TRY(ml_alloc(&S->X2, (size_t)cap * INP));
   M3_TRY(ml_alloc(&S->T, (size_t)cap * OUTP));
   M3_TRY(ml_alloc(&S->T2, (size_t)cap * OUTP));
   S->cap = cap;
-  S->count = 0;
   return M3SPH_OK;
 }
 

@@ -189,3 +189,28 @@ def test_trained_network_gain_per_sweep(built_lib):
     print("error left in the K-norm after one sweep:", m)
     assert m["learned"] < 0.9 * m["jacobi"]
     assert m["learned"] < 0.5 * m["untrained"]
+
+
+def test_training_samples_after_a_reservation_that_did_not_fit(tiny):
+    """Training samples after a reservation that device memory does not hold: none are left (their arrays
+    are gone), and a smaller reservation works."""
+    import ctypes as C
+    from m3tet_sph_gb300 import _lib as L, stokes
+    w = tiny
+    dm = stokes.DeviceMesh(w['levels'])
+    try:
+        dm.setup(w['visc'], w['dens'], w['ifix'], w['vfix'], w['phys'], precision=1)
+        n = C.c_int64()
+
+        def collect():
+            L.check(L.lib().m3sph_ml_collect(dm.h, 1, 1, 1, C.byref(n)))
+            return n.value
+
+        L.check(L.lib().m3sph_ml_reserve(dm.h, 500))
+        assert collect() == 500
+        assert L.lib().m3sph_ml_reserve(dm.h, 10 ** 13) == L.ERR_CUDA
+        assert collect() == 0
+        L.check(L.lib().m3sph_ml_reserve(dm.h, 300))
+        assert collect() == 300
+    finally:
+        dm.close()
