@@ -490,9 +490,10 @@ __device__ __forceinline__ void ring_visit(const SlmMesh &m, int e0, int depth, 
 // (placed points) or with any of those (points the walk could not place).
 //
 // FP64 bounds it: an FP64 instruction takes the SM 16 cycles whatever the number of active lanes. So a
-// block takes 32 points at a time: one warp forms the X-90 frames of all of them, one point per lane;
-// then the warps (4 points each) filter the rings in FP32 and list what is left, about 8 elements a
-// point; the FP64 coordinates of the 4 points' lists are then formed together by the lanes of a warp,
+// block takes 32 points at a time: one warp forms the X-90 frames of all of them, one point per lane, beside
+// the work on the 32 before (formed at the point where they are needed: 2.45 ms for the location of 1.5M
+// points, now 2.41); the warps (4 points each) filter the rings in FP32 and list what is left, about 8
+// elements a point; the FP64 coordinates of the 4 points' lists are then formed together by the lanes of a warp,
 // and one lane per point applies the rules. (One warp per point, every lane forming the point's frames
 // and each round of 32 ring elements its FP64 coordinates, took 1,069 us for the 43,554 departure points of
 // the 30,720-element shell and 6,464 us for the listed ones of 1.5M random points there; now 316 and
@@ -500,7 +501,7 @@ __device__ __forceinline__ void ring_visit(const SlmMesh &m, int e0, int depth, 
 constexpr int RING_WARPS = 8, RING_PTS = 32, RING_PPW = RING_PTS / RING_WARPS;
 constexpr int RING_CAP = 48;     // listed elements per point; more (a point with NaN coordinates): one by one
 struct RingSmem {
-  double px[3][RING_PTS];
+  double px[2][3][RING_PTS];     // X-90 frames of these 32 points and of the next
   double need[RING_PTS][RING_CAP], step[RING_PTS][RING_CAP], lc[RING_PTS][RING_CAP][3];
   int id[RING_PTS][RING_CAP];
   int n[RING_PTS];
@@ -514,23 +515,27 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 2) k_resolve_ring(SlmMesh m, 
   RingSmem &S = *reinterpret_cast<RingSmem *>(ring_raw);
   const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int total = *ntodo;
-  // frames of point pt of the 32 (its X-90 frame is in S.px)
+  int buf = 0;
+  // X-90 frames of the points from b on, into buffer k: by one warp, one point per lane
+  auto form_x90 = [&](int b, int k) {
+    if (wl != 0 || b + lane >= total) return;
+    const int i = todo[b + lane];
+    double x[3];
+    frame_x90(P[i], P[npt + i], P[2 * (size_t)npt + i], x);
+    for (int c = 0; c < 3; ++c) S.px[k][c][lane] = x[c];
+  };
+  // frames of point pt of the 32
   auto frames = [&](int i, int pt, PointFrames &f) {
     f.p0[0] = P[i];
     f.p0[1] = P[npt + i];
     f.p0[2] = P[2 * (size_t)npt + i];
     frame_z180(f.p0[0], f.p0[1], f.p0[2], f.pz);
-    for (int c = 0; c < 3; ++c) f.px[c] = S.px[c][pt];
+    for (int c = 0; c < 3; ++c) f.px[c] = S.px[buf][c][pt];
   };
-  for (int base = blockIdx.x * RING_PTS; base < total; base += gridDim.x * RING_PTS) {
+  form_x90(blockIdx.x * RING_PTS, 0);
+  __syncthreads();
+  for (int base = blockIdx.x * RING_PTS; base < total; base += gridDim.x * RING_PTS, buf ^= 1) {
     const int nloc = min(RING_PTS, total - base);
-    if (wl == 0 && lane < nloc) {
-      const int i = todo[base + lane];
-      double x[3];
-      frame_x90(P[i], P[npt + i], P[2 * (size_t)npt + i], x);
-      for (int k = 0; k < 3; ++k) S.px[k][lane] = x[k];
-    }
-    __syncthreads();
     for (int w = 0; w < RING_PPW; ++w) {
       const int pt = wl * RING_PPW + w;
       int cnt = 0;
@@ -550,6 +555,7 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 2) k_resolve_ring(SlmMesh m, 
       if (lane == 0) S.n[pt] = cnt;
     }
     __syncthreads();
+    if (base < total - (int)gridDim.x * RING_PTS) form_x90(base + gridDim.x * RING_PTS, buf ^ 1);
     // FP64 coordinates of the listed elements of the warp's points
     int off[RING_PPW + 1];
     off[0] = 0;
