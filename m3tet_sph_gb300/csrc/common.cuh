@@ -177,7 +177,7 @@ int cuda_fail(cudaError_t e, const char *what);
 // A grid that leaves half of the SMs free allows its successor's start at once; with larger ones the early
 // blocks take room and bandwidth from it (one velocity solve at 30,720 elements: 161 ms if they do, 144 if not),
 // and the successor starts as its blocks end. An iteration of the velocity solve is about 30 short kernels, whose
-// gaps and start-up latencies were a quarter of its time: 156 -> 144 ms at 30,720 elements, 87 -> 77 ms at 3,840.
+// gaps and start-up latencies were a quarter of its time: 156 -> 148 ms at 30,720 elements, 87 -> 75 ms at 3,840.
 #ifdef __CUDACC__
 constexpr unsigned PDL_EARLY_GRID = 76;
 __device__ __forceinline__ void grid_dep() {

@@ -204,8 +204,8 @@ __global__ void __launch_bounds__(DP_WARPS * 32) k_diff_pattern(int nnod, int ns
   }
 }
 // Row values, 16 lanes per node: a lane sums its column's entries over the node's elements in element order.
-// Latency of the three dependent loads per element bounds it: 0.41 ms at 338k nodes one element at a time, 0.37 ms
-// with four in flight
+// FP64 additions (pipe 74 % busy), L1 (63 %) and the latency of the three dependent loads per element bound it:
+// 0.41 ms at 338k nodes one element at a time, 0.37 ms with four in flight
 __global__ void __launch_bounds__(256) k_diff_rows(int nnod, int nsub, const int *__restrict__ sub,
                                                    const double *__restrict__ C, const int *__restrict__ gptr,
                                                    const int *__restrict__ gidx, const int *__restrict__ sptr,

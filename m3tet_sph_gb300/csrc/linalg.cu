@@ -356,7 +356,8 @@ __global__ void k_dense_from_bsr(const int *__restrict__ ptr, const int *__restr
 // the work of the full form): C_i of an unswept panel i is the stored tile, of a swept one minus the
 // transpose of tile (k, i), and R_j = +-D^-1 C_j'. The upper triangle is filled in at the end.
 //
-// Three launches per panel:
+// Three launches per panel, and from 48 FP32 panels on k_gjb_diag of the next panel beside the update of this
+// one (gj_blocked_inverse):
 //  * k_gjb_diag inverts D in one CTA, the block held in registers (an RT x RT piece per thread), by
 //    16-wide sub-panels: the 16 x 16 pivot block by one warp through shuffles, the rest as rank-16
 //    updates. (One pivot at a time in shared memory took 975 us per panel in FP32 and 3,941 us in FP64;
@@ -382,9 +383,12 @@ constexpr int WARPS = 16, THREADS = (WARPS + 2) * 32;     // two groups of 8 epi
 constexpr int STAGE_LD = 20;                               // floats per row of a warp's staging tile of 16 rows
 constexpr int OFF_A = 0, OFF_B = IMAGE, OFF_ST = OFF_B + 2 * HALF;
 constexpr int OFF_BAR = OFF_ST + WARPS * 16 * STAGE_LD * 4;  // a_full, b_full[2], b_empty[2], acc_full[4], acc_empty[2], drain
-// The accumulators round towards zero: sums of the magnitude of the result are cut four times per half of K, by
-// half a unit in the last place on average (a unit is 2^-24 to 2^-23 of the value). The third part of C gives
-// this back.
+// The accumulators round towards zero. In a half of K the large product comes last, in four instructions of
+// K = 16, and after each the sum is cut; for terms of one sign the sums are 1/4, 1/2, 3/4 and all of the result, a
+// cut takes half a unit of the last place on average, and that is 2^-24 / (2 ln 2) = 4.3e-8 of the value:
+// 2.5 x 4.3e-8 = 1.07e-7 of the result is lost. The third part of C gives 1e-7 back. Error of a V-cycle with
+// the inverse of 3,210 free dofs: 5.2e-7 with nothing given back, 3.6e-7 with half of it, 2.4e-7 with this;
+// 3.3e-7 with an update by FP32 multiply-adds (tests: 1 to 48 panels).
 constexpr float ROUNDING = 1e-7f;
 constexpr int OFF_TM = OFF_BAR + 12 * 8;
 constexpr int SMEM = OFF_TM + 8, SMEM_ALLOC = SMEM + 1024;
@@ -751,11 +755,11 @@ __global__ void __launch_bounds__(256, 2) k_gjb_update(T *__restrict__ A, int ld
 // the two halves are added in FP32, and what rounding towards zero takes is given back (gu::ROUNDING). Against
 // FP64 inverses of difference matrices of 129 to 14,801 unknowns and contrasts of 1e2 to 1e4 the error of the
 // whole inverse is 0 to 10 % below that of FP32 multiply-adds (without ROUNDING 1 to 4 % above); on the coarsest
-// levels of shells, 630 to 17,334 dofs, a V-cycle's error from the inverse is 8 to 40 % below.
+// levels of shells, 378 to 17,334 dofs, a V-cycle's error from the inverse is 5 % above to 50 % below.
 // A persistent CTA takes a run of tiles of the triangle, row by row: the row's operand stays in shared memory
 // (96 KB), the column's comes in halves of 48 KB through a ring of two, and the accumulators of two tiles
 // alternate in TMEM between two groups of epilogue warps, which subtract through a staging tile. At 14.8k free
-// dofs 223 us per panel, FP32 multiply-adds 589 us; the triangle read and written at the copy rate would be
+// dofs 223 us per panel (248 us on 151 SMs with the next diagonal block beside it), FP32 multiply-adds 589 us; the triangle read and written at the copy rate would be
 // 130 us, the MMAs alone are 82 us: what is left is the latency of the A accesses (272 us with chunks fetched when
 // they were needed, 255 us without the prefetch of the next tile into L2).
 __global__ void __launch_bounds__(gu::THREADS, 1) k_gjb_update_tc(float *__restrict__ A, int ld, int n, int kblk,

@@ -113,7 +113,7 @@ __device__ __forceinline__ void forward_strip(int row0, const __nv_bfloat16 *sX,
 }
 
 // ---------------------------------------------------------------------------------------
-// features of one element from a residual vector 
+// features of one element from a residual vector
 // ---------------------------------------------------------------------------------------
 struct FeatLevel {
   int nel;
@@ -715,7 +715,7 @@ __global__ void k_ml_publish(const float *p, int n, __nv_bfloat16 *W1, __nv_bflo
 namespace m3sph {
 
 struct MlLevel {
-  int *n2e_ptr = nullptr, *n2e_code = nullptr;   // node -> (stored element * 10 + local node)
+  int *n2e_ptr = nullptr, *n2e_code = nullptr;   // node -> (element * 10 + local node)
   float *lvisc = nullptr, *geo = nullptr;         // [10][nel], [12][nel]
   float *C = nullptr;                             // 30 corrections per element ([30][nel] or [nel][30])
   float *z = nullptr;                             // [3 nnod] Jacobi-scaled residual (fused sweep)

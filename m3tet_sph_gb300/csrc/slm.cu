@@ -37,7 +37,6 @@ constexpr double IFACE_TRIGGER = 15e-3;  // the same for elements next to anothe
 constexpr double GAP_STEP = 1e-6;
 constexpr int GAP_QMAX = 15000;          // 15e-3 in 1e-6 steps
 constexpr int MAX_CAND = 64;             // candidates within the tie band kept per point
-constexpr int MAX_RING_VERTS = 96;       // vertices of the 1-ring gathered for the 2-ring search
 
 struct SlmMesh {
   int nel, nnod, nvnod;
@@ -496,8 +495,8 @@ __device__ __forceinline__ void ring_visit(const SlmMesh &m, int e0, int depth, 
 // elements a point; the FP64 coordinates of the 4 points' lists are then formed together by the lanes of a warp,
 // and one lane per point applies the rules. (One warp per point, every lane forming the point's frames
 // and each round of 32 ring elements its FP64 coordinates, took 1,069 us for the 43,554 departure points of
-// the 30,720-element shell and 6,464 us for the listed ones of 1.5M random points there; now 316 and
-// 1,287 us.)
+// the 30,720-element shell and 6,464 us for the listed ones of 1.5M random points there; now 328 and
+// 1,326 us.)
 constexpr int RING_WARPS = 8, RING_PTS = 32, RING_PPW = RING_PTS / RING_WARPS;
 constexpr int RING_CAP = 48;     // listed elements per point; more (a point with NaN coordinates): one by one
 struct RingSmem {
